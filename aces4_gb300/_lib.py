@@ -83,6 +83,7 @@ SIGNATURES = {
     "a4g_batch_timings": (ctypes.c_int, None),
     "a4g_batch_info": (ctypes.c_int, None),
     "a4g_batch_form": (ctypes.c_int, None),
+    "a4g_batch_products": (ctypes.c_int, [c_void_p]),
     "a4g_batch_destroy": (None, [c_void_p]),
     "a4g_batch_rebind": (ctypes.c_int, [c_void_p, c_void_p, ctypes.c_int64, c_void_p]),
     "a4g_batch_hold": (ctypes.c_int, [c_void_p, ctypes.c_int, ctypes.c_int, c_void_p]),

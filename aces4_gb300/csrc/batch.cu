@@ -38,6 +38,11 @@ struct a4g_batch {
   int store_mode() const { return beta | (negate << 1); }
   int variant = 0;  // tensor-core GEMM form: 0 autotuned, else 1 + index into forms
   int pipeline = 0;  // requested GEMM parts (0/1: one launch)
+  // Residue form (residue.cu): `products` moduli instead of the digits' levels.
+  bool residue = false;
+  int products = 0;  // planes of a panel and of the workspace: slices, or the moduli
+  OzResidues res{};
+  OzCrt crt{};
   int64_t pairs = 0;
   double flops = 0.0;
   int64_t device_bytes = 0;
@@ -226,6 +231,7 @@ uint64_t batch_signature(const a4g_batch* b, const int* ptrn, const a4g_triple* 
   f.put(b->precision), f.put(b->slices), f.put(b->beta), f.put(b->negate), f.put(b->pipeline);
   f.put(b->drank), f.put(b->lrank), f.put(b->rrank);
   f.add(ptrn, sizeof(int) * size_t(b->lrank + b->rrank));
+  if (b->residue) f.put(uint32_t(0x52455331)), f.put(b->products);
   f.put(n);
   std::unordered_map<const void*, int> id;
   auto ident = [&](const void* p) -> int {
@@ -442,7 +448,46 @@ int build_f64(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector
   return rc;
 }
 
-int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector<const DevPlan*>& plans) {
+// Whether the batch's products run modulo coprime numbers (residue.cu) or as
+// digit levels.  Residues need 5 or more slices (at 4 they take as many
+// products as the digits) and a k range long enough that fewer products pay
+// for the wider panels and the reconstruction: kResidueMinKb 64-wide k blocks
+// in every destination.  A pinned variant names a digit form.
+constexpr int kResidueMinKb = 24;
+void choose_products(a4g_batch* b, const std::vector<OzTile>& dinfo, bool allow) {
+  b->residue = false;
+  b->products = b->slices;
+  if (!allow || b->variant || b->slices < 5 || dinfo.empty()) return;
+  int min_kb = 1 << 30, max_kb = 0;
+  for (const OzTile& t : dinfo) min_kb = std::min(min_kb, t.kb_total), max_kb = std::max(max_kb, t.kb_total);
+  if (min_kb < kResidueMinKb) return;
+  const int L = oz_residue_count(b->slices, int64_t(max_kb) * kOzBK);
+  if (L <= 0 || L >= b->slices * (b->slices + 1) / 2) return;
+  b->residue = true;
+  b->products = L;
+  oz_residue_tables(b->slices, L, int64_t(max_kb) * kOzBK, &b->res, &b->crt);
+}
+
+// Operand side of a job set: digits or residues.
+int launch_split(const a4g_batch* b, const a4g_batch::JobSet& js, cudaStream_t s) {
+  const OzPanel* panels = js.left ? b->d_pa : b->d_pb_view;
+  return b->residue ? oz_launch_residues(js.layout, js.d_jobs, js.d_prefix_split, js.njobs, js.tiles_split, panels,
+                                         b->res, s)
+                    : oz_launch_split(js.layout, js.d_jobs, js.d_prefix_split, js.njobs, js.tiles_split, panels,
+                                      b->slices, s);
+}
+
+// Result side of a workspace form.
+int launch_recombine(const a4g_batch* b, const a4g_batch::GemmForm& gf, const OzDBlock* dblocks, const int* ws,
+                     int nsplit, cudaStream_t s) {
+  return b->residue ? oz_launch_residue_recombine(gf.d_tiles, gf.n_tiles, gf.tile_rows, gf.tile_cols, dblocks, b->d_pa,
+                                                  b->d_pb, ws, b->crt, nsplit, b->store_mode(), s)
+                    : oz_launch_recombine(gf.d_tiles, gf.n_tiles, gf.tile_rows, gf.tile_cols, dblocks, b->d_pa,
+                                          b->d_pb, ws, b->slices, nsplit, b->store_mode(), s);
+}
+
+int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector<const DevPlan*>& plans,
+                const int* ptrn, bool allow_residue) {
   std::vector<PanelBuild> pa, pb;
   std::map<std::vector<const double*>, int> ia, ib;
   std::vector<OzDBlock> dblocks;
@@ -578,7 +623,10 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     b->h_colptr = colptr_host;
     b->h_dblocks = dblocks;
   }
+  choose_products(b, dinfo, allow_residue);
+  b->signature = batch_signature(b, ptrn, b->bound.data(), int64_t(b->bound.size()));
   const int S = b->slices;
+  const int NP = b->products;  // planes: slices of the panels, levels or moduli of the workspace
   int rc0 = oz_prepare();
   if (rc0) return rc0;
   // panels: slices (BF16, zero padded), exponents, tensor maps
@@ -609,17 +657,17 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
       p.rows = src[i].rows;
       p.rows_pad = int(ceil_to(src[i].rows, rows_tile));
       p.kpad = src[i].kpad;
-      const size_t bytes = size_t(S) * p.rows_pad * size_t(p.kpad) * 2;
+      const size_t bytes = size_t(NP) * p.rows_pad * size_t(p.kpad) * 2;
       void* mem = nullptr;
       int r = device_alloc(b, bytes, &mem, true);
       if (r) return r;
       p.base = static_cast<__nv_bfloat16*>(mem);
       p.exps = b->d_exps + eoff;
       eoff += p.rows_pad;
-      r = oz_make_tensor_map(maps[i].b, mem, p.kpad, int64_t(S) * p.rows_pad, kOzBM);
+      r = oz_make_tensor_map(maps[i].b, mem, p.kpad, int64_t(NP) * p.rows_pad, kOzBM);
       if (r) return r;
-      if (maps2 && (r = oz_make_tensor_map((*maps2)[i].b, mem, p.kpad, int64_t(S) * p.rows_pad, 64))) return r;
-      if (maps3 && (r = oz_make_tensor_map((*maps3)[i].b, mem, p.kpad, int64_t(S) * p.rows_pad, 256))) return r;
+      if (maps2 && (r = oz_make_tensor_map((*maps2)[i].b, mem, p.kpad, int64_t(NP) * p.rows_pad, 64))) return r;
+      if (maps3 && (r = oz_make_tensor_map((*maps3)[i].b, mem, p.kpad, int64_t(NP) * p.rows_pad, 256))) return r;
       dst.push_back(p);
     }
     return A4G_OK;
@@ -638,10 +686,10 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     b->err_groups.push_back(eg);
   }
   for (auto& p : hpa)
-    if (p.kpad > 0x7fffffffLL || int64_t(S) * p.rows_pad > 0x7fffffffLL)
+    if (p.kpad > 0x7fffffffLL || int64_t(NP) * p.rows_pad > 0x7fffffffLL)
       return fail(A4G_ERR_RANGE, "panel exceeds TMA coordinate range");
   for (auto& p : hpb)
-    if (p.kpad > 0x7fffffffLL || int64_t(S) * p.rows_pad > 0x7fffffffLL)
+    if (p.kpad > 0x7fffffffLL || int64_t(NP) * p.rows_pad > 0x7fffffffLL)
       return fail(A4G_ERR_RANGE, "panel exceeds TMA coordinate range");
   // split jobs (one per block per panel), grouped by side and source layout
   auto layout_of = [](const DevPlan* dp, bool left) {
@@ -737,7 +785,7 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
   if ((rc = upload(b, hpa, &b->d_pa)) || (rc = upload(b, hpb, &b->d_pb)) || (rc = upload(b, trips, &d_trips)) ||
       (rc = upload(b, dblocks, &b->d_dblocks)) || (rc = upload(b, hpb_view, &b->d_pb_view)))
     return rc;
-  for (int t = 0; t < S; ++t)
+  for (int t = 0; t < S && !b->residue; ++t)
     if (oz_chunk_kb(t) < 1) return fail(A4G_ERR_ARG, "slice count too large for exact accumulation");
   int pairs = 0;
   if ((rc = oz_max_pairs(&pairs))) return rc;
@@ -748,7 +796,7 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
   auto make_units = [&](const std::vector<OzTile>& tiles, int nsplit, bool tile_major = false) {
     std::vector<OzUnit> units;
     const int nt = int(tiles.size());
-    for (int lv = 0; lv < S; ++lv)
+    for (int lv = 0; lv < NP; ++lv)
       for (int sp = 0; sp < nsplit; ++sp)
         for (int ti = 0; ti < nt; ++ti) {
           const OzTile& t = tiles[ti];
@@ -774,7 +822,7 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
   //   sum_t S_t 256^(S-1-t),  |S_t| <= (t+1) * K * 2^14  (digits |d| <= 128),
   // so they need |sum| < 2^63 for the longest k range (kept below 2^62 here),
   // and at least one k block per tile.
-  bool direct_ok = S <= 6;
+  bool direct_ok = S <= 6 && !b->residue;
   {
     long double weight = 0.0L;
     for (int t = 0; t < S; ++t) weight += (long double)(t + 1) * std::pow(2.0L, 8 * (S - 1 - t));
@@ -811,17 +859,22 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     // smallest split count that gives every worker the same number of equal
     // units per level (the workers then stay in step through the k panels),
     // keeping at least 16 k blocks per unit and the workspace below 6 GB.
+    // Residue form: the running residues never grow (no lower bound on the
+    // count), all products cost the same, so the units of all of them are
+    // dealt together; 8 k blocks per unit suffice (the epilogue keeps one
+    // register per column and stores 2 bytes).
     const int max_unit_kb = int(((1LL << 31) - 1) / (int64_t(S) * 128 * 128 * kOzBK));
     int min_kb = 1 << 30, max_kb = 0;
     for (const OzTile& t : tiles) min_kb = std::min(min_kb, t.kb_total), max_kb = std::max(max_kb, t.kb_total);
-    const int ns_min = std::max(1, (max_kb + max_unit_kb - 1) / max_unit_kb);
-    const double tile_bytes = double(gf.tile_rows) * gf.tile_cols * sizeof(int);
+    const int ns_min = b->residue ? 1 : std::max(1, (max_kb + max_unit_kb - 1) / max_unit_kb);
+    const int unit_kb = b->residue ? 8 : 16;
+    const double tile_bytes = double(gf.tile_rows) * gf.tile_cols * (b->residue ? sizeof(int16_t) : sizeof(int));
     int nsplit = ns_min;
     double best = -1.0;
     for (int ns = ns_min; !gf.direct && ns <= std::max(64, ns_min); ++ns) {
-      if (ns > ns_min && min_kb / ns < 16) break;
-      if (ns > ns_min && double(gf.n_tiles) * S * ns * tile_bytes > 6.0 * (1u << 30)) break;
-      const int64_t units = int64_t(gf.n_tiles) * ns;
+      if (ns > ns_min && min_kb / ns < unit_kb) break;
+      if (ns > ns_min && double(gf.n_tiles) * NP * ns * tile_bytes > 6.0 * (1u << 30)) break;
+      const int64_t units = int64_t(gf.n_tiles) * ns * (b->residue ? NP : 1);
       const double eff = double(units) / double(P * ((units + P - 1) / P));
       if (eff > best + 1e-9) best = eff, nsplit = ns;
       if (eff >= 0.999) break;
@@ -831,7 +884,8 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     gf.nsplit = nsplit;
     std::vector<OzUnit>& units = form_units[f];
     units = make_units(tiles, nsplit, gf.direct);
-    if (!gf.direct) ws_elems = std::max(ws_elems, size_t(gf.n_tiles) * S * nsplit * gf.tile_rows * gf.tile_cols);
+    if (!gf.direct)  // in ints
+      ws_elems = std::max(ws_elems, size_t(gf.n_tiles) * NP * nsplit * gf.tile_rows * gf.tile_cols / (b->residue ? 2 : 1));
     OzUnit* d_units = nullptr;
     if ((rc = upload(b, tiles, &gf.d_tiles)) || (rc = upload(b, units, &d_units))) return rc;
     OzGemmArgs& ga = gf.args;
@@ -842,9 +896,12 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     ga.n_tiles = gf.n_tiles;
     ga.units = d_units;
     ga.n_units = int(units.size());
-    ga.slices = S;
+    ga.slices = NP;
     ga.nsplit = nsplit;
-    for (int t = 0; t < kOzMaxSlices; ++t) ga.chunk_kb[t] = t < S ? oz_chunk_kb(t) : 1;
+    ga.residue = b->residue ? 1 : 0;
+    for (int t = 0; t < kOzMaxResidues; ++t)
+      ga.chunk_kb[t] = b->residue ? kOzResidueChunkKb : t < S ? oz_chunk_kb(t) : 1, ga.res_p[t] = b->crt.p[t],
+      ga.res_inv[t] = b->crt.inv[t];
     ga.err_flag = ctx()->d_error_flag;
     ga.direct = gf.direct ? 1 : 0;
     ga.mode = b->store_mode();
@@ -883,8 +940,7 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
         if (!rc) rc = oz_launch_exp(js.layout, js.d_jobs, js.d_prefix_exp, js.njobs, js.tiles_exp,
                                     js.left ? b->d_pa : b->d_pb_view, s);
       for (const auto& js : b->jobsets)
-        if (!rc) rc = oz_launch_split(js.layout, js.d_jobs, js.d_prefix_split, js.njobs, js.tiles_split,
-                                      js.left ? b->d_pa : b->d_pb_view, S, s);
+        if (!rc) rc = launch_split(b, js, s);
       if (!rc) rc = check_device_flag(s);
     }
     for (const auto& js : b->jobsets) {
@@ -958,16 +1014,15 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
         if (rep == 1 && cudaEventRecord(e0, s) != cudaSuccess) return cuda_fail(cudaGetLastError(), "event");
         r = oz_launch_gemm(ta, grid, gf.pair, gf.tile_cols, s);
         if (!r && !gf.direct && sdb)
-          r = oz_launch_recombine(gf.d_tiles, gf.n_tiles, gf.tile_rows, gf.tile_cols, sdb, b->d_pa,
-                                  b->d_pb, ta.ws, S, ta.nsplit, b->store_mode(), s);
+          r = launch_recombine(b, gf, sdb, ta.ws, ta.nsplit, s);
       }
       if (r) return r;
       A4G_CUDA(cudaEventRecord(e1, s));
       A4G_CUDA(cudaEventSynchronize(e1));
       A4G_CUDA(cudaEventElapsedTime(ms, e0, e1));
       if (!sdb) {
-        const double ws_bytes = gf.direct ? 0.0 : double(gf.n_tiles) * S * ta.nsplit * gf.tile_rows *
-                                                      gf.tile_cols * sizeof(int);
+        const double ws_bytes = gf.direct ? 0.0 : double(gf.n_tiles) * NP * ta.nsplit * gf.tile_rows *
+                                                      gf.tile_cols * (b->residue ? sizeof(int16_t) : sizeof(int));
         *ms += float((ws_bytes + d_bytes) * ms_per_byte);
       }
       return check_device_flag(s);
@@ -988,12 +1043,13 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     int min_kb = 1 << 30;
     for (const OzTile& t : tiles) min_kb = std::min(min_kb, t.kb_total);
     const int ns1 = gf.nsplit, ns2 = 2 * ns1;
-    const double ws2 = 2.0 * double(gf.n_tiles) * S * ns1 * gf.tile_rows * gf.tile_cols * sizeof(int);
+    const double ws2 = 2.0 * double(gf.n_tiles) * NP * ns1 * gf.tile_rows * gf.tile_cols *
+                       (b->residue ? sizeof(int16_t) : sizeof(int));
     if (!rc && !gf.direct) {
       b->split_candidates[0] = ns1;
       b->split_cost_ms[0] = gf.score_ms;
     }
-    if (!rc && !gf.direct && gf.n_tiles > 0 && ns2 <= 64 && min_kb / ns2 >= 16 && ws2 <= 6.0 * (1u << 30)) {
+    if (!rc && !gf.direct && gf.n_tiles > 0 && ns2 <= 64 && min_kb / ns2 >= (b->residue ? 8 : 16) && ws2 <= 6.0 * (1u << 30)) {
       std::vector<OzUnit> units2 = make_units(tiles, ns2);
       OzUnit* d_units2 = nullptr;
       void* ws2p = nullptr;
@@ -1105,7 +1161,7 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     std::vector<size_t> start;
     for (int p = 0; p < P; ++p) {
       start.push_back(units.size());
-      for (int lv = S - 1; lv >= 0; --lv)
+      for (int lv = NP - 1; lv >= 0; --lv)
         for (int sp = ns * p / P; sp < ns * (p + 1) / P; ++sp)
           for (int ti = 0; ti < gf.n_tiles; ++ti) units.push_back(all[(size_t(lv) * ns + sp) * gf.n_tiles + ti]);
     }
@@ -1241,8 +1297,7 @@ int slice_side(a4g_batch* b, int side, cudaStream_t s) {
                          js.left ? b->d_pa : b->d_pb_view, s);
   for (const auto& js : b->jobsets)
     if (!rc && (side < 0 || side == (js.left ? 0 : 1)))
-      rc = oz_launch_split(js.layout, js.d_jobs, js.d_prefix_split, js.njobs, js.tiles_split,
-                           js.left ? b->d_pa : b->d_pb_view, b->slices, s);
+      rc = launch_split(b, js, s);
   return rc;
 }
 
@@ -1290,8 +1345,7 @@ int run(a4g_batch* b, cudaStream_t s, const cudaEvent_t* ev = nullptr) {
   auto split_group = [&](int g, cudaStream_t st) -> int {
     for (const auto& js : b->jobsets)
       if (js.group == g && sliced(js)) {
-        const int r = oz_launch_split(js.layout, js.d_jobs, js.d_prefix_split, js.njobs, js.tiles_split,
-                                      js.left ? b->d_pa : b->d_pb_view, b->slices, st);
+        const int r = launch_split(b, js, st);
         if (r) return r;
       }
     return A4G_OK;
@@ -1319,8 +1373,7 @@ int run(a4g_batch* b, cudaStream_t s, const cudaEvent_t* ev = nullptr) {
   }
   if ((rc = mark(4))) return rc;
   if (gf.n_tiles > 0 && !gf.direct &&
-      (rc = oz_launch_recombine(gf.d_tiles, gf.n_tiles, gf.tile_rows, gf.tile_cols, b->d_dblocks,
-                                b->d_pa, b->d_pb, b->d_ws, b->slices, gf.nsplit, b->store_mode(), s)))
+      (rc = launch_recombine(b, gf, b->d_dblocks, b->d_ws, gf.nsplit, s)))
     return rc;
   return mark(5);
 }
@@ -1329,12 +1382,9 @@ int run(a4g_batch* b, cudaStream_t s, const cudaEvent_t* ev = nullptr) {
 
 extern "C" {
 
-int a4g_batch_create(a4g_batch** out, const int* ptrn, int drank, int lrank, int rrank,
-                     const a4g_triple* trip, int64_t n, const a4g_batch_opts* opts) {
-  if (!out) return fail(A4G_ERR_ARG, "null output handle");
-  *out = nullptr;
-  int rc = ensure_init();
-  if (rc) return rc;
+static int create_batch(a4g_batch** out, const int* ptrn, int drank, int lrank, int rrank, const a4g_triple* trip,
+                        int64_t n, const a4g_batch_opts* opts, bool allow_residue, bool* residue) {
+  int rc = A4G_OK;
   if (!ptrn || (n > 0 && !trip)) return fail(A4G_ERR_ARG, "null argument");
   if (drank < 1 || drank > 6 || lrank < 1 || lrank > 6 || rrank < 1 || rrank > 6)
     return fail(A4G_ERR_UNSUPPORTED, "batched contraction needs tensor operands of rank 1..6");
@@ -1353,7 +1403,6 @@ int a4g_batch_create(a4g_batch** out, const int* ptrn, int drank, int lrank, int
   if (b->slices < 1 || b->slices > kOzMaxUsableSlices) return fail(A4G_ERR_ARG, "slices must be 1..7");
   b->drank = drank, b->lrank = lrank, b->rrank = rrank;
   if (n > 0) b->bound.assign(trip, trip + n);
-  if (b->precision == A4G_PREC_OZAKI_BF16) b->signature = batch_signature(b.get(), ptrn, trip, n);
 
   std::vector<const DevPlan*> plans;
   std::map<const DevPlan*, int> plan_index;
@@ -1428,10 +1477,28 @@ int a4g_batch_create(a4g_batch** out, const int* ptrn, int drank, int lrank, int
   std::vector<PlanRef> refs;
   for (const DevPlan* p : plans) refs.push_back(ref_of(p));
   if ((rc = upload(b.get(), refs, &b->d_plans))) return rc;
-  rc = b->precision == A4G_PREC_FP64 ? build_f64(b.get(), groups, plans) : build_ozaki(b.get(), groups, plans);
+  rc = b->precision == A4G_PREC_FP64 ? build_f64(b.get(), groups, plans)
+                                     : build_ozaki(b.get(), groups, plans, ptrn, allow_residue);
+  *residue = b->residue;
   if (rc) return rc;
   *out = b.release();
   return A4G_OK;
+}
+
+int a4g_batch_create(a4g_batch** out, const int* ptrn, int drank, int lrank, int rrank,
+                     const a4g_triple* trip, int64_t n, const a4g_batch_opts* opts) {
+  if (!out) return fail(A4G_ERR_ARG, "null output handle");
+  *out = nullptr;
+  int rc = ensure_init();
+  if (rc) return rc;
+  bool residue = false;
+  rc = create_batch(out, ptrn, drank, lrank, rrank, trip, n, opts, true, &residue);
+  if (rc == A4G_ERR_NOMEM && residue) {
+    // the residue panels are 11 / 5 of the digits': where they do not fit, the digits may
+    cudaGetLastError();
+    rc = create_batch(out, ptrn, drank, lrank, rrank, trip, n, opts, false, &residue);
+  }
+  return rc;
 }
 
 int a4g_batch_run(a4g_batch* b, void* stream) {
@@ -1532,6 +1599,11 @@ int a4g_batch_form(const a4g_batch* b, int* form, float* tuned_ms, int n) {
   if (form) *form = b->precision == A4G_PREC_FP64 ? 0 : b->form + 1;
   for (int f = 0; f < n && tuned_ms; ++f) tuned_ms[f] = f < a4g_batch::kForms ? b->forms[f].score_ms : -1.f;
   return A4G_OK;
+}
+
+int a4g_batch_products(const a4g_batch* b) {
+  if (!b || b->precision == A4G_PREC_FP64) return 0;
+  return b->residue ? b->products : b->slices * (b->slices + 1) / 2;
 }
 
 int a4g_batch_rebind(a4g_batch* b, const a4g_triple* trip, int64_t n, void* stream) {

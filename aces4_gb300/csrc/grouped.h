@@ -140,6 +140,26 @@ struct OzEnergyBlock {
   int last_row;
 };
 
+// Residue form (residue.cu): what the operand side and the GEMM need of the
+// moduli, and what the reconstruction needs.
+constexpr int kOzMaxResidues = 15;
+constexpr int kOzResidueChunkKb = 4;  // 64-wide k blocks per exact FP32 chunk (256 k, |residues| <= 255)
+constexpr int kOzResidueBias = 256;     // added to a residue stored in the workspace (0 .. 512)
+struct OzResidues {
+  int L, slices;
+  // each twice, as the packed FP32 instructions take them: -p, the FP32
+  // reciprocal of p, and 2^14, 2^28, 2^42 modulo p
+  float2 np[kOzMaxResidues], inv[kOzMaxResidues], c[3][kOzMaxResidues];
+};
+struct OzCrt {
+  int L, slices;
+  int words;  // 32-bit words of the reconstruction: 3 when |sum| < 2^95, else 4
+  float p[kOzMaxResidues], inv[kOzMaxResidues];
+  float cinv[kOzMaxResidues];  // (P / p)^-1 modulo p, P the product of the moduli
+  int m[kOzMaxResidues][4];    // P / p modulo 2^128, signed 32-bit words
+  int prod[4];                 // P modulo 2^128
+};
+
 struct OzGemmArgs {
   const void* maps_a;  // CUtensorMap[n_panels_a], 64-byte aligned, device memory
   const void* maps_b;
@@ -152,7 +172,7 @@ struct OzGemmArgs {
   int n_tiles;
   int slices;
   int nsplit;
-  int chunk_kb[kOzMaxSlices];  // k blocks per exact flush at each level
+  int chunk_kb[kOzMaxResidues];  // k blocks per exact flush at each level (or modulus)
   int* ws;                     // [tile][level][split][col 128][row 128] exact integer level sums
   int* err_flag;
   // Direct form (128-column tiles, one split): the levels of a tile are folded
@@ -162,6 +182,11 @@ struct OzGemmArgs {
   int mode;  // direct: bit 0 accumulate into D, bit 1 negate
   int dry;   // direct: compute everything but store nothing (timing)
   const OzDBlock* dblocks;
+  // Residue form: slices = the number of moduli; "level" t of a unit is the
+  // product of slice t of A with slice t of B, reduced modulo res_p[t] in the
+  // epilogue and stored as int16 plus kOzResidueBias (ws: [tile][modulus][split][col][row] int16).
+  int residue;
+  float res_p[kOzMaxResidues], res_inv[kOzMaxResidues];
   // Energy form (direct, one SM per tile): nothing is stored; each epilogue
   // thread accumulates sum D(x) * fl(D(x) / eps(x)) over its elements in FP64
   // and writes it to epart[(blockIdx.x * 16 + epilogue warp) * 32 + lane].

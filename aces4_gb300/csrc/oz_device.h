@@ -1,0 +1,70 @@
+// Device helpers shared by the split-precision kernels (digits in ozaki.cu,
+// residues in residue.cu): locating a split job, loading its tile, the
+// fixed-point value of an element.
+#pragma once
+
+#include "grouped.h"
+
+namespace a4g {
+namespace {
+
+constexpr int kDigitBits = 8;
+
+// A row or column exponent of 2047 (the field of Inf and NaN) marks a panel
+// row that holds a non-finite value: digits cannot carry it, so every result
+// that row or column feeds is stored as NaN (in FP64 a NaN or an infinity in
+// an operand makes the whole row or column of the product NaN or infinite).
+constexpr int kNonFiniteExp = 2047;
+
+// Tiles of 64 rows x 64 k over the jobs; job_tiles[j] is the prefix count.
+__device__ __forceinline__ int find_job(const int64_t* prefix, int njobs, int64_t t) {
+  int lo = 0, hi = njobs;  // prefix[lo] <= t < prefix[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (prefix[mid] <= t) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
+constexpr int kSplitT = 64;
+
+// Loads one 64x64 (row, k) tile of a job into shared memory as raw bits.
+__device__ __forceinline__ void load_job_tile(const OzSplitJob& jb, int r0, int k0,
+                                              unsigned long long (*tile)[kSplitT + 1]) {
+  const int t = threadIdx.x;  // 256 threads
+  for (int p = 0; p < 16; ++p) {
+    int r, k;
+    if (jb.kfast) {
+      k = t & 63;
+      r = (t >> 6) + 4 * p;
+    } else {
+      r = t & 63;
+      k = (t >> 6) + 4 * p;
+    }
+    unsigned long long v = 0;
+    if (r0 + r < jb.rows && k0 + k < jb.K)
+      v = __double_as_longlong(__ldg(&jb.src[__ldg(&jb.offRow[r0 + r]) + __ldg(&jb.offK[k0 + k])]));
+    tile[r][k] = v ^ (jb.negate ? (1ull << 63) : 0ull);  // -x: the sign bit (exponents unchanged)
+  }
+}
+
+// Signed fixed-point value of one double against its row exponent (biased
+// max exponent mx, |x| < 2^E with E = mx - 1022):
+//     n = round_half_away(x * 2^(8*slices - E - 1)),   |n| <= 2^(8*slices - 1).
+__device__ __forceinline__ long long quantize(unsigned long long bits, int mx, int slices) {
+  const int be = int((bits >> 52) & 0x7FF);
+  const unsigned long long frac = bits & ((1ull << 52) - 1);
+  const unsigned long long mant = be ? (frac | (1ull << 52)) : frac;
+  const int ex = be ? be : 1;
+  const int E = (mx ? mx : 1) - 1022;
+  const int sh = ex - 1076 + kDigitBits * slices - E;  // |x| * 2^(8s-E-1) = mant * 2^sh
+  unsigned long long m;
+  if (sh >= 0) m = mant << sh;  // only for 7 slices: sh <= 2, mant << 2 < 2^55
+  else if (-sh >= 63) m = 0ull;
+  else m = (mant + (1ull << (-sh - 1))) >> (-sh);
+  return (bits >> 63) ? -static_cast<long long>(m) : static_cast<long long>(m);
+}
+
+}  // namespace
+}  // namespace a4g

@@ -45,13 +45,14 @@
 
 #include "a4g_internal.h"
 #include "exact_fp.h"
+#include "f32x2.h"
 #include "grouped.h"
+#include "oz_device.h"
 #include "ozaki.h"
 
 namespace a4g {
 namespace {
 
-constexpr int kDigitBits = 8;
 constexpr int kThreadsOz = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
 // Direct forms: warps 2..17 epilogue (four per TMEM lane quadrant, 32 columns
 // each): their epilogue also rounds and stores every result.
@@ -110,10 +111,10 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) { mbar_expect_tx(smem_u32(bar), bytes); }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -146,12 +147,59 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, SM& sm
     }
   }
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const void* map, uint64_t* bar, int c0, int c1) {
+// The same wait by a whole warp (shared-memory address of the barrier): every
+// lane returns the same answer, so the warp stays converged around the
+// single-thread issues that follow.
+template <class SM>
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, SM& sm, int* err, int code) {
+  auto done = [&]() {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return __all_sync(0xffffffffu, ok != 0) != 0;
+  };
+  if (done()) return true;
+  const unsigned long long t0 = now_ns();
+#pragma unroll 1
+  for (uint32_t it = 1;; ++it) {
+    if (done()) return true;
+    if ((it & 255) == 0) {
+      const bool late = now_ns() - t0 > kWaitLimitNs;
+      if (__any_sync(0xffffffffu, sm.abort || late)) {
+        if (!sm.abort) {
+          sm.abort = 1;
+          atomicExch(err, code);
+        }
+        __syncwarp();
+        return false;
+      }
+    }
+  }
+}
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          smem_u32(dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
+          dst),
+      "l"(map), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(void* dst, const void* map, uint64_t* bar, int c0, int c1) {
+  tma_load_2d(smem_u32(dst), map, smem_u32(bar), c0, c1);
 }
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -159,11 +207,10 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void tc_commit(uint64_t* bar) { tc_commit(smem_u32(bar)); }
 template <int N>
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accum) {
   asm volatile(
@@ -196,11 +243,11 @@ __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar_cluster, uin
 }
 // TMA load into this CTA's shared memory that signals an mbarrier which may
 // live in either CTA of the pair
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* map, uint32_t bar_cluster, int c0,
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* map, uint32_t bar_cluster, int c0,
                                                  int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          smem_u32(dst)),
+          dst),
       "l"(map), "r"(bar_cluster), "r"(c0), "r"(c1)
       : "memory");
 }
@@ -214,24 +261,25 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t adesc, uin
 }
 // arrive on the mbarrier at the same offset in both CTAs of the pair once
 // this thread's tcgen05 operations complete
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
+          bar),
       "h"(uint16_t(3))
       : "memory");
 }
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) { tc_commit_pair(smem_u32(bar)); }
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, rows of 128 B,
 // 8-row core groups 1024 B apart (SBO), descriptor version 1 (bits 46-48).
-__device__ __forceinline__ uint64_t sw128_desc(const void* tile) {
-  const uint32_t addr = smem_u32(tile);
-  uint64_t d = uint64_t((addr & 0x3FFFF) >> 4);
-  d |= uint64_t(1) << 16;            // leading byte offset (unused for SW128 K-major)
-  d |= uint64_t(1024 >> 4) << 32;    // stride byte offset
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(2) << 61;            // SWIZZLE_128B
-  return d;
+// The low word holds the tile's address (in 16-byte units) and the leading
+// byte offset (unused for SW128 K-major); the high word is the same for all.
+__device__ __forceinline__ uint32_t sw128_desc_lo(const void* tile) {
+  return ((smem_u32(tile) & 0x3FFFF) >> 4) | (1u << 16);
+}
+__device__ __forceinline__ uint64_t sw128_desc(uint32_t lo) {
+  constexpr uint32_t hi = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);  // SBO, version 1, SWIZZLE_128B
+  return (uint64_t(hi) << 32) | lo;
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -265,12 +313,6 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
   hi = s;
   lo = __fadd_rn(lo, e);
 }
-
-// A row or column exponent of 2047 (the field of Inf and NaN) marks a panel
-// row that holds a non-finite value: digits cannot carry it, so every result
-// that row or column feeds is stored as NaN (in FP64 a NaN or an infinity in
-// an operand makes the whole row or column of the product NaN or infinite).
-constexpr int kNonFiniteExp = 2047;
 
 // ------------------------------------------------------------------ roles
 // Walks the k blocks of one unit: calls f(koff_a, koff_b, kb) per 64-wide
@@ -312,11 +354,20 @@ __device__ __forceinline__ void for_units(const OzGemmArgs& a, F&& f) {
   }
 }
 
-template <bool PAIR, int BN>
+// Both single-issuer roles run as whole, converged warps: every lane keeps the
+// loop's counters and waits, one elected lane issues.  Stage addresses,
+// barriers and descriptors are the first stage's plus a multiple of the stage
+// index, with no division and no address conversion in the loop: a role whose
+// instructions for one stage (64 k: 512 clocks of MMAs for a 256-column tile)
+// take longer than the stage itself starves the tensor cores.
+template <bool PAIR, int BN, bool RES>
 __device__ void producer(const OzGemmArgs& a, OzSmemT<PAIR, BN>& sm, uint32_t rank) {
   using SM = OzSmemT<PAIR, BN>;
   constexpr uint32_t kBytes = kTileBytes + SM::kBBytes;
-  uint32_t it = 0;
+  const bool leader = elect_one();
+  const uint32_t a0 = smem_u32(sm.a[0]), b0 = smem_u32(sm.b[0]), empty0 = smem_u32(&sm.empty[0]);
+  const uint32_t full0 = PAIR ? mapa_shared(&sm.full[0], 0) : smem_u32(&sm.full[0]);  // pair: the leader CTA's
+  uint32_t s = 0, free_parity = 1;
   for_units<PAIR>(a, [&](int u) {
     const OzUnit un = a.units[u];
     const OzTile tl = a.tiles[un.tile];
@@ -324,25 +375,30 @@ __device__ void producer(const OzGemmArgs& a, OzSmemT<PAIR, BN>& sm, uint32_t ra
     const void* ma = static_cast<const uint8_t*>(a.maps_a) + size_t(tl.panel_a) * 128;
     const void* mb = static_cast<const uint8_t*>(a.maps_b) + size_t(tl.panel_b) * 128;
     const int rpa = a.panels_a[tl.panel_a].rows_pad, rpb = a.panels_b[tl.panel_b].rows_pad;
-    const int arow = tl.m0 + int(rank) * kOzBM;          // this CTA's 128 rows of A
-    const int brow = tl.n0 + int(rank) * (BN / 2);       // this CTA's half of B (pair form)
+    const int first = RES ? level : 0;
+    const int arow = tl.m0 + int(rank) * kOzBM + first * rpa;  // this CTA's 128 rows of A
+    // this CTA's rows of B (pair form: half of them); slice level - i, or the modulus' own
+    const int brow = tl.n0 + (PAIR ? int(rank) * (BN / 2) : 0) + level * rpb;
     bool ok = true;
     for_unit_kblocks(a, un, tl, [&](int ka, int kb, int) {
-      for (int i = 0; i <= level; ++i) {
-        const int s = it % SM::kSt;
-        const uint32_t ph = (it / SM::kSt) & 1;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1, sm, a.err_flag, 1)) return ok = false;
-        if constexpr (PAIR) {
-          const uint32_t fb = mapa_shared(&sm.full[s], 0);  // the leader CTA's barrier
-          mbar_expect_tx_cluster(fb, kBytes);
-          tma_load_2d_pair(sm.a[s], ma, fb, ka, i * rpa + arow);
-          tma_load_2d_pair(sm.b[s], mb, fb, kb, (level - i) * rpb + brow);
-        } else {
-          mbar_expect_tx(&sm.full[s], kBytes);
-          tma_load_2d(sm.a[s], ma, &sm.full[s], ka, i * rpa + arow);
-          tma_load_2d(sm.b[s], mb, &sm.full[s], kb, (level - i) * rpb + tl.n0);
+      int ar = arow, br = brow;
+      for (int i = first; i <= level; ++i) {
+        if (!warp_wait(empty0 + 8 * s, free_parity, sm, a.err_flag, 1)) return ok = false;
+        if (leader) {
+          const uint32_t fb = full0 + 8 * s;
+          if constexpr (PAIR) {
+            mbar_expect_tx_cluster(fb, kBytes);
+            tma_load_2d_pair(a0 + s * kTileBytes, ma, fb, ka, ar);
+            tma_load_2d_pair(b0 + s * SM::kBBytes, mb, fb, kb, br);
+          } else {
+            mbar_expect_tx(fb, kBytes);
+            tma_load_2d(a0 + s * kTileBytes, ma, fb, ka, ar);
+            tma_load_2d(b0 + s * SM::kBBytes, mb, fb, kb, br);
+          }
         }
-        ++it;
+        __syncwarp();
+        ar += rpa, br -= rpb;
+        if (++s == uint32_t(SM::kSt)) s = 0, free_parity ^= 1;
       }
       return true;
     });
@@ -350,49 +406,57 @@ __device__ void producer(const OzGemmArgs& a, OzSmemT<PAIR, BN>& sm, uint32_t ra
   });
 }
 
-// One thread issues every MMA (the leader CTA's in the pair form).
-template <bool PAIR, int BN>
+// One lane issues every MMA (in the leader CTA's warp in the pair form).
+template <bool PAIR, int BN, bool RES>
 __device__ void mma_issuer(const OzGemmArgs& a, OzSmemT<PAIR, BN>& sm, uint32_t tmem) {
   using SM = OzSmemT<PAIR, BN>;
-  uint32_t it = 0, chunk = 0;
+  const bool leader = elect_one();
+  const uint32_t full0 = smem_u32(&sm.full[0]), empty0 = smem_u32(&sm.empty[0]);
+  const uint32_t acc_full0 = smem_u32(&sm.acc_full[0]), acc_empty0 = smem_u32(&sm.acc_empty[0]);
+  const uint32_t ad0 = sw128_desc_lo(sm.a[0]), bd0 = sw128_desc_lo(sm.b[0]);
+  uint32_t s = 0, full_parity = 0, chunk = 0;
   for_units<PAIR>(a, [&](int u) {
     const OzUnit un = a.units[u];
     const OzTile tl = a.tiles[un.tile];
-    const int level = un.level;
-    const int ckb = a.chunk_kb[level];
-    int in_chunk = 0;
+    const int ckb = a.chunk_kb[un.level];
+    const int products = RES ? 1 : un.level + 1;
+    int left = 0;  // k blocks left in the chunk (0: a new chunk)
     uint32_t buf = 0;
     bool ok = true;
     for_unit_kblocks(a, un, tl, [&](int, int, int kb) {
-      if (in_chunk == 0) {
+      uint32_t acc = 1;
+      if (left == 0) {
         buf = chunk & 1;
-        if (!mbar_wait(&sm.acc_empty[buf], ((chunk >> 1) & 1) ^ 1, sm, a.err_flag, 2)) return ok = false;
+        if (!warp_wait(acc_empty0 + 8 * buf, ((chunk >> 1) & 1) ^ 1, sm, a.err_flag, 2)) return ok = false;
         tc_fence_after();
+        left = min(ckb, un.kb_end - kb);
+        acc = 0;
       }
       const uint32_t d_tmem = tmem + buf * BN;
-      for (int i = 0; i <= level; ++i) {
-        const int s = it % SM::kSt;
-        const uint32_t ph = (it / SM::kSt) & 1;
-        if (!mbar_wait(&sm.full[s], ph, sm, a.err_flag, 3)) return ok = false;
+      --left;
+      for (int i = 0; i < products; ++i) {
+        if (!warp_wait(full0 + 8 * s, full_parity, sm, a.err_flag, 3)) return ok = false;
         tc_fence_after();
-        const uint64_t ad = sw128_desc(sm.a[s]), bd = sw128_desc(sm.b[s]);
+        if (leader) {
+          const uint32_t ad = ad0 + s * (kTileBytes >> 4), bd = bd0 + s * (SM::kBBytes >> 4);
 #pragma unroll
-        for (int kk = 0; kk < kOzBK / 16; ++kk) {
-          const uint32_t acc = (in_chunk == 0 && i == 0 && kk == 0) ? 0u : 1u;
-          if constexpr (PAIR) tc_mma_pair<BN>(d_tmem, ad + 2 * kk, bd + 2 * kk, acc);
-          else tc_mma<BN>(d_tmem, ad + 2 * kk, bd + 2 * kk, acc);
+          for (int kk = 0; kk < kOzBK / 16; ++kk) {
+            const uint32_t ac = kk == 0 ? acc : 1u;
+            if constexpr (PAIR) tc_mma_pair<BN>(d_tmem, sw128_desc(ad + 2 * kk), sw128_desc(bd + 2 * kk), ac);
+            else tc_mma<BN>(d_tmem, sw128_desc(ad + 2 * kk), sw128_desc(bd + 2 * kk), ac);
+          }
+          if constexpr (PAIR) tc_commit_pair(empty0 + 8 * s);
+          else tc_commit(empty0 + 8 * s);
+          if (left == 0 && i == products - 1) {
+            if constexpr (PAIR) tc_commit_pair(acc_full0 + 8 * buf);
+            else tc_commit(acc_full0 + 8 * buf);
+          }
         }
-        if constexpr (PAIR) tc_commit_pair(&sm.empty[s]);
-        else tc_commit(&sm.empty[s]);
-        ++it;
+        __syncwarp();
+        acc = 1;
+        if (++s == uint32_t(SM::kSt)) s = 0, full_parity ^= 1;
       }
-      ++in_chunk;
-      if (in_chunk == ckb || kb + 1 == un.kb_end) {
-        if constexpr (PAIR) tc_commit_pair(&sm.acc_full[buf]);
-        else tc_commit(&sm.acc_full[buf]);
-        ++chunk;
-        in_chunk = 0;
-      }
+      if (left == 0) ++chunk;
       return true;
     });
     return ok;
@@ -779,7 +843,76 @@ __device__ void epilogue_int(const OzGemmArgs& a, OzSmemT<PAIR, 256>& sm, uint32
   });
 }
 
-template <bool PAIR, int BN, bool DIRECT = false, bool ENERGY = false>
+// Residue form, every tile shape: a chunk (256 k) of the modulus' product is an
+// exact FP32 integer below 2^24 - 256; the thread's running residue (at most
+// p / 2 in magnitude, one FP32 register per column) is added to it, exactly,
+// and the sum reduced modulo p again: four packed FP32 instructions per two
+// columns.  (The conversion to int32 that the level form uses runs at a
+// quarter of the FP32 rate's 128 per clock and would take as long as the
+// chunk's MMAs: 2048 clocks for a 128 x 256 accumulator.)  A chunk has to be
+// drained within the next one's MMAs: the pair 256 x 256 form keeps its tensor
+// pipe 90 % busy (95 % with the drain left out; sixteen epilogue warps instead
+// of eight, with loads of eight columns in flight, measured the same).  Stored
+// as the non-negative int16 r + kOzResidueBias.
+template <bool PAIR, int BN>
+__device__ void epilogue_residue(const OzGemmArgs& a, OzSmemT<PAIR, BN>& sm, uint32_t tmem, int warp, int lane,
+                                 uint32_t rank) {
+  constexpr int kRows = PAIR ? 2 * kOzBM : kOzBM;
+  constexpr int kCols = BN / 2;  // columns of a thread
+  const int q = warp & 3, h = (warp - 2) >> 2;
+  const int row = int(rank) * kOzBM + 32 * q + lane;
+  const uint32_t lane_addr = tmem + (uint32_t(32 * q) << 16) + uint32_t(kCols * h);
+  uint32_t empty_bar[2];
+  for (int b = 0; b < 2; ++b) empty_bar[b] = PAIR ? mapa_shared(&sm.acc_empty[b], 0) : smem_u32(&sm.acc_empty[b]);
+  const F32x2 magic = pack2(kRintMagic, kRintMagic), unmagic = pack2(-kRintMagic, -kRintMagic);
+  const F32x2 biased = pack2(kRintMagic + kOzResidueBias, kRintMagic + kOzResidueBias);
+  uint32_t chunk = 0;
+  for_units<PAIR>(a, [&](int u) {
+    const OzUnit un = a.units[u];
+    const int nchunks = (un.kb_end - un.kb_begin + kOzResidueChunkKb - 1) / kOzResidueChunkKb;
+    const float p = a.res_p[un.level], ip = a.res_inv[un.level];
+    const F32x2 inv = pack2(ip, ip), np = pack2(-p, -p);
+    int16_t* w = reinterpret_cast<int16_t*>(a.ws) +
+                 ((size_t(un.tile) * a.slices + un.level) * a.nsplit + un.split) * BN * kRows +
+                 size_t(kCols * h) * kRows + row;
+    F32x2 r[kCols / 2];
+#pragma unroll
+    for (int j = 0; j < kCols / 2; ++j) r[j] = 0ull;  // two +0
+    for (int c = 0; c < nchunks; ++c) {
+      const uint32_t buf = chunk & 1;
+      if (!mbar_wait(&sm.acc_full[buf], (chunk >> 1) & 1, sm, a.err_flag, 4)) return false;
+      tc_fence_after();
+      uint32_t xg[16];
+#pragma unroll
+      for (int g = 0; g < kCols / 16; ++g) {
+        tc_ld16_nowait(lane_addr + buf * BN + 16 * g, xg);
+        tc_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const F32x2 y = add2(pack2(__uint_as_float(xg[2 * j]), __uint_as_float(xg[2 * j + 1])), r[8 * g + j]);
+          r[8 * g + j] = fma2(np, add2(fma2(y, inv, magic), unmagic), y);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_cluster(empty_bar[buf]);
+        else mbar_arrive(&sm.acc_empty[buf]);
+      }
+      ++chunk;
+    }
+#pragma unroll
+    for (int j = 0; j < kCols / 2; ++j) {
+      float lo, hi;
+      unpack2(add2(r[j], biased), lo, hi);  // the low 16 bits of 1.5 2^23 + x are x
+      w[size_t(2 * j) * kRows] = int16_t(__float_as_uint(lo));
+      w[size_t(2 * j + 1) * kRows] = int16_t(__float_as_uint(hi));
+    }
+    return true;
+  });
+}
+
+template <bool PAIR, int BN, bool DIRECT = false, bool ENERGY = false, bool RES = false>
 __global__ void __launch_bounds__(DIRECT ? kThreadsOzDirect : kThreadsOz, 1)
     oz_gemm_kernel(const __grid_constant__ OzGemmArgs a) {
   using SM = OzSmemT<PAIR, BN>;
@@ -821,17 +954,21 @@ __global__ void __launch_bounds__(DIRECT ? kThreadsOzDirect : kThreadsOz, 1)
   const uint32_t tmem = sm.tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) producer<PAIR, BN>(a, sm, rank);
+    producer<PAIR, BN, RES>(a, sm, rank);
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      mma_issuer<PAIR, BN>(a, sm, tmem);
-      // all MMAs this thread issued have completed before TMEM is released
-      if constexpr (PAIR) tc_commit_pair(&sm.drain);
-      else tc_commit(&sm.drain);
-      mbar_wait(&sm.drain, 0, sm, a.err_flag, 5);
+    if (rank == 0) {
+      mma_issuer<PAIR, BN, RES>(a, sm, tmem);
+      // all MMAs this warp issued have completed before TMEM is released
+      if (elect_one()) {
+        if constexpr (PAIR) tc_commit_pair(&sm.drain);
+        else tc_commit(&sm.drain);
+      }
+      __syncwarp();
+      warp_wait(smem_u32(&sm.drain), 0, sm, a.err_flag, 5);
     }
   } else {
-    if constexpr (BN == 256) epilogue_int<PAIR>(a, sm, tmem, warp, lane, rank);
+    if constexpr (RES) epilogue_residue<PAIR, BN>(a, sm, tmem, warp, lane, rank);
+    else if constexpr (BN == 256) epilogue_int<PAIR>(a, sm, tmem, warp, lane, rank);
     else epilogue<PAIR, DIRECT, ENERGY>(a, sm, tmem, warp, lane, rank);
   }
   tc_fence_before();
@@ -1135,39 +1272,6 @@ __global__ void __launch_bounds__(kThreadsOzDirect, 1) oz_levels_kernel(const __
 }
 
 // ------------------------------------------------------------------ split side
-// Tiles of 64 rows x 64 k over the jobs; job_tiles[j] is the prefix count.
-__device__ __forceinline__ int find_job(const int64_t* prefix, int njobs, int64_t t) {
-  int lo = 0, hi = njobs;  // prefix[lo] <= t < prefix[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (prefix[mid] <= t) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-constexpr int kSplitT = 64;
-
-// Loads one 64x64 (row, k) tile of a job into shared memory as raw bits.
-__device__ __forceinline__ void load_job_tile(const OzSplitJob& jb, int r0, int k0,
-                                              unsigned long long (*tile)[kSplitT + 1]) {
-  const int t = threadIdx.x;  // 256 threads
-  for (int p = 0; p < 16; ++p) {
-    int r, k;
-    if (jb.kfast) {
-      k = t & 63;
-      r = (t >> 6) + 4 * p;
-    } else {
-      r = t & 63;
-      k = (t >> 6) + 4 * p;
-    }
-    unsigned long long v = 0;
-    if (r0 + r < jb.rows && k0 + k < jb.K)
-      v = __double_as_longlong(__ldg(&jb.src[__ldg(&jb.offRow[r0 + r]) + __ldg(&jb.offK[k0 + k])]));
-    tile[r][k] = v ^ (jb.negate ? (1ull << 63) : 0ull);  // -x: the sign bit (exponents unchanged)
-  }
-}
-
 __global__ void __launch_bounds__(256) oz_exp_kernel(const OzSplitJob* __restrict__ jobs,
                                                      const int64_t* __restrict__ prefix, int njobs,
                                                      const OzPanel* __restrict__ panels) {
@@ -1187,23 +1291,6 @@ __global__ void __launch_bounds__(256) oz_exp_kernel(const OzSplitJob* __restric
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
   if (part == 0 && r0 + r < jb.rows && m > 0) atomicMax(&panels[jb.panel].exps[r0 + r], m);
-}
-
-// Signed fixed-point value of one double against its row exponent (biased
-// max exponent mx, |x| < 2^E with E = mx - 1022):
-//     n = round_half_away(x * 2^(8*slices - E - 1)),   |n| <= 2^(8*slices - 1).
-__device__ __forceinline__ long long quantize(unsigned long long bits, int mx, int slices) {
-  const int be = int((bits >> 52) & 0x7FF);
-  const unsigned long long frac = bits & ((1ull << 52) - 1);
-  const unsigned long long mant = be ? (frac | (1ull << 52)) : frac;
-  const int ex = be ? be : 1;
-  const int E = (mx ? mx : 1) - 1022;
-  const int sh = ex - 1076 + kDigitBits * slices - E;  // |x| * 2^(8s-E-1) = mant * 2^sh
-  unsigned long long m;
-  if (sh >= 0) m = mant << sh;  // only for 7 slices: sh <= 2, mant << 2 < 2^55
-  else if (-sh >= 63) m = 0ull;
-  else m = (mant + (1ull << (-sh - 1))) >> (-sh);
-  return (bits >> 63) ? -static_cast<long long>(m) : static_cast<long long>(m);
 }
 
 // Balanced base-256 digits of n, most significant first: d[0] in [-128, 128],
@@ -1850,9 +1937,9 @@ int oz_launch_split(int layout, const OzSplitJob* jobs, const int64_t* prefix, i
   return A4G_OK;
 }
 
-template <bool PAIR, int BN, bool DIRECT = false, bool ENERGY = false>
+template <bool PAIR, int BN, bool DIRECT = false, bool ENERGY = false, bool RES = false>
 int set_smem_attr() {
-  A4G_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<PAIR, BN, DIRECT, ENERGY>,
+  A4G_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<PAIR, BN, DIRECT, ENERGY, RES>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(OzSmemT<PAIR, BN>)) + 1024));
   return A4G_OK;
 }
@@ -1880,6 +1967,8 @@ int oz_prepare() {
     if ((rc = set_smem_attr<false, 128>()) || (rc = set_smem_attr<true, 128>()) ||
         (rc = set_smem_attr<false, 256>()) || (rc = set_smem_attr<true, 256>()) ||
         (rc = set_smem_attr<false, 128, true>()) || (rc = set_smem_attr<true, 128, true>()) ||
+        (rc = set_smem_attr<false, 128, false, false, true>()) || (rc = set_smem_attr<true, 128, false, false, true>()) ||
+        (rc = set_smem_attr<false, 256, false, false, true>()) || (rc = set_smem_attr<true, 256, false, false, true>()) ||
         (rc = set_smem_attr<false, 128, true, true>()) || (rc = set_levels_attr<false>()) ||
         (rc = set_levels_attr<true>())) {
       done.store(0);
@@ -1909,11 +1998,11 @@ int oz_max_pairs(int* pairs) {
   return A4G_OK;
 }
 
-template <bool PAIR, int BN, bool DIRECT = false, bool ENERGY = false>
+template <bool PAIR, int BN, bool DIRECT = false, bool ENERGY = false, bool RES = false>
 int launch_form(const OzGemmArgs& args, int grid, cudaStream_t s) {
   const size_t smem = sizeof(OzSmemT<PAIR, BN>) + 1024;
   if constexpr (!PAIR) {
-    oz_gemm_kernel<false, BN, DIRECT, ENERGY><<<grid, DIRECT ? kThreadsOzDirect : kThreadsOz, smem, s>>>(args);
+    oz_gemm_kernel<false, BN, DIRECT, ENERGY, RES><<<grid, DIRECT ? kThreadsOzDirect : kThreadsOz, smem, s>>>(args);
   } else {
     if (grid % 2) return fail(A4G_ERR_ARG, "CTA-pair grid must be even");
     cudaLaunchConfig_t cfg = {};
@@ -1926,17 +2015,25 @@ int launch_form(const OzGemmArgs& args, int grid, cudaStream_t s) {
     attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    A4G_CUDA(cudaLaunchKernelEx(&cfg, oz_gemm_kernel<true, BN, DIRECT>, args));
+    A4G_CUDA(cudaLaunchKernelEx(&cfg, oz_gemm_kernel<true, BN, DIRECT, false, RES>, args));
   }
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
 }
 
 int oz_launch_gemm(const OzGemmArgs& args, int grid, bool pair, int tile_cols, cudaStream_t s) {
-  if (args.slices > kOzMaxUsableSlices) return fail(A4G_ERR_ARG, "at most 7 slices");
+  if (!args.residue && args.slices > kOzMaxUsableSlices) return fail(A4G_ERR_ARG, "at most 7 slices");
   int rc = oz_prepare();
   if (rc) return rc;
   if (args.n_units <= 0) return A4G_OK;
+  if (args.residue) {
+    if (args.direct || args.slices > kOzMaxResidues) return fail(A4G_ERR_ARG, "residue form: workspace, at most 15 moduli");
+    if (tile_cols == 256)
+      return pair ? launch_form<true, 256, false, false, true>(args, grid, s)
+                  : launch_form<false, 256, false, false, true>(args, grid, s);
+    return pair ? launch_form<true, 128, false, false, true>(args, grid, s)
+                : launch_form<false, 128, false, false, true>(args, grid, s);
+  }
   if (args.direct) {
     if (tile_cols != 128 || args.nsplit != 1 || args.n_units % args.slices)
       return fail(A4G_ERR_ARG, "direct form: 128-column tiles, one split, whole tiles");

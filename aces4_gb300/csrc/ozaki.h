@@ -30,6 +30,16 @@ int oz_launch_gemm(const OzGemmArgs& args, int grid, bool pair, int tile_cols, c
 constexpr int kOzLevelsTileCols = 64;
 bool oz_levels_fit(int slices, int kb_total);
 int oz_launch_levels(const OzGemmArgs& args, int grid, cudaStream_t s);
+// Residue form (residue.cu): the number of products for K columns at `slices`
+// slices (0: not possible), its tables, the operand side and the
+// reconstruction (ws as int16, see OzGemmArgs).
+int oz_residue_count(int slices, int64_t K);
+void oz_residue_tables(int slices, int L, int64_t K, OzResidues* r, OzCrt* t);
+int oz_launch_residues(int layout, const OzSplitJob* jobs, const int64_t* prefix, int njobs, int64_t ntiles,
+                       const OzPanel* panels, const OzResidues& r, cudaStream_t s);
+int oz_launch_residue_recombine(const OzTile* tiles, int ntiles, int tile_rows, int tile_cols,
+                                const OzDBlock* dblocks, const OzPanel* pa, const OzPanel* pb, const void* ws,
+                                const OzCrt& t, int nsplit, int mode, cudaStream_t s);
 int oz_wait_timeout_selftest(int limit_ms, int* waited_ms, cudaStream_t s);
 // device runs of the one-rounding helpers (exact_fp.h) over device arrays
 int oz_round_selftest(int n, const long long* v, const int* e2, const int* neg, double* out, cudaStream_t s);

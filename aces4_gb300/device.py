@@ -428,6 +428,10 @@ class Batch:
         return {"form": f.value, "name": self.FORMS.get(f.value),
                 "tuned_ms": {self.FORMS[i + 1]: float(ms[i]) for i in range(n) if ms[i] >= 0}}
 
+    def products(self) -> int:
+        """Tensor-core products per block pair (a4g_batch_products; 0 for FP64)."""
+        return int(lib().a4g_batch_products(self._h))
+
     def close(self):
         if getattr(self, "_h", None) and self._h.value:
             lib().a4g_batch_destroy(self._h)

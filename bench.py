@@ -658,7 +658,8 @@ def run_ladder_full(args, world, rank, local):
     t0 = time.perf_counter()
     b = create()
     cold_ms = (time.perf_counter() - t0) * 1e3
-    cold = {"create_ms": cold_ms, **b.tuning(), "form": b.form(), "split_k": b.splits(), "info": b.info()}
+    cold = {"create_ms": cold_ms, **b.tuning(), "form": b.form(), "split_k": b.splits(), "info": b.info(),
+            "products": b.products()}
     launches_full = b.launches()["kernels_per_run"]
     b.close()
 
@@ -919,7 +920,7 @@ def run_ladder_full(args, world, rank, local):
 
     if rank == 0:
         gemm_ms = phases["gemm"]
-        bf16_flops = S * (S + 1) / 2 * slab_flop
+        bf16_flops = cold["products"] * slab_flop
         achieved = bf16_flops / (gemm_ms * 1e-3) / 1e12
         long_run = ms * args.steps >= 2000.0
         peak_key = "bf16_tflops_sustained" if long_run else "bf16_tflops"
@@ -932,7 +933,7 @@ def run_ladder_full(args, world, rank, local):
             "vs_baseline": None, "dtype": f"f64 (Ozaki, {S} BF16 slices)", "data": "synthetic",
             "config": {"workload": full_workload_name(nv, no, len(all_slabs)), "slices": S,
                        "slabs_per_run": k_run,
-                       "digits": "balanced base-256 (8-bit)", "slabs": len(all_slabs), "slabs_this_rank": len(slabs),
+                       "products": cold["products"], "slabs": len(all_slabs), "slabs_this_rank": len(slabs),
                        "block_pairs_per_slab": cold["info"]["pairs"],
                        "l2": f"per slab V {n_v * 8 / 1e9:.2f} GB + T {T.buf.numel() * 8 / 1e9:.2f} GB > 126 MB L2 "
                              "(no flush needed)",
@@ -943,7 +944,7 @@ def run_ladder_full(args, world, rank, local):
             "roofline": {"kernel": "oz_gemm_kernel (tcgen05 BF16 slice products)", "bound": "tensor",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_kind": f"{peak_key} of {peak_kind} (timed region {ms * args.steps / 1e3:.1f} s)",
-                         "algorithmic_per_launch": f"{S * (S + 1) // 2} slice-pair GEMMs x {k_run} slab(s) x "
+                         "algorithmic_per_launch": f"{cold['products']} BF16 products x {k_run} slab(s) x "
                                                    f"{slab_flop:.3e} flop",
                          "traffic": _traffic("oz_gemm_kernel") if k_run == 1 else None},
             "fp64_plain": ({"value": fp64_value, "unit": "TFLOP/s", "ms_per_slab": fp64_ms,
@@ -1424,6 +1425,7 @@ def main():
     barrier()
     ms = max_over_ranks(ev0.elapsed_time(ev1) / args.steps)
     phases = split.timings()
+    products = split.products()
     value = world * flops / (ms * 1e-3) / 1e12
     R_split = R.buf.clone()
     bound = split.error_bound(stream=stream)
@@ -1541,7 +1543,7 @@ def main():
                              f"(OpenMP) + numpy OpenBLAS dgemm, all {cores} host threads"}
         runs = max(1, phases["runs"])
         gemm_ms = phases["gemm"] / runs
-        bf16_flops = S * (S + 1) / 2 * flops
+        bf16_flops = products * flops
         achieved = bf16_flops / (gemm_ms * 1e-3) / 1e12
         # the burst peak for a short timed region, the sustained one once the
         # timed region runs long enough for the power cap to act
@@ -1549,21 +1551,22 @@ def main():
         peak_key = "bf16_tflops_sustained" if long_run else "bf16_tflops"
         peak = peaks.get(peak_key, 1743.3 if long_run else 1933.6)
         n_elem = sum(V.size(k) for k in V.keys()) + sum(T.size(k) for k in T.keys())
-        split_bytes = n_elem * (8 + 2 * S)
+        planes = S if products == S * (S + 1) // 2 else products  # digit slices or residues
+        split_bytes = n_elem * (8 + 2 * planes)
         exp_bytes = n_elem * 8
         ck = clk.summary()
         out = {
             "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": f"f64 (Ozaki, {S} BF16 slices)", "data": "synthetic",
-            "config": {"workload": workload, "slices": S, "digits": "balanced base-256 (8-bit)", "block_pairs": info["pairs"],
+            "config": {"workload": workload, "slices": S, "products": products, "block_pairs": info["pairs"],
                        "l2": f"inputs {n_elem * 8 / 1e9:.2f} GB > 126 MB L2 (no flush needed)",
                        "parallelism": f"replicas x{world}"},
             "e2e": e2e,
             "roofline": {"kernel": "oz_gemm_kernel (tcgen05 BF16 slice products)", "bound": "tensor",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_kind": f"{peak_key} of {peak_kind} (timed region {ms * args.steps / 1e3:.2f} s)",
-                         "algorithmic_per_launch": f"{S * (S + 1) // 2} slice-pair GEMMs x {flops:.3e} flop",
+                         "algorithmic_per_launch": f"{products} BF16 products x {flops:.3e} flop",
                          "traffic": _traffic("oz_gemm_kernel")},
             "fp64_plain": ({"value": fp64_value, "unit": "TFLOP/s", "ms_per_step": fp64_ms,
                             "kernel": "grouped DMMA (mma.sync f64)",

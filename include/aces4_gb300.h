@@ -284,8 +284,12 @@ typedef struct a4g_triple {
 typedef struct a4g_batch_opts {
   int precision;   /* A4G_PREC_*                                              */
   int slices;      /* BF16 digit slices per operand (Ozaki), 1..7; 0 = 5.
-                      Each slice is a balanced base-256 digit; 5 slices keep
-                      the relative error near 1e-11, 6 near 1e-13.          */
+                      An operand element is rounded to 8 * slices bits of its
+                      row's largest element; 5 slices keep the relative error
+                      near 1e-11, 6 near 1e-13.  At 5 and more slices and k
+                      ranges of 1536 and more the products run modulo coprime
+                      numbers (a4g_batch_products) unless `variant` names a
+                      digit form; both round the operands alike.            */
   int beta;        /* 0: D = sum of products (overwrite); 1: D += sum        */
   int variant;     /* split precision, tensor-core GEMM form: 0 autotuned at
                       creation (each form timed once and scored with the
@@ -339,6 +343,12 @@ int a4g_batch_launches(const a4g_batch* b, int* kernels_per_run, int* gemm_parts
  * batches) and the autotuner's score of each form in ms (-1: not run): the
  * GEMM's measured time + the workspace read and D traffic at the copy rate. */
 int a4g_batch_form(const a4g_batch* b, int* form, float* tuned_ms, int n);
+/* Tensor-core products (one BF16 matrix product each) a split-precision run
+ * takes per block pair: slices (slices + 1) / 2 digit products, or, from 5
+ * slices on and for k ranges of at least 1536, one product per modulus of the
+ * residue form (11 at 5 slices; the same operand rounding, no dropped terms).
+ * 0 for FP64 batches. */
+int a4g_batch_products(const a4g_batch* b);
 void a4g_batch_destroy(a4g_batch* b);
 
 /* ----------------------------------------------------------------------------
