@@ -824,11 +824,11 @@ int a4g_fused_create(a4g_fused** out, int drank, int lrank, int rrank, const a4g
     for (size_t i = 0; i < hp.size(); ++i) {
       hp[i].base = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(p) + at[i]);
       hp[i].exps = f->d_exps + offset_of(hp[i].exps);
-      // all-levels form: 32-wide k boxes of 128 rows (A) or 64 columns (B)
-      const int box_rows = P.levels && int(i) >= P.nA ? kOzLevelsTileCols : kOzBM;
-      if ((rc = oz_make_tensor_map_k(maps[i].b, hp[i].base, hp[i].kpad, int64_t(S) * hp[i].rows_pad, box_rows,
-                                     P.levels ? 32 : kOzBK)))
-        return rc;
+      // all-levels form: every slice's 32-wide k box of 128 rows (A) or 64 columns (B)
+      rc = P.levels ? oz_make_levels_map(maps[i].b, hp[i].base, hp[i].kpad, hp[i].rows_pad, S,
+                                         int(i) >= P.nA ? kOzLevelsTileCols : kOzBM)
+                    : oz_make_tensor_map(maps[i].b, hp[i].base, hp[i].kpad, int64_t(S) * hp[i].rows_pad, kOzBM);
+      if (rc) return rc;
     }
     MapImage* d_maps = nullptr;
     if ((rc = fupload(f.get(), maps, &d_maps))) return rc;

@@ -198,8 +198,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, uint3
       "l"(map), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const void* map, uint64_t* bar, int c0, int c1) {
-  tma_load_2d(smem_u32(dst), map, smem_u32(bar), c0, c1);
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+          dst),
+      "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -989,12 +993,18 @@ __global__ void __launch_bounds__(DIRECT ? kThreadsOzDirect : kThreadsOz, 1)
 // of a 128 x 64 tile lives in TMEM at once (levels 0-2 one each; levels 3 and
 // 4, whose sums over 320 k could pass 2^24, one per half of the k range:
 // 7 x 64 = 448 columns).  Each 32-wide k block of the tile's S A-slices and S
-// B-slices is then loaded once for all S (S + 1) / 2 slice pairs, where the
-// level-by-level form loads two tiles per pair.  When the tile's MMAs
-// complete, the epilogue reads each accumulator once, forms the exact sum
-// over levels (the same 64-bit integer as the level-by-level Horner sum) in
-// registers and releases TMEM before it rounds and divides, sums or stores:
-// the tensor cores run the next tile meanwhile.
+// B-slices is loaded once (one 3-D copy per operand) for all S (S + 1) / 2
+// slice pairs, where the level-by-level form loads two tiles per pair.
+// A slice i multiplies B slices 0, 1, ... into levels i, i + 1, ...: B slices
+// lie one after another in shared memory (rows of one taller operand) and the
+// levels' accumulators side by side in TMEM, so one MMA of up to 256 columns
+// covers up to four slice pairs and reads A slice i from shared memory once
+// for all of them: 6 MMAs (8 in the second half of the k range) and 54 KB (62)
+// of operand reads per 16 k instead of 15 MMAs of 64 columns and 90 KB.  When
+// the tile's MMAs complete, the epilogue reads each accumulator once, forms
+// the exact sum over levels (the same 64-bit integer as the level-by-level
+// Horner sum) in registers and releases TMEM before it rounds and divides,
+// sums or stores: the tensor cores run the next tile meanwhile.
 constexpr int kLvBN = 64, kLvBK = 32, kLvMaxS = 5, kLvSt = 3, kLvAcc = 7;
 constexpr uint32_t kLvATile = kOzBM * kLvBK * 2;  // 8 KB: 128 rows x 32 k
 constexpr uint32_t kLvBTile = kLvBN * kLvBK * 2;  // 4 KB: 64 columns x 32 k
@@ -1007,95 +1017,115 @@ struct __align__(1024) LvSmem {
   volatile int abort;
 };
 static_assert(kLvBN == kOzLevelsTileCols, "tile columns of the all-levels form");
-// TMEM accumulator (in 64-column units) of level t; levels 3 and 4: of k half h.
-__device__ __forceinline__ int lv_acc(int t, int h) { return t < 3 ? t : 2 * t - 3 + h; }
+// TMEM accumulator (in 64-column units) of level t; levels 3 and 4: of k half
+// h.  The levels of each half lie side by side: 0 1 2 3 4 | 3' 4'.
+__device__ __forceinline__ int lv_acc(int t, int h) { return t + (t >= 3 && h ? 2 : 0); }
 
 // Shared-memory matrix descriptor: K-major, 64-byte swizzle, rows of 64 B,
-// 8-row core groups 512 B apart.
-__device__ __forceinline__ uint64_t sw64_desc(const void* tile) {
-  const uint32_t addr = smem_u32(tile);
-  uint64_t d = uint64_t((addr & 0x3FFFF) >> 4);
-  d |= uint64_t(1) << 16;          // leading byte offset (unused for swizzled K-major)
-  d |= uint64_t(512 >> 4) << 32;   // stride byte offset
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(4) << 61;          // SWIZZLE_64B
-  return d;
+// 8-row core groups 512 B apart; `lo` as sw128_desc_lo.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t lo) {
+  constexpr uint32_t hi = uint32_t(512 >> 4) | (1u << 14) | (4u << 29);  // SBO, version 1, SWIZZLE_64B
+  return (uint64_t(hi) << 32) | lo;
 }
 
 // Per 32-wide k block of a tile, one stage: the S A-slices (rows m0..m0+127)
-// and the S B-slices (columns n0..n0+63).
+// and the S B-slices (columns n0..n0+63).  Converged warp, one lane issues.
 __device__ void lv_producer(const OzGemmArgs& a, LvSmem& sm) {
-  const int S = a.slices;
-  const uint32_t bytes = uint32_t(S) * (kLvATile + kLvBTile);
-  uint32_t it = 0;
+  const uint32_t bytes = uint32_t(a.slices) * (kLvATile + kLvBTile);
+  const bool leader = elect_one();
+  const uint32_t a0 = smem_u32(sm.a[0][0]), b0 = smem_u32(sm.b[0][0]);
+  const uint32_t full0 = smem_u32(&sm.full[0]), empty0 = smem_u32(&sm.empty[0]);
+  uint32_t s = 0, free_parity = 1;
   for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x)) {
     const OzTile tl = a.tiles[g];
     const void* ma = static_cast<const uint8_t*>(a.maps_a) + size_t(tl.panel_a) * 128;
     const void* mb = static_cast<const uint8_t*>(a.maps_b) + size_t(tl.panel_b) * 128;
-    const int rpa = a.panels_a[tl.panel_a].rows_pad, rpb = a.panels_b[tl.panel_b].rows_pad;
     for (int q = tl.trip_begin; q < tl.trip_end; ++q) {
       const OzTrip tr = a.trips[q];
-      for (int j = 0; j < 2 * tr.nkb; ++j) {
-        const int s = int(it % kLvSt);
-        const uint32_t ph = (it / kLvSt) & 1;
-        if (!mbar_wait(&sm.empty[s], ph ^ 1, sm, a.err_flag, 1)) return;
-        mbar_expect_tx(&sm.full[s], bytes);
-        const int ka = int(tr.koff_a) + j * kLvBK, kb = int(tr.koff_b) + j * kLvBK;
-        for (int i = 0; i < S; ++i) {
-          tma_load_2d(sm.a[s][i], ma, &sm.full[s], ka, i * rpa + tl.m0);
-          tma_load_2d(sm.b[s][i], mb, &sm.full[s], kb, i * rpb + tl.n0);
+      int ka = int(tr.koff_a), kb = int(tr.koff_b);
+      for (int j = 0; j < 2 * tr.nkb; ++j, ka += kLvBK, kb += kLvBK) {
+        if (!warp_wait(empty0 + 8 * s, free_parity, sm, a.err_flag, 1)) return;
+        if (leader) {
+          const uint32_t fb = full0 + 8 * s;
+          mbar_expect_tx(fb, bytes);
+          tma_load_3d(a0 + s * (kLvMaxS * kLvATile), ma, fb, ka, tl.m0, 0);
+          tma_load_3d(b0 + s * (kLvMaxS * kLvBTile), mb, fb, kb, tl.n0, 0);
         }
-        ++it;
+        __syncwarp();
+        if (++s == uint32_t(kLvSt)) s = 0, free_parity ^= 1;
       }
     }
   }
 }
 
-// One thread issues every MMA: per stage, slice pair (i, j) with i + j < S
-// into the accumulator of level i + j (k half h for levels 3 and 4: the
-// tile's 2 kb_total 32-wide blocks split in two equal halves, at most 160 k
-// each).  The first MMA into an accumulator overwrites it.
-__device__ void lv_mma(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem) {
-  const int S = a.slices;
-  uint32_t it = 0, nt = 0;
-  for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x), ++nt) {
-    const OzTile tl = a.tiles[g];
-    const int half = tl.kb_total;
-    if (!mbar_wait(&sm.acc_empty, (nt & 1) ^ 1, sm, a.err_flag, 2)) return;
-    tc_fence_after();
-    int kb = 0;
-    for (int q = tl.trip_begin; q < tl.trip_end; ++q) {
-      const int nk = 2 * a.trips[q].nkb;
-      for (int j = 0; j < nk; ++j, ++kb) {
-        const int s = int(it % kLvSt);
-        const uint32_t ph = (it / kLvSt) & 1;
-        if (!mbar_wait(&sm.full[s], ph, sm, a.err_flag, 3)) return;
-        tc_fence_after();
-        // one issue slot per MMA: the slices' descriptors are the stage's first
-        // plus the tile offset (in 16-byte units), the accumulator columns and
-        // the overwrite flags fixed per stage
-        const uint32_t h64 = kb >= half ? uint32_t(kLvBN) : 0u;  // levels 3, 4: second k half
-        const uint32_t acc_lo = kb == 0 ? 0u : 1u;                // levels 0-2: overwrite at the first block
-        const uint32_t acc_hi = kb == 0 || kb == half ? 0u : 1u;  // levels 3, 4: at the first block of a half
-        const uint64_t ad0 = sw64_desc(sm.a[s][0]), bd0 = sw64_desc(sm.b[s][0]);
+// One MMA (16 k) of 64 * levels columns.
+__device__ __forceinline__ void lv_mma_one(uint32_t d, uint32_t ad, uint32_t bd, int levels, uint32_t acc) {
+  const uint32_t idesc = idesc_bf16<128, 0>() | (uint32_t(levels) << 20);  // N >> 3 = 8 * levels at bit 17
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(sw64_desc(ad)), "l"(sw64_desc(bd)), "r"(idesc), "r"(acc));
+}
+
+// The MMAs of one 16-k step of S slices: A slice i against B slices j into
+// levels i + j < S, as few and as wide as the accumulators' order allows
+// (second half of the k range: levels 3 and 4 have accumulators of their own).
+// acc_lo / acc_hi: 0 where the first MMA into levels 0-2 / 3-4 overwrites.
+template <int S, bool SECOND>
+__device__ __forceinline__ void lv_step(uint32_t tmem, uint32_t ad, uint32_t bd, uint32_t acc_lo, uint32_t acc_hi) {
+  constexpr uint32_t kA = kLvATile >> 4, kB = kLvBTile >> 4;
 #pragma unroll
-        for (int i = 0; i < kLvMaxS; ++i) {
-#pragma unroll
-          for (int jj = 0; jj < kLvMaxS - i; ++jj) {
-            const int t = i + jj;
-            if (t >= S) continue;
-            const uint32_t d = tmem + uint32_t(kLvBN * lv_acc(t, 0)) + (t >= 3 ? h64 : 0u);
-            const uint32_t acc = i > 0 ? 1u : (t < 3 ? acc_lo : acc_hi);
-            const uint64_t ad = ad0 + uint64_t(i) * (kLvATile >> 4), bd = bd0 + uint64_t(jj) * (kLvBTile >> 4);
-            tc_mma<kLvBN>(d, ad, bd, acc);
-            tc_mma<kLvBN>(d, ad + 2, bd + 2, 1u);  // the block's second 16 k: 32 B further
-          }
-        }
-        tc_commit(&sm.empty[s]);
-        ++it;
-      }
+  for (int i = 0; i < S; ++i) {
+    const uint32_t ai = ad + uint32_t(i) * kA;
+    if constexpr (!SECOND) {
+      const int n = S - i < 4 ? S - i : 4;  // levels i .. i + n - 1: at most 256 columns
+      lv_mma_one(tmem + uint32_t(kLvBN * i), ai, bd, n, i == 0 ? acc_lo : 1u);
+      if (n < S - i) lv_mma_one(tmem + uint32_t(kLvBN * (i + n)), ai, bd + uint32_t(n) * kB, S - i - n, i == 0 ? acc_hi : 1u);
+    } else {
+      const int lo = (S < 3 ? S : 3) - i;  // levels i .. 2
+      if (lo > 0) lv_mma_one(tmem + uint32_t(kLvBN * i), ai, bd, lo, i == 0 ? acc_lo : 1u);
+      const int t = i > 3 ? i : 3;         // levels t .. S - 1
+      if (S - t > 0)
+        lv_mma_one(tmem + uint32_t(kLvBN * (t + 2)), ai, bd + uint32_t(t - i) * kB, S - t, i == 0 ? acc_hi : 1u);
     }
-    tc_commit(&sm.acc_full);
+  }
+}
+
+// The tile's 2 kb_total 32-wide k blocks in two equal halves (at most 160 k
+// each); the first MMA into an accumulator overwrites it.  Converged warp, one
+// lane issues.
+template <int S>
+__device__ void lv_mma(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem) {
+  const bool leader = elect_one();
+  const uint32_t full0 = smem_u32(&sm.full[0]), empty0 = smem_u32(&sm.empty[0]);
+  const uint32_t acc_full = smem_u32(&sm.acc_full), acc_empty = smem_u32(&sm.acc_empty);
+  const uint32_t ad0 = sw128_desc_lo(sm.a[0][0]), bd0 = sw128_desc_lo(sm.b[0][0]);
+  uint32_t s = 0, full_parity = 0, free_parity = 1;
+  for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x)) {
+    const int half = a.tiles[g].kb_total;
+    if (!warp_wait(acc_empty, free_parity, sm, a.err_flag, 2)) return;
+    free_parity ^= 1;
+    tc_fence_after();
+    for (int kb = 0; kb < 2 * half; ++kb) {
+      if (!warp_wait(full0 + 8 * s, full_parity, sm, a.err_flag, 3)) return;
+      tc_fence_after();
+      if (leader) {
+        const uint32_t ad = ad0 + s * (kLvMaxS * kLvATile >> 4), bd = bd0 + s * (kLvMaxS * kLvBTile >> 4);
+        if (kb < half) {
+          const uint32_t acc = kb == 0 ? 0u : 1u;
+          lv_step<S, false>(tmem, ad, bd, acc, acc);
+          lv_step<S, false>(tmem, ad + 2, bd + 2, 1u, 1u);  // the block's second 16 k: 32 B further
+        } else {
+          lv_step<S, true>(tmem, ad, bd, 1u, kb == half ? 0u : 1u);
+          lv_step<S, true>(tmem, ad + 2, bd + 2, 1u, 1u);
+        }
+        tc_commit(empty0 + 8 * s);
+        if (kb + 1 == 2 * half) tc_commit(acc_full);
+      }
+      __syncwarp();
+      if (++s == uint32_t(kLvSt)) s = 0, full_parity ^= 1;
+    }
   }
 }
 
@@ -1118,14 +1148,13 @@ struct LvCol {
 //   quotient exactly rounded; zeros add nothing);
 //   store form: D = x or D += x.
 // A non-finite operand value in the row or column makes x NaN.
-template <bool ENERGY>
+template <bool ENERGY, int S>
 __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int warp, int lane) {
   __shared__ LvCol lv_cols[kThreadsOzDirect / 32 - 2][16];
   LvCol* tab = lv_cols[warp - 2];
   const int q = warp & 3, h = (warp - 2) >> 2;
   const int row = 32 * q + lane;
   const uint32_t lane_addr = tmem + (uint32_t(32 * q) << 16) + uint32_t(16 * h);
-  const int S = a.slices;
   [[maybe_unused]] double eacc = 0.0;
   uint32_t nt = 0;
   for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x), ++nt) {
@@ -1188,12 +1217,11 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
         // 3 and 4: the sum of the two halves)
         long long r = 0;
 #pragma unroll
-        for (int t = 0; t < kLvMaxS; ++t)
-          if (t < S) {
+        for (int t = 0; t < S; ++t) {
             long long st = __float2int_rz(__uint_as_float(v[lv_acc(t, 0)][j]));
             if (t >= 3) st += __float2int_rz(__uint_as_float(v[lv_acc(t, 1)][j]));
             r = r * 256 + st;
-          }
+        }
         sum[8 * gg + j] = r;
       }
     }
@@ -1227,7 +1255,7 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
   if constexpr (ENERGY) a.epart[(size_t(blockIdx.x) * 16 + size_t(warp - 2)) * 32 + lane] = eacc;
 }
 
-template <bool ENERGY>
+template <bool ENERGY, int S>
 __global__ void __launch_bounds__(kThreadsOzDirect, 1) oz_levels_kernel(const __grid_constant__ OzGemmArgs a) {
   extern __shared__ uint8_t smem_raw[];
   LvSmem& sm = *reinterpret_cast<LvSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1253,15 +1281,14 @@ __global__ void __launch_bounds__(kThreadsOzDirect, 1) oz_levels_kernel(const __
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   if (warp == 0) {
-    if (lane == 0) lv_producer(a, sm);
+    lv_producer(a, sm);
   } else if (warp == 1) {
-    if (lane == 0) {
-      lv_mma(a, sm, tmem);
-      tc_commit(&sm.drain);  // all MMAs this thread issued have completed before TMEM is released
-      mbar_wait(&sm.drain, 0, sm, a.err_flag, 5);
-    }
+    lv_mma<S>(a, sm, tmem);
+    if (elect_one()) tc_commit(&sm.drain);  // all MMAs of this warp have completed before TMEM is released
+    __syncwarp();
+    warp_wait(smem_u32(&sm.drain), 0, sm, a.err_flag, 5);
   } else {
-    lv_epilogue<ENERGY>(a, sm, tmem, warp, lane);
+    lv_epilogue<ENERGY, S>(a, sm, tmem, warp, lane);
   }
   tc_fence_before();
   __syncthreads();
@@ -1869,24 +1896,36 @@ int oz_chunk_kb(int level) {
 }
 
 int oz_make_tensor_map(void* map128, const void* base, int64_t kpad, int64_t rows_total, int box_rows) {
-  return oz_make_tensor_map_k(map128, base, kpad, rows_total, box_rows, kOzBK);
-}
-
-int oz_make_tensor_map_k(void* map128, const void* base, int64_t kpad, int64_t rows_total, int box_rows, int box_k) {
   EncodeTiled enc = get_encoder();
   if (!enc) return fail(A4G_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-  if (box_k != kOzBK && box_k != kLvBK) return fail(A4G_ERR_ARG, "tensor map: k box of 64 or 32");
   if (kpad % kOzBK != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0)
     return fail(A4G_ERR_ARG, "panel not aligned for TMA");
   cuuint64_t dims[2] = {cuuint64_t(kpad), cuuint64_t(rows_total)};
   cuuint64_t strides[1] = {cuuint64_t(kpad) * 2};
-  cuuint32_t box[2] = {cuuint32_t(box_k), cuuint32_t(box_rows)};
+  cuuint32_t box[2] = {cuuint32_t(kOzBK), cuuint32_t(box_rows)};
   cuuint32_t estr[2] = {1, 1};
-  // rows of 128 B (64 k) with the 128-byte swizzle, of 64 B (32 k) with the 64-byte one
   CUresult r = enc(reinterpret_cast<CUtensorMap*>(map128), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   box_k == kOzBK ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(A4G_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(int(r)));
+  return A4G_OK;
+}
+
+int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t rows_pad, int slices, int box_rows) {
+  EncodeTiled enc = get_encoder();
+  if (!enc) return fail(A4G_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+  if (kpad % kOzBK != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0)
+    return fail(A4G_ERR_ARG, "panel not aligned for TMA");
+  cuuint64_t dims[3] = {cuuint64_t(kpad), cuuint64_t(rows_pad), cuuint64_t(slices)};
+  cuuint64_t strides[2] = {cuuint64_t(kpad) * 2, cuuint64_t(rows_pad) * cuuint64_t(kpad) * 2};
+  cuuint32_t box[3] = {cuuint32_t(kLvBK), cuuint32_t(box_rows), cuuint32_t(slices)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  // rows of 64 B (32 k) with the 64-byte swizzle
+  CUresult r = enc(reinterpret_cast<CUtensorMap*>(map128), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(A4G_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(int(r)));
   return A4G_OK;
 }
@@ -1944,11 +1983,24 @@ int set_smem_attr() {
   return A4G_OK;
 }
 
-template <bool ENERGY>
+template <bool ENERGY, int S = kLvMaxS>
 int set_levels_attr() {
-  A4G_CUDA(cudaFuncSetAttribute(oz_levels_kernel<ENERGY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  A4G_CUDA(cudaFuncSetAttribute(oz_levels_kernel<ENERGY, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 int(sizeof(LvSmem)) + 1024));
-  return A4G_OK;
+  if constexpr (S > 1) return set_levels_attr<ENERGY, S - 1>();
+  else return A4G_OK;
+}
+
+template <bool ENERGY>
+void launch_levels(const OzGemmArgs& args, int grid, cudaStream_t s) {
+  const size_t smem = sizeof(LvSmem) + 1024;
+  switch (args.slices) {
+    case 1: oz_levels_kernel<ENERGY, 1><<<grid, kThreadsOzDirect, smem, s>>>(args); break;
+    case 2: oz_levels_kernel<ENERGY, 2><<<grid, kThreadsOzDirect, smem, s>>>(args); break;
+    case 3: oz_levels_kernel<ENERGY, 3><<<grid, kThreadsOzDirect, smem, s>>>(args); break;
+    case 4: oz_levels_kernel<ENERGY, 4><<<grid, kThreadsOzDirect, smem, s>>>(args); break;
+    default: oz_levels_kernel<ENERGY, 5><<<grid, kThreadsOzDirect, smem, s>>>(args); break;
+  }
 }
 
 // Function attributes are set once per device (they belong to the device's
@@ -2054,12 +2106,11 @@ int oz_launch_levels(const OzGemmArgs& args, int grid, cudaStream_t s) {
   int rc = oz_prepare();
   if (rc) return rc;
   if (args.n_tiles <= 0) return A4G_OK;
-  const size_t smem = sizeof(LvSmem) + 1024;
   if (args.energy) {
     if (!args.eblocks || !args.epart) return fail(A4G_ERR_ARG, "energy form: tables");
-    oz_levels_kernel<true><<<grid, kThreadsOzDirect, smem, s>>>(args);
+    launch_levels<true>(args, grid, s);
   } else {
-    oz_levels_kernel<false><<<grid, kThreadsOzDirect, smem, s>>>(args);
+    launch_levels<false>(args, grid, s);
   }
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
