@@ -42,6 +42,13 @@ struct Context {
   // every synchronisation, so a synchronous call would allocate from scratch
   // each time.
   cudaMemPool_t pool = nullptr;
+  // Scratch of the deterministic reductions: rings of slots, one per launch in
+  // turn, so that launches on several streams (or from several threads) that
+  // overlap do not share one.  The counters' ring is the longer one: a counter
+  // that two launches shared would not come back to zero.
+  static constexpr int kReducePartials = 1024, kReduceSlots = 256, kReduceCounters = 65536;
+  double* reduce_partials = nullptr;  // [slot][kReducePartials + 8]
+  unsigned* reduce_counters = nullptr;
   // Kernels can read and write pageable host memory through the host's page
   // tables (address translation services over the CPU-GPU link): the
   // drop-ins then run on the caller's host blocks in place.
@@ -112,29 +119,33 @@ int launch_permute(int rank, const int* ext, const int* o2n_1based, const double
                    cudaStream_t s);
 int launch_add_sub_permuted(int subtract, int rank, const int* r_ext, const int* o2n_1based,
                             double* d, const double* l, const double* r, cudaStream_t s);
-int launch_dot(const double* a, const double* b, const int64_t* offA, const int64_t* offB,
-               int64_t n, double* d_out, double* d_scratch, int64_t scratch_len, cudaStream_t s);
+// Scratch of one reduction: partial sums of its CTAs, the counter of those that
+// have written theirs (zero between launches) and room for a result.
+struct ReductionSlot {
+  double* partial = nullptr;
+  double* result = nullptr;
+  unsigned* counter = nullptr;
+};
+// The next slot of the context's rings (after ensure_init).
+ReductionSlot reduction_slot();
+int launch_dot(const double* a, const double* b, const int64_t* offA, const int64_t* offB, int64_t n, double* d_out,
+               const ReductionSlot& slot, int beta, cudaStream_t s);
+int launch_norm2(const double* a, int64_t n, double* d_out, const ReductionSlot& slot, cudaStream_t s);
 int launch_slice_insert(int insert, int rank, double* tens, const int* tens_ext, double* slice,
                         const int* slice_ext, const int* ext_beg, cudaStream_t s);
 int launch_update_t2(const int* off, const int* ext, const double* t2new, const double* t2new_pair,
                      const double* t2old, const double* t2old_pair, double* err, double* next, int rank1, int ld1,
-                     const double* e_or_fock, double* norm2, double* d_scratch, int64_t scratch_len,
-                     cudaStream_t s);
+                     const double* e_or_fock, double* norm2, const ReductionSlot& slot, cudaStream_t s);
 int launch_energy_contract(int rank0, const int* off, const int* ext0, const int* pos, const double* w,
                            int rank1, int ld1, const double* e_or_fock, double efact, double* esum,
-                           double* d_scratch, int scratch_len, cudaStream_t s);
+                           const ReductionSlot& slot, cudaStream_t s);
 int launch_denominator(int rank0, const int* off, const int* ext0, double* data, int rank1,
                        int ld1, const double* e_or_fock, cudaStream_t s);
-int launch_dot_beta(const double* a, const double* b, const int64_t* offA, const int64_t* offB,
-                    int64_t n, double* d_out, double* d_scratch, int64_t scratch_len, int beta,
-                    cudaStream_t s);
-int dot_scratch_len();  // doubles of scratch launch_dot needs
-
 // Permute-fused FP64 contraction (kernels_dmma.cu).
 int launch_contract_f64(const DevPlan* p, const double* L, const double* R, double* D, int beta,
                         cudaStream_t s);
 // Scalar cases of tensor_block_contract_ (kernels_block.cu).
 int launch_scalar_cases(const DevPlan* p, const double* L, const double* R, double* D, int beta,
-                        double* d_scratch, cudaStream_t s);
+                        const ReductionSlot& slot, cudaStream_t s);
 
 }  // namespace a4g

@@ -158,21 +158,12 @@ std::mutex g_predef_mu;
 
 int contract_device(const int* ptrn, const double* l, int lrank, const int* lext, const double* r,
                     int rrank, const int* rext, double* d, int drank, const int* dext, int beta,
-                    double* scratch, cudaStream_t s) {
+                    cudaStream_t s) {
   const DevPlan* p = nullptr;
   int rc = get_dev_plan(ptrn, lrank, lext, rrank, rext, drank, dext, &p);
   if (rc) return rc;
   if (p->host.kind == ContractKind::kTensorTensor) return launch_contract_f64(p, l, r, d, beta, s);
-  return launch_scalar_cases(p, l, r, d, beta, scratch, s);
-}
-
-// Per-context scratch for the deterministic reductions of the device API.
-double* reduction_scratch() {
-  static double* p = nullptr;
-  if (!p) {
-    if (cudaMalloc(&p, sizeof(double) * (dot_scratch_len() + 8)) != cudaSuccess) p = nullptr;
-  }
-  return p;
+  return launch_scalar_cases(p, l, r, d, beta, reduction_slot(), s);
 }
 
 }  // namespace
@@ -248,12 +239,11 @@ double tensor_block_norm2__(int* nthreads, double* tens, int* tens_rank, int* ex
   double result = 0.0;
   HostIO io;
   double* d = nullptr;
-  if (!rc) rc = io.begin(rounded(n) + rounded(dot_scratch_len() + 1));
+  if (!rc) rc = io.begin(rounded(n) + rounded(1));
   if (!rc) rc = io.in(tens, n, &d);
   if (!rc) {
-    double* scratch = io.scratch(dot_scratch_len());
     double* out = io.scratch(1);
-    rc = launch_dot(d, d, nullptr, nullptr, n, out, scratch, dot_scratch_len(), io.s);
+    rc = launch_norm2(d, n, out, reduction_slot(), io.s);
     if (!rc) rc = d2h(&result, out, 1, io.s);
     if (!rc) rc = io.finish();
   }
@@ -348,13 +338,12 @@ void tensor_block_contract__(int* nthreads, int* ptrn, double* ltens, int* lrank
   const int64_t nl = count(*lrank, lext), nr = count(*rrank, rext), nd = count(*drank, dext);
   HostIO io;
   double *dl = nullptr, *dr = nullptr, *dd = nullptr;
-  if (!rc) rc = io.begin(rounded(nl) + rounded(nr) + rounded(nd) + rounded(dot_scratch_len()));
+  if (!rc) rc = io.begin(rounded(nl) + rounded(nr) + rounded(nd));
   if (!rc) rc = io.in(ltens, nl, &dl);
   if (!rc) rc = io.in(rtens, nr, &dr);
   if (!rc) rc = io.out(dtens, nd, false, false, &dd);
   if (!rc)
-    rc = contract_device(ptrn, dl, *lrank, lext, dr, *rrank, rext, dd, *drank, dext, 0,
-                         io.scratch(dot_scratch_len()), io.s);
+    rc = contract_device(ptrn, dl, *lrank, lext, dr, *rrank, rext, dd, *drank, dext, 0, io.s);
   if (!rc) rc = io.finish();
   *ierr = rc == A4G_ERR_PATTERN ? 1 : runtime_ierr(rc);
 }
@@ -547,10 +536,7 @@ int a4g_contract(const int* ptrn, const double* l, int lrank, const int* lext, c
   int rc = ensure_init();
   if (rc) return rc;
   if (!l || !r || !d || !ptrn) return fail(A4G_ERR_ARG, "null pointer");
-  double* scratch = reduction_scratch();
-  if (!scratch) return fail(A4G_ERR_NOMEM, "reduction scratch");
-  return contract_device(ptrn, l, lrank, lext, r, rrank, rext, d, drank, dext, beta ? 1 : 0,
-                         scratch, pick(stream));
+  return contract_device(ptrn, l, lrank, lext, r, rrank, rext, d, drank, dext, beta ? 1 : 0, pick(stream));
 }
 
 int a4g_contract_labels(const int* d_labels, const int* l_labels, const int* r_labels,
@@ -630,11 +616,10 @@ int a4g_add_sub(int subtract, int rank, const int* d_labels, const int* r_labels
 int a4g_norm2(const double* t, int64_t n, double* h_result, void* stream) {
   int rc = ensure_init();
   if (rc) return rc;
-  double* scratch = reduction_scratch();
-  if (!scratch) return fail(A4G_ERR_NOMEM, "reduction scratch");
+  const ReductionSlot slot = reduction_slot();
   cudaStream_t s = pick(stream);
-  double* out = scratch + dot_scratch_len();
-  rc = launch_dot(t, t, nullptr, nullptr, n, out, scratch, dot_scratch_len(), s);
+  double* out = slot.result;
+  rc = launch_norm2(t, n, out, slot, s);
   if (rc) return rc;
   A4G_CUDA(cudaMemcpyAsync(h_result, out, sizeof(double), cudaMemcpyDeviceToHost, s));
   return check_device_flag(s);
@@ -687,10 +672,8 @@ int a4g_update_t2(const int* iv, const int* ext, const double* t2new, const doub
   int off[6];
   rc = denominator_offsets(4, iv, ext, rank1, ext1, std::vector<int>(segs, segs + std::max(nsegs, 0)), off);
   if (rc) return rc;
-  double* scratch = reduction_scratch();
-  if (!scratch) return fail(A4G_ERR_NOMEM, "reduction scratch");
   return launch_update_t2(off, ext, t2new, t2new_pair, t2old, t2old_pair, diis_err, t2old_next, rank1, ext1[0],
-                          e_or_fock, norm2, scratch, dot_scratch_len(), pick(stream));
+                          e_or_fock, norm2, reduction_slot(), pick(stream));
 }
 
 int a4g_selftest_wait_timeout(int limit_ms, int* waited_ms, void* stream) {
@@ -736,10 +719,8 @@ int a4g_energy_contract(int rank0, const int* iv, const int* ext0, const double*
   int off[6];
   rc = denominator_offsets(rank0, iv, ext0, rank1, ext1, std::vector<int>(segs, segs + std::max(nsegs, 0)), off);
   if (rc) return rc;
-  double* scratch = reduction_scratch();
-  if (!scratch) return fail(A4G_ERR_NOMEM, "reduction scratch");
-  return launch_energy_contract(rank0, off, ext0, pos, data0, rank1, ext1[0], e, efact, esum, scratch,
-                                dot_scratch_len(), pick(stream));
+  return launch_energy_contract(rank0, off, ext0, pos, data0, rank1, ext1[0], e, efact, esum, reduction_slot(),
+                                pick(stream));
 }
 
 }  // extern "C"

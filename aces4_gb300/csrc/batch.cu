@@ -1741,16 +1741,16 @@ int a4g_batch_error_bound(a4g_batch* b, double target, double* h_bound, void* st
   std::vector<int> ex(b->exps_bytes / sizeof(int));
   const size_t ng = b->err_groups.size();
   double* dev = nullptr;
-  const int64_t scratch = dot_scratch_len();
-  if (const int rc_ = async_alloc(reinterpret_cast<void**>(&dev), (ng + size_t(scratch)) * sizeof(double), s)) return rc_;
+  if (const int rc_ = async_alloc(reinterpret_cast<void**>(&dev), std::max<size_t>(ng, 1) * sizeof(double), s)) return rc_;
+  const ReductionSlot slot = reduction_slot();  // one block after another on this stream
   int rc = A4G_OK;
   for (size_t i = 0; i < ng && !rc; ++i) {
     const a4g_batch::ErrGroup& eg = b->err_groups[i];
-    rc = launch_dot(eg.d, eg.d, nullptr, nullptr, eg.size, dev + scratch + i, dev, scratch, s);
+    rc = launch_norm2(eg.d, eg.size, dev + i, slot, s);
   }
   std::vector<double> nrm2(ng);
   if (!rc && ng) {
-    A4G_CUDA(cudaMemcpyAsync(nrm2.data(), dev + scratch, ng * sizeof(double), cudaMemcpyDeviceToHost, s));
+    A4G_CUDA(cudaMemcpyAsync(nrm2.data(), dev, ng * sizeof(double), cudaMemcpyDeviceToHost, s));
   }
   if (!rc) A4G_CUDA(cudaMemcpyAsync(ex.data(), b->d_exps, b->exps_bytes, cudaMemcpyDeviceToHost, s));
   cudaFreeAsync(dev, s);

@@ -49,15 +49,6 @@ A4G_HD double double_of(unsigned long long u) {
   return x;
 #endif
 }
-// 1/x rounded to the nearest float
-A4G_HD float frcp_rn(float x) {
-#if defined(__CUDA_ARCH__)
-  return __frcp_rn(x);
-#else
-  return 1.0f / x;
-#endif
-}
-
 // The double nearest (ties to even) to u * 2^e2 with sign `neg`, u an
 // unsigned 64-bit magnitude, rounded once: to 53 bits in the normal range, to
 // a multiple of 2^-1074 below it (subnormal results and zero), to infinity
@@ -132,6 +123,17 @@ A4G_HD double i64_scaled_to_double(long long v, int e2, bool neg) {
   return double_of(bits);
 }
 
+#if defined(__CUDACC__)
+// v * 2^e2 rounded once, branch-free: valid (the return value) for v != 0 and
+// a normal result; the same bits as i64_scaled_to_double there.
+__device__ __forceinline__ bool i64_scaled_normal(long long v, int e2, double* x) {
+  const unsigned long long b = bits_of(__ll2double_rn(v));
+  const int field = int((b >> 52) & 0x7FF) + e2;
+  *x = double_of(b + ((unsigned long long)(long long)e2 << 52));
+  return v != 0 && uint32_t(field - 1) < 2046u;
+}
+#endif
+
 // The same for a two's-complement 128-bit integer N.
 A4G_HD double i128_scaled_to_double(__int128 N, int e2) {
   const bool neg = N < 0;
@@ -146,86 +148,126 @@ A4G_HD double i128_scaled_to_double(__int128 N, int e2) {
   return u64_scaled_to_double((top << 1) | (sticky ? 1ull : 0ull), neg, e2 + sh - 1);
 }
 
-// a / b rounded to the nearest double (ties to even; a quotient of two
-// doubles is never exactly halfway) for normal a, b and a normal result;
-// false otherwise (the caller divides in FP64).  With A = ma or 2 ma (the
-// dividend's significand doubled when it is below the divisor's, so that
-// A / mb lies in [1, 2)), the 55-bit quotient Q = floor(A 2^54 / mb) is
-// formed in two digits, each estimated through a 32-bit reciprocal
-// R32 ~ 2^84 / mb and the next one taken from the exact remainder (Knuth,
-// TAOCP vol. 2, 4.3.1: estimate a quotient digit, then continue from the
-// remainder), and the last one corrected from the remainder, which also gives
-// the sticky bit for the rounding.  R32 comes from Newton-Raphson,
-// x' = x + x (1 - d x), in fixed point: the FP32 reciprocal of mb's top 24
-// bits (relative error below 2^-22), one step in 32-bit arithmetic on mb's top
-// 32 bits (below 2^-30).  Digit 1, q1 = (A's top 32 bits) R32 / 2^32, lies
-// within (-2, 4.01) units of A 2^30 / mb, so s1 = A 2^30 - q1 mb (exact in
-// wrapping 64-bit arithmetic) is below 4.01 mb in magnitude; digit 2,
-// q2 = floor((s1 >> 25) R32 / 2^35), lies within one unit of s1 2^24 / mb
-// (the estimate is off by less than 0.19 below and 0.07 above).  So
-// Q = q1 2^24 + q2 is off by at most one unit, one correction each way
-// suffices, and the remainder, below 2 mb < 2^54 in magnitude, is exact in
-// wrapping 64-bit arithmetic.
-A4G_HD bool div_rn_sig(unsigned long long ma, int ea, unsigned long long mb, int eb, unsigned long long sign,
-                       double* q) {
-  const int adj = ma < mb ? 1 : 0;
-  const unsigned long long A = ma << adj;  // [mb, 2 mb)
-  const int field = ea - eb + 1023 - adj;  // biased exponent of the quotient's leading bit
-  if (field < 1 || field > 2045) return false;
-  // seed R32 ~ 2^84 / mb: the FP32 reciprocal of mb's top 24 bits (exact in
-  // FP32) lies in (2^-24, 2^-23]; its significand shifted into place, 2^-23
-  // itself (2^32) clamped to 2^32 - 1
-  const float rf = frcp_rn(float(uint32_t(mb >> 29)));
-  uint32_t rb;
-  memcpy(&rb, &rf, 4);
-  uint32_t R32 = ((rb >> 23) & 0xFFu) == 103u ? (((rb & 0x7FFFFFu) | 0x800000u) << 8) : 0xFFFFFFFFu;
-  // 32-bit step on m32 = mb's top 32 bits: R32 += R32 (2^63 - m32 R32) / 2^63,
-  // the correction formed from e's top 32 bits (|e| < 2^42: the seed is within
-  // 2^-21 of 2^63 / m32)
-  {
-    const uint32_t m32 = uint32_t(mb >> 21);
-    const unsigned long long t = (unsigned long long)m32 * R32;  // ~2^63
-    const bool up = t < (1ull << 63);
-    const unsigned long long e = up ? (1ull << 63) - t : t - (1ull << 63);
-    const unsigned long long d = ((unsigned long long)R32 * uint32_t(e >> 10)) >> 53;
-    const unsigned long long r = up ? (unsigned long long)R32 + d : (unsigned long long)R32 - d;
-    R32 = r > 0xFFFFFFFFull ? 0xFFFFFFFFu : uint32_t(r);
-  }
-  // digit 1: the quotient's top 31 bits; s1 = A 2^30 - q1 mb
-  const uint32_t q1 = uint32_t(((unsigned long long)uint32_t(A >> 22) * R32) >> 32);
-  const long long s1 = (long long)((A << 30) - (unsigned long long)q1 * mb);
-  // digit 2: floor(s1 2^24 / mb), within one unit
-  const long long q2 = ((s1 >> 25) * (long long)R32) >> 35;
-  unsigned long long Q = ((unsigned long long)q1 << 24) + (unsigned long long)q2;
-  long long rem = (long long)(((A & 0x3FFull) << 54) - Q * mb);  // A 2^54 - Q mb, exact: |.| < 2 mb
-  if (rem < 0) --Q, rem += (long long)mb;
-  if (rem >= (long long)mb) ++Q, rem -= (long long)mb;
-  unsigned long long mant = Q >> 2;
-  const unsigned long long guard = (Q >> 1) & 1ull, sticky = (Q & 1ull) | (rem != 0 ? 1ull : 0ull);
-  mant += (guard && (sticky || (mant & 1ull))) ? 1ull : 0ull;
-  *q = double_of((sign << 63) | ((((unsigned long long)(field - 1)) << 52) + mant));
-  return true;
+A4G_HD uint32_t mulhi32(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  return __umulhi(a, b);
+#else
+  return uint32_t(((unsigned long long)a * b) >> 32);
+#endif
+}
+A4G_HD float float_of(uint32_t u) {
+#if defined(__CUDA_ARCH__)
+  return __uint_as_float(u);
+#else
+  float x;
+  memcpy(&x, &u, 4);
+  return x;
+#endif
+}
+A4G_HD uint32_t bits_of(float x) {
+#if defined(__CUDA_ARCH__)
+  return __float_as_uint(x);
+#else
+  uint32_t u;
+  memcpy(&u, &x, 4);
+  return u;
+#endif
+}
+// 1/x, 1 < x < 2, to within one unit in the last place (the GPU's approximate
+// reciprocal; on the host the nearest float, or A4G_RCP_ULP units off it, so
+// that a test can show that the division needs no more than this)
+A4G_HD float rcp_approx(float x) {
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+#ifndef A4G_RCP_ULP
+#define A4G_RCP_ULP 0
+#endif
+  return float_of(bits_of(1.0f / x) + uint32_t(A4G_RCP_ULP));
+#endif
 }
 
+// a / b rounded to the nearest double (ties to even; a quotient of two
+// doubles is never exactly halfway) where a, b and the quotient are normal
+// numbers; the return value says whether it is valid.  Branch-free, so that a
+// kernel can run several divisions interleaved (the FP64 pipe of this GPU
+// takes 5 clocks per division and SM).
+//
+// With significands ma, mb in [2^52, 2^53) and A = ma or 2 ma (doubled when ma
+// < mb, so that v = A 2^52 / mb lies in [2^52, 2^53)), the result's
+// significand is RN(v).  Two quotient digits are estimated through a 31-bit
+// reciprocal and the exact remainder decides the rounding (Knuth, TAOCP vol.
+// 2, 4.3.1: a digit's estimate, then continue from the remainder):
+//  1. R ~ R* = 2^83 / mb, 2^30 < R* <= 2^31: the FP32 reciprocal of f = mb's
+//     top 24 bits with the last two set (f in (1 + 2^-22, 2), so 1/f + 1 lies
+//     below 2 and its fraction field is 2^23 / f; relative error below
+//     2^-20.6), then one Newton-Raphson step R + R (1 - R / R*) in 32-bit
+//     integers on mb's top 32 bits: with t = floor(m32 R / 2^32) and
+//     e = 2^30 - 2 - t, |e| <= 640, R += ((R >> 10) e) >> 20 lands in
+//     (R* - 5.1, R* - 0.9).
+//  2. q1 = floor((A >> 22) R / 2^32) lies in (A 2^29 / mb - 6.6, A 2^29 / mb],
+//     so s1 = A 2^29 - q1 mb (exact in wrapping 64-bit arithmetic) in
+//     [0, 6.6 mb), below 2^56.
+//  3. h = floor((s1 >> 24) R / 2^32) lies in (16 w - 5.7, 16 w] with
+//     w = s1 2^23 / mb = v - q1 2^23; m0 = q1 2^23 + ((h + 10) >> 4) is within
+//     0.67 of v.
+//  4. r = A 2^52 - m0 mb, |r| < 0.67 mb, exact in wrapping 64-bit arithmetic:
+//     RN(v) = m0 + 1 where 2 r > mb, m0 - 1 where 2 r < -mb, else m0.
 A4G_HD bool div_rn_int(double a, double b, double* q) {
   const unsigned long long ua = bits_of(a), ub = bits_of(b);
-  const int ea = int((ua >> 52) & 0x7FF), eb = int((ub >> 52) & 0x7FF);
-  if (ea == 0 || ea == 2047 || eb == 0 || eb == 2047) return false;
-  const unsigned long long ma = (ua & ((1ull << 52) - 1)) | (1ull << 52);
+  const uint32_t ah = uint32_t(ua >> 32), bh = uint32_t(ub >> 32);
   const unsigned long long mb = (ub & ((1ull << 52) - 1)) | (1ull << 52);
-  return div_rn_sig(ma, ea, mb, eb, (ua ^ ub) >> 63, q);
+  unsigned long long A = (ua & ((1ull << 52) - 1)) | (1ull << 52);
+  const int adj = A < mb ? 1 : 0;
+  A += adj ? A : 0ull;  // [mb, 2 mb)
+  const float f = float_of(0x3F800000u | (uint32_t(mb >> 29) & 0x7FFFFFu) | 3u);
+  uint32_t R = (bits_of(rcp_approx(f) + 1.0f) & 0x7FFFFFu) << 8;
+  const int e = int((1u << 30) - 2u - mulhi32(uint32_t(mb >> 21), R));
+  R += uint32_t((int(R >> 10) * e) >> 20);
+  const uint32_t q1 = mulhi32(uint32_t(A >> 22), R);
+  const unsigned long long s1 = (A << 29) - (unsigned long long)q1 * mb;
+  const uint32_t h = mulhi32(uint32_t(s1 >> 24), R);
+  const unsigned long long m0 = (unsigned long long)q1 * (1u << 23) + ((h + 10u) >> 4);
+  const long long r2 = (long long)(((A << 52) - m0 * mb) << 1);
+  const uint32_t up = uint32_t((unsigned long long)((long long)mb - r2) >> 63);
+  const uint32_t down = uint32_t((unsigned long long)((long long)mb + r2) >> 63);
+  // the exponents and the sign in the high word: field = ea - eb + 1023 - adj,
+  // one less because the significand's leading bit adds one
+  const int ea = int((ah >> 20) & 0x7FFu), eb = int((bh >> 20) & 0x7FFu);
+  const int field = ea - eb + 1023 - adj;
+  const uint32_t high = (uint32_t(field - 1) << 20) + ((ah ^ bh) & 0x80000000u);
+  const unsigned long long bits = m0 + (((unsigned long long)high << 32) + up - down);
+  *q = double_of(bits);
+  return uint32_t(ea - 1) < 2046u && uint32_t(eb - 1) < 2046u && uint32_t(field - 1) < 2045u;
 }
 
 // a / b rounded to the nearest double: div_rn_int where it applies, the FP64
 // divide otherwise (zero, subnormal or non-finite operands or results).
-A4G_HD double div_rn(double a, double b) {
-  double q;
-  if (div_rn_int(a, b, &q)) return q;
+A4G_HD double div_rn_slow(double a, double b) {
 #if defined(__CUDA_ARCH__)
   return __ddiv_rn(a, b);
 #else
   return a / b;
 #endif
+}
+A4G_HD double div_rn(double a, double b) {
+  double q;
+  return div_rn_int(a, b, &q) ? q : div_rn_slow(a, b);
+}
+
+// N quotients a[i] / b[i], their steps interleaved; the rare operands that
+// div_rn_int does not take go through the FP64 divide afterwards.
+template <int N>
+A4G_HD void div_rn_n(const double (&a)[N], const double (&b)[N], double (&q)[N]) {
+  bool ok[N], all = true;
+#pragma unroll
+  for (int i = 0; i < N; ++i) ok[i] = div_rn_int(a[i], b[i], &q[i]), all = all && ok[i];
+  if (all) return;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (!ok[i]) q[i] = div_rn_slow(a[i], b[i]);
 }
 
 // x != 0 without the FP64 pipe

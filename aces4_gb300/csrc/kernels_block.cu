@@ -281,43 +281,97 @@ int launch_perm_op(const PermParams& p, const double* in, double* out, const dou
   return A4G_OK;
 }
 
-// ---------------------------------------------------------------- dot / norm
-constexpr int kDotBlocks = 1024;
-__global__ void __launch_bounds__(kThreads) dot_partial_kernel(const double* __restrict__ a,
-                                                               const double* __restrict__ b,
-                                                               const int64_t* __restrict__ offA,
-                                                               const int64_t* __restrict__ offB,
-                                                               int64_t n, double* partial) {
-  double acc = 0.0;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const double x = a[offA ? offA[i] : i];
-    const double y = b[offB ? offB[i] : i];
-    acc = fma(x, y, acc);
-  }
-  __shared__ double red[kThreads / 32];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+// ---------------------------------------------------------------- reductions
+constexpr int kDotBlocks = Context::kReducePartials;  // partials of a reduction: at most so many CTAs
+
+// Deterministic sum of acc over the grid, in the launch that forms it: every
+// CTA writes its sum, and the last one to arrive adds them in a fixed order.
+// True, with the total, in one thread of the grid; the counter is back at zero
+// afterwards.  (A second kernel for the partials cost 4 us a call.)
+__device__ __forceinline__ bool grid_sum(double acc, double* partial, unsigned* counter, double* total) {
+  __shared__ double red[32];
+  __shared__ unsigned last;
+  const int nw = int(blockDim.x + 31) / 32, lane = int(threadIdx.x) & 31;
+  const unsigned blocks = gridDim.x * gridDim.y, self = blockIdx.y * gridDim.x + blockIdx.x;
+  auto block_sum = [&]() {  // in thread 0
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
     double s = 0.0;
-    for (int w = 0; w < kThreads / 32; ++w) s += red[w];
-    partial[blockIdx.x] = s;
+    if (threadIdx.x == 0)
+      for (int w = 0; w < nw; ++w) s += red[w];
+    return s;
+  };
+  const double s = block_sum();
+  if (threadIdx.x == 0) {
+    __stcg(partial + self, s);
+    unsigned arrived;  // releases the partial, and acquires the others' for the last one
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(counter) : "memory");
+    last = arrived == blocks - 1 ? 1u : 0u;
   }
+  __syncthreads();
+  if (!last) return false;
+  acc = 0.0;
+  for (unsigned q = threadIdx.x; q < blocks; q += 8 * blockDim.x) {  // eight loads in flight
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = q + k * blockDim.x < blocks ? __ldcg(partial + q + k * blockDim.x) : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) acc += v[k] + v[k + 1];
+  }
+  const double sum = block_sum();
+  if (threadIdx.x != 0) return false;
+  *counter = 0u;
+  *total = sum;
+  return true;
 }
 
-__global__ void dot_final_kernel(const double* partial, int np, double* out, int beta) {
-  // fixed-order sum of the partials: deterministic for a fixed grid size
-  __shared__ double red[kThreads];
+// ---------------------------------------------------------------- dot / norm
+// *out (=|+=) sum_i a[offA[i]] b[offB[i]] (full contraction).
+__global__ void __launch_bounds__(kThreads) dot_kernel(const double* __restrict__ a, const double* __restrict__ b,
+                                                       const int64_t* __restrict__ offA,
+                                                       const int64_t* __restrict__ offB, int64_t n, double* out,
+                                                       int beta, double* partial, unsigned* counter) {
   double acc = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) acc += partial[i];
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+    acc = fma(a[offA[i]], b[offB[i]], acc);
+  double total;
+  if (grid_sum(acc, partial, counter, &total)) *out = beta ? *out + total : total;
+}
+
+// *out = sum_i a[i]^2: eight 16-byte loads in flight per thread (one 8-byte
+// load at a time ran at 61 % of the copy bandwidth), four running sums.
+__global__ void __launch_bounds__(kThreads) norm2_kernel(const double* __restrict__ a, int64_t n, int vec, double* out,
+                                                         double* partial, unsigned* counter) {
+  constexpr int kLoads = 8;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x, first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  int64_t done = 0;  // elements taken as pairs
+  if (vec) {
+    const double2* a2 = reinterpret_cast<const double2*>(a);
+    const int64_t n2 = n / 2;
+    done = 2 * n2;
+    int64_t i = first;
+    for (; i + (kLoads - 1) * stride < n2; i += kLoads * stride) {
+      double2 v[kLoads];
+#pragma unroll
+      for (int k = 0; k < kLoads; ++k) v[k] = __ldg(a2 + i + k * stride);
+#pragma unroll
+      for (int k = 0; k < kLoads; ++k) {
+        acc[2 * (k & 1)] = fma(v[k].x, v[k].x, acc[2 * (k & 1)]);
+        acc[2 * (k & 1) + 1] = fma(v[k].y, v[k].y, acc[2 * (k & 1) + 1]);
+      }
+    }
+    for (; i < n2; i += stride) {
+      const double2 v = __ldg(a2 + i);
+      acc[0] = fma(v.x, v.x, acc[0]);
+      acc[1] = fma(v.y, v.y, acc[1]);
+    }
   }
-  if (threadIdx.x == 0) *out = beta ? *out + red[0] : red[0];
+  for (int64_t i = done + first; i < n; i += stride) acc[0] = fma(a[i], a[i], acc[0]);
+  double total;
+  if (grid_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), partial, counter, &total)) *out = total;
 }
 
 // ---------------------------------------------------------------- slice/insert
@@ -434,19 +488,6 @@ __global__ void __launch_bounds__(kThreads) denominator_kernel(DenParams p, doub
 // (one fused multiply-add per element).  Each CTA writes one partial sum; the
 // partials are added in a fixed order, so a GPU gives the same bits every run.
 
-// Deterministic CTA sum of acc into partial[slot].
-__device__ __forceinline__ void block_sum_to(double acc, double* partial, int64_t slot) {
-  __shared__ double red[32];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double sum = 0.0;
-    for (int q = 0; q < int(blockDim.x + 31) / 32; ++q) sum += red[q];
-    partial[slot] = sum;
-  }
-}
-
 // Storage in the denominator's order (position q = storage dimension q), rank
 // 4 or 6: eps = ((((e1 + e3) + e5) - e0) - e2) - e4, or ((e1 + e3) - e0) - e2.
 // The chain's prefix is formed where its terms are fixed: a thread owns one
@@ -458,15 +499,16 @@ __device__ __forceinline__ void block_sum_to(double acc, double* partial, int64_
 // divide).  (An integer form of the subtraction, exact as well, ran slower
 // than the FP64 one.)  Units (x3 [x5], a range of x2) are spread over
 // gridDim.y CTAs in a fixed order.
-constexpr int kEnLoads = 4;  // loads in flight per thread
-constexpr int kEnThreads = 512;
+constexpr int kEnLoads = 4;  // loads in flight per thread, and divisions interleaved
+constexpr int kEnThreads = 384;  // two CTAs per SM at 80 registers: four divisions in flight per thread
 // DIVIDE: the denominator drop-in on the same walk, in place: each element
 // becomes fl(w / eps) (zeros included: 0 / eps keeps the IEEE sign), nothing
 // is summed.
 template <bool DIVIDE>
 __global__ void __launch_bounds__(kEnThreads, 2) energy_chain_kernel(DenParams p, double* w,
                                                             const double* __restrict__ e, int x2_per_unit,
-                                                            int64_t nunits, double* partial) {
+                                                            int64_t nunits, double efact, double* esum,
+                                                            double* partial, unsigned* counter) {
   extern __shared__ double en[];  // e2 energies [ext2], then e4 energies [ext4]
   const int n0 = p.ext[0], n1 = p.ext[1], n2 = p.ext[2], n3 = p.ext[3];
   const bool r6 = p.rank0 == 6;
@@ -495,44 +537,48 @@ __global__ void __launch_bounds__(kEnThreads, 2) energy_chain_kernel(DenParams p
       if (r6) t = __dadd_rn(t, eps_at(p, e, x5 + p.off[5]));
       t = __dsub_rn(t, e0v);
       const int x2b = chunk * x2_per_unit, x2e = min(n2, x2b + x2_per_unit);
-      if (!r6) {
-        double* base = w + pp + n01 * (int64_t(n2) * x3);
-        for (int x2 = x2b; x2 < x2e; x2 += kEnLoads) {
-          double v[kEnLoads];
+      // one run of elements at stride st whose denominators are tt - es[k]
+      auto run = [&](double* base, int64_t st, double tt, const double* es, int n) {
+        int k0 = 0;
+        for (; k0 + kEnLoads <= n; k0 += kEnLoads) {
+          double v[kEnLoads], d[kEnLoads], q[kEnLoads];
 #pragma unroll
-          for (int k = 0; k < kEnLoads; ++k) v[k] = x2 + k < x2e ? load(base + n01 * (x2 + k)) : 0.0;
+          for (int k = 0; k < kEnLoads; ++k) v[k] = load(base + st * (k0 + k));
 #pragma unroll
-          for (int k = 0; k < kEnLoads; ++k) {
-            if constexpr (DIVIDE) {
-              if (x2 + k < x2e) base[n01 * (x2 + k)] = div_rn(v[k], __dsub_rn(t, en[x2 + k]));
-            } else if (nonzero(v[k])) {
-              acc = fma(v[k], div_rn(v[k], __dsub_rn(t, en[x2 + k])), acc);
-            }
+          for (int k = 0; k < kEnLoads; ++k) d[k] = __dsub_rn(tt, es[k0 + k]);
+          if constexpr (DIVIDE) {
+            div_rn_n<kEnLoads>(v, d, q);
+#pragma unroll
+            for (int k = 0; k < kEnLoads; ++k) base[st * (k0 + k)] = q[k];
+          } else {
+            bool ok[kEnLoads];
+#pragma unroll
+            for (int k = 0; k < kEnLoads; ++k) ok[k] = div_rn_int(v[k], d[k], &q[k]);
+#pragma unroll
+            for (int k = 0; k < kEnLoads; ++k)
+              if (ok[k]) acc = fma(v[k], q[k], acc);
+              else if (nonzero(v[k])) acc = fma(v[k], div_rn_slow(v[k], d[k]), acc);
           }
         }
+        for (; k0 < n; ++k0) {
+          const double v = load(base + st * k0);
+          if constexpr (DIVIDE) base[st * k0] = div_rn(v, __dsub_rn(tt, es[k0]));
+          else if (nonzero(v)) acc = fma(v, div_rn(v, __dsub_rn(tt, es[k0])), acc);
+        }
+      };
+      if (!r6) {
+        run(w + pp + n01 * (x2b + int64_t(n2) * x3), n01, t, en + x2b, x2e - x2b);
       } else {
         const int64_t s4 = n01 * int64_t(n2) * n3;  // stride of x4
-        for (int x2 = x2b; x2 < x2e; ++x2) {
-          const double t2 = __dsub_rn(t, en[x2]);
-          double* base = w + pp + n01 * (x2 + int64_t(n2) * x3) + s4 * int64_t(n4) * x5;
-          for (int x4 = 0; x4 < n4; x4 += kEnLoads) {
-            double v[kEnLoads];
-#pragma unroll
-            for (int k = 0; k < kEnLoads; ++k) v[k] = x4 + k < n4 ? load(base + s4 * (x4 + k)) : 0.0;
-#pragma unroll
-            for (int k = 0; k < kEnLoads; ++k) {
-              if constexpr (DIVIDE) {
-                if (x4 + k < n4) base[s4 * (x4 + k)] = div_rn(v[k], __dsub_rn(t2, en[n2 + x4 + k]));
-              } else if (nonzero(v[k])) {
-                acc = fma(v[k], div_rn(v[k], __dsub_rn(t2, en[n2 + x4 + k])), acc);
-              }
-            }
-          }
-        }
+        for (int x2 = x2b; x2 < x2e; ++x2)
+          run(w + pp + n01 * (x2 + int64_t(n2) * x3) + s4 * int64_t(n4) * x5, s4, __dsub_rn(t, en[x2]), en + n2, n4);
       }
     }
   }
-  if constexpr (!DIVIDE) block_sum_to(acc, partial, int64_t(blockIdx.y) * gridDim.x + blockIdx.x);
+  if constexpr (!DIVIDE) {
+    double total;
+    if (grid_sum(acc, partial, counter, &total)) *esum = __dadd_rn(*esum, __dmul_rn(total, efact));
+  }
 }
 
 // Any other storage order or rank: the whole chain per element (den_eps, the
@@ -540,7 +586,8 @@ __global__ void __launch_bounds__(kEnThreads, 2) energy_chain_kernel(DenParams p
 // denominator kernel; a fixed grid, one partial per CTA.
 __global__ void __launch_bounds__(kThreads) energy_generic_kernel(DenParams p, const double* __restrict__ w,
                                                                   const double* __restrict__ e, int64_t n,
-                                                                  double* partial) {
+                                                                  double efact, double* esum, double* partial,
+                                                                  unsigned* counter) {
   const int64_t stride = int64_t(gridDim.x) * blockDim.x * kDenRun;
   double acc = 0.0;
   for (int64_t i0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * kDenRun; i0 < n; i0 += stride) {
@@ -561,7 +608,8 @@ __global__ void __launch_bounds__(kThreads) energy_generic_kernel(DenParams p, c
       }
     }
   }
-  block_sum_to(acc, partial, blockIdx.x);
+  double total;
+  if (grid_sum(acc, partial, counter, &total)) *esum = __dadd_rn(*esum, __dmul_rn(total, efact));
 }
 
 // ---------------------------------------------------------------- amplitude update
@@ -573,15 +621,30 @@ __global__ void __launch_bounds__(kThreads) energy_generic_kernel(DenParams p, c
 //   T2old'(a,i,b,j) = (0.5 * t) / eps            (next amplitudes, a separate buffer:
 //                                                 the partner block still reads T2old)
 //   partial[block] = sum of E^2                  (its residual norm, deterministic)
-// eps = ((e_i + e_j) - e_a) - e_b, energy_denominator_rhf's rank-4 order.  Each
-// CTA handles a 32x32 (a,b) tile at fixed (i,j); the partner tiles are read
-// along b and transposed through shared memory so all loads coalesce.
+// eps = ((e_i + e_j) - e_a) - e_b, energy_denominator_rhf's rank-4 order.
 // (0.5 t)/eps is formed as 0.5 (t/eps): both are t/(2 eps) correctly rounded
 // while the quotient is a normal number; below that the division is redone.
+//
+// A work unit is one (a,b) tile at fixed (i,j).  The plane is cut evenly into
+// tiles of at most 48 x 24 (a 33 x 37 plane is two of 33 x 19, 96 x 96 eight of
+// 48 x 24): threads walk the tile's own elements, so the lanes are as full as
+// the plane allows (32 x 32 tiles left 73 % of the lanes of a 33 x 33 plane
+// idle).  The partner tiles are read along b and transposed through shared
+// memory so that all loads coalesce.  Four elements per thread at a time, their
+// loads (the first own ones before the partner's) and divisions in flight
+// together.  One resident wave of CTAs, each over several units;
+// the last one to finish adds the partial norms in a fixed order.
+// o=40/v=300 (400 blocks of about 33 x 20 x 33 x 20, 48 B an element):
+// 20 us a block before.
+constexpr int kUpdA = 48, kUpdB = 24, kUpdGroup = 4, kUpdThreads = 128;
 struct UpdParams {
   int ea, ei, eb, ej;   // extents
   int oa, oi, ob, oj;   // first orbitals
   int rank1, ld1;
+  int ta, tb;           // tile extents
+  int tiles_a, tiles_b;
+  int64_t units;
+  uint32_t mul_a, mul_b;  // ceil(2^20 / ta), ceil(2^20 / tb): e / t = (e mul) >> 20 for e < 48 * 24 + 512
 };
 
 __device__ __forceinline__ double eps_at_upd(const UpdParams& p, const double* e, int orb) {
@@ -596,87 +659,124 @@ __device__ __forceinline__ double half_of(double x) {
   return f >= 2u && f != 0x7FFu ? double_of(b - (1ull << 52)) : __dmul_rn(x, 0.5);
 }
 
-__global__ void __launch_bounds__(256) update_t2_kernel(UpdParams p, const double* __restrict__ xn,
-                                                        const double* __restrict__ xnp,
-                                                        const double* __restrict__ xo,
-                                                        const double* __restrict__ xop, double* __restrict__ err,
-                                                        double* __restrict__ next, const double* __restrict__ e,
-                                                        double* partial) {
-  __shared__ double pn[32][33], po[32][33];  // [a][b] of the partner tiles
-  const int tiles_a = (p.ea + 31) / 32;
-  const int ta = blockIdx.x % tiles_a, tb = blockIdx.x / tiles_a;
-  const int i = blockIdx.y % p.ei, j = blockIdx.y / p.ei;
-  const int a0 = ta * 32, b0 = tb * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  // partner block (b,j,a,i): element (b, j, a, i) at b + eb*(j + ej*(a + ea*i))
-  for (int k = ty; k < 32; k += 8) {
-    const int b = b0 + tx, a = a0 + k;
-    double vn = 0.0, vo = 0.0;
-    if (a < p.ea && b < p.eb) {
-      const int64_t q = b + int64_t(p.eb) * (j + int64_t(p.ej) * (a + int64_t(p.ea) * i));
-      vn = __ldg(xnp + q);
-      vo = __ldg(xop + q);
+__global__ void __launch_bounds__(kUpdThreads, 6) update_t2_kernel(UpdParams p, const double* __restrict__ xn,
+                                                           const double* __restrict__ xnp,
+                                                           const double* __restrict__ xo,
+                                                           const double* __restrict__ xop, double* __restrict__ err,
+                                                           double* __restrict__ next, const double* __restrict__ e,
+                                                           double* norm2, double* partial, unsigned* counter) {
+  __shared__ double pn[kUpdA][kUpdB + 1], po[kUpdA][kUpdB + 1];  // [a][b] of the partner tiles
+  __shared__ double sa[kUpdA], sb[kUpdB];  // (e_i + e_j) - e_a of the tile's a, e_b of its b
+  double acc = 0.0;
+  for (int64_t u = blockIdx.x; u < p.units; u += gridDim.x) {
+    int64_t r = u;
+    const int at = int(r % p.tiles_a);
+    r /= p.tiles_a;
+    const int bt = int(r % p.tiles_b);
+    r /= p.tiles_b;
+    const int i = int(r % p.ei), j = int(r / p.ei);
+    const int a0 = at * p.ta, b0 = bt * p.tb;
+    const int na = min(p.ta, p.ea - a0), nb = min(p.tb, p.eb - b0), n = p.ta * p.tb;
+    __syncthreads();  // the previous unit's tiles are read
+    if (threadIdx.x < kUpdA) {
+      const int k = threadIdx.x;
+      if (k < na)
+        sa[k] = __dsub_rn(__dadd_rn(eps_at_upd(p, e, p.oi + i), eps_at_upd(p, e, p.oj + j)),
+                          eps_at_upd(p, e, p.oa + a0 + k));
+      if (k < nb) sb[k] = eps_at_upd(p, e, p.ob + b0 + k);
     }
-    pn[k][tx] = vn;
-    po[k][tx] = vo;
-  }
-  __syncthreads();
-  // (e_i + e_j) - e_a once per thread (a is fixed per thread), - e_b per element
-  const int a = a0 + tx;
-  const double eija = a < p.ea ? __dsub_rn(__dadd_rn(eps_at_upd(p, e, p.oi + i), eps_at_upd(p, e, p.oj + j)),
-                                           eps_at_upd(p, e, p.oa + a))
-                               : 0.0;
-  double acc = 0.0;
-  for (int k = ty; k < 32; k += 8) {
-    const int b = b0 + k;
-    if (a >= p.ea || b >= p.eb) continue;
-    const int64_t q = a + int64_t(p.ea) * (i + int64_t(p.ei) * (b + int64_t(p.eb) * j));
-    const double t = __dadd_rn(pn[tx][k], __ldg(xn + q));
-    const double t1 = __dadd_rn(po[tx][k], __ldg(xo + q));
-    const double eps = __dsub_rn(eija, eps_at_upd(p, e, p.ob + b));
-    const double td = div_rn(t, eps);
-    const double ev = double_of(bits_of(half_of(__dsub_rn(t1, td))) ^ (1ull << 63));  // -0.5 (t1 - td)
-    if (err) err[q] = ev;
-    next[q] = fabs(td) >= 0x1p-1021 ? half_of(td) : __ddiv_rn(__dmul_rn(t, 0.5), eps);
-    acc = fma(ev, ev, acc);
-  }
-  __shared__ double red[8];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double sum = 0.0;
-    for (int q = 0; q < 8; ++q) sum += red[q];
-    partial[int64_t(blockIdx.y) * gridDim.x + blockIdx.x] = sum;
-  }
-}
-
-// *out += fixed-order sum of the partials (out may be null: nothing)
-__global__ void sum_partials_kernel(const double* partial, int64_t np, double* out) {
-  __shared__ double red[kThreads];
-  double acc = 0.0;
-  for (int64_t q = threadIdx.x; q < np; q += blockDim.x) acc += partial[q];
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+    const int64_t qb = a0 + int64_t(p.ea) * (i + int64_t(p.ei) * (b0 + int64_t(p.eb) * j));
+    const int64_t qsb = int64_t(p.ea) * p.ei;
+    double t[kUpdGroup], t1[kUpdGroup];
+    auto load_own = [&](int e0) {
+#pragma unroll
+      for (int g = 0; g < kUpdGroup; ++g) {
+        const int el = e0 + kUpdThreads * g, b = int((uint32_t(el) * p.mul_a) >> 20), a = el - b * p.ta;
+        const bool live = el < n && a < na && b < nb;
+        t[g] = live ? __ldg(xn + qb + a + qsb * b) : 1.0;
+        t1[g] = live ? __ldg(xo + qb + a + qsb * b) : 0.0;
+      }
+    };
+    load_own(threadIdx.x);
+    // partner block (b,j,a,i): element (b, j, a, i) at b + eb*(j + ej*(a + ea*i))
+    const int64_t pb = b0 + int64_t(p.eb) * (j + int64_t(p.ej) * (a0 + int64_t(p.ea) * i));
+    const int64_t psa = int64_t(p.eb) * p.ej;
+#pragma unroll 1
+    for (int e0 = threadIdx.x; e0 < n; e0 += kUpdThreads * kUpdGroup) {
+      double vn[kUpdGroup], vo[kUpdGroup];
+#pragma unroll
+      for (int g = 0; g < kUpdGroup; ++g) {
+        const int el = e0 + kUpdThreads * g, a = int((uint32_t(el) * p.mul_b) >> 20), b = el - a * p.tb;
+        const bool live = el < n && a < na && b < nb;
+        vn[g] = live ? __ldg(xnp + pb + b + psa * a) : 0.0;
+        vo[g] = live ? __ldg(xop + pb + b + psa * a) : 0.0;
+      }
+#pragma unroll
+      for (int g = 0; g < kUpdGroup; ++g) {
+        const int el = e0 + kUpdThreads * g, a = int((uint32_t(el) * p.mul_b) >> 20), b = el - a * p.tb;
+        if (el < n) pn[a][b] = vn[g], po[a][b] = vo[g];
+      }
+    }
     __syncthreads();
+#pragma unroll 1
+    for (int e0 = threadIdx.x; e0 < n; e0 += kUpdThreads * kUpdGroup) {
+      if (e0 != int(threadIdx.x)) load_own(e0);
+      int64_t q[kUpdGroup];
+      double eps[kUpdGroup], td[kUpdGroup];
+      bool live[kUpdGroup];
+#pragma unroll
+      for (int g = 0; g < kUpdGroup; ++g) {
+        const int el = e0 + kUpdThreads * g, b = int((uint32_t(el) * p.mul_a) >> 20), a = el - b * p.ta;
+        live[g] = el < n && a < na && b < nb;
+        q[g] = qb + a + qsb * b;
+        eps[g] = 1.0;  // outside the tile: 1 / 1, dropped
+        if (live[g]) {
+          t[g] = __dadd_rn(pn[a][b], t[g]);
+          t1[g] = __dadd_rn(po[a][b], t1[g]);
+          eps[g] = __dsub_rn(sa[a], sb[b]);
+        }
+      }
+      div_rn_n<kUpdGroup>(t, eps, td);
+      // -0.5 (t1 - td) and 0.5 td by their exponent fields where both halves
+      // are normal numbers (a multiplication or a comparison would take the
+      // FP64 pipe, 16 clocks a warp)
+      double ev[kUpdGroup], nx[kUpdGroup];
+      bool all = true;
+#pragma unroll
+      for (int g = 0; g < kUpdGroup; ++g) {
+        const unsigned long long x = bits_of(__dsub_rn(t1[g], td[g])), y = bits_of(td[g]);
+        ev[g] = double_of((x - (1ull << 52)) ^ (1ull << 63));
+        nx[g] = double_of(y - (1ull << 52));
+        t1[g] = double_of(x);
+        all = all && (uint32_t(x >> 52) & 0x7FFu) - 2u < 2045u && (uint32_t(y >> 52) & 0x7FFu) - 2u < 2045u;
+      }
+      if (!all) {
+#pragma unroll 1
+        for (int g = 0; g < kUpdGroup; ++g) {
+          double x = 0.0, y = 0.0, tg = 0.0, eg = 0.0;
+#pragma unroll
+          for (int k = 0; k < kUpdGroup; ++k)
+            if (k == g) x = t1[k], y = td[k], tg = t[k], eg = eps[k];
+          const unsigned f = uint32_t(bits_of(y) >> 52) & 0x7FFu;
+          x = double_of(bits_of(half_of(x)) ^ (1ull << 63));
+          y = f >= 2u ? half_of(y) : __ddiv_rn(__dmul_rn(tg, 0.5), eg);
+#pragma unroll
+          for (int k = 0; k < kUpdGroup; ++k)
+            if (k == g) ev[k] = x, nx[k] = y;
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < kUpdGroup; ++g) {
+        if (!live[g]) continue;
+        if (err) err[q[g]] = ev[g];
+        next[q[g]] = nx[g];
+        if (norm2) acc = fma(ev[g], ev[g], acc);
+      }
+    }
   }
-  if (threadIdx.x == 0 && out) *out = __dadd_rn(*out, red[0]);
-}
-
-// *esum += efact * (fixed-order sum of the partials)
-__global__ void energy_final_kernel(const double* partial, int np, double efact, double* esum) {
-  __shared__ double red[kThreads];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) acc += partial[i];
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *esum = __dadd_rn(*esum, __dmul_rn(red[0], efact));
+  if (!norm2) return;
+  double total;
+  if (grid_sum(acc, partial, counter, &total)) *norm2 = __dadd_rn(*norm2, total);
 }
 
 // ---------------------------------------------------------------- scalar cases
@@ -783,20 +883,19 @@ int launch_add_sub_permuted(int subtract, int rank, const int* r_ext, const int*
   return subtract ? launch_perm_op<2>(p, r, d, l, total, s) : launch_perm_op<1>(p, r, d, l, total, s);
 }
 
-int dot_scratch_len() { return kDotBlocks; }
-
-int launch_dot(const double* a, const double* b, const int64_t* offA, const int64_t* offB,
-               int64_t n, double* d_out, double* d_scratch, int64_t scratch_len, cudaStream_t s) {
-  return launch_dot_beta(a, b, offA, offB, n, d_out, d_scratch, scratch_len, 0, s);
+int launch_dot(const double* a, const double* b, const int64_t* offA, const int64_t* offB, int64_t n, double* d_out,
+               const ReductionSlot& slot, int beta, cudaStream_t s) {
+  const int g = std::min<int>(kDotBlocks, grid_for(n, 8));
+  dot_kernel<<<g, kThreads, 0, s>>>(a, b, offA, offB, n, d_out, beta, slot.partial, slot.counter);
+  A4G_CUDA(cudaGetLastError());
+  return A4G_OK;
 }
 
-int launch_dot_beta(const double* a, const double* b, const int64_t* offA, const int64_t* offB,
-                    int64_t n, double* d_out, double* d_scratch, int64_t scratch_len, int beta,
-                    cudaStream_t s) {
-  if (scratch_len < kDotBlocks) return fail(A4G_ERR_ARG, "dot scratch too small");
-  const int g = std::min<int>(kDotBlocks, grid_for(n, 8));
-  dot_partial_kernel<<<g, kThreads, 0, s>>>(a, b, offA, offB, n, d_scratch);
-  dot_final_kernel<<<1, kThreads, 0, s>>>(d_scratch, g, d_out, beta);
+int launch_norm2(const double* a, int64_t n, double* d_out, const ReductionSlot& slot, cudaStream_t s) {
+  // 6 CTAs per SM: one resident wave
+  const int sms = ctx()->num_sms > 0 ? ctx()->num_sms : 152;
+  const int g = std::min<int>({kDotBlocks, 6 * sms, grid_for(n, 8)});
+  norm2_kernel<<<g, kThreads, 0, s>>>(a, n, aligned16(a) ? 1 : 0, d_out, slot.partial, slot.counter);
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
 }
@@ -842,8 +941,12 @@ static DenParams den_params(int rank0, const int* off, const int* ext0, const in
 
 // Grid of the chain walk (rank 4 or 6 in the denominator's order): a thread
 // per (x0, x1) position (the positions split evenly over gx CTAs of at most
-// 512 threads); units (x3 [x5], an x2 range) spread over enough CTAs to fill
-// the GPU a few times, at most max_ctas in all.
+// kEnThreads threads); units (x3 [x5], an x2 range) spread over one resident
+// wave of CTAs (2 per SM), at most max_ctas in all.  The x2 ranges are cut so
+// that a CTA gets 16 units or more where the block has them (the last round is
+// then nearly full), at rank 4 in multiples of the elements a thread divides
+// together (a 48 x 42 x 53 x 42 block in ranges of 6 left 2 of 6 elements to
+// the one-by-one tail).
 struct ChainGrid {
   int64_t gx = 0, gy = 0, nunits = 0;
   int threads = 0, per = 0;
@@ -856,11 +959,12 @@ ChainGrid chain_grid(int rank0, const int* ext0, int64_t max_ctas) {
   g.gx = (n01 + kEnThreads - 1) / kEnThreads;
   g.threads = int(((n01 + g.gx - 1) / g.gx + 31) / 32 * 32);
   const int64_t nocc = rank0 == 6 ? int64_t(ext0[3]) * ext0[5] : ext0[3];
-  const int64_t want = 16LL * sms;  // CTAs
-  const int chunks = int(std::max<int64_t>(1, std::min<int64_t>(ext0[2], (want / g.gx + nocc - 1) / nocc)));
-  g.per = (ext0[2] + chunks - 1) / chunks;
+  const int64_t wave = std::max<int64_t>(1, std::min<int64_t>(2LL * sms / g.gx, max_ctas / g.gx));
+  const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(ext0[2], (16 * wave + nocc - 1) / nocc));
+  g.per = int((ext0[2] + chunks - 1) / chunks);
+  if (rank0 == 4) g.per = (g.per + kEnLoads - 1) / kEnLoads * kEnLoads;
   g.nunits = nocc * ((ext0[2] + g.per - 1) / g.per);
-  g.gy = std::max<int64_t>(1, std::min<int64_t>({g.nunits, std::max<int64_t>(1, want / g.gx), max_ctas / g.gx}));
+  g.gy = std::min(g.nunits, wave);
   g.smem = size_t(ext0[2] + (rank0 == 6 ? ext0[4] : 0)) * sizeof(double);
   return g;
 }
@@ -875,7 +979,7 @@ int launch_denominator(int rank0, const int* off, const int* ext0, double* data,
     const ChainGrid g = chain_grid(rank0, ext0, 0x7fffffffLL);
     if (g.smem <= 48 * 1024 && g.gx <= 0x7fffffffLL && g.gy <= 65535) {
       energy_chain_kernel<true><<<dim3(unsigned(g.gx), unsigned(g.gy)), g.threads, g.smem, s>>>(
-          p, data, e_or_fock, g.per, g.nunits, nullptr);
+          p, data, e_or_fock, g.per, g.nunits, 0.0, nullptr, nullptr, nullptr);
       A4G_CUDA(cudaGetLastError());
       return A4G_OK;
     }
@@ -887,32 +991,28 @@ int launch_denominator(int rank0, const int* off, const int* ext0, double* data,
 
 int launch_update_t2(const int* off, const int* ext, const double* t2new, const double* t2new_pair,
                      const double* t2old, const double* t2old_pair, double* err, double* next, int rank1, int ld1,
-                     const double* e_or_fock, double* norm2, double* d_scratch, int64_t scratch_len,
-                     cudaStream_t s) {
+                     const double* e_or_fock, double* norm2, const ReductionSlot& slot, cudaStream_t s) {
   UpdParams p{};
   p.ea = ext[0], p.ei = ext[1], p.eb = ext[2], p.ej = ext[3];
   p.oa = off[0], p.oi = off[1], p.ob = off[2], p.oj = off[3];
   p.rank1 = rank1, p.ld1 = ld1;
-  const int64_t gx = int64_t((p.ea + 31) / 32) * ((p.eb + 31) / 32), gy = int64_t(p.ei) * p.ej;
-  if (gx * gy == 0) return A4G_OK;
-  if (gx > 0x7fffffffLL || gy > 65535) return fail(A4G_ERR_RANGE, "amplitude update: block too large");
-  double* partial = d_scratch;
-  bool own = false;
-  if (gx * gy > scratch_len) {  // more CTAs than the reduction scratch holds
-    if (const int rc_ = async_alloc(reinterpret_cast<void**>(&partial), size_t(gx * gy) * sizeof(double), s)) return rc_;
-    own = true;
-  }
-  update_t2_kernel<<<dim3(unsigned(gx), unsigned(gy)), 256, 0, s>>>(p, t2new, t2new_pair, t2old, t2old_pair, err,
-                                                                     next, e_or_fock, partial);
-  sum_partials_kernel<<<1, kThreads, 0, s>>>(partial, gx * gy, norm2);
-  if (own) A4G_CUDA(cudaFreeAsync(partial, s));
+  p.tiles_a = (p.ea + kUpdA - 1) / kUpdA, p.tiles_b = (p.eb + kUpdB - 1) / kUpdB;
+  p.ta = (p.ea + p.tiles_a - 1) / p.tiles_a, p.tb = (p.eb + p.tiles_b - 1) / p.tiles_b;
+  p.mul_a = ((1u << 20) + p.ta - 1) / p.ta, p.mul_b = ((1u << 20) + p.tb - 1) / p.tb;
+  p.units = int64_t(p.tiles_a) * p.tiles_b * p.ei * p.ej;
+  if (p.units == 0) return A4G_OK;
+  // one resident wave (6 CTAs of 128 threads per SM): its CTAs share the units evenly
+  const int sms = ctx()->num_sms > 0 ? ctx()->num_sms : 152;
+  const int64_t wave = std::min<int64_t>(kDotBlocks, 6 * int64_t(sms));
+  update_t2_kernel<<<unsigned(std::min(p.units, wave)), kUpdThreads, 0, s>>>(
+      p, t2new, t2new_pair, t2old, t2old_pair, err, next, e_or_fock, norm2, slot.partial, slot.counter);
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
 }
 
 int launch_energy_contract(int rank0, const int* off, const int* ext0, const int* pos, const double* w,
                            int rank1, int ld1, const double* e_or_fock, double efact, double* esum,
-                           double* d_scratch, int scratch_len, cudaStream_t s) {
+                           const ReductionSlot& slot, cudaStream_t s) {
   int64_t n = 0;
   const DenParams p = den_params(rank0, off, ext0, pos, rank1, ld1, &n);
   if (n == 0) return A4G_OK;
@@ -920,29 +1020,27 @@ int launch_energy_contract(int rank0, const int* off, const int* ext0, const int
   for (int q = 0; q < rank0; ++q) identity &= p.pos[q] == q;
   const int sms = ctx()->num_sms > 0 ? ctx()->num_sms : 152;
   const int64_t n01 = rank0 >= 2 ? int64_t(ext0[0]) * ext0[1] : n;
-  if (identity && (rank0 == 4 || rank0 == 6) && n01 <= kEnThreads * int64_t(scratch_len)) {
-    // at most scratch_len partials (one per CTA)
-    const ChainGrid g = chain_grid(rank0, ext0, scratch_len);
+  if (identity && (rank0 == 4 || rank0 == 6) && n01 <= kEnThreads * int64_t(kDotBlocks)) {
+    // at most kDotBlocks partials (one per CTA)
+    const ChainGrid g = chain_grid(rank0, ext0, kDotBlocks);
     if (g.smem > 48 * 1024) return fail(A4G_ERR_RANGE, "energy contraction: segments too large");
     energy_chain_kernel<false><<<dim3(unsigned(g.gx), unsigned(g.gy)), g.threads, g.smem, s>>>(
-        p, const_cast<double*>(w), e_or_fock, g.per, g.nunits, d_scratch);
-    energy_final_kernel<<<1, kThreads, 0, s>>>(d_scratch, int(g.gx * g.gy), efact, esum);
+        p, const_cast<double*>(w), e_or_fock, g.per, g.nunits, efact, esum, slot.partial, slot.counter);
   } else {
-    const int g = int(std::min<int64_t>({int64_t(scratch_len), 8LL * sms,
+    const int g = int(std::min<int64_t>({int64_t(kDotBlocks), 8LL * sms,
                                          std::max<int64_t>(1, (n + kThreads * kDenRun - 1) / (kThreads * kDenRun))}));
-    energy_generic_kernel<<<g, kThreads, 0, s>>>(p, w, e_or_fock, n, d_scratch);
-    energy_final_kernel<<<1, kThreads, 0, s>>>(d_scratch, g, efact, esum);
+    energy_generic_kernel<<<g, kThreads, 0, s>>>(p, w, e_or_fock, n, efact, esum, slot.partial, slot.counter);
   }
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
 }
 
 int launch_scalar_cases(const DevPlan* p, const double* L, const double* R, double* D, int beta,
-                        double* d_scratch, cudaStream_t s) {
+                        const ReductionSlot& slot, cudaStream_t s) {
   const GemmPlan& h = p->host;
   switch (h.kind) {
     case ContractKind::kFull:
-      return launch_dot_beta(L, R, p->offLk, p->offRk, h.K, D, d_scratch, kDotBlocks, beta, s);
+      return launch_dot(L, R, p->offLk, p->offRk, h.K, D, slot, beta, s);
     case ContractKind::kRightScalar:
       scalar_case_kernel<<<grid_for(h.M), kThreads, 0, s>>>(L, R, p->offLm, p->offDm, D, h.M, beta);
       break;

@@ -635,16 +635,32 @@ __device__ __forceinline__ void energy_direct(const OzGemmArgs& a, const DirectT
     tc_ld8_nowait(w0addr + (kTmemW1 - kTmemW0) + 8 * p, w1);
     tc_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const EnergyCol ec = t.ecols[8 * p + j];
-      if (!t.mlive || ec.ck < 0) continue;
-      const int F = t.cols[8 * p + j].F;
-      const long long v = (long long)(((unsigned long long)w1[j] << 32) | w0[j]);
-      double x = i64_scaled_to_double(v, t.ebase + F, false);
-      if (t.nonfinite || F == kNonFiniteExp) x = __longlong_as_double(0x7FF8000000000000ll);
-      if (!nonzero(x)) continue;
-      const double eps = __dsub_rn(t.prow[ec.ck], t.last_row ? t.er : ec.ec);
-      acc = fma(x, div_rn(x, eps), acc);
+    for (int j0 = 0; j0 < 8; j0 += 2) {  // two elements at a time without a branch between them
+      double x[2], qv[2];
+      bool ok[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int j = j0 + i, F = t.cols[8 * p + j].F;
+        const EnergyCol ec = t.ecols[8 * p + j];
+        const long long v = (long long)(((unsigned long long)w1[j] << 32) | w0[j]);
+        ok[i] = i64_scaled_normal(v, t.ebase + F, &x[i]);
+        const double eps = __dsub_rn(t.prow[max(ec.ck, 0)], t.last_row ? t.er : ec.ec);
+        ok[i] = div_rn_int(x[i], eps, &qv[i]) && ok[i] && t.mlive && ec.ck >= 0 && !t.nonfinite && F != kNonFiniteExp;
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (ok[i]) {
+          acc = fma(x[i], qv[i], acc);
+          continue;
+        }
+        const int j = j0 + i, F = t.cols[8 * p + j].F;
+        const EnergyCol ec = t.ecols[8 * p + j];
+        if (!t.mlive || ec.ck < 0) continue;
+        double y = i64_scaled_to_double((long long)(((unsigned long long)w1[j] << 32) | w0[j]), t.ebase + F, false);
+        if (t.nonfinite || F == kNonFiniteExp) y = __longlong_as_double(0x7FF8000000000000ll);
+        if (!nonzero(y)) continue;
+        acc = fma(y, div_rn(y, __dsub_rn(t.prow[ec.ck], t.last_row ? t.er : ec.ec)), acc);
+      }
     }
   }
 }
@@ -1138,6 +1154,8 @@ struct LvCol {
   int ck;        // energy form: prefix-table column (-1: outside D)
 };
 
+constexpr int kLvGroup = 4;  // elements whose energy work overlaps
+
 // Sixteen warps, four per TMEM lane quadrant; a thread owns one row and 16
 // columns.  Per tile: the row's scale and tables, the 16 columns' table, the
 // wait for the tile's MMAs, the exact sums (two groups of 8 columns, each
@@ -1172,6 +1190,7 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
     if constexpr (ENERGY) {
       eb = a.eblocks[tl.dblock];
       last_row = eb.last_row != 0;
+      prow = eb.ptab;  // rows outside the block read (and drop) the table's first row
     }
     if (mlive) {
       const int e = a.panels_a[tl.panel_a].exps[m];
@@ -1229,15 +1248,40 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
     __syncwarp();
     if (lane == 0) mbar_arrive(&sm.acc_empty);  // the next tile's MMAs may start
     if constexpr (ENERGY) {
+      // groups of kLvGroup elements without a branch between them, so that
+      // their conversions, denominators and divisions overlap; zeros, dead rows
+      // and columns, non-finite rows and results beyond the normal range are
+      // done one by one afterwards
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const LvCol c = tab[j];
-        if (!mlive || c.ck < 0) continue;
-        double x = i64_scaled_to_double(sum[j], ebase + c.F, false);
-        if (nonfinite || c.F == kNonFiniteExp) x = __longlong_as_double(0x7FF8000000000000ll);
-        if (!nonzero(x)) continue;
-        const double eps = __dsub_rn(prow[c.ck], last_row ? er : c.ec);
-        eacc = fma(x, div_rn(x, eps), eacc);
+      for (int j0 = 0; j0 < 16; j0 += kLvGroup) {
+        double x[kLvGroup], qv[kLvGroup];
+        bool ok[kLvGroup], all = mlive && !nonfinite;
+#pragma unroll
+        for (int i = 0; i < kLvGroup; ++i) {
+          const LvCol c = tab[j0 + i];
+          ok[i] = i64_scaled_normal(sum[j0 + i], ebase + c.F, &x[i]);
+          const double eps = __dsub_rn(prow[max(c.ck, 0)], last_row ? er : c.ec);
+          ok[i] = div_rn_int(x[i], eps, &qv[i]) && ok[i] && c.ck >= 0 && c.F != kNonFiniteExp;
+          all = all && ok[i];
+        }
+        if (all) {
+#pragma unroll
+          for (int i = 0; i < kLvGroup; ++i) eacc = fma(x[i], qv[i], eacc);
+        } else if (mlive) {
+#pragma unroll
+          for (int i = 0; i < kLvGroup; ++i) {
+            if (ok[i] && !nonfinite) {
+              eacc = fma(x[i], qv[i], eacc);
+              continue;
+            }
+            const LvCol c = tab[j0 + i];
+            if (c.ck < 0) continue;
+            double y = i64_scaled_to_double(sum[j0 + i], ebase + c.F, false);
+            if (nonfinite || c.F == kNonFiniteExp) y = __longlong_as_double(0x7FF8000000000000ll);
+            if (!nonzero(y)) continue;
+            eacc = fma(y, div_rn(y, __dsub_rn(prow[c.ck], last_row ? er : c.ec)), eacc);
+          }
+        }
       }
     } else {
       const bool acc = a.mode & 1;

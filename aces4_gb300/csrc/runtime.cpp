@@ -1,6 +1,7 @@
 // Runtime support: error reporting, the process context, the contraction
 // pattern planner and the device plan cache.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <unordered_map>
@@ -44,6 +45,11 @@ int ensure_init() {
   A4G_CUDA(cudaStreamCreateWithFlags(&g_ctx.stream, cudaStreamNonBlocking));
   A4G_CUDA(cudaMalloc(&g_ctx.d_error_flag, sizeof(int)));
   A4G_CUDA(cudaMemset(g_ctx.d_error_flag, 0, sizeof(int)));
+  A4G_CUDA(cudaMalloc(&g_ctx.reduce_partials,
+                      sizeof(double) * (Context::kReducePartials + 8) * size_t(Context::kReduceSlots)));
+  A4G_CUDA(cudaMalloc(&g_ctx.reduce_counters, sizeof(unsigned) * Context::kReduceCounters));
+  A4G_CUDA(cudaMemset(g_ctx.reduce_counters, 0, sizeof(unsigned) * Context::kReduceCounters));
+  A4G_CUDA(cudaDeviceSynchronize());
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
@@ -63,6 +69,13 @@ int ensure_init() {
 int async_alloc(void** p, size_t bytes, cudaStream_t s) {
   A4G_CUDA(cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 8), g_ctx.pool, s));
   return A4G_OK;
+}
+
+ReductionSlot reduction_slot() {
+  static std::atomic<unsigned> next{0};
+  const unsigned q = next.fetch_add(1, std::memory_order_relaxed);
+  double* p = g_ctx.reduce_partials + size_t(Context::kReducePartials + 8) * (q % Context::kReduceSlots);
+  return {p, p + Context::kReducePartials, g_ctx.reduce_counters + q % Context::kReduceCounters};
 }
 
 cudaStream_t pick(void* stream) {
