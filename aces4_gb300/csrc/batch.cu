@@ -105,14 +105,14 @@ struct a4g_batch {
   cudaEvent_t stage_ev[kStageRing] = {};
   bool stage_busy[kStageRing] = {};
   // split jobs grouped by operand side (A: left blocks, B: right blocks) and
-  // source layout; each set has its own CTA prefix sums for both passes
+  // source layout; each set has its own list of CTA pieces for both passes
   struct JobSet {
     bool left;
     int layout;
     int group = 0;  // split pipeline group: 0 before the GEMM, g > 0 with GEMM part g-1
     OzSplitJob* d_jobs = nullptr;
-    int64_t* d_prefix_exp = nullptr;
-    int64_t* d_prefix_split = nullptr;
+    OzTileRef* d_refs_exp = nullptr;
+    OzTileRef* d_refs_split = nullptr;
     int njobs = 0;
     int64_t tiles_exp = 0, tiles_split = 0;
     std::vector<OzSplitJob> h_jobs;  // host copy (a rebind rewrites the source pointers)
@@ -450,31 +450,58 @@ int build_f64(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector
 
 // Whether the batch's products run modulo coprime numbers (residue.cu) or as
 // digit levels.  Residues need 5 or more slices (at 4 they take as many
-// products as the digits) and a k range long enough that fewer products pay
-// for the wider panels and the reconstruction: kResidueMinKb 64-wide k blocks
-// in every destination.  A pinned variant names a digit form.
+// products as the digits) and kResidueMinKb 64-wide k blocks in every
+// destination (below, the direct forms' digits need no workspace).  Then the
+// products saved have to pay for the wider panels, L instead of S planes
+// written by every run: both sides at measured rates (a tensor-core product
+// at 1.6 PFLOP/s, panel bytes at 5.5 TB/s), with 30 % for the reconstruction.  A 529 x 2304 x 6241 step lies just
+// below the line (381 us with digits, 397 with residues), the o=64/v=512 slab
+// (1024 x 4096 x 262144) well above it (20.8 -> 18.1 ms).  Where the digits'
+// products take less than kResidueSmallUs in all, units and launches count and
+// not bytes: all residue products cost the same, so the GEMM has more and equal
+// units (o=10/v=48 step: 64 -> 44 us).  A pinned variant names a digit form.
 constexpr int kResidueMinKb = 24;
-void choose_products(a4g_batch* b, const std::vector<OzTile>& dinfo, bool allow) {
+constexpr double kResidueSmallUs = 40.0;
+void choose_products(a4g_batch* b, const std::vector<OzTile>& dinfo, const std::vector<PanelBuild>& pa,
+                     const std::vector<PanelBuild>& pb, bool allow) {
   b->residue = false;
   b->products = b->slices;
   if (!allow || b->variant || b->slices < 5 || dinfo.empty()) return;
   int min_kb = 1 << 30, max_kb = 0;
-  for (const OzTile& t : dinfo) min_kb = std::min(min_kb, t.kb_total), max_kb = std::max(max_kb, t.kb_total);
+  double macs = 0.0, elems = 0.0;  // per product, in whole 128 x 128 tiles; panel elements
+  for (const OzTile& t : dinfo) {
+    min_kb = std::min(min_kb, t.kb_total), max_kb = std::max(max_kb, t.kb_total);
+    macs += double(ceil_to(t.m0, kOzBM)) * double(ceil_to(t.n0, kOzBN)) * t.kb_total * kOzBK;
+  }
+  for (const auto& p : pa) elems += double(p.rows) * double(p.kpad);
+  for (const auto& p : pb)
+    if (p.used) elems += double(p.rows) * double(p.kpad);
   if (min_kb < kResidueMinKb) return;
-  const int L = oz_residue_count(b->slices, int64_t(max_kb) * kOzBK);
-  if (L <= 0 || L >= b->slices * (b->slices + 1) / 2) return;
+  const int L = oz_residue_count(b->slices, int64_t(max_kb) * kOzBK), P = b->slices * (b->slices + 1) / 2;
+  if (L <= 0 || L >= P) return;
+  const double product_us = 2.0 * macs / 1.6e9;
+  if (P * product_us > kResidueSmallUs && (P - L) * product_us < 1.3 * (2.0 * (L - b->slices) * elems / 5.5e6))
+    return;
   b->residue = true;
   b->products = L;
   oz_residue_tables(b->slices, L, int64_t(max_kb) * kOzBK, &b->res, &b->crt);
 }
 
-// Operand side of a job set: digits or residues.
-int launch_split(const a4g_batch* b, const a4g_batch::JobSet& js, cudaStream_t s) {
-  const OzPanel* panels = js.left ? b->d_pa : b->d_pb_view;
-  return b->residue ? oz_launch_residues(js.layout, js.d_jobs, js.d_prefix_split, js.njobs, js.tiles_split, panels,
-                                         b->res, s)
-                    : oz_launch_split(js.layout, js.d_jobs, js.d_prefix_split, js.njobs, js.tiles_split, panels,
-                                      b->slices, s);
+// The exponent or the split pass (digits or residues) of the job sets that
+// `take` picks, in one launch.
+template <class F>
+int launch_exps(const a4g_batch* b, cudaStream_t s, F&& take) {
+  OzJobSetRefs sets;
+  for (const auto& js : b->jobsets)
+    if (take(js)) sets.add(js.d_jobs, js.d_refs_exp, js.tiles_exp, js.left ? b->d_pa : b->d_pb_view, js.layout);
+  return oz_launch_exp(sets, s);
+}
+template <class F>
+int launch_split(const a4g_batch* b, cudaStream_t s, F&& take) {
+  OzJobSetRefs sets;
+  for (const auto& js : b->jobsets)
+    if (take(js)) sets.add(js.d_jobs, js.d_refs_split, js.tiles_split, js.left ? b->d_pa : b->d_pb_view, js.layout);
+  return b->residue ? oz_launch_residues(sets, b->res, s) : oz_launch_split(sets, b->slices, s);
 }
 
 // Result side of a workspace form.
@@ -623,7 +650,7 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     b->h_colptr = colptr_host;
     b->h_dblocks = dblocks;
   }
-  choose_products(b, dinfo, allow_residue);
+  choose_products(b, dinfo, pa, pb, allow_residue);
   b->signature = batch_signature(b, ptrn, b->bound.data(), int64_t(b->bound.size()));
   const int S = b->slices;
   const int NP = b->products;  // planes: slices of the panels, levels or moduli of the workspace
@@ -755,18 +782,18 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     js.left = left;
     js.layout = lay;
     js.group = group;
-    std::vector<int64_t> pe(1, 0), ps(1, 0);
-    for (const OzSplitJob& j : jobs) {
-      pe.push_back(pe.back() + oz_exp_tiles(lay, j.rows, j.K));
-      ps.push_back(ps.back() + oz_split_tiles(lay, j.rows, j.K));
+    std::vector<OzTileRef> re, rs;
+    for (size_t q = 0; q < jobs.size(); ++q) {
+      oz_add_refs(&re, int(q), oz_exp_tiles(lay, jobs[q].rows, jobs[q].K));
+      oz_add_refs(&rs, int(q), (b->residue ? oz_residue_tiles : oz_split_tiles)(lay, jobs[q].rows, jobs[q].K));
     }
     js.njobs = int(jobs.size());
-    js.tiles_exp = pe.back();
-    js.tiles_split = ps.back();
+    js.tiles_exp = int64_t(re.size());
+    js.tiles_split = int64_t(rs.size());
     js.h_jobs = jobs;
     int r;
-    if ((r = upload(b, jobs, &js.d_jobs)) || (r = upload(b, pe, &js.d_prefix_exp)) ||
-        (r = upload(b, ps, &js.d_prefix_split)))
+    if ((r = upload(b, jobs, &js.d_jobs)) || (r = upload(b, re, &js.d_refs_exp)) ||
+        (r = upload(b, rs, &js.d_refs_split)))
       return r;
     b->jobsets.push_back(js);
     return A4G_OK;
@@ -936,17 +963,15 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     if (!rc) {
       cudaStream_t s = ctx()->stream;
       A4G_CUDA(cudaMemsetAsync(b->d_exps, 0, b->exps_bytes, s));
-      for (const auto& js : b->jobsets)
-        if (!rc) rc = oz_launch_exp(js.layout, js.d_jobs, js.d_prefix_exp, js.njobs, js.tiles_exp,
-                                    js.left ? b->d_pa : b->d_pb_view, s);
-      for (const auto& js : b->jobsets)
-        if (!rc) rc = launch_split(b, js, s);
+      const auto every = [](const a4g_batch::JobSet&) { return true; };
+      rc = launch_exps(b, s, every);
+      if (!rc) rc = launch_split(b, s, every);
       if (!rc) rc = check_device_flag(s);
     }
     for (const auto& js : b->jobsets) {
       release(b, js.d_jobs, size_t(js.njobs) * sizeof(OzSplitJob));
-      release(b, js.d_prefix_exp, size_t(js.njobs + 1) * sizeof(int64_t));
-      release(b, js.d_prefix_split, size_t(js.njobs + 1) * sizeof(int64_t));
+      release(b, js.d_refs_exp, size_t(js.tiles_exp) * sizeof(OzTileRef));
+      release(b, js.d_refs_split, size_t(js.tiles_split) * sizeof(OzTileRef));
     }
     b->jobsets.clear();
     if (rc) return rc;
@@ -1291,13 +1316,11 @@ int clear_exps(a4g_batch* b, bool side_a, bool side_b, cudaStream_t s) {
 // both (side < 0), split pipeline groups included.
 int slice_side(a4g_batch* b, int side, cudaStream_t s) {
   int rc = clear_exps(b, side != 1, side != 0, s);
-  for (const auto& js : b->jobsets)
-    if (!rc && (side < 0 || side == (js.left ? 0 : 1)))
-      rc = oz_launch_exp(js.layout, js.d_jobs, js.d_prefix_exp, js.njobs, js.tiles_exp,
-                         js.left ? b->d_pa : b->d_pb_view, s);
-  for (const auto& js : b->jobsets)
-    if (!rc && (side < 0 || side == (js.left ? 0 : 1)))
-      rc = launch_split(b, js, s);
+  const auto take = [&](const a4g_batch::JobSet& js) { return side < 0 || side == (js.left ? 0 : 1); };
+  if (!rc) rc = launch_exps(b, s, take);
+  if (rc) return rc;
+  for (int g = 0; g < b->parts && !rc; ++g)  // one launch per group: at most six job sets in each
+    rc = launch_split(b, s, [&](const a4g_batch::JobSet& js) { return js.group == g && take(js); });
   return rc;
 }
 
@@ -1336,19 +1359,11 @@ int run(a4g_batch* b, cudaStream_t s, const cudaEvent_t* ev = nullptr) {
   auto sliced = [&](const a4g_batch::JobSet& js) { return !b->held[js.left ? 0 : 1]; };
   if (gf.n_tiles > 0) {
     if ((rc = clear_exps(b, !b->held[0], !b->held[1], s))) return rc;
-    for (const auto& js : b->jobsets)
-      if (sliced(js) && (rc = oz_launch_exp(js.layout, js.d_jobs, js.d_prefix_exp, js.njobs, js.tiles_exp,
-                                            js.left ? b->d_pa : b->d_pb_view, s)))
-        return rc;
+    if ((rc = launch_exps(b, s, sliced))) return rc;
   }
   if ((rc = mark(2))) return rc;
   auto split_group = [&](int g, cudaStream_t st) -> int {
-    for (const auto& js : b->jobsets)
-      if (js.group == g && sliced(js)) {
-        const int r = launch_split(b, js, st);
-        if (r) return r;
-      }
-    return A4G_OK;
+    return launch_split(b, st, [&](const a4g_batch::JobSet& js) { return js.group == g && sliced(js); });
   };
   if (gf.n_tiles > 0 && (rc = split_group(0, s))) return rc;
   if (gf.n_tiles > 0 && b->parts > 1) {
@@ -1574,10 +1589,11 @@ int a4g_batch_launches(const a4g_batch* b, int* kernels_per_run, int* gemm_parts
     k += b->n_f64_reds > 0 ? 1 : 0;
   } else if (b->forms[b->form].n_tiles > 0) {
     parts = b->parts;
-    int sliced = 0;  // job sets of a held side are not run
-    for (const auto& js : b->jobsets) sliced += b->held[js.left ? 0 : 1] ? 0 : 1;
-    // exponents + splits, GEMM parts, recombine (folded into the GEMM by direct forms)
-    k += 2 * sliced + parts + (b->forms[b->form].direct ? 0 : 1);
+    std::set<int> groups;  // one split launch per pipeline group; a held side's job sets are not run
+    for (const auto& js : b->jobsets)
+      if (!b->held[js.left ? 0 : 1]) groups.insert(js.group);
+    // exponents, splits, GEMM parts, recombine (folded into the GEMM by direct forms)
+    k += (groups.empty() ? 0 : 1) + int(groups.size()) + parts + (b->forms[b->form].direct ? 0 : 1);
   }
   if (kernels_per_run) *kernels_per_run = k;
   if (gemm_parts) *gemm_parts = parts;

@@ -74,8 +74,8 @@ struct a4g_fused {
   size_t exps_bytes = 0;
   OzPanel* d_panels = nullptr;  // A panels, then B panels (split jobs index the whole array)
   OzSplitJob* d_jobs = nullptr;
-  int64_t* d_prefix_exp = nullptr;
-  int64_t* d_prefix_split = nullptr;
+  OzTileRef* d_refs_exp = nullptr;
+  OzTileRef* d_refs_split = nullptr;
   int njobs = 0;
   int64_t tiles_exp = 0, tiles_split = 0;
   int64_t* d_offs = nullptr;        // split-job address tables
@@ -839,15 +839,15 @@ int a4g_fused_create(a4g_fused** out, int drank, int lrank, int rrank, const a4g
   // ---- split jobs (generic layout: any strides, the sign)
   if ((rc = fupload(f.get(), P.offs, &f->d_offs))) return rc;
   f->h_jobs = relocated_jobs(P, f->d_offs);
-  std::vector<int64_t> pe(1, 0), ps(1, 0);
-  for (const OzSplitJob& j : f->h_jobs) {
-    pe.push_back(pe.back() + oz_exp_tiles(kOzGeneric, j.rows, j.K));
-    ps.push_back(ps.back() + oz_split_tiles(kOzGeneric, j.rows, j.K));
+  std::vector<OzTileRef> re, rs;
+  for (size_t q = 0; q < f->h_jobs.size(); ++q) {
+    oz_add_refs(&re, int(q), oz_exp_tiles(kOzGeneric, f->h_jobs[q].rows, f->h_jobs[q].K));
+    oz_add_refs(&rs, int(q), oz_split_tiles(kOzGeneric, f->h_jobs[q].rows, f->h_jobs[q].K));
   }
   f->njobs = int(f->h_jobs.size());
-  f->tiles_exp = pe.back(), f->tiles_split = ps.back();
-  if ((rc = fupload(f.get(), f->h_jobs, &f->d_jobs)) || (rc = fupload(f.get(), pe, &f->d_prefix_exp)) ||
-      (rc = fupload(f.get(), ps, &f->d_prefix_split)))
+  f->tiles_exp = int64_t(re.size()), f->tiles_split = int64_t(rs.size());
+  if ((rc = fupload(f.get(), f->h_jobs, &f->d_jobs)) || (rc = fupload(f.get(), re, &f->d_refs_exp)) ||
+      (rc = fupload(f.get(), rs, &f->d_refs_split)))
     return rc;
   // ---- destination sub-blocks
   int64_t* d_rowoffs = nullptr;
@@ -967,9 +967,10 @@ int a4g_fused_run(a4g_fused* f, double* esum, void* stream) {
     if ((rc = launch_fill(z.first, z.second, 0.0, s))) return rc;
   if (f->args.n_tiles <= 0) return A4G_OK;
   A4G_CUDA(cudaMemsetAsync(f->d_exps, 0, f->exps_bytes, s));
-  if ((rc = oz_launch_exp(kOzGeneric, f->d_jobs, f->d_prefix_exp, f->njobs, f->tiles_exp, f->d_panels, s)) ||
-      (rc = oz_launch_split(kOzGeneric, f->d_jobs, f->d_prefix_split, f->njobs, f->tiles_split, f->d_panels,
-                            f->slices, s)) ||
+  OzJobSetRefs exps, split;
+  exps.add(f->d_jobs, f->d_refs_exp, f->tiles_exp, f->d_panels, kOzGeneric);
+  split.add(f->d_jobs, f->d_refs_split, f->tiles_split, f->d_panels, kOzGeneric);
+  if ((rc = oz_launch_exp(exps, s)) || (rc = oz_launch_split(split, f->slices, s)) ||
       (rc = f->levels ? oz_launch_levels(f->args, f->grid, s) : oz_launch_gemm(f->args, f->grid, false, kOzBN, s)))
     return rc;
   if (f->energy) return oz_launch_energy_reduce(f->d_epart, f->epart_len, f->efact, esum, s);

@@ -75,11 +75,42 @@ struct OzSplitJob {
   int pad;
 };
 
+// What CTA t of an exponent or split pass works on: piece `tile` of job `job`
+// (one 8-byte load; a search in the jobs' prefix sums took one dependent load
+// per halving, a microsecond at 256 jobs, before the first element was read).
+struct OzTileRef {
+  int job, tile;
+};
+
 // Memory layout of a split job's source block, detected on the host from the
 // address tables: a plain column-major [rows x K] matrix (rows contiguous), a
 // [K x rows] matrix (k contiguous), or anything else (gathered through the
 // tables).
 enum OzLayout { kOzGeneric = 0, kOzRowsMajor = 1, kOzKMajor = 2 };
+
+// The job sets (one per operand side and layout) that one launch of a pass
+// covers, one after another in the grid: a set that follows the first starts
+// while that one drains, and a small step pays for one launch, not for three.
+struct OzJobSetRef {
+  const OzSplitJob* jobs;
+  const OzTileRef* refs;
+  const OzPanel* panels;
+  int layout;
+  unsigned end;  // first CTA after this set
+};
+constexpr int kOzMaxJobSets = 16;  // 3 layouts a side, the right k-major set once per pipeline part
+struct OzJobSetRefs {
+  int n = 0;
+  int64_t total = 0;  // CTAs
+  OzJobSetRef s[kOzMaxJobSets];
+  void add(const OzSplitJob* jobs, const OzTileRef* refs, int64_t tiles, const OzPanel* panels, int layout) {
+    if (tiles <= 0) return;
+    total += tiles;
+    if (n < kOzMaxJobSets) s[n] = {jobs, refs, panels, layout, unsigned(total)};
+    ++n;
+  }
+  bool fits() const { return n <= kOzMaxJobSets && total <= 0x7fffffff; }
+};
 
 // One output tile (the GEMM form's tile_rows x tile_cols) of one destination block.
 struct OzTile {

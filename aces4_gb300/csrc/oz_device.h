@@ -16,15 +16,23 @@ constexpr int kDigitBits = 8;
 // an operand makes the whole row or column of the product NaN or infinite).
 constexpr int kNonFiniteExp = 2047;
 
-// Tiles of 64 rows x 64 k over the jobs; job_tiles[j] is the prefix count.
-__device__ __forceinline__ int find_job(const int64_t* prefix, int njobs, int64_t t) {
-  int lo = 0, hi = njobs;  // prefix[lo] <= t < prefix[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (prefix[mid] <= t) lo = mid;
-    else hi = mid;
-  }
-  return lo;
+// What this CTA works on.
+struct JobPiece {
+  OzSplitJob jb;
+  OzPanel pn;
+  int layout, tile;
+};
+__device__ __forceinline__ JobPiece job_piece(const OzJobSetRefs& sets) {
+  int q = 0;
+  unsigned base = 0;
+  while (q + 1 < sets.n && blockIdx.x >= sets.s[q].end) base = sets.s[q++].end;
+  const OzTileRef ref = sets.s[q].refs[blockIdx.x - base];
+  JobPiece p;
+  p.jb = sets.s[q].jobs[ref.job];
+  p.pn = sets.s[q].panels[p.jb.panel];
+  p.layout = sets.s[q].layout;
+  p.tile = ref.tile;
+  return p;
 }
 
 constexpr int kSplitT = 64;

@@ -23,9 +23,10 @@
 // Versions", ISC 2020 (slices on tensor cores with exact FP32 accumulation).
 //
 // Kernels:
-//   oz_exp_*_kernel     max exponent per panel row          (HBM: 8 B/elem read)
-//   oz_split_*_kernel   FP64 -> BF16 digit slices, K-major   (HBM: 8 B read + 2*slices B write)
-//                       with the block's index permute folded into the gather
+//   oz_exp_kernel       max exponent per panel row          (HBM: 8 B/elem read)
+//   oz_split_kernel     FP64 -> BF16 digit slices, K-major   (HBM: 8 B read + 2*slices B write)
+//                       with the block's index permute folded into the gather; both take every
+//                       operand side and source layout of a step in one launch
 //   oz_gemm_kernel<PAIR, BN, DIRECT, ENERGY>
 //                       persistent warp-specialised tcgen05 GEMM: TMA (SW128)
 //                       -> smem ring -> tcgen05.mma into TMEM (2 accumulators)
@@ -1343,16 +1344,11 @@ __global__ void __launch_bounds__(kThreadsOzDirect, 1) oz_levels_kernel(const __
 }
 
 // ------------------------------------------------------------------ split side
-__global__ void __launch_bounds__(256) oz_exp_kernel(const OzSplitJob* __restrict__ jobs,
-                                                     const int64_t* __restrict__ prefix, int njobs,
-                                                     const OzPanel* __restrict__ panels) {
-  __shared__ unsigned long long tile[kSplitT][kSplitT + 1];
-  const int64_t t = blockIdx.x;
-  const int j = find_job(prefix, njobs, t);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = t - prefix[j];
+// Row maxima of any source layout: 64 x 64 tiles gathered through the tables.
+__device__ __forceinline__ void exp_generic(const OzSplitJob& jb, const OzPanel& pn, int t,
+                                            unsigned long long (*tile)[kSplitT + 1]) {
   const int ktiles = (jb.K + kSplitT - 1) / kSplitT;
-  const int r0 = int(local / ktiles) * kSplitT, k0 = int(local % ktiles) * kSplitT;
+  const int r0 = (t / ktiles) * kSplitT, k0 = (t % ktiles) * kSplitT;
   load_job_tile(jb, r0, k0, tile);
   __syncthreads();
   // 4 threads per row, 16 k each
@@ -1361,7 +1357,90 @@ __global__ void __launch_bounds__(256) oz_exp_kernel(const OzSplitJob* __restric
   for (int k = part * 16; k < part * 16 + 16; ++k) m = max(m, int((tile[r][k] >> 52) & 0x7FF));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
   m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-  if (part == 0 && r0 + r < jb.rows && m > 0) atomicMax(&panels[jb.panel].exps[r0 + r], m);
+  if (part == 0 && r0 + r < jb.rows && m > 0) atomicMax(&pn.exps[r0 + r], m);
+}
+
+// Row maxima of a column-major [rows x K] block (rows contiguous) over a
+// kExpRowsK-wide k range: a thread owns two rows (one 16-byte load per k) and every
+// KG-th k, KG as many as 256 threads allow for the block's rows (a 144-row
+// block: 96 threads for the rows, 2 k at a time), eight loads in flight; the
+// row maxima meet in shared memory.
+constexpr int kExpRowsK = 32;
+__device__ __forceinline__ void exp_rows(const OzSplitJob& jb, const OzPanel& pn, int t, int* best) {
+  const int ktiles = (jb.K + kExpRowsK - 1) / kExpRowsK;
+  const int r0 = (t / ktiles) * 512, k0 = (t % ktiles) * kExpRowsK;
+  const int rows = min(512, jb.rows - r0), kn = min(kExpRowsK, jb.K - k0);
+  const int rp = ((rows + 1) / 2 + 31) & ~31, kg = 256 / rp;
+  const int lane = threadIdx.x % rp, kq = threadIdx.x / rp;
+  if (kg > 1) {
+    for (int i = threadIdx.x; i < rows; i += 256) best[i] = 0;
+    __syncthreads();
+  }
+  const int r = 2 * lane;
+  unsigned long long m0 = 0, m1 = 0;
+  constexpr unsigned long long kExp = 0x7FF0000000000000ull;
+  if (kq < kg && r < rows) {
+    const double* base = jb.src + size_t(k0) * jb.rows + r0 + r;
+    if (r + 1 < rows && (jb.rows & 1) == 0) {
+#pragma unroll 8
+      for (int k = kq; k < kn; k += kg) {
+        const double2 v = __ldg(reinterpret_cast<const double2*>(base + size_t(k) * jb.rows));
+        m0 = max(m0, __double_as_longlong(v.x) & kExp);
+        m1 = max(m1, __double_as_longlong(v.y) & kExp);
+      }
+    } else {
+      const bool two = r + 1 < rows;
+#pragma unroll 4
+      for (int k = kq; k < kn; k += kg) {
+        m0 = max(m0, __double_as_longlong(__ldg(base + size_t(k) * jb.rows)) & kExp);
+        if (two) m1 = max(m1, __double_as_longlong(__ldg(base + size_t(k) * jb.rows + 1)) & kExp);
+      }
+    }
+    int* e = kg > 1 ? best : pn.exps + r0;
+    if (m0) atomicMax(&e[r], int(m0 >> 52));
+    if (m1) atomicMax(&e[r + 1], int(m1 >> 52));
+  }
+  if (kg > 1) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < rows; i += 256)
+      if (best[i]) atomicMax(&pn.exps[r0 + i], best[i]);
+  }
+}
+
+// Row maxima of a [K x rows] block (k contiguous): one warp per row.
+__device__ __forceinline__ void exp_kmaj(const OzSplitJob& jb, const OzPanel& pn, int t) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool vec = (jb.K & 1) == 0;
+  for (int rr = 0; rr < 4; ++rr) {
+    const int r = t * 32 + warp * 4 + rr;
+    if (r >= jb.rows) return;
+    const double* row = jb.src + size_t(r) * jb.K;
+    unsigned long long m = 0;
+    if (vec) {
+      const double2* row2 = reinterpret_cast<const double2*>(row);
+#pragma unroll 4
+      for (int k = lane; k < jb.K / 2; k += 32) {
+        const double2 v = __ldg(row2 + k);
+        m = max(m, max(__double_as_longlong(v.x) & 0x7FF0000000000000ull,
+                       __double_as_longlong(v.y) & 0x7FF0000000000000ull));
+      }
+    } else {
+#pragma unroll 4
+      for (int k = lane; k < jb.K; k += 32)
+        m = max(m, __double_as_longlong(__ldg(row + k)) & 0x7FF0000000000000ull);
+    }
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0 && m) atomicMax(&pn.exps[r], int(m >> 52));
+  }
+}
+
+__global__ void __launch_bounds__(256) oz_exp_kernel(const __grid_constant__ OzJobSetRefs sets) {
+  extern __shared__ __align__(16) unsigned long long exp_smem[];
+  auto* tile = reinterpret_cast<unsigned long long(*)[kSplitT + 1]>(exp_smem);
+  const JobPiece p = job_piece(sets);
+  if (p.layout == kOzRowsMajor) exp_rows(p.jb, p.pn, p.tile, reinterpret_cast<int*>(tile));
+  else if (p.layout == kOzKMajor) exp_kmaj(p.jb, p.pn, p.tile);
+  else exp_generic(p.jb, p.pn, p.tile, tile);
 }
 
 // Balanced base-256 digits of n, most significant first: d[0] in [-128, 128],
@@ -1411,20 +1490,14 @@ __device__ __forceinline__ uint32_t digits_bf16x2(int d0, int d1) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// Slices of any source layout: 64 x 64 tiles gathered through the tables.
 template <int S>
-__global__ void __launch_bounds__(256) oz_split_kernel(const OzSplitJob* __restrict__ jobs,
-                                                       const int64_t* __restrict__ prefix, int njobs,
-                                                       const OzPanel* __restrict__ panels) {
-  __shared__ unsigned long long tile[kSplitT][kSplitT + 1];
-  const int64_t t = blockIdx.x;
-  const int j = find_job(prefix, njobs, t);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = t - prefix[j];
+__device__ __forceinline__ void split_generic(const OzSplitJob& jb, const OzPanel& pn, int tl,
+                                              unsigned long long (*tile)[kSplitT + 1]) {
   const int ktiles = (jb.K + kSplitT - 1) / kSplitT;
-  const int r0 = int(local / ktiles) * kSplitT, k0 = int(local % ktiles) * kSplitT;
+  const int r0 = (tl / ktiles) * kSplitT, k0 = (tl % ktiles) * kSplitT;
   load_job_tile(jb, r0, k0, tile);
   __syncthreads();
-  const OzPanel pn = panels[jb.panel];
   // each thread: one row, two consecutive k -> one bf16x2 store per slice
   const int kp = threadIdx.x & 31;
   for (int p = 0; p < 8; ++p) {
@@ -1444,87 +1517,13 @@ __global__ void __launch_bounds__(256) oz_split_kernel(const OzSplitJob* __restr
   }
 }
 
-// ------------------------------------------------------------------ fast split paths
-// Row maxima of a column-major [rows x K] block (rows contiguous): each thread
-// owns two rows (one 16-byte load per k) over a 64-wide k range.
-__global__ void __launch_bounds__(256) oz_exp_rows_kernel(const OzSplitJob* __restrict__ jobs,
-                                                          const int64_t* __restrict__ prefix, int njobs,
-                                                          const OzPanel* __restrict__ panels) {
-  const int j = find_job(prefix, njobs, blockIdx.x);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = int64_t(blockIdx.x) - prefix[j];
-  const int ktiles = (jb.K + 63) / 64;
-  const int r = int(local / ktiles) * 512 + 2 * threadIdx.x;
-  const int k0 = int(local % ktiles) * 64;
-  if (r >= jb.rows) return;
-  const int k1 = min(jb.K, k0 + 64);
-  const bool pair = r + 1 < jb.rows && (jb.rows & 1) == 0;
-  unsigned long long m0 = 0, m1 = 0;
-  const double* base = jb.src + r;
-  if (pair) {
-#pragma unroll 8
-    for (int k = k0; k < k1; ++k) {
-      const double2 v = __ldg(reinterpret_cast<const double2*>(base + size_t(k) * jb.rows));
-      m0 = max(m0, __double_as_longlong(v.x) & 0x7FF0000000000000ull);
-      m1 = max(m1, __double_as_longlong(v.y) & 0x7FF0000000000000ull);
-    }
-  } else {
-    for (int k = k0; k < k1; ++k) {
-      m0 = max(m0, __double_as_longlong(__ldg(base + size_t(k) * jb.rows)) & 0x7FF0000000000000ull);
-      if (r + 1 < jb.rows)
-        m1 = max(m1, __double_as_longlong(__ldg(base + 1 + size_t(k) * jb.rows)) & 0x7FF0000000000000ull);
-    }
-  }
-  int* e = panels[jb.panel].exps;
-  if (m0) atomicMax(&e[r], int(m0 >> 52));
-  if (m1 && r + 1 < jb.rows) atomicMax(&e[r + 1], int(m1 >> 52));
-}
-
-// Row maxima of a [K x rows] block (k contiguous): one warp per row.
-__global__ void __launch_bounds__(256) oz_exp_kmaj_kernel(const OzSplitJob* __restrict__ jobs,
-                                                          const int64_t* __restrict__ prefix, int njobs,
-                                                          const OzPanel* __restrict__ panels) {
-  const int j = find_job(prefix, njobs, blockIdx.x);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = int64_t(blockIdx.x) - prefix[j];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int* e = panels[jb.panel].exps;
-  const bool vec = (jb.K & 1) == 0;
-  for (int rr = 0; rr < 4; ++rr) {
-    const int r = int(local) * 32 + warp * 4 + rr;
-    if (r >= jb.rows) return;
-    const double* row = jb.src + size_t(r) * jb.K;
-    unsigned long long m = 0;
-    if (vec) {
-      const double2* row2 = reinterpret_cast<const double2*>(row);
-#pragma unroll 4
-      for (int k = lane; k < jb.K / 2; k += 32) {
-        const double2 v = __ldg(row2 + k);
-        m = max(m, max(__double_as_longlong(v.x) & 0x7FF0000000000000ull,
-                       __double_as_longlong(v.y) & 0x7FF0000000000000ull));
-      }
-    } else {
-      for (int k = lane; k < jb.K; k += 32)
-        m = max(m, __double_as_longlong(__ldg(row + k)) & 0x7FF0000000000000ull);
-    }
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0 && m) atomicMax(&e[r], int(m >> 52));
-  }
-}
-
 // Slices of a [K x rows] block: one warp per row, each lane four consecutive k
 // (two 16-byte loads, one 8-byte store per slice).
 template <int S>
-__global__ void __launch_bounds__(256) oz_split_kmaj_kernel(const OzSplitJob* __restrict__ jobs,
-                                                            const int64_t* __restrict__ prefix, int njobs,
-                                                            const OzPanel* __restrict__ panels) {
-  const int j = find_job(prefix, njobs, blockIdx.x);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = int64_t(blockIdx.x) - prefix[j];
+__device__ __forceinline__ void split_kmaj(const OzSplitJob& jb, const OzPanel& pn, int tl) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = int(local) * 8 + warp;
+  const int r = tl * 8 + warp;
   if (r >= jb.rows) return;
-  const OzPanel pn = panels[jb.panel];
   const int mx = pn.exps[r];
   const double* row = jb.src + size_t(r) * jb.K;
   uint2* dst = reinterpret_cast<uint2*>(pn.base + (size_t(r) * pn.kpad + jb.koff));
@@ -1563,15 +1562,10 @@ __device__ __forceinline__ int rows_tile_col(int k) { return (k & ~3) | (((k & 3
 // Slices of a column-major [rows x K] block: 64x64 tiles transposed through
 // shared memory (16-byte loads along rows, 8-byte stores along k).
 template <int S>
-__global__ void __launch_bounds__(256) oz_split_rows_kernel(const OzSplitJob* __restrict__ jobs,
-                                                            const int64_t* __restrict__ prefix, int njobs,
-                                                            const OzPanel* __restrict__ panels) {
-  __shared__ unsigned long long tile[64][65];
-  const int j = find_job(prefix, njobs, blockIdx.x);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = int64_t(blockIdx.x) - prefix[j];
+__device__ __forceinline__ void split_rows(const OzSplitJob& jb, const OzPanel& pn, int tl,
+                                           unsigned long long (*tile)[kSplitT + 1]) {
   const int ktiles = (jb.K + 63) / 64;
-  const int r0 = int(local / ktiles) * 64, k0 = int(local % ktiles) * 64;
+  const int r0 = (tl / ktiles) * 64, k0 = (tl % ktiles) * 64;
   const int t = threadIdx.x;
   // load: thread -> (row pair, k): 32 row pairs x 8 k per pass, 8 passes
   const bool vec = (jb.rows & 1) == 0;
@@ -1595,7 +1589,6 @@ __global__ void __launch_bounds__(256) oz_split_rows_kernel(const OzSplitJob* __
   }
   __syncthreads();
   // store: thread -> (row, 4 consecutive k): 16 k-quads x 16 rows per pass, 4 passes
-  const OzPanel pn = panels[jb.panel];
   const size_t slice_stride = size_t(pn.rows_pad) * pn.kpad / 4;
 #pragma unroll 1
   for (int p = 0; p < 4; ++p) {
@@ -1617,6 +1610,15 @@ __global__ void __launch_bounds__(256) oz_split_rows_kernel(const OzSplitJob* __
       dst[i * slice_stride] = o;
     }
   }
+}
+
+template <int S>
+__global__ void __launch_bounds__(256) oz_split_kernel(const __grid_constant__ OzJobSetRefs sets) {
+  __shared__ unsigned long long tile[kSplitT][kSplitT + 1];
+  const JobPiece p = job_piece(sets);
+  if (p.layout == kOzRowsMajor) split_rows<S>(p.jb, p.pn, p.tile, tile);
+  else if (p.layout == kOzKMajor) split_kmaj<S>(p.jb, p.pn, p.tile);
+  else split_generic<S>(p.jb, p.pn, p.tile, tile);
 }
 
 // ------------------------------------------------------------------ recombine
@@ -1975,7 +1977,7 @@ int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t row
 }
 
 int64_t oz_exp_tiles(int layout, int rows, int K) {
-  if (layout == kOzRowsMajor) return int64_t((rows + 511) / 512) * ((K + 63) / 64);
+  if (layout == kOzRowsMajor) return int64_t((rows + 511) / 512) * ((K + kExpRowsK - 1) / kExpRowsK);
   if (layout == kOzKMajor) return (rows + 31) / 32;
   return int64_t((rows + 63) / 64) * ((K + 63) / 64);
 }
@@ -1985,35 +1987,29 @@ int64_t oz_split_tiles(int layout, int rows, int K) {
   return int64_t((rows + 63) / 64) * ((K + 63) / 64);
 }
 
-int oz_launch_exp(int layout, const OzSplitJob* jobs, const int64_t* prefix, int njobs, int64_t ntiles,
-                  const OzPanel* panels, cudaStream_t s) {
-  if (ntiles <= 0) return A4G_OK;
-  if (ntiles > 0x7fffffffLL) return fail(A4G_ERR_RANGE, "too many split tiles");
-  if (layout == kOzRowsMajor) oz_exp_rows_kernel<<<unsigned(ntiles), 256, 0, s>>>(jobs, prefix, njobs, panels);
-  else if (layout == kOzKMajor) oz_exp_kmaj_kernel<<<unsigned(ntiles), 256, 0, s>>>(jobs, prefix, njobs, panels);
-  else oz_exp_kernel<<<unsigned(ntiles), 256, 0, s>>>(jobs, prefix, njobs, panels);
+int oz_launch_exp(const OzJobSetRefs& sets, cudaStream_t s) {
+  if (!sets.total) return A4G_OK;
+  if (!sets.fits()) return fail(A4G_ERR_RANGE, "too many split tiles");
+  // what the layouts at hand need (the row maxima, or a gathered tile): it bounds the CTAs per SM
+  size_t smem = 512 * sizeof(int);
+  for (int q = 0; q < sets.n; ++q)
+    if (sets.s[q].layout == kOzGeneric) smem = kSplitT * (kSplitT + 1) * sizeof(unsigned long long);
+  oz_exp_kernel<<<unsigned(sets.total), 256, smem, s>>>(sets);
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
 }
 
-int oz_launch_split(int layout, const OzSplitJob* jobs, const int64_t* prefix, int njobs, int64_t ntiles,
-                    const OzPanel* panels, int slices, cudaStream_t s) {
-  if (ntiles <= 0) return A4G_OK;
-  if (ntiles > 0x7fffffffLL) return fail(A4G_ERR_RANGE, "too many split tiles");
-  auto go = [&](auto sc) {
-    constexpr int S = decltype(sc)::value;
-    if (layout == kOzRowsMajor) oz_split_rows_kernel<S><<<unsigned(ntiles), 256, 0, s>>>(jobs, prefix, njobs, panels);
-    else if (layout == kOzKMajor) oz_split_kmaj_kernel<S><<<unsigned(ntiles), 256, 0, s>>>(jobs, prefix, njobs, panels);
-    else oz_split_kernel<S><<<unsigned(ntiles), 256, 0, s>>>(jobs, prefix, njobs, panels);
-  };
+int oz_launch_split(const OzJobSetRefs& sets, int slices, cudaStream_t s) {
+  if (!sets.total) return A4G_OK;
+  if (!sets.fits()) return fail(A4G_ERR_RANGE, "too many split tiles");
   switch (slices) {
-    case 1: go(std::integral_constant<int, 1>()); break;
-    case 2: go(std::integral_constant<int, 2>()); break;
-    case 3: go(std::integral_constant<int, 3>()); break;
-    case 4: go(std::integral_constant<int, 4>()); break;
-    case 5: go(std::integral_constant<int, 5>()); break;
-    case 6: go(std::integral_constant<int, 6>()); break;
-    case 7: go(std::integral_constant<int, 7>()); break;
+    case 1: oz_split_kernel<1><<<unsigned(sets.total), 256, 0, s>>>(sets); break;
+    case 2: oz_split_kernel<2><<<unsigned(sets.total), 256, 0, s>>>(sets); break;
+    case 3: oz_split_kernel<3><<<unsigned(sets.total), 256, 0, s>>>(sets); break;
+    case 4: oz_split_kernel<4><<<unsigned(sets.total), 256, 0, s>>>(sets); break;
+    case 5: oz_split_kernel<5><<<unsigned(sets.total), 256, 0, s>>>(sets); break;
+    case 6: oz_split_kernel<6><<<unsigned(sets.total), 256, 0, s>>>(sets); break;
+    case 7: oz_split_kernel<7><<<unsigned(sets.total), 256, 0, s>>>(sets); break;
     default: return fail(A4G_ERR_ARG, "slices must be 1..7");
   }
   A4G_CUDA(cudaGetLastError());
@@ -2066,7 +2062,7 @@ int oz_prepare() {
         (rc = set_smem_attr<false, 128, false, false, true>()) || (rc = set_smem_attr<true, 128, false, false, true>()) ||
         (rc = set_smem_attr<false, 256, false, false, true>()) || (rc = set_smem_attr<true, 256, false, false, true>()) ||
         (rc = set_smem_attr<false, 128, true, true>()) || (rc = set_levels_attr<false>()) ||
-        (rc = set_levels_attr<true>())) {
+        (rc = set_levels_attr<true>()) || (rc = oz_residue_prepare())) {
       done.store(0);
       return rc;
     }

@@ -1,6 +1,8 @@
 // Host launchers of the split-precision (Ozaki) contraction kernels.
 #pragma once
 
+#include <vector>
+
 #include "grouped.h"
 
 namespace a4g {
@@ -13,13 +15,15 @@ int oz_make_tensor_map(void* map128, const void* base, int64_t kpad, int64_t row
 // the all-levels form's map of a panel: boxes of 32 k x box_rows rows x every slice (64-byte swizzle)
 int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t rows_pad, int slices, int box_rows);
 int oz_max_pairs(int* pairs);  // CTA pairs of the 2-SM kernel that fit on the GPU at once
-// CTA counts of the exponent / split kernels for one job of a given layout.
+// CTA counts of the exponent / split kernels for one job of a given layout, and
+// the list of pieces of a job set's CTAs.
 int64_t oz_exp_tiles(int layout, int rows, int K);
 int64_t oz_split_tiles(int layout, int rows, int K);
-int oz_launch_exp(int layout, const OzSplitJob* jobs, const int64_t* prefix, int njobs, int64_t ntiles,
-                  const OzPanel* panels, cudaStream_t s);
-int oz_launch_split(int layout, const OzSplitJob* jobs, const int64_t* prefix, int njobs, int64_t ntiles,
-                    const OzPanel* panels, int slices, cudaStream_t s);
+inline void oz_add_refs(std::vector<OzTileRef>* refs, int job, int64_t tiles) {
+  for (int64_t t = 0; t < tiles; ++t) refs->push_back({job, int(t)});
+}
+int oz_launch_exp(const OzJobSetRefs& sets, cudaStream_t s);
+int oz_launch_split(const OzJobSetRefs& sets, int slices, cudaStream_t s);
 // pair = false: 1-SM kernel, 128 x tile_cols tiles; pair = true: CTA-pair
 // kernel (cluster of 2, cta_group::2), 256 x tile_cols tiles, grid even.
 // tile_cols: 128 (exact sums kept in TMEM) or 256 (exact sums in registers).
@@ -35,8 +39,10 @@ int oz_launch_levels(const OzGemmArgs& args, int grid, cudaStream_t s);
 // reconstruction (ws as int16, see OzGemmArgs).
 int oz_residue_count(int slices, int64_t K);
 void oz_residue_tables(int slices, int L, int64_t K, OzResidues* r, OzCrt* t);
-int oz_launch_residues(int layout, const OzSplitJob* jobs, const int64_t* prefix, int njobs, int64_t ntiles,
-                       const OzPanel* panels, const OzResidues& r, cudaStream_t s);
+int oz_residue_prepare();  // kernel attributes (oz_prepare calls it)
+int oz_launch_residues(const OzJobSetRefs& sets, const OzResidues& r, cudaStream_t s);
+// residue pieces of one job (the digits': oz_split_tiles)
+int64_t oz_residue_tiles(int layout, int rows, int K);
 int oz_launch_residue_recombine(const OzTile* tiles, int ntiles, int tile_rows, int tile_cols,
                                 const OzDBlock* dblocks, const OzPanel* pa, const OzPanel* pb, const void* ws,
                                 const OzCrt& t, int nsplit, int mode, cudaStream_t s);

@@ -140,19 +140,12 @@ __device__ __forceinline__ void store_residues(const OzResidues& R, const unsign
 
 // Any source layout: 64 x 64 tiles gathered through the address tables.
 template <int NP>
-__global__ void __launch_bounds__(256) oz_residue_generic_kernel(const __grid_constant__ OzResidues R,
-                                                                 const OzSplitJob* __restrict__ jobs,
-                                                                 const int64_t* __restrict__ prefix, int njobs,
-                                                                 const OzPanel* __restrict__ panels) {
-  __shared__ unsigned long long tile[kSplitT][kSplitT + 1];
-  const int j = find_job(prefix, njobs, blockIdx.x);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = int64_t(blockIdx.x) - prefix[j];
+__device__ __forceinline__ void residues_generic(const OzResidues& R, const OzSplitJob& jb, const OzPanel& pn, int t,
+                                                 unsigned long long (*tile)[kSplitT + 1]) {
   const int ktiles = (jb.K + kSplitT - 1) / kSplitT;
-  const int r0 = int(local / ktiles) * kSplitT, k0 = int(local % ktiles) * kSplitT;
+  const int r0 = (t / ktiles) * kSplitT, k0 = (t % ktiles) * kSplitT;
   load_job_tile(jb, r0, k0, tile);
   __syncthreads();
-  const OzPanel pn = panels[jb.panel];
   const size_t plane = size_t(pn.rows_pad) * pn.kpad / 8;
 #pragma unroll 1
   for (int p = 0; p < 2; ++p) {
@@ -162,21 +155,15 @@ __global__ void __launch_bounds__(256) oz_residue_generic_kernel(const __grid_co
 #pragma unroll
     for (int u = 0; u < 8; ++u) b[u] = tile[r][k + u];  // zero beyond K
     store_residues<NP>(R, b, row_scale(pn.exps[r0 + r], R.slices),
-                         reinterpret_cast<uint4*>(pn.base + (size_t(r0 + r) * pn.kpad + jb.koff + k0 + k)), plane);
+                       reinterpret_cast<uint4*>(pn.base + (size_t(r0 + r) * pn.kpad + jb.koff + k0 + k)), plane);
   }
 }
 
 // A [K x rows] block (k contiguous): eight rows per CTA, eight consecutive k
 // per thread, threads over the rows' k octets in turn (a row of 144 k has 18).
 template <int NP>
-__global__ void __launch_bounds__(256) oz_residue_kmaj_kernel(const __grid_constant__ OzResidues R,
-                                                              const OzSplitJob* __restrict__ jobs,
-                                                              const int64_t* __restrict__ prefix, int njobs,
-                                                              const OzPanel* __restrict__ panels) {
-  const int j = find_job(prefix, njobs, blockIdx.x);
-  const OzSplitJob jb = jobs[j];
-  const int r0 = int(int64_t(blockIdx.x) - prefix[j]) * 8;
-  const OzPanel pn = panels[jb.panel];
+__device__ __forceinline__ void residues_kmaj(const OzResidues& R, const OzSplitJob& jb, const OzPanel& pn, int t) {
+  const int r0 = t * 8;
   const size_t plane = size_t(pn.rows_pad) * pn.kpad / 8;
   const int octs = (jb.K + 7) / 8, rows = min(8, jb.rows - r0);
   const bool vec = (jb.K & 1) == 0;
@@ -196,62 +183,88 @@ __global__ void __launch_bounds__(256) oz_residue_kmaj_kernel(const __grid_const
       for (int u = 0; u < 8; ++u) b[u] = k + u < jb.K ? __double_as_longlong(__ldg(src + u)) : 0ull;
     }
     store_residues<NP>(R, b, row_scale(pn.exps[r], R.slices),
-                         reinterpret_cast<uint4*>(pn.base + (size_t(r) * pn.kpad + jb.koff + k)), plane);
+                       reinterpret_cast<uint4*>(pn.base + (size_t(r) * pn.kpad + jb.koff + k)), plane);
   }
 }
 
-// Column of k inside a row of the transpose tile: the low three bits are
-// rotated by the octet, so that the eight octets of a row that a quarter warp
-// reads (columns 8 q + u) fall into eight different banks.
-__device__ __forceinline__ int oct_col(int k) { return (k & ~7) | ((k + (k >> 3)) & 7); }
-
-// A column-major [rows x K] block: 64 x 64 tiles transposed through shared
-// memory (16-byte loads along rows, 16-byte stores along k).
+// A column-major [rows x K] block (rows contiguous), transposed through shared
+// memory: 32 rows and up to eight tiles of 64 k per CTA, two tiles copied
+// asynchronously (16 or 8 bytes at a time) while a third is reduced; one tile
+// per CTA, loaded, then reduced, ran at 57 % of the memory bandwidth.  Element
+// (k, row) of a tile lies at [k][(row + 2 (k / 8)) mod 32]: the copies' 16-byte
+// pieces stay whole, and the eight octets of two rows that a half warp reads
+// fall into 16 different banks.
+constexpr int kRowTiles = 8, kRowStages = 3, kRowRows = 32;
+__device__ __forceinline__ void copy_async(uint32_t dst, const double* src, int bytes, bool live) {
+  const int n = live ? bytes : 0;  // what is left out is zero
+  if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
 template <int NP>
-__global__ void __launch_bounds__(256) oz_residue_rows_kernel(const __grid_constant__ OzResidues R,
-                                                              const OzSplitJob* __restrict__ jobs,
-                                                              const int64_t* __restrict__ prefix, int njobs,
-                                                              const OzPanel* __restrict__ panels) {
-  __shared__ unsigned long long tile[64][65];
-  const int j = find_job(prefix, njobs, blockIdx.x);
-  const OzSplitJob jb = jobs[j];
-  const int64_t local = int64_t(blockIdx.x) - prefix[j];
-  const int ktiles = (jb.K + 63) / 64;
-  const int r0 = int(local / ktiles) * 64, k0 = int(local % ktiles) * 64;
-  const int t = threadIdx.x;
+__device__ __forceinline__ void residues_rows(const OzResidues& R, const OzSplitJob& jb, const OzPanel& pn, int t,
+                                              unsigned long long (*tiles)[64][kRowRows]) {
+  const int kchunks = (jb.K + 64 * kRowTiles - 1) / (64 * kRowTiles);
+  const int r0 = (t / kchunks) * kRowRows, kfirst = (t % kchunks) * 64 * kRowTiles;
+  const int n = min(kRowTiles, (jb.K - kfirst + 63) / 64);
+  const size_t plane = size_t(pn.rows_pad) * pn.kpad / 8;
   const bool vec = (jb.rows & 1) == 0;
+  auto load = [&](int i, int stage) {
+    if (i < n) {
+      const int k0 = kfirst + 64 * i;
+      const uint32_t dst = uint32_t(__cvta_generic_to_shared(tiles[stage]));
+      const int rp = threadIdx.x & 15, r = r0 + 2 * rp;
 #pragma unroll
-  for (int p = 0; p < 8; ++p) {
-    const int rp = t & 31, k = (t >> 5) + 8 * p;
-    const int r = r0 + 2 * rp;
-    unsigned long long x0 = 0, x1 = 0;
-    if (k0 + k < jb.K && r < jb.rows) {
-      const double* src = jb.src + size_t(k0 + k) * jb.rows + r;
-      if (vec) {
-        const double2 v = __ldg(reinterpret_cast<const double2*>(src));
-        x0 = __double_as_longlong(v.x), x1 = __double_as_longlong(v.y);
-      } else {
-        x0 = __double_as_longlong(__ldg(src));
-        if (r + 1 < jb.rows) x1 = __double_as_longlong(__ldg(src + 1));
+      for (int p = 0; p < 4; ++p) {
+        const int k = (threadIdx.x >> 4) + 16 * p;
+        const bool live = k0 + k < jb.K && r < jb.rows;
+        const double* src = live ? jb.src + size_t(k0 + k) * jb.rows + r : jb.src;
+        const uint32_t at = dst + 8u * uint32_t(kRowRows * k + ((2 * rp + 2 * (k >> 3)) & (kRowRows - 1)));
+        if (vec) {
+          copy_async(at, src, 16, live);
+        } else {
+          copy_async(at, src, 8, live);
+          copy_async(at + 8, live && r + 1 < jb.rows ? src + 1 : jb.src, 8, live && r + 1 < jb.rows);
+        }
       }
     }
-    tile[2 * rp][oct_col(k)] = x0;
-    tile[2 * rp + 1][oct_col(k)] = x1;
-  }
-  __syncthreads();
-  const OzPanel pn = panels[jb.panel];
-  const size_t plane = size_t(pn.rows_pad) * pn.kpad / 8;
-#pragma unroll 1
-  for (int p = 0; p < 2; ++p) {
-    const int k = 8 * (t & 7), r = (t >> 3) + 32 * p;
-    if (r0 + r >= jb.rows || k0 + k >= jb.K) continue;
-    unsigned long long b[8];
+    asm volatile("cp.async.commit_group;" ::: "memory");  // one group per tile, empty ones too
+  };
+  for (int i = 0; i < kRowStages - 1; ++i) load(i, i);
+  const int o = threadIdx.x & 7, row = threadIdx.x >> 3;  // this thread's octet and row
+  const bool live = r0 + row < jb.rows;
+  const RowScale rs = row_scale(live ? pn.exps[r0 + row] : 0, R.slices);
+  uint4* dst = reinterpret_cast<uint4*>(pn.base + (size_t(r0 + row) * pn.kpad + jb.koff + kfirst + 8 * o));
+  int stage = 0, next = kRowStages - 1;
+  for (int i = 0; i < n; ++i) {
+    load(i + kRowStages - 1, next);
+    next = next + 1 == kRowStages ? 0 : next + 1;
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRowStages - 1) : "memory");
+    __syncthreads();
+    if (live && kfirst + 64 * i + 8 * o < jb.K) {
+      unsigned long long b[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) b[u] = tile[r][oct_col(k + u)];  // zero beyond K
-    store_residues<NP>(R, b, row_scale(pn.exps[r0 + r], R.slices),
-                         reinterpret_cast<uint4*>(pn.base + (size_t(r0 + r) * pn.kpad + jb.koff + k0 + k)), plane);
+      for (int u = 0; u < 8; ++u) b[u] = tiles[stage][8 * o + u][(row + 2 * o) & (kRowRows - 1)];  // zero beyond K
+      store_residues<NP>(R, b, rs, dst + 8 * i, plane);
+    }
+    __syncthreads();  // the tile is read before a later one lands in it
+    stage = stage + 1 == kRowStages ? 0 : stage + 1;
   }
 }
+
+template <int NP>
+__global__ void __launch_bounds__(256, 4) oz_residue_kernel(const __grid_constant__ OzResidues R,
+                                                            const __grid_constant__ OzJobSetRefs sets) {
+  extern __shared__ __align__(16) unsigned long long residue_smem[];
+  const JobPiece p = job_piece(sets);
+  if (p.layout == kOzRowsMajor)
+    residues_rows<NP>(R, p.jb, p.pn, p.tile, reinterpret_cast<unsigned long long(*)[64][kRowRows]>(residue_smem));
+  else if (p.layout == kOzKMajor)
+    residues_kmaj<NP>(R, p.jb, p.pn, p.tile);
+  else
+    residues_generic<NP>(R, p.jb, p.pn, p.tile, reinterpret_cast<unsigned long long(*)[kSplitT + 1]>(residue_smem));
+}
+constexpr size_t kRowsSmem = kRowStages * 64 * kRowRows * sizeof(unsigned long long);
+constexpr size_t kGenericSmem = kSplitT * (kSplitT + 1) * sizeof(unsigned long long);
 
 // ------------------------------------------------------------------ result side
 // The integer X with X = s_i (mod p_i), |X| < prod p / 2 (the host admits only
@@ -426,20 +439,28 @@ void oz_residue_tables(int slices, int L, int64_t K, OzResidues* r, OzCrt* t) {
   }
 }
 
-int oz_launch_residues(int layout, const OzSplitJob* jobs, const int64_t* prefix, int njobs, int64_t ntiles,
-                       const OzPanel* panels, const OzResidues& r, cudaStream_t s) {
-  if (ntiles <= 0) return A4G_OK;
-  if (ntiles > 0x7fffffffLL) return fail(A4G_ERR_RANGE, "too many split tiles");
-  auto go = [&](auto np) {
-    constexpr int NP = decltype(np)::value;
-    const unsigned g = unsigned(ntiles);
-    if (layout == kOzRowsMajor) oz_residue_rows_kernel<NP><<<g, 256, 0, s>>>(r, jobs, prefix, njobs, panels);
-    else if (layout == kOzKMajor) oz_residue_kmaj_kernel<NP><<<g, 256, 0, s>>>(r, jobs, prefix, njobs, panels);
-    else oz_residue_generic_kernel<NP><<<g, 256, 0, s>>>(r, jobs, prefix, njobs, panels);
-  };
-  if (r.slices <= 5) go(std::integral_constant<int, 3>());
-  else go(std::integral_constant<int, 4>());
+int64_t oz_residue_tiles(int layout, int rows, int K) {
+  if (layout == kOzRowsMajor) return int64_t((rows + kRowRows - 1) / kRowRows) * ((K + 64 * kRowTiles - 1) / (64 * kRowTiles));
+  return oz_split_tiles(layout, rows, K);
+}
+
+int oz_launch_residues(const OzJobSetRefs& sets, const OzResidues& r, cudaStream_t s) {
+  if (!sets.total) return A4G_OK;
+  if (!sets.fits()) return fail(A4G_ERR_RANGE, "too many split tiles");
+  size_t smem = 0;  // what the layouts at hand need: it bounds the CTAs per SM
+  for (int q = 0; q < sets.n; ++q) {
+    if (sets.s[q].layout == kOzRowsMajor) smem = std::max(smem, kRowsSmem);
+    if (sets.s[q].layout == kOzGeneric) smem = std::max(smem, kGenericSmem);
+  }
+  if (r.slices <= 5) oz_residue_kernel<3><<<unsigned(sets.total), 256, smem, s>>>(r, sets);
+  else oz_residue_kernel<4><<<unsigned(sets.total), 256, smem, s>>>(r, sets);
   A4G_CUDA(cudaGetLastError());
+  return A4G_OK;
+}
+
+int oz_residue_prepare() {
+  A4G_CUDA(cudaFuncSetAttribute(oz_residue_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(std::max(kRowsSmem, kGenericSmem))));
+  A4G_CUDA(cudaFuncSetAttribute(oz_residue_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(std::max(kRowsSmem, kGenericSmem))));
   return A4G_OK;
 }
 
