@@ -39,6 +39,7 @@
 #include "a4g_internal.h"
 #include "grouped.h"
 #include "ozaki.h"
+#include "stage.h"
 
 using namespace a4g;
 
@@ -85,9 +86,7 @@ struct a4g_fused {
   // energy form
   const double* e_dev = nullptr;
   int rank1 = 1, ld1 = 0;
-  double* d_elast = nullptr;
-  size_t n_elast = 0;
-  double* d_ptab = nullptr;
+  double* d_ptab = nullptr;  // prefix tables, and the last terms' energies of each block
   PtabTable* d_ptabs = nullptr;
   int n_ptabs = 0;
   int64_t max_ptab_n = 0;
@@ -96,8 +95,11 @@ struct a4g_fused {
   double* d_epart = nullptr;
   int epart_len = 0;
   std::vector<std::pair<double*, int64_t>> zero_blocks;  // store mode, beta 0: blocks no pair feeds
+  TableStage stage;  // a rebind's tables on their way to the device
+  cudaEvent_t ev_default = nullptr;
   ~a4g_fused() {
     for (void* p : allocs) cudaFree(p);
+    if (ev_default) cudaEventDestroy(ev_default);
   }
 };
 
@@ -196,14 +198,6 @@ struct TablePool {
   }
 };
 
-// Host copy of the orbital energies a denominator reads (e or the diagonal
-// of the Fock block).
-struct Energies {
-  int rank1 = 1, ld1 = 0;
-  std::vector<double> h;
-  double at(int orb) const { return rank1 == 2 ? h[size_t(orb) + size_t(orb) * size_t(ld1)] : h[size_t(orb)]; }
-};
-
 // 64-bit FNV-1a over the inputs that decide a fused step's device structure.
 struct Fnv64 {
   uint64_t h = 1469598103934665603ull;
@@ -268,7 +262,6 @@ struct Plan {
   const double* e_dev = nullptr;
   int rank1 = 1, ld1 = 0;
   std::vector<int> ikeys;
-  std::vector<double> elast;
   std::vector<PtabTable> ptabs;
   int64_t ptab_n = 0;
   std::vector<OzEnergyBlock> eblocks;  // ptab / rk / ck / elast as offsets
@@ -369,7 +362,6 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
   for (const WBlock& w : wb) sig.add(w.dext, sizeof(int) * size_t(drank));
 
   // ---- energy inputs
-  Energies en;
   int pos[6] = {0, 1, 2, 3, 4, 5};
   std::vector<std::vector<int>> wb_off(wb.size());  // orbital offset per destination dim
   int dl = -1;                                      // destination dim of the chain's last term
@@ -398,12 +390,8 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
     dl = pos[drank - 2];
     if (cat[size_t(dl)] != kRow && cat[size_t(dl)] != kCol)
       return fail(A4G_ERR_UNSUPPORTED, "fused energy: the denominator's last term is a fixed (batch) index");
-    en.rank1 = energy->rank1, en.ld1 = energy->ext1[0];
     const int64_t ne = energy->rank1 == 2 ? int64_t(energy->ext1[0]) * energy->ext1[1] : energy->ext1[0];
     if (ne <= 0) return fail(A4G_ERR_ARG, "fused energy: empty energy array");
-    sig.put(energy->rank1), sig.put(energy->ext1[0]), sig.put(energy->rank1 == 2 ? energy->ext1[1] : 0);
-    en.h.resize(size_t(ne));
-    A4G_CUDA(cudaMemcpy(en.h.data(), energy->e_or_fock, size_t(ne) * sizeof(double), cudaMemcpyDeviceToHost));
     const std::vector<int> segs(energy->seg_sizes, energy->seg_sizes + std::max(energy->nsegs, 0));
     for (int64_t i = 0; i < energy->n_blocks; ++i) {
       auto it = widx.find(energy->blocks[i]);
@@ -418,7 +406,7 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
       if (wb_off[w].empty()) return fail(A4G_ERR_ARG, "fused energy: a destination block without index values");
     P.efact = energy->efact;
     P.e_dev = energy->e_or_fock;
-    P.rank1 = en.rank1, P.ld1 = en.ld1;
+    P.rank1 = energy->rank1, P.ld1 = energy->ext1[0];
   }
 
   // ---- panels, split jobs, sub-problems, tiles
@@ -640,6 +628,7 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
     const bool last_row = cat[size_t(dl)] == kRow;
     TablePool<int> ikeys;
     std::map<std::vector<int>, size_t> ptab_index;  // orbital offsets and extents -> table offset
+    int64_t prefix_n = 0;
     for (size_t w = 0; w < wb.size(); ++w) {
       const WBlock& W = wb[w];
       const WInfo& I = wi[w];
@@ -664,20 +653,23 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
       EW& E = ew[w];
       E.rk_at = ikeys.add(keys(dims[kRow], erow, I.M));
       E.ck_at = ikeys.add(keys(dims[kCol], ecol, I.N));
-      // the last term's energies along its own dim (one array per block: its
-      // values change with the block's segments, its place must not)
+      // the last term's energies along its own dim: a table of one term over the
+      // rows (columns), read on the device like the prefix tables (one per
+      // block: its values change with the block's segments, its place must not)
       {
         const std::vector<int>& cd = last_row ? dims[kRow] : dims[kCol];
         const std::vector<int>& ex = last_row ? erow : ecol;
-        const int64_t n = last_row ? I.M : I.N;
+        PtabTable el{};
+        el.n = last_row ? I.M : I.N;
+        el.rkn = int(el.n), el.ckn = 1, el.nb1 = 1, el.nb2 = 1, el.nterms = 1;
+        int stride = 1;
         size_t qd = 0;
-        while (cd[qd] != dl) ++qd;
-        int c[kMaxRank];
-        E.el_at = P.elast.size();
-        for (int64_t i = 0; i < n; ++i) {
-          coords_of(i, ex, c);
-          P.elast.push_back(en.at(off[size_t(dl)] + c[qd]));
-        }
+        while (cd[qd] != dl) stride *= ex[qd++];
+        el.t[0] = {0, stride, ex[qd], off[size_t(dl)], 1};
+        el.at = P.ptab_n;
+        P.ptab_n += el.n;
+        P.ptabs.push_back(el);
+        E.el_at = size_t(el.at);
       }
       // prefix table [b][j][rk][ck] (the chain without its last term), shared by
       // the blocks whose other dims have the same segments
@@ -704,9 +696,9 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
         if (d != dl) key.push_back(off[size_t(d)]), key.push_back(W.dext[d]);
       auto it = ptab_index.find(key);
       if (it == ptab_index.end()) {
-        if (P.ptab_n + tab.n > (int64_t(1) << 28)) return fail(A4G_ERR_RANGE, "fused energy: denominator tables beyond 2 GB");
+        if (prefix_n + tab.n > (int64_t(1) << 28)) return fail(A4G_ERR_RANGE, "fused energy: denominator tables beyond 2 GB");
         tab.at = P.ptab_n;
-        P.ptab_n += tab.n;
+        P.ptab_n += tab.n, prefix_n += tab.n;
         P.ptabs.push_back(tab);
         it = ptab_index.emplace(key, size_t(tab.at)).first;
       }
@@ -770,9 +762,11 @@ std::vector<OzSplitJob> relocated_jobs(const Plan& P, const int64_t* d_offs) {
 int launch_ptab(const a4g_fused* f, cudaStream_t s) {
   if (f->n_ptabs == 0) return A4G_OK;
   const unsigned gx = unsigned(std::min<int64_t>(4096, (f->max_ptab_n + 255) / 256));
-  ptab_kernel<<<dim3(std::max(1u, gx), unsigned(f->n_ptabs)), 256, 0, s>>>(f->d_ptabs, f->e_dev, f->rank1, f->ld1,
-                                                                           f->d_ptab);
-  A4G_CUDA(cudaGetLastError());
+  for (int i = 0; i < f->n_ptabs; i += 65535) {
+    const unsigned gy = unsigned(std::min(65535, f->n_ptabs - i));
+    ptab_kernel<<<dim3(std::max(1u, gx), gy), 256, 0, s>>>(f->d_ptabs + i, f->e_dev, f->rank1, f->ld1, f->d_ptab);
+    A4G_CUDA(cudaGetLastError());
+  }
   return A4G_OK;
 }
 
@@ -860,10 +854,9 @@ int a4g_fused_create(a4g_fused** out, int drank, int lrank, int rrank, const a4g
   std::vector<OzEnergyBlock> eblocks = P.eblocks;
   if (f->energy) {
     int* d_ikeys = nullptr;
-    if ((rc = fupload(f.get(), P.ikeys, &d_ikeys)) || (rc = fupload(f.get(), P.elast, &f->d_elast)) ||
+    if ((rc = fupload(f.get(), P.ikeys, &d_ikeys)) ||
         (rc = fupload(f.get(), P.ptabs, &f->d_ptabs)))
       return rc;
-    f->n_elast = P.elast.size();
     void* p = nullptr;
     if ((rc = falloc(f.get(), size_t(P.ptab_n) * sizeof(double), &p))) return rc;
     f->d_ptab = static_cast<double*>(p);
@@ -875,7 +868,7 @@ int a4g_fused_create(a4g_fused** out, int drank, int lrank, int rrank, const a4g
       eb.ptab = f->d_ptab + offset_of(eb.ptab);
       eb.rk = d_ikeys + offset_of(eb.rk);
       eb.ck = d_ikeys + offset_of(eb.ck);
-      eb.elast = f->d_elast + offset_of(eb.elast);
+      eb.elast = f->d_ptab + offset_of(eb.elast);
     }
   }
 
@@ -939,22 +932,30 @@ int a4g_fused_rebind(a4g_fused* f, const a4g_term* terms, int nterms, const a4g_
   int rc = plan_fused(f->drank, f->lrank, f->rrank, terms, nterms, energy, f->slices, f->beta, f->variant, &P);
   if (rc) return rc;
   if (P.sig != f->signature || P.jobs.size() != f->h_jobs.size() || P.colptr.size() != f->n_colptr ||
-      P.elast.size() != f->n_elast || int(P.ptabs.size()) != f->n_ptabs)
+      int(P.ptabs.size()) != f->n_ptabs)
     return fail(A4G_ERR_ARG, "fused rebind: the triples' structure differs from the creation's");
   cudaStream_t s = pick(stream);
-  // only what depends on the blocks: split-job sources, column bases, energy tables
+  // only what depends on the blocks: split-job sources, column bases, energy
+  // tables (their energies are read on the device: nothing waits for the
+  // stream, so the host plans the next step while this one runs: 2.7 ms of
+  // planning hidden behind an 18 ms step of o=24/v=240)
+  static_assert(sizeof(OzSplitJob) % 8 == 0 && sizeof(PtabTable) % 8 == 0, "tables are copied in 8-byte words");
   f->h_jobs = relocated_jobs(P, f->d_offs);
-  A4G_CUDA(cudaMemcpyAsync(f->d_jobs, f->h_jobs.data(), f->h_jobs.size() * sizeof(OzSplitJob), cudaMemcpyHostToDevice, s));
-  if (!P.colptr.empty())
-    A4G_CUDA(cudaMemcpyAsync(f->d_colptr, P.colptr.data(), P.colptr.size() * sizeof(double*), cudaMemcpyHostToDevice, s));
+  const size_t bytes_j = f->h_jobs.size() * sizeof(OzSplitJob), bytes_c = P.colptr.size() * sizeof(double*),
+               bytes_t = f->energy ? P.ptabs.size() * sizeof(PtabTable) : 0;
+  if ((rc = f->stage.begin(bytes_j + bytes_c + bytes_t)) || (rc = f->stage.add(f->d_jobs, f->h_jobs.data(), bytes_j)) ||
+      (rc = f->stage.add(f->d_colptr, P.colptr.data(), bytes_c)) ||
+      (rc = f->stage.add(f->d_ptabs, P.ptabs.data(), bytes_t)) || (rc = f->stage.launch(s)))
+    return rc;
   f->zero_blocks = P.zero_blocks;
   if (f->energy) {
-    A4G_CUDA(cudaMemcpyAsync(f->d_elast, P.elast.data(), P.elast.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-    A4G_CUDA(cudaMemcpyAsync(f->d_ptabs, P.ptabs.data(), P.ptabs.size() * sizeof(PtabTable), cudaMemcpyHostToDevice, s));
-    f->e_dev = P.e_dev, f->efact = P.efact;
+    f->e_dev = P.e_dev, f->efact = P.efact, f->rank1 = P.rank1, f->ld1 = P.ld1;
+    // energies that the default stream is still writing are waited for there
+    if (!f->ev_default) A4G_CUDA(cudaEventCreateWithFlags(&f->ev_default, cudaEventDisableTiming));
+    A4G_CUDA(cudaEventRecord(f->ev_default, cudaStreamLegacy));
+    A4G_CUDA(cudaStreamWaitEvent(s, f->ev_default, 0));
     if ((rc = launch_ptab(f, s))) return rc;
   }
-  // the host vectors must outlive the copies: pageable sources are staged before these calls return
   return A4G_OK;
 }
 
