@@ -733,7 +733,9 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
       db.d = base;
       db.rowoff = as_offset<const int64_t>(I.rowoff_at);
       db.colptr = as_offset<double* const>(P.colptr.size());
-      for (int64_t o : enum_offsets(ex, st)) P.colptr.push_back(base + o);
+      const std::vector<int64_t> cols = enum_offsets(ex, st);
+      for (int64_t o : cols) P.colptr.push_back(base + o);
+      db.col_fast = cols.size() > 1 && cols[1] == 1;  // D is unit-stride along a column index
     } else {
       const EW& E = ew[sb.w];
       OzEnergyBlock eb{};

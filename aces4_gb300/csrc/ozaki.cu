@@ -1032,7 +1032,9 @@ struct __align__(1024) LvSmem {
   uint64_t acc_full, acc_empty, drain;
   uint32_t tmem_base;
   volatile int abort;
+  double out[kThreadsOzDirect / 32 - 2][32][9];  // per epilogue warp: 32 rows x 8 columns on their way to D
 };
+static_assert(sizeof(LvSmem) + 1024 + 6144 <= 232448, "with the static column tables: one CTA's shared memory");
 static_assert(kLvBN == kOzLevelsTileCols, "tile columns of the all-levels form");
 // TMEM accumulator (in 64-column units) of level t; levels 3 and 4: of k half
 // h.  The levels of each half lie side by side: 0 1 2 3 4 | 3' 4'.
@@ -1286,14 +1288,51 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
       }
     } else {
       const bool acc = a.mode & 1;
+      auto result = [&](int j) {
+        const int F = tab[j].F;
+        double x = i64_scaled_to_double(sum[j], ebase + F, a.mode & 2);
+        if (nonfinite || F == kNonFiniteExp) x = __longlong_as_double(0x7FF8000000000000ll);
+        return x;
+      };
+      if (!db.col_fast) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const LvCol c = tab[j];
-        if (!mlive || !c.colp) continue;
-        double x = i64_scaled_to_double(sum[j], ebase + c.F, a.mode & 2);
-        if (nonfinite || c.F == kNonFiniteExp) x = __longlong_as_double(0x7FF8000000000000ll);
-        double* p = c.colp + roff;
-        *p = acc ? *p + x : x;
+        for (int j = 0; j < 16; ++j) {
+          double* cp = tab[j].colp;
+          if (!mlive || !cp) continue;
+          const double x = result(j);
+          double* p = cp + roff;
+          *p = acc ? *p + x : x;
+        }
+      } else {
+        // D runs along the columns: the warp's 32 x 8 results turn in shared
+        // memory, so that a store covers four rows of 64 contiguous bytes
+        // instead of 32 rows of one element each, 32 cycles of the load / store
+        // unit per instruction (o=12/v=63 step, 413 MB of W: 666 -> 459 us;
+        // rows that are contiguous already store directly)
+        double(*buf)[9] = sm.out[warp - 2];
+        const int c = lane & 7;
+        const long long ro = mlive ? roff : -1;
+#pragma unroll
+        for (int h8 = 0; h8 < 2; ++h8) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) buf[lane][j] = result(8 * h8 + j);
+          __syncwarp();
+          double* cp = tab[8 * h8 + c].colp;
+          double* p[8];
+          double old[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const long long o = __shfl_sync(0xffffffffu, ro, 4 * i + (lane >> 3));
+            p[i] = cp && o >= 0 ? cp + o : nullptr;
+            old[i] = acc && p[i] ? *p[i] : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const double x = buf[4 * i + (lane >> 3)][c];
+            if (p[i]) *p[i] = acc ? old[i] + x : x;
+          }
+          __syncwarp();
+        }
       }
     }
   }
