@@ -93,9 +93,20 @@ struct GemmPlan {
 int build_gemm_plan(const int* ptrn, int lrank, const int* lext, int rrank, const int* rext,
                     int drank, const int* dext, GemmPlan* p);
 
+// How a plain FP64 contraction is divided (kernels_dmma.cu): tile rows and
+// columns in 8s, and the CTAs that share a tile's k steps.
+struct F64Form {
+  int h = 4, w = 4, cluster = 1;
+};
+struct F64Shape {
+  int64_t M, N, steps, count;  // steps: 16 k each, summed over the pairs; count: destinations like this
+};
+F64Form f64_form(const std::vector<F64Shape>& shapes, int sms);
+
 // Device copy of a plan's tables (cached by pattern + extents).
 struct DevPlan {
   GemmPlan host;
+  F64Form f64;
   int64_t* d_tables = nullptr;  // offLm | offLk | offRk | offRn | offDm | offDn
   const int64_t *offLm, *offLk, *offRk, *offRn, *offDm, *offDn;
 };
@@ -142,6 +153,7 @@ int launch_energy_contract(int rank0, const int* off, const int* ext0, const int
 int launch_denominator(int rank0, const int* off, const int* ext0, double* data, int rank1,
                        int ld1, const double* e_or_fock, cudaStream_t s);
 // Permute-fused FP64 contraction (kernels_dmma.cu).
+int launch_copy_two(const double* a, double* da, int64_t na, const double* b, double* db, int64_t nb, cudaStream_t s);
 int launch_contract_f64(const DevPlan* p, const double* L, const double* R, double* D, int beta,
                         cudaStream_t s);
 // Scalar cases of tensor_block_contract_ (kernels_block.cu).

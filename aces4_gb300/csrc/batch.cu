@@ -9,6 +9,7 @@
 // is one call: pairs that feed the same destination block are summed in the
 // kernel, zero blocks (NULL operand) are never touched.
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -59,13 +60,9 @@ struct a4g_batch {
   GroupedF64Tile* d_f64_tiles = nullptr;
   GroupedPair* d_f64_pairs = nullptr;
   int n_f64_tiles = 0;
-  double* d_f64_ws = nullptr;           // partial tiles when tiles are spread
-  GroupedF64Reduce* d_f64_reds = nullptr;
-  int n_f64_reds = 0;
-  int f64_tile_m = 64, f64_tile_n = 64;  // rows (64 or 48) and columns (64 or 32) of a grouped FP64 tile
+  int f64_cluster = 1;  // CTAs that share a tile's k steps
   std::vector<GroupedF64Tile> h_f64_tiles;
   std::vector<GroupedPair> h_f64_pairs;
-  std::vector<GroupedF64Reduce> h_f64_reds;
   // split precision
   OzPanel* d_pa = nullptr;
   OzPanel* d_pb = nullptr;
@@ -275,15 +272,6 @@ void release(a4g_batch* b, void* p, size_t bytes) {
   cudaFree(p);
 }
 
-PlanRef ref_of(const DevPlan* p) {
-  PlanRef r;
-  r.offLm = p->offLm, r.offLk = p->offLk, r.offRk = p->offRk, r.offRn = p->offRn;
-  r.offDm = p->offDm, r.offDn = p->offDn;
-  r.M = int(p->host.M), r.N = int(p->host.N), r.K = int(p->host.K);
-  r.a_kfast = p->host.a_kfast, r.b_kfast = p->host.b_kfast;
-  return r;
-}
-
 struct Pair {
   const double* l;
   const double* r;
@@ -460,57 +448,53 @@ Panels lay_panels(const std::vector<DGroup>& groups, const std::vector<const Dev
 }
 
 int build_f64(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector<const DevPlan*>& plans) {
-  std::vector<GroupedF64Tile> tiles;
   std::vector<GroupedPair> pairs;
-  int64_t max_n = 0, pad64 = 0, pad48 = 0;
-  for (const DGroup& g : groups) {
-    const int64_t M = plans[g.plan]->host.M;
-    max_n = std::max(max_n, plans[g.plan]->host.N);
-    pad64 += (M + 63) / 64 * 64, pad48 += (M + 47) / 48 * 48;
+  std::vector<F64Shape> shapes;
+  std::map<std::array<int64_t, 3>, size_t> shape_of;
+  std::vector<int64_t> total(groups.size(), 0);  // k steps of each destination
+  auto steps_of = [&](const Pair& p) { return (plans[p.plan]->host.K + 15) / 16; };
+  for (size_t i = 0; i < groups.size(); ++i) {
+    const GemmPlan& h = plans[groups[i].plan]->host;
+    for (const Pair& p : groups[i].pairs) total[i] += steps_of(p);
+    auto it = shape_of.emplace(std::array<int64_t, 3>{h.M, h.N, total[i]}, shapes.size());
+    if (it.second) shapes.push_back({h.M, h.N, total[i], 0});
+    ++shapes[it.first->second].count;
   }
-  const int TM = grouped_f64_tile_m(pad64, pad48), TN = grouped_f64_tile_n(int(std::min<int64_t>(max_n, 1 << 30)));
-  b->f64_tile_m = TM, b->f64_tile_n = TN;
-  for (const DGroup& g : groups) {
+  const F64Form f = f64_form(shapes, ctx()->num_sms > 0 ? ctx()->num_sms : 152);
+  std::vector<GroupedF64Tile> tiles;
+  for (size_t i = 0; i < groups.size(); ++i) {
+    const DGroup& g = groups[i];
     const int begin = int(pairs.size());
     for (const Pair& p : g.pairs) pairs.push_back({p.l, p.r, p.plan, 0});
-    const int end = int(pairs.size());
-    const GemmPlan& h = plans[g.plan]->host;
-    for (int64_t n0 = 0; n0 < h.N; n0 += TN)
-      for (int64_t m0 = 0; m0 < h.M; m0 += TM)
-        tiles.push_back({g.d, int(m0), int(n0), begin, end, g.plan, -1});
-  }
-  // Few tiles with many pairs each (small blocks, long sums): spread each
-  // tile's pairs over G CTAs writing partial tiles, summed in order after.
-  const int sms = ctx()->num_sms > 0 ? ctx()->num_sms : 152;
-  const int64_t want = 4LL * sms;
-  int min_pairs = 1 << 30;
-  for (const auto& t : tiles) min_pairs = std::min(min_pairs, t.pair_end - t.pair_begin);
-  const int G = tiles.empty() ? 1
-                              : int(std::max<int64_t>(1, std::min<int64_t>({16, int64_t(min_pairs),
-                                                                            (want + int64_t(tiles.size()) - 1) /
-                                                                                int64_t(tiles.size())})));
-  if (G > 1) {
-    std::vector<GroupedF64Tile> spread;
-    std::vector<GroupedF64Reduce> reds;
-    int slot = 0;
-    for (const auto& t : tiles) {
-      const int np = t.pair_end - t.pair_begin;
-      reds.push_back({t.d, t.m0, t.n0, t.dplan, slot, G, 0});
-      for (int q = 0; q < G; ++q)
-        spread.push_back({t.d, t.m0, t.n0, t.pair_begin + np * q / G, t.pair_begin + np * (q + 1) / G, t.dplan,
-                          slot++});
+    // the shares: ranges of the pairs' k steps laid end to end
+    struct Share {
+      int pb, pe, ks0, ks1;
+    };
+    std::vector<Share> shares;
+    for (int q = 0; q < f.cluster; ++q) {
+      const int64_t lo = total[i] * q / f.cluster, hi = total[i] * (q + 1) / f.cluster;
+      Share sh{begin, begin, 0, 0};
+      int64_t at = 0;
+      for (size_t k = 0; k < g.pairs.size() && lo < hi; ++k) {
+        const int64_t n = steps_of(g.pairs[k]);
+        if (lo >= at && lo < at + n) sh.pb = begin + int(k), sh.ks0 = int(lo - at);
+        if (hi > at && hi <= at + n) sh.pe = begin + int(k) + 1, sh.ks1 = int(hi - at);
+        at += n;
+      }
+      shares.push_back(sh);
     }
-    void* ws = nullptr;
-    int rc = device_alloc(b, size_t(slot) * TM * TN * sizeof(double), &ws, false);
-    if (rc) return rc;
-    b->d_f64_ws = static_cast<double*>(ws);
-    if ((rc = upload(b, reds, &b->d_f64_reds))) return rc;
-    b->n_f64_reds = int(reds.size());
-    b->h_f64_reds = reds;
-    tiles.swap(spread);
+    const GemmPlan& h = plans[g.plan]->host;
+    const int64_t um = (h.M + 7) / 8, un = (h.N + 7) / 8, tm = (um + f.h - 1) / f.h, tn = (un + f.w - 1) / f.w;
+    for (int64_t n = 0; n < tn; ++n)
+      for (int64_t m = 0; m < tm; ++m) {
+        const int u0 = int(um * m / tm), u1 = int(um * (m + 1) / tm), v0 = int(un * n / tn), v1 = int(un * (n + 1) / tn);
+        for (const Share& sh : shares)
+          tiles.push_back({g.d, 8 * u0, 8 * v0, u1 - u0, v1 - v0, sh.pb, sh.pe, sh.ks0, sh.ks1, g.plan, 0});
+      }
   }
   if (tiles.size() > 0x7fffffffu) return fail(A4G_ERR_RANGE, "too many tiles");
   b->n_f64_tiles = int(tiles.size());
+  b->f64_cluster = f.cluster;
   int rc = upload(b, tiles, &b->d_f64_tiles);
   if (!rc) rc = upload(b, pairs, &b->d_f64_pairs);
   b->h_f64_tiles = tiles;
@@ -1269,7 +1253,7 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
 }
 
 static_assert(sizeof(OzSplitJob) % 8 == 0 && sizeof(OzDBlock) % 8 == 0 && sizeof(GroupedPair) % 8 == 0 &&
-                  sizeof(GroupedF64Tile) % 8 == 0 && sizeof(GroupedF64Reduce) % 8 == 0,
+                  sizeof(GroupedF64Tile) % 8 == 0,
               "tables are copied in 8-byte words");
 
 // Zeroes the exponents of the A panels (side 0) and/or the B panels (side 1).
@@ -1321,8 +1305,8 @@ int run(a4g_batch* b, cudaStream_t s, const cudaEvent_t* ev = nullptr) {
   if ((rc = mark(1))) return rc;
   if (b->precision == A4G_PREC_FP64) {
     if ((rc = mark(2)) || (rc = mark(3))) return rc;
-    rc = launch_grouped_f64(b->d_f64_tiles, b->n_f64_tiles, b->d_f64_pairs, b->d_plans, b->store_mode(),
-                            b->d_f64_ws, b->d_f64_reds, b->n_f64_reds, b->f64_tile_m, b->f64_tile_n, s);
+    rc = launch_grouped_f64(b->d_f64_tiles, b->n_f64_tiles, b->f64_cluster, b->d_f64_pairs, b->d_plans,
+                            b->store_mode(), s);
     if (rc) return rc;
     if ((rc = mark(4)) || (rc = mark(5))) return rc;
     return A4G_OK;
@@ -1466,7 +1450,7 @@ static int create_batch(a4g_batch** out, const int* ptrn, int drank, int lrank, 
     }
   }
   std::vector<PlanRef> refs;
-  for (const DevPlan* p : plans) refs.push_back(ref_of(p));
+  for (const DevPlan* p : plans) refs.push_back(plan_ref(*p));
   if ((rc = upload(b.get(), refs, &b->d_plans))) return rc;
   rc = b->precision == A4G_PREC_FP64 ? build_f64(b.get(), groups, plans)
                                      : build_ozaki(b.get(), groups, plans, order[b->swapped ? 0 : 1], ptrn, allow_residue);
@@ -1562,7 +1546,6 @@ int a4g_batch_launches(const a4g_batch* b, int* kernels_per_run, int* gemm_parts
   int parts = 1;
   if (b->precision == A4G_PREC_FP64) {
     k += b->n_f64_tiles > 0 ? 1 : 0;
-    k += b->n_f64_reds > 0 ? 1 : 0;
   } else if (b->forms[b->form].n_tiles > 0) {
     parts = b->parts;
     std::set<int> groups;  // one split launch per pipeline group; a held side's job sets are not run
@@ -1642,8 +1625,7 @@ int a4g_batch_rebind(a4g_batch* b, const a4g_triple* trip, int64_t n, void* stre
   // (runs queued before on `stream` still read the old tables)
   size_t total = 0;
   if (b->precision == A4G_PREC_FP64) {
-    total = b->h_f64_pairs.size() * sizeof(GroupedPair) + b->h_f64_tiles.size() * sizeof(GroupedF64Tile) +
-            b->h_f64_reds.size() * sizeof(GroupedF64Reduce);
+    total = b->h_f64_pairs.size() * sizeof(GroupedPair) + b->h_f64_tiles.size() * sizeof(GroupedF64Tile);
   } else {
     for (const auto& js : b->jobsets) total += js.h_jobs.size() * sizeof(OzSplitJob);
     total += b->h_dblocks.size() * sizeof(OzDBlock) + b->h_colptr.size() * sizeof(double*);
@@ -1654,19 +1636,15 @@ int a4g_batch_rebind(a4g_batch* b, const a4g_triple* trip, int64_t n, void* stre
   if (b->precision == A4G_PREC_FP64) {
     std::vector<GroupedPair> pairs = b->h_f64_pairs;
     std::vector<GroupedF64Tile> tiles = b->h_f64_tiles;
-    std::vector<GroupedF64Reduce> reds = b->h_f64_reds;
     for (auto& p : pairs)
       p.l = static_cast<const double*>(mp(p.l)), p.r = static_cast<const double*>(mp(p.r));
     for (auto& t : tiles) t.d = const_cast<double*>(static_cast<const double*>(mp(t.d)));
-    for (auto& r : reds) r.d = const_cast<double*>(static_cast<const double*>(mp(r.d)));
     if ((rc = put(b->d_f64_pairs, pairs.data(), pairs.size() * sizeof(GroupedPair))) ||
         (rc = put(b->d_f64_tiles, tiles.data(), tiles.size() * sizeof(GroupedF64Tile))) ||
-        (rc = put(b->d_f64_reds, reds.data(), reds.size() * sizeof(GroupedF64Reduce))) ||
         (rc = b->stage.launch(s)))
       return rc;
     b->h_f64_pairs.swap(pairs);
     b->h_f64_tiles.swap(tiles);
-    b->h_f64_reds.swap(reds);
   } else {
     std::vector<std::vector<OzSplitJob>> jobs(b->jobsets.size());
     for (size_t i = 0; i < b->jobsets.size(); ++i) {

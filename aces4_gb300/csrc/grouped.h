@@ -5,6 +5,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "a4g_internal.h"
+
 namespace a4g {
 
 // Device copy of one contraction plan's address tables (see GemmPlan).
@@ -14,6 +16,15 @@ struct PlanRef {
   int a_kfast, b_kfast;
 };
 
+inline PlanRef plan_ref(const DevPlan& p) {
+  PlanRef r;
+  r.offLm = p.offLm, r.offLk = p.offLk, r.offRk = p.offRk, r.offRn = p.offRn;
+  r.offDm = p.offDm, r.offDn = p.offDn;
+  r.M = int(p.host.M), r.N = int(p.host.N), r.K = int(p.host.K);
+  r.a_kfast = p.host.a_kfast, r.b_kfast = p.host.b_kfast;
+  return r;
+}
+
 // ------------------------------------------------------------ FP64 grouped
 struct GroupedPair {
   const double* l;
@@ -21,30 +32,19 @@ struct GroupedPair {
   int plan;
   int pad;
 };
+// One CTA's share of a destination tile: rows m0.. (mi 8s), columns n0.. (nu
+// 8s), the k steps (of 16) from ks0 of pair pair_begin to ks1 of pair
+// pair_end - 1.  A tile's shares follow each other and make a cluster.
 struct GroupedF64Tile {
   double* d;
-  int m0, n0;
-  int pair_begin, pair_end;  // pairs summed into this tile
-  int dplan;                 // plan giving D's tables and M, N
-  int slot;                  // -1: store into D; else the partial-tile slot in the workspace
-};
-// Destination tiles whose pairs were spread over several CTAs: the partial
-// tiles in slots [slot0, slot0 + nparts) are summed in order and stored.
-struct GroupedF64Reduce {
-  double* d;
-  int m0, n0;
-  int dplan;
-  int slot0, nparts;
+  int m0, n0, mi, nu;
+  int pair_begin, pair_end, ks0, ks1;
+  int dplan;  // plan giving D's tables and M, N
   int pad;
 };
-// mode: bit 0 accumulate, bit 1 negate; tile_m: 64 or 48 (grouped_f64_tile_m), tile_n: 64 or 32
-// (grouped_f64_tile_n)
-int launch_grouped_f64(const GroupedF64Tile* tiles, int ntiles, const GroupedPair* pairs, const PlanRef* plans,
-                       int mode, double* ws, const GroupedF64Reduce* reds, int nreds, int tile_m, int tile_n,
-                       cudaStream_t s);
-// tile rows given the destination rows padded to 64- and to 48-row tiles (summed over the blocks)
-int grouped_f64_tile_m(int64_t padded64, int64_t padded48);
-int grouped_f64_tile_n(int max_n);  // tile columns for destination blocks of at most max_n columns
+// mode: bit 0 accumulate, bit 1 negate
+int launch_grouped_f64(const GroupedF64Tile* tiles, int ntiles, int cluster, const GroupedPair* pairs,
+                       const PlanRef* plans, int mode, cudaStream_t s);
 
 // ------------------------------------------------------------ split precision
 // A panel holds the BF16 slices of every left block that feeds one group of

@@ -803,11 +803,38 @@ __global__ void scalar_scalar_kernel(const double* l, const double* r, double* d
   *d = beta ? __dadd_rn(*d, v) : v;
 }
 
+// Two blocks copied side by side, each thread with four loads in flight: the
+// blocks are in host memory and the link's latency, not its rate, is to cover.
+__global__ void __launch_bounds__(256) copy_two_kernel(const double* __restrict__ a, double* __restrict__ da, int64_t na,
+                                                       const double* __restrict__ b, double* __restrict__ db, int64_t nb) {
+  constexpr int kLoads = 4;
+  const int64_t threads = int64_t(gridDim.x) * blockDim.x, n = na + nb;
+  for (int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i0 < n; i0 += kLoads * threads) {
+    double x[kLoads];
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      const int64_t i = i0 + q * threads;
+      if (i < n) x[q] = i < na ? a[i] : b[i - na];
+    }
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      const int64_t i = i0 + q * threads;
+      if (i < n) (i < na ? da[i] : db[i - na]) = x[q];
+    }
+  }
+}
+
 }  // namespace
 
 // ============================================================== launchers
 int launch_fill(double* d, int64_t n, double v, cudaStream_t s) {
   return launch_ew<EwOp::kFill>(d, nullptr, n, v, s);
+}
+int launch_copy_two(const double* a, double* da, int64_t na, const double* b, double* db, int64_t nb, cudaStream_t s) {
+  const int64_t want = (na + nb + 1023) / 1024, most = int64_t(ctx()->num_sms > 0 ? ctx()->num_sms : 152) * 8;
+  copy_two_kernel<<<unsigned(std::max<int64_t>(1, std::min(want, most))), 256, 0, s>>>(a, da, na, b, db, nb);
+  A4G_CUDA(cudaGetLastError());
+  return A4G_OK;
 }
 int launch_scale(double* d, int64_t n, double f, cudaStream_t s) {
   return launch_ew<EwOp::kScale>(d, nullptr, n, f, s);

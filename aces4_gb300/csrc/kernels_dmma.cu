@@ -5,17 +5,31 @@
 // so no transposed copy of L, R or D is ever written (the reference allocates
 // and fills transposed temporaries, tensor_dil_omp.F90:729-751, 782-785).
 //
-// CTA tile 64 or 48 rows x 64 or 32 columns (the smaller forms for small or
-// narrow destinations), k-step 16, 128 threads (2x2 warps, BM/16 x BN/16
-// m8n8k4 DMMA tiles per warp).  Tiles are gathered through the offset tables into
-// registers, then staged in double-buffered shared memory.  FP64 throughput on
-// GB300 is ~2 FMA/clk/SM, so the kernel is bound by the FP64 pipe; the gather
-// traffic is small in comparison.
+// The FP64 pipes bound both forms (1.046 TFLOP/s of m8n8k4 and 1.005 of FMAs
+// measured with all four of an SM's quarters busy, a quarter of that from one
+// warp), the gathers are small beside them.  So a tile pays for what lives in
+// it and no more, and every SM gets the same share:
+//   - a CTA holds at most 32 x 32 results as 8 x 8 DMMA tiles and runs only the
+//     live ones; up to 4 columns beyond the last whole 8 run as FMAs, a row per
+//     lane, where that is less than another DMMA column (25 columns cost 25);
+//   - its four warps share every k step (16 k, 4 each) and not the tile, so
+//     they stay equal whatever the tile's shape, and add up once at the end;
+//   - a cluster of 1, 2, 4 or 8 CTAs divides a tile's k steps and adds its
+//     partial tiles through distributed shared memory in rank order: one
+//     launch, no workspace, the same bits on every run.
+// Rows, columns and cluster size come from a model of the makespan (f64_form).
+// Against 64 x 64 (48, 32) tiles padded to their edges, 2 x 2 warps a tile, and
+// partial tiles through a workspace and a second launch: a 660 x 580 x 580 pair
+// 715 -> 502 us (425 at the pipes' rate), the o=10/v=48 step 1488 -> 1124 us
+// (1013), 108 x 96 x 96 pairs 43 -> 12 us.
 //
-// The grouped form runs a whole pardo step: one CTA owns one 64x64 tile of one
+// The grouped form runs a whole pardo step: one cluster owns one tile of one
 // destination block and sums the products of every block pair that feeds that
 // block (the contract-accumulate the interpreter lacks), then writes D once.
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <cmath>
 
 #include "a4g_internal.h"
 #include "grouped.h"
@@ -23,8 +37,12 @@
 namespace a4g {
 namespace {
 
-constexpr int BK = 16;
+namespace cg = cooperative_groups;
+
+constexpr int BK = 16;      // a k step: 4 k for each of the four warps
+constexpr int kStage = 32;  // k staged at a time
 constexpr int kThreadsF64 = 128;
+constexpr int kTile = 32;  // rows and columns of the largest tile
 
 __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -32,312 +50,313 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// Element e = threadIdx.x + 128 i of a ROWS x 16 operand tile: with the
+// Element e = threadIdx.x + 128 i of a 32 x kStage operand tile: with the
 // operand unit-stride along k (kfast) threads walk k fastest, else the rows.
-template <int ROWS>
 __device__ __forceinline__ void tile_coord(bool kfast, int e, int& r, int& kk) {
-  if (kfast) kk = e & (BK - 1), r = e >> 4;
-  else r = e % ROWS, kk = e / ROWS;
+  if (kfast) kk = e % kStage, r = e / kStage;
+  else r = e & 31, kk = e >> 5;
 }
 
-// Gathers one ROWS x 16 operand tile (rows x k) into ROWS/8 registers per thread.
-template <int ROWS>
-__device__ __forceinline__ void gather_tile(bool kfast, double (&reg)[ROWS / 8], const double* __restrict__ X,
+// Gathers one 32 x kStage operand tile (rows x k from k0, below kend).
+__device__ __forceinline__ void gather_tile(bool kfast, double (&reg)[kStage / 4], const double* __restrict__ X,
                                             const int64_t* __restrict__ offRow,  // smem, per row
                                             const int64_t* __restrict__ offK,    // global, per k
-                                            int rows_left, int k0, int K) {
+                                            int rows, int k0, int kend) {
 #pragma unroll
-  for (int i = 0; i < ROWS / 8; ++i) {
+  for (int i = 0; i < kStage / 4; ++i) {
     int r, kk;
-    tile_coord<ROWS>(kfast, int(threadIdx.x) + kThreadsF64 * i, r, kk);
+    tile_coord(kfast, int(threadIdx.x) + kThreadsF64 * i, r, kk);
     const int k = k0 + kk;
-    reg[i] = (r < rows_left && k < K) ? __ldg(&X[offRow[r] + __ldg(&offK[k])]) : 0.0;
+    reg[i] = (r < rows && k < kend) ? __ldg(&X[offRow[r] + __ldg(&offK[k])]) : 0.0;
   }
 }
 
-template <int ROWS, int LD>
-__device__ __forceinline__ void store_tile(bool kfast, double (*S)[LD], const double (&reg)[ROWS / 8]) {
+__device__ __forceinline__ void store_tile(bool kfast, double (*S)[kTile + 4], const double (&reg)[kStage / 4]) {
 #pragma unroll
-  for (int i = 0; i < ROWS / 8; ++i) {
+  for (int i = 0; i < kStage / 4; ++i) {
     int r, kk;
-    tile_coord<ROWS>(kfast, int(threadIdx.x) + kThreadsF64 * i, r, kk);
+    tile_coord(kfast, int(threadIdx.x) + kThreadsF64 * i, r, kk);
     S[kk][r] = reg[i];
   }
 }
 
-// Tile BM x BN: BM 64 or 48 rows (48 when it cuts the row padding: the small
-// ladder's 144 rows are three 48-row tiles, 75 % of three 64-row ones), BN
-// 64 or 32 columns (32 for narrow destinations: the ladder's i,j extent of 25
-// fills 78 % of a 32-column tile, 39 % of a 64-column one).  4 warps as 2 x 2,
-// each (BM/2) x (BN/2) = BM/16 x BN/16 m8n8k4 DMMA tiles.
-template <int BM, int BN>
-struct Smem {
-  double As[2][BK][BM + 4];  // +4 doubles: conflict-free fragment reads
-  double Bs[2][BK][BN + 4];
-  int64_t sLm[BM], sRn[BN];
+// FMA columns that `part` live columns beyond a tile's whole 8s run as (1, 2 or
+// 4), or 0 where another DMMA column costs less.
+__host__ __device__ inline int f64_fma_cols(int part, int mi) {
+  const int c = part == 3 ? 4 : part;
+  return c <= 4 && c < 2 * mi ? c : 0;
+}
+
+struct F64Smem {
+  union {
+    struct {
+      double As[2][kStage][kTile + 4];  // +4 doubles: conflict-free fragment reads
+      double Bs[2][kStage][kTile + 4];
+    };
+    double part[kThreadsF64 / 32][kTile][kTile + 2];  // each warp's share of the tile, column-major
+  };
+  int64_t sLm[kTile], sRn[kTile];
 };
 
-template <int BM, int BN>
-struct Acc {
-  double v[BM / 16][BN / 16][2];
-  __device__ __forceinline__ void zero() {
+// The first MI rows of 8 of a tile, one k4.  A body of its own per MI: a DMMA
+// that is predicated off takes its slot in the pipe all the same.
+template <int MI, int NJ>
+__device__ __forceinline__ void mma_rows(double (&acc)[kTile / 8][NJ][2], const double* a, const double* b) {
+  double bf[NJ];
 #pragma unroll
-    for (int i = 0; i < BM / 16; ++i)
+  for (int j = 0; j < NJ; ++j) bf[j] = b[8 * j];
 #pragma unroll
-      for (int j = 0; j < BN / 16; ++j) v[i][j][0] = v[i][j][1] = 0.0;
-  }
-};
-
-// acc += L_tile * R_tile over the k steps [ks0, ks1) (16 k each) of one pair.
-template <int BM, int BN>
-__device__ void accumulate_pair(Smem<BM, BN>& sm, Acc<BM, BN>& acc, const double* __restrict__ L,
-                                const double* __restrict__ R, const int64_t* __restrict__ offLm,
-                                const int64_t* __restrict__ offLk, const int64_t* __restrict__ offRk,
-                                const int64_t* __restrict__ offRn, int M, int N, int K, int m0, int n0,
-                                bool a_kfast, bool b_kfast, int ks0, int ks1) {
-  const int t = threadIdx.x;
-  __syncthreads();  // previous pair done with the tables / tiles
-  if (t < BM) sm.sLm[t] = (m0 + t < M) ? offLm[m0 + t] : 0;
-  if (t < BN) sm.sRn[t] = (n0 + t < N) ? offRn[n0 + t] : 0;
-  __syncthreads();
-  if (ks0 >= ks1) return;
-
-  const int warp = t >> 5, lane = t & 31;
-  const int g = lane >> 2, tig = lane & 3;
-  const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
-  double ra[BM / 8], rb[BN / 8];
-  gather_tile<BM>(a_kfast, ra, L, sm.sLm, offLk, M - m0, ks0 * BK, K);
-  gather_tile<BN>(b_kfast, rb, R, sm.sRn, offRk, N - n0, ks0 * BK, K);
-  store_tile<BM, BM + 4>(a_kfast, sm.As[0], ra);
-  store_tile<BN, BN + 4>(b_kfast, sm.Bs[0], rb);
-  __syncthreads();
-  for (int ks = ks0; ks < ks1; ++ks) {
-    const int cur = (ks - ks0) & 1;
-    if (ks + 1 < ks1) {
-      gather_tile<BM>(a_kfast, ra, L, sm.sLm, offLk, M - m0, (ks + 1) * BK, K);
-      gather_tile<BN>(b_kfast, rb, R, sm.sRn, offRk, N - n0, (ks + 1) * BK, K);
-    }
+  for (int i = 0; i < MI; ++i) {
+    const double af = a[8 * i];
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      double af[BM / 16], bf[BN / 16];
-#pragma unroll
-      for (int i = 0; i < BM / 16; ++i) af[i] = sm.As[cur][kk + tig][wm + i * 8 + g];
-#pragma unroll
-      for (int j = 0; j < BN / 16; ++j) bf[j] = sm.Bs[cur][kk + tig][wn + j * 8 + g];
-#pragma unroll
-      for (int i = 0; i < BM / 16; ++i)
-#pragma unroll
-        for (int j = 0; j < BN / 16; ++j) dmma_8x8x4(acc.v[i][j], af[i], bf[j]);
-    }
-    if (ks + 1 < ks1) {
-      store_tile<BM, BM + 4>(a_kfast, sm.As[cur ^ 1], ra);
-      store_tile<BN, BN + 4>(b_kfast, sm.Bs[cur ^ 1], rb);
-    }
-    __syncthreads();
+    for (int j = 0; j < NJ; ++j) dmma_8x8x4(acc[i][j], af, bf[j]);
   }
 }
 
-// mode bit 0: accumulate into D (beta = 1), bit 1: store the negated sum.
-template <int BM, int BN>
-__device__ void write_tile(const Acc<BM, BN>& acc, double* __restrict__ D, const int64_t* __restrict__ offDm,
-                           const int64_t* __restrict__ offDn, int M, int N, int m0, int n0, int mode) {
+// part = sum over the k steps [ks0 of pair pb, ks1 of pair pe - 1) of the
+// tile's rows m0.. (mi DMMA tiles) and columns n0.. (NJ DMMA tiles, then up to
+// NREM columns of FMAs, nrem of them live).  Warp w takes k = 4w..4w+3 of each
+// step.  NREM is a template parameter for the same reason.
+template <int NJ, int NREM>
+__device__ void accumulate_tile(F64Smem& sm, const GroupedPair* __restrict__ pairs, const PlanRef* __restrict__ plans,
+                                int pb, int pe, int ks0, int ks1, int m0, int n0, int mi, int nrem) {
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int g = lane >> 2, tig = lane & 3;
-  const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
+  double acc[kTile / 8][NJ ? NJ : 1][2];
+  double rem[NREM ? NREM : 1];
 #pragma unroll
-  for (int i = 0; i < BM / 16; ++i) {
-    const int m = m0 + wm + i * 8 + g;
-    if (m >= M) continue;
-    const int64_t om = offDm[m];
+  for (int i = 0; i < kTile / 8; ++i)
 #pragma unroll
-    for (int j = 0; j < BN / 16; ++j) {
+    for (int j = 0; j < (NJ ? NJ : 1); ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int n = n0 + wn + j * 8 + 2 * tig + h;
-        if (n >= N) continue;
-        double* p = &D[om + offDn[n]];
-        const double v = (mode & 2) ? -acc.v[i][j][h] : acc.v[i][j][h];
-        *p = (mode & 1) ? *p + v : v;
-      }
-    }
-  }
-}
+  for (int c = 0; c < (NREM ? NREM : 1); ++c) rem[c] = 0.0;
 
-// A partial tile, column-major BM x BN, into workspace slot `slot`.
-template <int BM, int BN>
-__device__ void write_partial(const Acc<BM, BN>& acc, double* __restrict__ ws, int64_t slot) {
-  double* w = ws + slot * BM * BN;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int g = lane >> 2, tig = lane & 3;
-  const int wm = (warp & 1) * (BM / 2), wn = (warp >> 1) * (BN / 2);
-#pragma unroll
-  for (int i = 0; i < BM / 16; ++i)
-#pragma unroll
-    for (int j = 0; j < BN / 16; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) w[(wn + j * 8 + 2 * tig + h) * BM + wm + i * 8 + g] = acc.v[i][j][h];
-}
-
-// One block pair.  CTA x = tile + tiles * split: with nsplit == 1 each CTA
-// computes a whole tile and stores it; otherwise each computes the tile over
-// its share of the k steps and writes a partial tile to the workspace, which
-// contract_f64_reduce_kernel sums in split order.  FP64 runs at a few FMA per
-// clock per SM on this GPU, so a small block (the ladder's 144 x 25 x 144)
-// needs its k range spread over many SMs to finish in microseconds.
-template <int BM, int BN>
-__global__ void __launch_bounds__(kThreadsF64) contract_f64_kernel(
-    const double* __restrict__ L, const double* __restrict__ R, double* __restrict__ D,
-    const int64_t* __restrict__ offLm, const int64_t* __restrict__ offLk,
-    const int64_t* __restrict__ offRk, const int64_t* __restrict__ offRn,
-    const int64_t* __restrict__ offDm, const int64_t* __restrict__ offDn, int M, int N, int K,
-    int tiles_m, int tiles, int nsplit, int mode, int a_kfast, int b_kfast, double* __restrict__ ws) {
-  __shared__ __align__(16) Smem<BM, BN> sm;
-  const int tile = blockIdx.x % tiles, split = blockIdx.x / tiles;
-  const int tm = tile % tiles_m, tn = tile / tiles_m;
-  const int m0 = tm * BM, n0 = tn * BN;
-  const int ksteps = (K + BK - 1) / BK;
-  const int ks0 = int(int64_t(ksteps) * split / nsplit), ks1 = int(int64_t(ksteps) * (split + 1) / nsplit);
-  Acc<BM, BN> acc;
-  acc.zero();
-  accumulate_pair<BM, BN>(sm, acc, L, R, offLm, offLk, offRk, offRn, M, N, K, m0, n0, a_kfast, b_kfast, ks0,
-                          ks1);
-  if (nsplit > 1) write_partial<BM, BN>(acc, ws, blockIdx.x);
-  else write_tile<BM, BN>(acc, D, offDm, offDn, M, N, m0, n0, mode);
-}
-
-// Sums tile `blockIdx.x`'s nsplit partials (slots tile + tiles * split) in
-// split order and stores it: the same bits on every run.
-template <int BM, int BN>
-__global__ void __launch_bounds__(256) contract_f64_reduce_kernel(const double* __restrict__ ws, int tiles,
-                                                                  int nsplit, int tiles_m, double* __restrict__ D,
-                                                                  const int64_t* __restrict__ offDm,
-                                                                  const int64_t* __restrict__ offDn, int M, int N,
-                                                                  int mode) {
-  const int tile = blockIdx.x, tm = tile % tiles_m, tn = tile / tiles_m;
-  for (int e = threadIdx.x; e < BM * BN; e += blockDim.x) {
-    const int ml = e % BM, nl = e / BM;
-    const int m = tm * BM + ml, n = tn * BN + nl;
-    if (m >= M || n >= N) continue;
-    double v = 0.0;
-    for (int q = 0; q < nsplit; ++q) v += ws[(int64_t(tile) + int64_t(tiles) * q) * BM * BN + e];
-    if (mode & 2) v = -v;
-    double* p = D + offDm[m] + offDn[n];
-    *p = (mode & 1) ? *p + v : v;
-  }
-}
-
-// One CTA per (destination block, tile, share of its pairs); the pairs are
-// summed and the tile stored into D, or into a workspace slot when the tile's
-// pairs are spread over several CTAs (few tiles, many pairs).
-template <int BM, int BN>
-__global__ void __launch_bounds__(kThreadsF64) grouped_f64_kernel(const GroupedF64Tile* __restrict__ tiles,
-                                                                  const GroupedPair* __restrict__ pairs,
-                                                                  const PlanRef* __restrict__ plans,
-                                                                  int mode, double* __restrict__ ws) {
-  __shared__ __align__(16) Smem<BM, BN> sm;
-  const GroupedF64Tile tl = tiles[blockIdx.x];
-  Acc<BM, BN> acc;
-  acc.zero();
-  for (int q = tl.pair_begin; q < tl.pair_end; ++q) {
+  for (int q = pb; q < pe; ++q) {
     const GroupedPair pr = pairs[q];
     const PlanRef pl = plans[pr.plan];
-    accumulate_pair<BM, BN>(sm, acc, pr.l, pr.r, pl.offLm, pl.offLk, pl.offRk, pl.offRn, pl.M, pl.N, pl.K,
-                            tl.m0, tl.n0, pl.a_kfast, pl.b_kfast, 0, (pl.K + BK - 1) / BK);
+    const int kend = q == pe - 1 ? min(pl.K, ks1 * BK) : pl.K;
+    const int rows = min(pl.M - m0, 8 * mi), cols = min(pl.N - n0, 8 * NJ + nrem);
+    int kb = q == pb ? ks0 * BK : 0;
+    __syncthreads();  // previous pair done with the tables / tiles
+    if (t < kTile) sm.sLm[t] = t < rows ? pl.offLm[m0 + t] : 0;
+    else if (t < 2 * kTile) sm.sRn[t - kTile] = t - kTile < cols ? pl.offRn[n0 + t - kTile] : 0;
+    __syncthreads();
+    if (kb >= kend) continue;
+    double ra[kStage / 4], rb[kStage / 4];
+    gather_tile(pl.a_kfast, ra, pr.l, sm.sLm, pl.offLk, rows, kb, kend);
+    gather_tile(pl.b_kfast, rb, pr.r, sm.sRn, pl.offRk, cols, kb, kend);
+    store_tile(pl.a_kfast, sm.As[0], ra);
+    store_tile(pl.b_kfast, sm.Bs[0], rb);
+    __syncthreads();
+    for (int cur = 0; kb < kend; kb += kStage, cur ^= 1) {
+      const bool more = kb + kStage < kend;
+      if (more) {
+        gather_tile(pl.a_kfast, ra, pr.l, sm.sLm, pl.offLk, rows, kb + kStage, kend);
+        gather_tile(pl.b_kfast, rb, pr.r, sm.sRn, pl.offRk, cols, kb + kStage, kend);
+      }
+#pragma unroll
+      for (int h = 0; h < kStage / BK; ++h) {
+        if (h && kb + h * BK >= kend) break;
+        const int k4 = h * BK + 4 * warp;
+        if constexpr (NJ > 0) {
+          const double *ak = &sm.As[cur][k4 + tig][g], *bk = &sm.Bs[cur][k4 + tig][g];
+          switch (mi) {
+            case 1: mma_rows<1>(acc, ak, bk); break;
+            case 2: mma_rows<2>(acc, ak, bk); break;
+            case 3: mma_rows<3>(acc, ak, bk); break;
+            default: mma_rows<4>(acc, ak, bk); break;
+          }
+        }
+        if constexpr (NREM > 0) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            const double a0 = sm.As[cur][k4 + kk][lane];
+#pragma unroll
+            for (int c = 0; c < NREM; ++c) rem[c] = fma(a0, sm.Bs[cur][k4 + kk][8 * NJ + c], rem[c]);
+          }
+        }
+      }
+      if (more) {
+        store_tile(pl.a_kfast, sm.As[cur ^ 1], ra);
+        store_tile(pl.b_kfast, sm.Bs[cur ^ 1], rb);
+      }
+      __syncthreads();
+    }
   }
-  if (tl.slot >= 0) {
-    write_partial<BM, BN>(acc, ws, tl.slot);
-    return;
-  }
-  const PlanRef dp = plans[tl.dplan];
-  write_tile<BM, BN>(acc, tl.d, dp.offDm, dp.offDn, dp.M, dp.N, tl.m0, tl.n0, mode);
+  __syncthreads();  // the staged operands are done with
+  if constexpr (NJ > 0)
+#pragma unroll
+    for (int i = 0; i < kTile / 8; ++i)
+      if (i < mi)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) sm.part[warp][8 * j + 2 * tig + h][8 * i + g] = acc[i][j][h];
+  if constexpr (NREM > 0)
+#pragma unroll
+    for (int c = 0; c < NREM; ++c) sm.part[warp][8 * NJ + c][lane] = rem[c];
 }
 
-// Sums a spread tile's partials in slot order (deterministic) and stores it.
-template <int BM, int BN>
-__global__ void __launch_bounds__(256) grouped_f64_reduce_kernel(const GroupedF64Reduce* __restrict__ reds,
-                                                                 const PlanRef* __restrict__ plans,
-                                                                 const double* __restrict__ ws, int mode) {
-  const GroupedF64Reduce rd = reds[blockIdx.x];
-  const PlanRef dp = plans[rd.dplan];
-  for (int e = threadIdx.x; e < BM * BN; e += blockDim.x) {
-    const int ml = e % BM, nl = e / BM;
-    const int m = rd.m0 + ml, n = rd.n0 + nl;
-    if (m >= dp.M || n >= dp.N) continue;
+template <int NREM, class... A>
+__device__ __forceinline__ void accumulate_cols(int nj, A&&... args) {
+  if constexpr (NREM > 0) {
+    switch (nj) {
+      case 0: return accumulate_tile<0, NREM>(args...);
+      case 1: return accumulate_tile<1, NREM>(args...);
+      case 2: return accumulate_tile<2, NREM>(args...);
+      default: return accumulate_tile<3, NREM>(args...);
+    }
+  } else {
+    switch (nj) {
+      case 1: return accumulate_tile<1, 0>(args...);
+      case 2: return accumulate_tile<2, 0>(args...);
+      case 3: return accumulate_tile<3, 0>(args...);
+      default: return accumulate_tile<4, 0>(args...);
+    }
+  }
+}
+
+// One CTA's share of one tile (nu columns of 8, the last one perhaps partial),
+// then the sum over the cluster's CTAs and their warps into D.  mode bit 0: accumulate into D (beta = 1),
+// bit 1: store the negated sum.
+__device__ void f64_tile(F64Smem& sm, const GroupedPair* pairs, const PlanRef* plans, int pb, int pe, int ks0, int ks1,
+                         const PlanRef& dp, double* __restrict__ D, int m0, int n0, int mi, int nu, int mode) {
+  const int rows = min(dp.M - m0, 8 * mi), cols = min(dp.N - n0, 8 * nu);
+  // columns beyond the last whole 8: up to four as FMAs (64 clk a column of 32
+  // rows and k on a quarter's pipe), else one more DMMA column (512 clk a tile
+  // of 8 rows and 4 k)
+  const int part = cols & 7, fma_cols = f64_fma_cols(part, mi);
+  if (fma_cols == 1) accumulate_cols<1>(nu - 1, sm, pairs, plans, pb, pe, ks0, ks1, m0, n0, mi, part);
+  else if (fma_cols == 2) accumulate_cols<2>(nu - 1, sm, pairs, plans, pb, pe, ks0, ks1, m0, n0, mi, part);
+  else if (fma_cols == 4) accumulate_cols<4>(nu - 1, sm, pairs, plans, pb, pe, ks0, ks1, m0, n0, mi, part);
+  else accumulate_cols<0>(nu, sm, pairs, plans, pb, pe, ks0, ks1, m0, n0, mi, 0);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = int(cluster.num_blocks()), rank = int(cluster.block_rank());
+  if (ranks > 1) cluster.sync();
+  else __syncthreads();
+  const bool col_fast = dp.N > 1 && dp.offDn[1] - dp.offDn[0] == 1;
+  const int total = rows * cols, lo = total * rank / ranks, hi = total * (rank + 1) / ranks;
+  for (int e = lo + int(threadIdx.x); e < hi; e += kThreadsF64) {
+    const int m = col_fast ? e / cols : e % rows, n = col_fast ? e % cols : e / rows;
     double v = 0.0;
-    for (int q = 0; q < rd.nparts; ++q) v += ws[size_t(rd.slot0 + q) * BM * BN + e];
+    for (int q = 0; q < ranks; ++q)
+#pragma unroll
+      for (int w = 0; w < kThreadsF64 / 32; ++w) {
+        double* x = &sm.part[w][n][m];
+        v += ranks > 1 ? *cluster.map_shared_rank(x, q) : *x;
+      }
     if (mode & 2) v = -v;
-    double* p = rd.d + dp.offDm[m] + dp.offDn[n];
+    double* p = D + dp.offDm[m0 + m] + dp.offDn[n0 + n];
     *p = (mode & 1) ? *p + v : v;
   }
+  if (ranks > 1) cluster.sync();  // no CTA leaves while its partial tile is read
 }
 
-template <int BM, int BN>
-void launch_single(const DevPlan* p, const double* L, const double* R, double* D, int M, int N, int K, int mode,
-                   int tiles_m, int64_t tiles, int nsplit, double* ws, cudaStream_t s) {
-  const GemmPlan& h = p->host;
-  contract_f64_kernel<BM, BN><<<unsigned(tiles * nsplit), kThreadsF64, 0, s>>>(
-      L, R, D, p->offLm, p->offLk, p->offRk, p->offRn, p->offDm, p->offDn, M, N, K, tiles_m, int(tiles), nsplit, mode,
-      h.a_kfast, h.b_kfast, ws);
-  if (nsplit > 1)
-    contract_f64_reduce_kernel<BM, BN><<<unsigned(tiles), 256, 0, s>>>(ws, int(tiles), nsplit, tiles_m, D, p->offDm,
-                                                                      p->offDn, M, N, mode);
+// One block pair: cluster x = tile, its CTAs share the tile's k steps.
+struct F64PairArgs {
+  GroupedPair pair;
+  PlanRef plan;
+  double* d;
+  int tiles_m, tiles_n, mode;
+};
+__global__ void __launch_bounds__(kThreadsF64, 4) contract_f64_kernel(const __grid_constant__ F64PairArgs a) {
+  __shared__ __align__(16) F64Smem sm;
+  const int ranks = int(cg::this_cluster().num_blocks()), rank = int(cg::this_cluster().block_rank());
+  const int tile = int(blockIdx.x) / ranks, tm = tile % a.tiles_m, tn = tile / a.tiles_m;
+  const int um = (a.plan.M + 7) / 8, un = (a.plan.N + 7) / 8, steps = (a.plan.K + BK - 1) / BK;
+  const int u0 = int(int64_t(um) * tm / a.tiles_m), u1 = int(int64_t(um) * (tm + 1) / a.tiles_m);
+  const int v0 = int(int64_t(un) * tn / a.tiles_n), v1 = int(int64_t(un) * (tn + 1) / a.tiles_n);
+  f64_tile(sm, &a.pair, &a.plan, 0, 1, int(int64_t(steps) * rank / ranks), int(int64_t(steps) * (rank + 1) / ranks),
+           a.plan, a.d, 8 * u0, 8 * v0, u1 - u0, v1 - v0, a.mode);
 }
 
-template <int BM, int BN>
-void launch_grouped(const GroupedF64Tile* tiles, int ntiles, const GroupedPair* pairs, const PlanRef* plans, int mode,
-                    double* ws, const GroupedF64Reduce* reds, int nreds, cudaStream_t s) {
-  grouped_f64_kernel<BM, BN><<<ntiles, kThreadsF64, 0, s>>>(tiles, pairs, plans, mode, ws);
-  if (nreds > 0) grouped_f64_reduce_kernel<BM, BN><<<nreds, 256, 0, s>>>(reds, plans, ws, mode);
+// A pardo step: one CTA per (destination block, tile, share of its pairs' k
+// steps), a tile's shares in one cluster.
+__global__ void __launch_bounds__(kThreadsF64, 4) grouped_f64_kernel(const GroupedF64Tile* __restrict__ tiles,
+                                                                     const GroupedPair* __restrict__ pairs,
+                                                                     const PlanRef* __restrict__ plans, int mode) {
+  __shared__ __align__(16) F64Smem sm;
+  const GroupedF64Tile tl = tiles[blockIdx.x];
+  f64_tile(sm, pairs, plans, tl.pair_begin, tl.pair_end, tl.ks0, tl.ks1, plans[tl.dplan], tl.d, tl.m0, tl.n0, tl.mi,
+           tl.nu, mode);
+}
+
+template <class... P, class... A>
+int launch_clusters(void (*kernel)(P...), int64_t ctas, int cluster, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(ctas));
+  cfg.blockDim = dim3(kThreadsF64);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = unsigned(cluster), at.val.clusterDim.y = 1, at.val.clusterDim.z = 1;
+  cfg.attrs = &at, cfg.numAttrs = 1;
+  A4G_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  return A4G_OK;
 }
 
 }  // namespace
 
-// Tile rows for destination rows m: 48 when it pads less than 64 by a tenth.
-int f64_tile_m_for(int64_t padded64, int64_t padded48) { return padded48 * 10 < padded64 * 9 ? 48 : 64; }
+// Tile rows and columns (in 8s) and the cluster size with the least estimated
+// time.  A CTA's cost on a quarter's pipe: 578 clk a DMMA, 300 for the FMAs of a
+// column and 16 k, 300 to add the shares of an 8 x 8 tile, 250 a step and 3000 at
+// its ends.  An SM runs up to four CTAs at once and needs them to fill the pipe;
+// up to that many the fullest SM decides, beyond it half a CTA more than the mean.
+// Over 12 shapes from 32^3 to 1024 x 256 x 1024, all 64 forms measured of each,
+// the forms it picks take 5.6 % more than the best ones (and up to 9x less than the worst).
+F64Form f64_form(const std::vector<F64Shape>& shapes, int sms) {
+  F64Form best;
+  double best_t = 0.0;
+  int64_t hm = 1, hn = 1;
+  for (const F64Shape& x : shapes) hm = std::max(hm, (x.M + 7) / 8), hn = std::max(hn, (x.N + 7) / 8);
+  for (int h = 1; h <= int(std::min<int64_t>(4, hm)); ++h)
+    for (int w = 1; w <= int(std::min<int64_t>(4, hn)); ++w) {
+      double tiles = 0.0, cost[4] = {0.0, 0.0, 0.0, 0.0}, largest[4] = {0.0, 0.0, 0.0, 0.0};
+      for (const F64Shape& x : shapes) {
+        const int64_t um = (x.M + 7) / 8, un = (x.N + 7) / 8, tm = (um + h - 1) / h, tn = (un + w - 1) / w;
+        const int mi = int((um + tm - 1) / tm), nu = int((un + tn - 1) / tn);  // the largest tile
+        const double n = double(x.count) * double(tm * tn), rows = double(um) / double(tm), cols = double(un) / double(tn);
+        const int fma_cols = f64_fma_cols(int(x.N & 7), mi);
+        const double saved = fma_cols ? (578.0 * rows - 300.0 * fma_cols) / double(tn) : 0.0;
+        tiles += n;
+        for (int c = 0; c < 4; ++c) {
+          const double steps = double((x.steps + (1 << c) - 1) >> c);  // the longest share's
+          cost[c] += n * (steps * (578.0 * rows * cols - saved + 250.0) + 300.0 * rows * cols + 3000.0);
+          largest[c] = std::max(largest[c], steps * (578.0 * mi * nu + 250.0) + 300.0 * mi * nu + 3000.0);
+        }
+      }
+      for (int c = 0; c < 4; ++c) {
+        const double ctas = tiles * double(1 << c), mean = ctas / sms;
+        if (ctas > double(0x7fffffff)) break;
+        const double per_sm = mean <= 4.0 ? std::ceil(mean) : mean + 0.5, own = cost[c] / tiles;
+        const double full = per_sm <= 1.0 ? 0.4 : per_sm <= 2.0 ? 0.7 : per_sm <= 3.0 ? 0.9 : 1.0;
+        const double t = per_sm * own / full + 0.5 * largest[c] + 0.01 * ((1 << c) - 1) * own + (c ? 3000.0 : 0.0);
+        if (best_t == 0.0 || t < best_t) best_t = t, best.h = h, best.w = w, best.cluster = 1 << c;
+      }
+    }
+  return best;
+}
 
 int launch_contract_f64(const DevPlan* p, const double* L, const double* R, double* D, int mode,
                         cudaStream_t s) {
   const GemmPlan& h = p->host;
   if (h.M > 0x7fffffff || h.N > 0x7fffffff || h.K > 0x7fffffff)
     return fail(A4G_ERR_RANGE, "matrix dimension exceeds 2^31");
-  const int M = int(h.M), N = int(h.N), K = int(h.K);
-  const int bn = N <= 32 ? 32 : 64;
-  const int bm = f64_tile_m_for((M + 63) / 64 * 64, (M + 47) / 48 * 48);
-  const int64_t tiles_m = (M + bm - 1) / bm, tiles_n = (N + bn - 1) / bn;
-  const int64_t tiles = tiles_m * tiles_n;
-  if (tiles > 0x3fffffffLL) return fail(A4G_ERR_RANGE, "contraction grid too large");
-  // split the k steps when the tiles alone would leave most SMs idle (about
-  // two CTAs per SM, at most 64 splits of at least one k step)
-  const int sms = ctx()->num_sms > 0 ? ctx()->num_sms : 152;
-  const int64_t ksteps = (K + BK - 1) / BK;
-  int nsplit = int(std::max<int64_t>(1, std::min<int64_t>({64, ksteps, (2LL * sms + tiles - 1) / tiles})));
-  if (tiles * nsplit > 0x7fffffffLL) nsplit = 1;
-  double* ws = nullptr;
-  if (nsplit > 1)
-    if (const int rc_ = async_alloc(reinterpret_cast<void**>(&ws), size_t(tiles * nsplit) * bm * bn * sizeof(double), s))
-      return rc_;
-  if (bm == 48 && bn == 32) launch_single<48, 32>(p, L, R, D, M, N, K, mode, int(tiles_m), tiles, nsplit, ws, s);
-  else if (bm == 48) launch_single<48, 64>(p, L, R, D, M, N, K, mode, int(tiles_m), tiles, nsplit, ws, s);
-  else if (bn == 32) launch_single<64, 32>(p, L, R, D, M, N, K, mode, int(tiles_m), tiles, nsplit, ws, s);
-  else launch_single<64, 64>(p, L, R, D, M, N, K, mode, int(tiles_m), tiles, nsplit, ws, s);
-  if (nsplit > 1) A4G_CUDA(cudaFreeAsync(ws, s));
-  A4G_CUDA(cudaGetLastError());
-  return A4G_OK;
+  const F64Form& f = p->f64;
+  const int64_t um = (h.M + 7) / 8, un = (h.N + 7) / 8, tm = (um + f.h - 1) / f.h, tn = (un + f.w - 1) / f.w;
+  if (tm * tn * f.cluster > 0x7fffffffLL) return fail(A4G_ERR_RANGE, "contraction grid too large");
+  F64PairArgs a{};
+  a.pair = {L, R, 0, 0};
+  a.plan = plan_ref(*p);
+  a.d = D;
+  a.tiles_m = int(tm), a.tiles_n = int(tn), a.mode = mode;
+  return launch_clusters(contract_f64_kernel, tm * tn * f.cluster, f.cluster, s, a);
 }
 
-int launch_grouped_f64(const GroupedF64Tile* tiles, int ntiles, const GroupedPair* pairs, const PlanRef* plans,
-                       int mode, double* ws, const GroupedF64Reduce* reds, int nreds, int tile_m, int tile_n,
-                       cudaStream_t s) {
+int launch_grouped_f64(const GroupedF64Tile* tiles, int ntiles, int cluster, const GroupedPair* pairs,
+                       const PlanRef* plans, int mode, cudaStream_t s) {
   if (ntiles <= 0) return A4G_OK;
-  if (tile_m == 48 && tile_n == 32) launch_grouped<48, 32>(tiles, ntiles, pairs, plans, mode, ws, reds, nreds, s);
-  else if (tile_m == 48) launch_grouped<48, 64>(tiles, ntiles, pairs, plans, mode, ws, reds, nreds, s);
-  else if (tile_n == 32) launch_grouped<64, 32>(tiles, ntiles, pairs, plans, mode, ws, reds, nreds, s);
-  else launch_grouped<64, 64>(tiles, ntiles, pairs, plans, mode, ws, reds, nreds, s);
-  A4G_CUDA(cudaGetLastError());
-  return A4G_OK;
+  return launch_clusters(grouped_f64_kernel, ntiles, cluster, s, tiles, pairs, plans, mode);
 }
-
-int grouped_f64_tile_m(int64_t padded64, int64_t padded48) { return f64_tile_m_for(padded64, padded48); }
-int grouped_f64_tile_n(int max_n) { return max_n <= 32 ? 32 : 64; }
 
 }  // namespace a4g

@@ -337,6 +337,7 @@ int get_dev_plan(const int* ptrn, int lrank, const int* lext, int rrank, const i
   dp->offRn = q, q += h.offRn.size();
   dp->offDm = q, q += h.offDm.size();
   dp->offDn = q;
+  dp->f64 = f64_form({{h.M, h.N, (h.K + 15) / 16, 1}}, g_ctx.num_sms > 0 ? g_ctx.num_sms : 152);
   g_plans.emplace(key, dp);
   *out = dp;
   return A4G_OK;
