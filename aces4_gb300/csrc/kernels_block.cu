@@ -40,25 +40,41 @@ __device__ __forceinline__ double ew(double d, double s, double a) {
   else return fma(a, s, d);  // _gpu_axpy: cuBLAS daxpy semantics
 }
 
+// Bound by HBM, or by the FP64 pipes where an element takes two operations
+// (add_scaled: 340 us for 96^4 elements, of 338 measured).  Two reads and a
+// write: a CTA per 2 x 256 pairs and no loop (358 us with the grid held to 8
+// CTAs per SM); fewer streams: the held grid (scale_copy 209 us, 241 without).
+template <EwOp OP>
+struct EwReads {
+  static constexpr bool d = !(OP == EwOp::kFill || OP == EwOp::kScaleCopy);
+  static constexpr bool s = OP == EwOp::kScaleCopy || OP == EwOp::kAddScaled || OP == EwOp::kAdd || OP == EwOp::kAxpy;
+  static constexpr int pairs = d && s ? 2 : 1;  // a thread's, all loaded before the first is stored
+};
 template <EwOp OP, bool VEC>
 __global__ void __launch_bounds__(kThreads) ew_kernel(double* __restrict__ d,
                                                       const double* __restrict__ s, int64_t n,
                                                       double a) {
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  constexpr bool kReadD = !(OP == EwOp::kFill || OP == EwOp::kScaleCopy);
-  constexpr bool kReadS = (OP == EwOp::kScaleCopy || OP == EwOp::kAddScaled || OP == EwOp::kAdd ||
-                           OP == EwOp::kAxpy);
+  constexpr bool kReadD = EwReads<OP>::d, kReadS = EwReads<OP>::s;
+  constexpr int kEwPairs = EwReads<OP>::pairs;
   if constexpr (VEC) {
     const int64_t n2 = n / 2;
     double2* d2 = reinterpret_cast<double2*>(d);
     const double2* s2 = reinterpret_cast<const double2*>(s);
-    for (int64_t k = i; k < n2; k += stride) {
-      double2 dv = kReadD ? d2[k] : make_double2(0.0, 0.0);
-      double2 sv = kReadS ? __ldg(&s2[k]) : make_double2(0.0, 0.0);
-      dv.x = ew<OP>(dv.x, sv.x, a);
-      dv.y = ew<OP>(dv.y, sv.y, a);
-      d2[k] = dv;
+    for (int64_t b = int64_t(blockIdx.x) * blockDim.x * kEwPairs + threadIdx.x; b < n2; b += kEwPairs * stride) {
+      double2 dv[kEwPairs], sv[kEwPairs];
+#pragma unroll
+      for (int u = 0; u < kEwPairs; ++u) {
+        const int64_t k = b + u * int64_t(blockDim.x);
+        dv[u] = kReadD && k < n2 ? d2[k] : make_double2(0.0, 0.0);
+        sv[u] = kReadS && k < n2 ? __ldg(&s2[k]) : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < kEwPairs; ++u) {
+        const int64_t k = b + u * int64_t(blockDim.x);
+        if (k < n2) d2[k] = make_double2(ew<OP>(dv[u].x, sv[u].x, a), ew<OP>(dv[u].y, sv[u].y, a));
+      }
     }
     if (i == 0 && (n & 1)) {
       const int64_t k = n - 1;
@@ -75,9 +91,11 @@ int launch_ew(double* d, const double* s, int64_t n, double a, cudaStream_t st) 
   if (n == 0) return A4G_OK;
   if (!d) return fail(A4G_ERR_ARG, "null block pointer");
   const bool vec = aligned16(d) && (s == nullptr || aligned16(s));
-  const int g = grid_for(vec ? n / 2 + 1 : n);
-  if (vec) ew_kernel<OP, true><<<g, kThreads, 0, st>>>(d, s, n, a);
-  else ew_kernel<OP, false><<<g, kThreads, 0, st>>>(d, s, n, a);
+  constexpr int kShare = EwReads<OP>::pairs * kThreads;
+  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((n / 2 + kShare - 1) / kShare, 0x7fffffff));
+  const int64_t g = EwReads<OP>::pairs > 1 ? ctas : grid_for(n / 2 + 1);
+  if (vec) ew_kernel<OP, true><<<unsigned(g), kThreads, 0, st>>>(d, s, n, a);
+  else ew_kernel<OP, false><<<grid_for(n), kThreads, 0, st>>>(d, s, n, a);
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
 }
@@ -380,8 +398,11 @@ struct SliceParams {
   int sext[kPermMax];
   int64_t tstride[kPermMax];
   int64_t tbase;
+  unsigned mul[kPermMax];  // slice_runs_kernel: division by sext
+  int shift[kPermMax];
 };
 
+// Beyond 2^31 slice elements: an element at a time, 64-bit divisions.
 __global__ void __launch_bounds__(kThreads) slice_insert_kernel(SliceParams p, int insert,
                                                                 double* tens, double* slice,
                                                                 int64_t n) {
@@ -395,6 +416,39 @@ __global__ void __launch_bounds__(kThreads) slice_insert_kernel(SliceParams p, i
     }
     if (insert) tens[o] = slice[i];
     else slice[i] = tens[o];
+  }
+}
+
+// Fewer than 2^31 slice elements, as T (pairs where every run starts on 16
+// bytes and has an even length, else single elements): kSliceLoads a thread, all
+// loaded before the first is stored, offsets by multiplications (x / d = x *
+// mul >> 31 + shift, exact below 2^31).  HBM bounds it; an element's 64-bit
+// divisions did: a 72^4 slice of a 96^4
+// block 190 -> 66 us, its insertion 190 -> 60.
+constexpr int kSliceLoads = 4;
+template <int INSERT, class T>
+__global__ void __launch_bounds__(kThreads) slice_runs_kernel(SliceParams p, T* __restrict__ tens,
+                                                              T* __restrict__ slice, unsigned n) {
+  const unsigned first = blockIdx.x * (kThreads * kSliceLoads) + threadIdx.x;
+  int64_t at[kSliceLoads];
+  T v[kSliceLoads];
+#pragma unroll
+  for (int u = 0; u < kSliceLoads; ++u) {
+    const unsigned i = first + u * kThreads;
+    unsigned rem = i;
+    int64_t o = p.tbase;
+    for (int q = 0; q < p.rank - 1; ++q) {
+      const unsigned d = unsigned((uint64_t(rem) * p.mul[q]) >> (31 + p.shift[q]));
+      o += int64_t(rem - d * unsigned(p.sext[q])) * p.tstride[q];
+      rem = d;
+    }
+    at[u] = o + int64_t(rem) * p.tstride[p.rank - 1];
+    if (i < n) v[u] = INSERT ? slice[i] : tens[at[u]];
+  }
+#pragma unroll
+  for (int u = 0; u < kSliceLoads; ++u) {
+    const unsigned i = first + u * kThreads;
+    if (i < n) (INSERT ? tens[at[u]] : slice[i]) = v[u];
   }
 }
 
@@ -944,7 +998,37 @@ int launch_slice_insert(int insert, int rank, double* tens, const int* tens_ext,
     st *= tens_ext[q];
     n *= slice_ext[q];
   }
-  slice_insert_kernel<<<grid_for(n), kThreads, 0, s>>>(p, insert, tens, slice, n);
+  if (n > 0x7fffffff - kThreads * kSliceLoads) {
+    slice_insert_kernel<<<grid_for(n), kThreads, 0, s>>>(p, insert, tens, slice, n);
+    A4G_CUDA(cudaGetLastError());
+    return A4G_OK;
+  }
+  // dims that are whole in the slice join their outer neighbour; unit dims go
+  SliceParams m{};
+  m.tbase = p.tbase;
+  bool whole = false;  // the last kept dim covers its extent of the block
+  for (int q = 0; q < rank; ++q) {
+    if (whole) m.sext[m.rank - 1] *= p.sext[q];
+    else if (p.sext[q] != 1 || m.rank == 0) m.sext[m.rank] = p.sext[q], m.tstride[m.rank++] = p.tstride[q];
+    else continue;
+    whole = p.sext[q] == tens_ext[q];
+  }
+  if (m.rank == 0) m.rank = 1, m.sext[0] = 1, m.tstride[0] = 1;
+  bool pairs = aligned16(tens) && aligned16(slice) && m.tstride[0] == 1 && (m.sext[0] & 1) == 0 && (m.tbase & 1) == 0;
+  for (int q = 1; q < m.rank; ++q) pairs = pairs && (m.tstride[q] & 1) == 0;
+  if (pairs) {
+    n /= 2, m.sext[0] /= 2, m.tbase /= 2;
+    for (int q = 1; q < m.rank; ++q) m.tstride[q] /= 2;
+  }
+  for (int q = 0; q < m.rank; ++q) {
+    while ((int64_t(1) << m.shift[q]) < m.sext[q]) ++m.shift[q];
+    m.mul[q] = unsigned(((uint64_t(1) << (31 + m.shift[q])) + uint64_t(m.sext[q]) - 1) / uint64_t(m.sext[q]));
+  }
+  const unsigned grid = unsigned((n + kThreads * kSliceLoads - 1) / (kThreads * kSliceLoads));
+  if (pairs && insert) slice_runs_kernel<1><<<grid, kThreads, 0, s>>>(m, reinterpret_cast<double2*>(tens), reinterpret_cast<double2*>(slice), unsigned(n));
+  else if (pairs) slice_runs_kernel<0><<<grid, kThreads, 0, s>>>(m, reinterpret_cast<double2*>(tens), reinterpret_cast<double2*>(slice), unsigned(n));
+  else if (insert) slice_runs_kernel<1><<<grid, kThreads, 0, s>>>(m, tens, slice, unsigned(n));
+  else slice_runs_kernel<0><<<grid, kThreads, 0, s>>>(m, tens, slice, unsigned(n));
   A4G_CUDA(cudaGetLastError());
   return A4G_OK;
 }
