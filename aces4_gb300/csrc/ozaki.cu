@@ -1025,16 +1025,33 @@ __global__ void __launch_bounds__(DIRECT ? kThreadsOzDirect : kThreadsOz, 1)
 constexpr int kLvBN = 64, kLvBK = 32, kLvMaxS = 5, kLvSt = 3, kLvAcc = 7;
 constexpr uint32_t kLvATile = kOzBM * kLvBK * 2;  // 8 KB: 128 rows x 32 k
 constexpr uint32_t kLvBTile = kLvBN * kLvBK * 2;  // 4 KB: 64 columns x 32 k
+// What the epilogue needs of a tile's rows and columns, laid out by the
+// producer warp while the tensor cores work on the tile: the chain of loads to
+// it (tile, panel and block, tables) is not in the sixteen epilogue warps' way.
+// (In their way it took, per step: o=24/v=240 with energy 17.8 ms instead of
+// 17.0, o=12/v=63 stored 459 us instead of 410, a third of that from rounding
+// eight results without a branch.)
+struct LvTab {
+  double rx[kOzBM];      // energy form: the row's last-term orbital energy
+  long long rp[kOzBM];   // energy: the row's line of the prefix table; store: its offset in D
+  double cx[kLvBN];      // energy form: the column's last-term orbital energy
+  long long cp[kLvBN];   // energy: the column in that line (-1: outside D); store: its base in D (0: outside)
+  int re[kOzBM];         // biased row exponent (at least 1; 0: outside D)
+  int cf[kLvBN];         // biased column exponent (at least 1)
+  int flag;              // energy: the last term runs over the rows; store: D is unit-stride along the columns
+};
 struct __align__(1024) LvSmem {
   uint8_t a[kLvSt][kLvMaxS][kLvATile];
   uint8_t b[kLvSt][kLvMaxS][kLvBTile];
   uint64_t full[kLvSt], empty[kLvSt];
   uint64_t acc_full, acc_empty, drain;
+  uint64_t tab_full[2], tab_empty[2];
+  LvTab tab[2];
   uint32_t tmem_base;
   volatile int abort;
   double out[kThreadsOzDirect / 32 - 2][32][9];  // per epilogue warp: 32 rows x 8 columns on their way to D
 };
-static_assert(sizeof(LvSmem) + 1024 + 6144 <= 232448, "with the static column tables: one CTA's shared memory");
+static_assert(sizeof(LvSmem) + 1024 <= 232448, "one CTA's shared memory");
 static_assert(kLvBN == kOzLevelsTileCols, "tile columns of the all-levels form");
 // TMEM accumulator (in 64-column units) of level t; levels 3 and 4: of k half
 // h.  The levels of each half lie side by side: 0 1 2 3 4 | 3' 4'.
@@ -1049,16 +1066,22 @@ __device__ __forceinline__ uint64_t sw64_desc(uint32_t lo) {
 
 // Per 32-wide k block of a tile, one stage: the S A-slices (rows m0..m0+127)
 // and the S B-slices (columns n0..n0+63).  Converged warp, one lane issues.
-__device__ void lv_producer(const OzGemmArgs& a, LvSmem& sm) {
+// Then the tile's tables.
+template <bool ENERGY>
+__device__ void lv_producer(const OzGemmArgs& a, LvSmem& sm, int lane) {
   const uint32_t bytes = uint32_t(a.slices) * (kLvATile + kLvBTile);
   const bool leader = elect_one();
   const uint32_t a0 = smem_u32(sm.a[0][0]), b0 = smem_u32(sm.b[0][0]);
   const uint32_t full0 = smem_u32(&sm.full[0]), empty0 = smem_u32(&sm.empty[0]);
-  uint32_t s = 0, free_parity = 1;
-  for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x)) {
+  uint32_t s = 0, free_parity = 1, nt = 0;
+  for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x), ++nt) {
     const OzTile tl = a.tiles[g];
     const void* ma = static_cast<const uint8_t*>(a.maps_a) + size_t(tl.panel_a) * 128;
     const void* mb = static_cast<const uint8_t*>(a.maps_b) + size_t(tl.panel_b) * 128;
+    const int *exps_a = a.panels_a[tl.panel_a].exps, *exps_b = a.panels_b[tl.panel_b].exps;
+    const OzDBlock db = a.dblocks[tl.dblock];
+    [[maybe_unused]] OzEnergyBlock eb{};
+    if constexpr (ENERGY) eb = a.eblocks[tl.dblock];
     for (int q = tl.trip_begin; q < tl.trip_end; ++q) {
       const OzTrip tr = a.trips[q];
       int ka = int(tr.koff_a), kb = int(tr.koff_b);
@@ -1074,6 +1097,46 @@ __device__ void lv_producer(const OzGemmArgs& a, LvSmem& sm) {
         if (++s == uint32_t(kLvSt)) s = 0, free_parity ^= 1;
       }
     }
+    const uint32_t slot = nt & 1;
+    if (!warp_wait(smem_u32(&sm.tab_empty[slot]), ((nt >> 1) & 1) ^ 1, sm, a.err_flag, 1)) return;
+    LvTab& t = sm.tab[slot];
+#pragma unroll
+    for (int i = 0; i < kOzBM / 32; ++i) {
+      const int row = 32 * i + lane, m = tl.m0 + row;
+      int e = 0;
+      long long p = ENERGY ? reinterpret_cast<long long>(eb.ptab) : 0;  // rows outside read (and drop) the first line
+      double x = 0.0;
+      if (m < db.M) {
+        e = max(exps_a[m], 1);
+        if constexpr (ENERGY) {
+          p = reinterpret_cast<long long>(eb.ptab + int64_t(eb.rk[m]) * eb.ckn);
+          if (eb.last_row) x = eb.elast[m];
+        } else {
+          p = db.rowoff[m];
+        }
+      }
+      t.re[row] = e, t.rp[row] = p, t.rx[row] = x;
+    }
+#pragma unroll
+    for (int i = 0; i < kLvBN / 32; ++i) {
+      const int col = 32 * i + lane, n = tl.n0 + col;
+      int f = 1;
+      long long p = ENERGY ? -1 : 0;
+      double x = 0.0;
+      if (n < db.N) {
+        f = max(exps_b[n], 1);
+        if constexpr (ENERGY) {
+          p = eb.ck[n];
+          if (!eb.last_row) x = eb.elast[n];
+        } else {
+          p = reinterpret_cast<long long>(db.colptr[n]);
+        }
+      }
+      t.cf[col] = f, t.cp[col] = p, t.cx[col] = x;
+    }
+    if (lane == 0) t.flag = ENERGY ? eb.last_row : db.col_fast;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.tab_full[slot]);
   }
 }
 
@@ -1148,20 +1211,10 @@ __device__ void lv_mma(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem) {
   }
 }
 
-// What a thread needs of one of its warp's 16 columns (a table per warp in
-// shared memory, filled while the tensor cores work on the tile).
-struct LvCol {
-  double* colp;  // store form: column base in D (null: outside D)
-  double ec;     // energy form: the column's last-term orbital energy
-  int F;         // biased column exponent (at least 1)
-  int ck;        // energy form: prefix-table column (-1: outside D)
-};
-
 constexpr int kLvGroup = 4;  // elements whose energy work overlaps
 
 // Sixteen warps, four per TMEM lane quadrant; a thread owns one row and 16
-// columns.  Per tile: the row's scale and tables, the 16 columns' table, the
-// wait for the tile's MMAs, the exact sums (two groups of 8 columns, each
+// columns.  Per tile: the wait for the tile's tables and MMAs, the exact sums (two groups of 8 columns, each
 // accumulator read once), TMEM released, then per element the rounding to
 // FP64 with the row and column scales and
 //   energy form: acc += x * fl(x / eps), eps = fl(prefix - e_last)
@@ -1171,59 +1224,20 @@ constexpr int kLvGroup = 4;  // elements whose energy work overlaps
 // A non-finite operand value in the row or column makes x NaN.
 template <bool ENERGY, int S>
 __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int warp, int lane) {
-  __shared__ LvCol lv_cols[kThreadsOzDirect / 32 - 2][16];
-  LvCol* tab = lv_cols[warp - 2];
   const int q = warp & 3, h = (warp - 2) >> 2;
   const int row = 32 * q + lane;
   const uint32_t lane_addr = tmem + (uint32_t(32 * q) << 16) + uint32_t(16 * h);
   [[maybe_unused]] double eacc = 0.0;
   uint32_t nt = 0;
   for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x), ++nt) {
-    const OzTile tl = a.tiles[g];
-    const OzDBlock db = a.dblocks[tl.dblock];
-    const int m = tl.m0 + row;
-    const bool mlive = m < db.M;
-    int Em = 1;
-    bool nonfinite = false;
-    [[maybe_unused]] long long roff = 0;
-    [[maybe_unused]] const double* prow = nullptr;
-    [[maybe_unused]] double er = 0.0;
-    [[maybe_unused]] bool last_row = false;
-    [[maybe_unused]] OzEnergyBlock eb{};
-    if constexpr (ENERGY) {
-      eb = a.eblocks[tl.dblock];
-      last_row = eb.last_row != 0;
-      prow = eb.ptab;  // rows outside the block read (and drop) the table's first row
-    }
-    if (mlive) {
-      const int e = a.panels_a[tl.panel_a].exps[m];
-      Em = e ? e : 1;
-      nonfinite = e == kNonFiniteExp;
-      if constexpr (ENERGY) {
-        prow = eb.ptab + int64_t(eb.rk[m]) * eb.ckn;
-        if (last_row) er = eb.elast[m];
-      } else {
-        roff = db.rowoff[m];
-      }
-    }
-    const int ebase = Em - 1022 - 1022 + 2 - kDigitBits * (S + 1);
-    __syncwarp();  // the previous tile's entries are read
-    if (lane < 16) {
-      const int n = tl.n0 + 16 * h + lane;
-      LvCol c{nullptr, 0.0, 1, -1};
-      if (n < db.N) {
-        const int f = a.panels_b[tl.panel_b].exps[n];
-        c.F = f ? f : 1;
-        if constexpr (ENERGY) {
-          c.ck = eb.ck[n];
-          if (!last_row) c.ec = eb.elast[n];
-        } else {
-          c.colp = db.colptr[n];
-        }
-      }
-      tab[lane] = c;
-    }
-    __syncwarp();
+    const uint32_t slot = nt & 1;
+    if (!mbar_wait(&sm.tab_full[slot], (nt >> 1) & 1, sm, a.err_flag, 4)) break;
+    const LvTab& t = sm.tab[slot];
+    const int re = t.re[row];
+    const bool mlive = re != 0, nonfinite = re == kNonFiniteExp, flag = t.flag != 0;
+    const int ebase = max(re, 1) - 1022 - 1022 + 2 - kDigitBits * (S + 1);
+    const int* cf = t.cf + 16 * h;
+    const long long* cp = t.cp + 16 * h;
     if (!mbar_wait(&sm.acc_full, nt & 1, sm, a.err_flag, 4)) break;
     tc_fence_after();
     long long sum[16];
@@ -1255,16 +1269,19 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
       // their conversions, denominators and divisions overlap; zeros, dead rows
       // and columns, non-finite rows and results beyond the normal range are
       // done one by one afterwards
+      const double* prow = reinterpret_cast<const double*>(t.rp[row]);
+      const double er = t.rx[row];
+      const double* ec = t.cx + 16 * h;
 #pragma unroll
       for (int j0 = 0; j0 < 16; j0 += kLvGroup) {
         double x[kLvGroup], qv[kLvGroup];
         bool ok[kLvGroup], all = mlive && !nonfinite;
 #pragma unroll
         for (int i = 0; i < kLvGroup; ++i) {
-          const LvCol c = tab[j0 + i];
-          ok[i] = i64_scaled_normal(sum[j0 + i], ebase + c.F, &x[i]);
-          const double eps = __dsub_rn(prow[max(c.ck, 0)], last_row ? er : c.ec);
-          ok[i] = div_rn_int(x[i], eps, &qv[i]) && ok[i] && c.ck >= 0 && c.F != kNonFiniteExp;
+          const int F = cf[j0 + i], ck = int(cp[j0 + i]);
+          ok[i] = i64_scaled_normal(sum[j0 + i], ebase + F, &x[i]);
+          const double eps = __dsub_rn(prow[max(ck, 0)], flag ? er : ec[j0 + i]);
+          ok[i] = div_rn_int(x[i], eps, &qv[i]) && ok[i] && ck >= 0 && F != kNonFiniteExp;
           all = all && ok[i];
         }
         if (all) {
@@ -1277,64 +1294,76 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
               eacc = fma(x[i], qv[i], eacc);
               continue;
             }
-            const LvCol c = tab[j0 + i];
-            if (c.ck < 0) continue;
-            double y = i64_scaled_to_double(sum[j0 + i], ebase + c.F, false);
-            if (nonfinite || c.F == kNonFiniteExp) y = __longlong_as_double(0x7FF8000000000000ll);
+            const int F = cf[j0 + i], ck = int(cp[j0 + i]);
+            if (ck < 0) continue;
+            double y = i64_scaled_to_double(sum[j0 + i], ebase + F, false);
+            if (nonfinite || F == kNonFiniteExp) y = __longlong_as_double(0x7FF8000000000000ll);
             if (!nonzero(y)) continue;
-            eacc = fma(y, div_rn(y, __dsub_rn(prow[c.ck], last_row ? er : c.ec)), eacc);
+            eacc = fma(y, div_rn(y, __dsub_rn(prow[ck], flag ? er : ec[j0 + i])), eacc);
           }
         }
       }
     } else {
-      const bool acc = a.mode & 1;
-      auto result = [&](int j) {
-        const int F = tab[j].F;
-        double x = i64_scaled_to_double(sum[j], ebase + F, a.mode & 2);
-        if (nonfinite || F == kNonFiniteExp) x = __longlong_as_double(0x7FF8000000000000ll);
-        return x;
-      };
-      if (!db.col_fast) {
+      const bool acc = a.mode & 1, neg = a.mode & 2;
+      const long long roff = t.rp[row];
+      double(*buf)[9] = sm.out[warp - 2];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          double* cp = tab[j].colp;
-          if (!mlive || !cp) continue;
-          const double x = result(j);
-          double* p = cp + roff;
-          *p = acc ? *p + x : x;
+      for (int h8 = 0; h8 < 2; ++h8) {
+        // eight roundings without a branch between them; results beyond the
+        // normal range one by one afterwards
+        double x[8];
+        uint32_t slow = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const long long v = sum[8 * h8 + j];
+          const int F = cf[8 * h8 + j];
+          const bool ok = i64_scaled_normal(v, ebase + F, &x[j]) || v == 0;
+          if (v == 0) x[j] = 0.0;
+          x[j] = __longlong_as_double(__double_as_longlong(x[j]) ^ (neg ? (1ll << 63) : 0ll));
+          if (nonfinite || F == kNonFiniteExp) x[j] = __longlong_as_double(0x7FF8000000000000ll);
+          else if (!ok) slow |= 1u << j;
         }
-      } else {
+        if (slow) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (slow >> j & 1) x[j] = i64_scaled_to_double(sum[8 * h8 + j], ebase + cf[8 * h8 + j], neg);
+        }
+        if (!flag) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            double* p = reinterpret_cast<double*>(cp[8 * h8 + j]);
+            if (mlive && p) p[roff] = acc ? p[roff] + x[j] : x[j];
+          }
+          continue;
+        }
         // D runs along the columns: the warp's 32 x 8 results turn in shared
         // memory, so that a store covers four rows of 64 contiguous bytes
         // instead of 32 rows of one element each, 32 cycles of the load / store
         // unit per instruction (o=12/v=63 step, 413 MB of W: 666 -> 459 us;
         // rows that are contiguous already store directly)
-        double(*buf)[9] = sm.out[warp - 2];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) buf[lane][j] = x[j];
+        __syncwarp();
         const int c = lane & 7;
-        const long long ro = mlive ? roff : -1;
+        double* base = reinterpret_cast<double*>(cp[8 * h8 + c]);
+        double* p[8];
+        double old[8];
 #pragma unroll
-        for (int h8 = 0; h8 < 2; ++h8) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) buf[lane][j] = result(8 * h8 + j);
-          __syncwarp();
-          double* cp = tab[8 * h8 + c].colp;
-          double* p[8];
-          double old[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const long long o = __shfl_sync(0xffffffffu, ro, 4 * i + (lane >> 3));
-            p[i] = cp && o >= 0 ? cp + o : nullptr;
-            old[i] = acc && p[i] ? *p[i] : 0.0;
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const double x = buf[4 * i + (lane >> 3)][c];
-            if (p[i]) *p[i] = acc ? old[i] + x : x;
-          }
-          __syncwarp();
+        for (int i = 0; i < 8; ++i) {
+          const int rr = 32 * q + 4 * i + (lane >> 3);
+          p[i] = base && t.re[rr] ? base + t.rp[rr] : nullptr;
+          old[i] = acc && p[i] ? *p[i] : 0.0;
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const double y = buf[4 * i + (lane >> 3)][c];
+          if (p[i]) *p[i] = acc ? old[i] + y : y;
+        }
+        __syncwarp();
       }
     }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.tab_empty[slot]);
   }
   if constexpr (ENERGY) a.epart[(size_t(blockIdx.x) * 16 + size_t(warp - 2)) * 32 + lane] = eacc;
 }
@@ -1352,6 +1381,7 @@ __global__ void __launch_bounds__(kThreadsOzDirect, 1) oz_levels_kernel(const __
     mbar_init(&sm.acc_full, 1);
     mbar_init(&sm.acc_empty, 16);  // one arrive per epilogue warp
     mbar_init(&sm.drain, 1);
+    for (int s = 0; s < 2; ++s) mbar_init(&sm.tab_full[s], 1), mbar_init(&sm.tab_empty[s], 16);
     sm.abort = 0;
     fence_mbar_init();
   }
@@ -1365,7 +1395,7 @@ __global__ void __launch_bounds__(kThreadsOzDirect, 1) oz_levels_kernel(const __
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   if (warp == 0) {
-    lv_producer(a, sm);
+    lv_producer<ENERGY>(a, sm, lane);
   } else if (warp == 1) {
     lv_mma<S>(a, sm, tmem);
     if (elect_one()) tc_commit(&sm.drain);  // all MMAs of this warp have completed before TMEM is released
