@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "_build", "libaces4gb300.so")
@@ -19,20 +20,41 @@ def build(verbose: bool = False) -> str:
     return _b.build(verbose=verbose)
 
 
+# Integer arrays as a call takes them: packed bytes, whose address ctypes
+# passes (a ctypes array of the same values took 1 to 2 us to build, most of an
+# update_t2 call's 13 us went into its nine arguments of this kind).  Values
+# that struct does not take (floats, beyond 32 bits) go through int() and wrap,
+# as ctypes does.
+_PACK = [struct.Struct("%di" % n).pack for n in range(33)]
+
+
+def ints(seq):
+    try:
+        return _PACK[len(seq)](*seq)
+    except (TypeError, IndexError, struct.error):
+        seq = [int(v) for v in seq]
+        return (ctypes.c_int * max(1, len(seq)))(*seq)
+
+
+INT = [struct.pack("i", n) for n in range(65)]  # INT[n]: n by reference
+
+
+_I, _P = ctypes.c_int, c_void_p
+
 # (name, restype, argtypes) of every exported entry point; argtypes None means
-# "plain ctypes conversion" for the by-pointer Fortran-style drop-ins.
+# "plain ctypes conversion".
 SIGNATURES = {
     # tensor_ops_c_prototypes.h drop-ins
     "tensor_size_by_shape_": (ctypes.c_longlong, None),
     "get_contraction_ptrn_": (None, None),
-    "tensor_block_init__": (None, None),
-    "tensor_block_scale__": (None, None),
-    "tensor_block_norm2__": (ctypes.c_double, None),
-    "tensor_block_slice__": (None, None),
-    "tensor_block_insert__": (None, None),
-    "tensor_block_add__": (None, None),
-    "tensor_block_copy__": (None, None),
-    "tensor_block_contract__": (None, None),
+    "tensor_block_init__": (None, [_P] * 6),
+    "tensor_block_scale__": (None, [_P] * 6),
+    "tensor_block_norm2__": (ctypes.c_double, [_P] * 5),
+    "tensor_block_slice__": (None, [_P] * 8),
+    "tensor_block_insert__": (None, [_P] * 8),
+    "tensor_block_add__": (None, [_P] * 7),
+    "tensor_block_copy__": (None, [_P] * 7),
+    "tensor_block_contract__": (None, [_P] * 12),
     # gpu_super_instructions.h drop-ins
     "_init_gpu": (None, None),
     "_gpu_axpy": (None, [c_void_p, c_void_p, ctypes.c_double, ctypes.c_int]),
@@ -54,27 +76,27 @@ SIGNATURES = {
     "a4g_init": (ctypes.c_int, [ctypes.c_int]),
     "a4g_sync": (ctypes.c_int, [c_void_p]),
     "a4g_default_stream": (c_void_p, []),
-    "a4g_contract": (ctypes.c_int, None),
-    "a4g_contract_labels": (ctypes.c_int, None),
-    "a4g_permute": (ctypes.c_int, None),
+    "a4g_contract": (_I, [_P, _P, _I, _P, _P, _I, _P, _P, _I, _P, _I, _P]),
+    "a4g_contract_labels": (_I, [_P, _P, _P, _P, _I, _P, _P, _I, _P, _P, _I, _P, _I, _P]),
+    "a4g_permute": (_I, [_I, _P, _P, _P, _P, _P]),
     "a4g_fill": (ctypes.c_int, [c_void_p, ctypes.c_int64, ctypes.c_double, c_void_p]),
     "a4g_scale": (ctypes.c_int, [c_void_p, ctypes.c_int64, ctypes.c_double, c_void_p]),
     "a4g_scale_copy": (ctypes.c_int, [c_void_p, c_void_p, ctypes.c_int64, ctypes.c_double, c_void_p]),
     "a4g_increment": (ctypes.c_int, [c_void_p, ctypes.c_int64, ctypes.c_double, c_void_p]),
     "a4g_add_scaled": (ctypes.c_int, [c_void_p, c_void_p, ctypes.c_int64, ctypes.c_double, c_void_p]),
-    "a4g_add_sub": (ctypes.c_int, None),
+    "a4g_add_sub": (_I, [_I, _I, _P, _P, _P, _P, _P, _P, _P]),
     "a4g_add_sub_noalloc": (ctypes.c_int, None),
     "a4g_norm2": (ctypes.c_int, [c_void_p, ctypes.c_int64, c_double_p, c_void_p]),
-    "a4g_slice": (ctypes.c_int, None),
-    "a4g_insert": (ctypes.c_int, None),
-    "a4g_energy_denominator": (ctypes.c_int, None),
-    "a4g_energy_contract": (ctypes.c_int, None),
+    "a4g_slice": (_I, [_I, _P, _P, _P, _P, _P, _P]),
+    "a4g_insert": (_I, [_I, _P, _P, _P, _P, _P, _P]),
+    "a4g_energy_denominator": (_I, [_I, _P, _P, _P, _I, _P, _P, _I, _P, _P]),
+    "a4g_energy_contract": (_I, [_I, _P, _P, _P, _P, _I, _P, _P, _I, _P, ctypes.c_double, _P, _P]),
     "a4g_batch_splits": (ctypes.c_int, None),
     "a4g_selftest_wait_timeout": (ctypes.c_int, None),
     "a4g_selftest_round": (ctypes.c_int, [ctypes.c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "a4g_selftest_div": (ctypes.c_int, [ctypes.c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     "a4g_clear_error": (None, []),
-    "a4g_update_t2": (ctypes.c_int, None),
+    "a4g_update_t2": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _P, _P, _P]),
     "a4g_batch_launches": (ctypes.c_int, None),
     "a4g_batch_create": (ctypes.c_int, None),
     "a4g_batch_run": (ctypes.c_int, [c_void_p, c_void_p]),

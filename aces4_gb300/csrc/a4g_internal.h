@@ -35,7 +35,10 @@ struct Context {
   cudaStream_t stream = nullptr;
   void* arena = nullptr;
   size_t arena_bytes = 0;
-  int* d_error_flag = nullptr;  // device int: nonzero = a kernel gave up a wait
+  // nonzero: a kernel gave up a wait.  In mapped host memory, so that a synchronous
+  // call reads it without a copy (and the synchronisation that copy makes)
+  int* d_error_flag = nullptr;
+  volatile int* h_error_flag = nullptr;
   // Stream-ordered allocations of the library (split-K workspaces, block
   // copies, reduction partials) come from a pool of its own that keeps freed
   // memory for reuse: the default pool hands memory back to the driver at

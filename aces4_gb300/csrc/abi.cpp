@@ -535,6 +535,7 @@ int a4g_init(int device) {
 int a4g_sync(void* stream) {
   int rc = ensure_init();
   if (rc) return rc;
+  A4G_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the default stream's work is done too
   return check_device_flag(pick(stream));
 }
 

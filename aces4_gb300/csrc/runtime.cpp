@@ -43,8 +43,11 @@ int ensure_init() {
     return fail(A4G_ERR_UNSUPPORTED, "aces4_gb300 needs a Blackwell GPU (sm_103a); found sm_" +
                                          std::to_string(prop.major) + std::to_string(prop.minor));
   A4G_CUDA(cudaStreamCreateWithFlags(&g_ctx.stream, cudaStreamNonBlocking));
-  A4G_CUDA(cudaMalloc(&g_ctx.d_error_flag, sizeof(int)));
-  A4G_CUDA(cudaMemset(g_ctx.d_error_flag, 0, sizeof(int)));
+  void *flag = nullptr, *d_flag = nullptr;
+  A4G_CUDA(cudaHostAlloc(&flag, sizeof(int), cudaHostAllocMapped));
+  A4G_CUDA(cudaHostGetDevicePointer(&d_flag, flag, 0));
+  g_ctx.h_error_flag = static_cast<volatile int*>(flag), g_ctx.d_error_flag = static_cast<int*>(d_flag);
+  *g_ctx.h_error_flag = 0;
   A4G_CUDA(cudaMalloc(&g_ctx.reduce_partials,
                       sizeof(double) * (Context::kReducePartials + 8) * size_t(Context::kReduceSlots)));
   A4G_CUDA(cudaMalloc(&g_ctx.reduce_counters, sizeof(unsigned) * Context::kReduceCounters));
@@ -101,10 +104,9 @@ int arena_reserve(size_t bytes, void** out) {
 
 int check_device_flag(cudaStream_t s) {
   A4G_CUDA(cudaStreamSynchronize(s));
-  int flag = 0;
-  A4G_CUDA(cudaMemcpy(&flag, g_ctx.d_error_flag, sizeof(int), cudaMemcpyDeviceToHost));
+  const int flag = *g_ctx.h_error_flag;
   if (flag) {
-    A4G_CUDA(cudaMemset(g_ctx.d_error_flag, 0, sizeof(int)));
+    *g_ctx.h_error_flag = 0;
     return fail(A4G_ERR_TIMEOUT, "a device-side wait reached its iteration limit (code " +
                                      std::to_string(flag) + "); the kernel returned early");
   }

@@ -11,7 +11,7 @@ import ctypes
 
 import numpy as np
 
-from ._lib import lib, last_error
+from ._lib import ints, last_error, lib
 
 _i = ctypes.c_int
 
@@ -22,7 +22,13 @@ class A4GError(RuntimeError):
         self.rc = rc
 
 
+_F64 = [None]  # torch.float64, once seen
+
+
 def _ptr(x) -> int:
+    dtype = getattr(x, "dtype", None)
+    if dtype is not None and dtype is _F64[0] and x.is_cuda:
+        return x.data_ptr()
     if x is None:
         return 0
     if isinstance(x, int):
@@ -31,6 +37,8 @@ def _ptr(x) -> int:
         raise TypeError("device API expects CUDA tensors")
     if str(getattr(x, "dtype", "torch.float64")) != "torch.float64":
         raise TypeError(f"device API expects float64 tensors, got {x.dtype}")
+    if str(dtype) == "torch.float64":
+        _F64[0] = dtype
     return x.data_ptr()
 
 
@@ -53,6 +61,15 @@ def _stream(stream) -> ctypes.c_void_p:
     return ctypes.c_void_p(int(stream))
 
 
+def _on(stream) -> int:
+    """_stream's handle as an integer, for the calls with declared arguments."""
+    if stream is None:
+        return 0
+    if hasattr(stream, "cuda_stream"):
+        return stream.cuda_stream or _LEGACY_DEFAULT_STREAM
+    return int(stream)
+
+
 def _check(rc: int, what: str):
     if rc != 0:
         raise A4GError(rc, what)
@@ -68,77 +85,77 @@ def sync(stream=None):
 
 def contract(ptrn, l, lext, r, rext, d, dext, beta: int = 0, stream=None):
     """D (=|+=) contract(L, R) with the reference pattern format."""
-    rc = lib().a4g_contract(_iarr(ptrn), ctypes.c_void_p(_ptr(l)), _i(len(lext)), _iarr(lext),
-                            ctypes.c_void_p(_ptr(r)), _i(len(rext)), _iarr(rext),
-                            ctypes.c_void_p(_ptr(d)), _i(len(dext)), _iarr(dext), _i(beta), _stream(stream))
+    rc = lib().a4g_contract(ints(ptrn), _ptr(l), len(lext), ints(lext),
+                            _ptr(r), len(rext), ints(rext),
+                            _ptr(d), len(dext), ints(dext), _i(beta), _on(stream))
     _check(rc, "a4g_contract")
 
 
 def contract_labels(dlab, llab, rlab, l, lext, r, rext, d, dext, beta: int = 0, stream=None):
-    rc = lib().a4g_contract_labels(_iarr(dlab), _iarr(llab), _iarr(rlab), ctypes.c_void_p(_ptr(l)),
-                                   _i(len(lext)), _iarr(lext), ctypes.c_void_p(_ptr(r)), _i(len(rext)),
-                                   _iarr(rext), ctypes.c_void_p(_ptr(d)), _i(len(dext)), _iarr(dext),
-                                   _i(beta), _stream(stream))
+    rc = lib().a4g_contract_labels(ints(dlab), ints(llab), ints(rlab), _ptr(l),
+                                   len(lext), ints(lext), _ptr(r), len(rext),
+                                   ints(rext), _ptr(d), len(dext), ints(dext),
+                                   _i(beta), _on(stream))
     _check(rc, "a4g_contract_labels")
 
 
 def permute(ext, perm_o2n_1based, src, dst, stream=None):
-    rc = lib().a4g_permute(_i(len(ext)), _iarr(ext), _iarr([1] + list(perm_o2n_1based)),
-                           ctypes.c_void_p(_ptr(src)), ctypes.c_void_p(_ptr(dst)), _stream(stream))
+    rc = lib().a4g_permute(len(ext), ints(ext), ints([1] + list(perm_o2n_1based)),
+                           _ptr(src), _ptr(dst), _on(stream))
     _check(rc, "a4g_permute")
 
 
 def fill(d, value: float, stream=None):
-    _check(lib().a4g_fill(_ptr(d), d.numel(), float(value), _stream(stream)), "a4g_fill")
+    _check(lib().a4g_fill(_ptr(d), d.numel(), float(value), _on(stream)), "a4g_fill")
 
 
 def scale(d, factor: float, stream=None):
-    _check(lib().a4g_scale(_ptr(d), d.numel(), float(factor), _stream(stream)), "a4g_scale")
+    _check(lib().a4g_scale(_ptr(d), d.numel(), float(factor), _on(stream)), "a4g_scale")
 
 
 def scale_copy(d, s, factor: float, stream=None):
-    _check(lib().a4g_scale_copy(_ptr(d), _ptr(s), d.numel(), float(factor), _stream(stream)), "a4g_scale_copy")
+    _check(lib().a4g_scale_copy(_ptr(d), _ptr(s), d.numel(), float(factor), _on(stream)), "a4g_scale_copy")
 
 
 def increment(d, delta: float, stream=None):
-    _check(lib().a4g_increment(_ptr(d), d.numel(), float(delta), _stream(stream)), "a4g_increment")
+    _check(lib().a4g_increment(_ptr(d), d.numel(), float(delta), _on(stream)), "a4g_increment")
 
 
 def add_scaled(t0, t1, scale_fac: float, stream=None):
-    _check(lib().a4g_add_scaled(_ptr(t0), _ptr(t1), t0.numel(), float(scale_fac), _stream(stream)),
+    _check(lib().a4g_add_scaled(_ptr(t0), _ptr(t1), t0.numel(), float(scale_fac), _on(stream)),
            "a4g_add_scaled")
 
 
 def add_sub(subtract: bool, d_labels, r_labels, r_ext, d, l, r, stream=None):
-    rc = lib().a4g_add_sub(_i(int(subtract)), _i(len(r_ext)), _iarr(d_labels), _iarr(r_labels), _iarr(r_ext),
-                           ctypes.c_void_p(_ptr(d)), ctypes.c_void_p(_ptr(l)), ctypes.c_void_p(_ptr(r)),
-                           _stream(stream))
+    rc = lib().a4g_add_sub(int(subtract), len(r_ext), ints(d_labels), ints(r_labels), ints(r_ext),
+                           _ptr(d), _ptr(l), _ptr(r),
+                           _on(stream))
     _check(rc, "a4g_add_sub")
 
 
 def norm2(t, stream=None) -> float:
     out = ctypes.c_double(0.0)
-    _check(lib().a4g_norm2(_ptr(t), t.numel(), ctypes.byref(out), _stream(stream)), "a4g_norm2")
+    _check(lib().a4g_norm2(_ptr(t), t.numel(), ctypes.byref(out), _on(stream)), "a4g_norm2")
     return out.value
 
 
 def slice_block(tens, text, slice_, sext, beg, stream=None):
-    rc = lib().a4g_slice(_i(len(text)), ctypes.c_void_p(_ptr(tens)), _iarr(text), ctypes.c_void_p(_ptr(slice_)),
-                         _iarr(sext), _iarr(beg), _stream(stream))
+    rc = lib().a4g_slice(len(text), _ptr(tens), ints(text), _ptr(slice_),
+                         ints(sext), ints(beg), _on(stream))
     _check(rc, "a4g_slice")
 
 
 def insert_block(tens, text, slice_, sext, beg, stream=None):
-    rc = lib().a4g_insert(_i(len(text)), ctypes.c_void_p(_ptr(tens)), _iarr(text), ctypes.c_void_p(_ptr(slice_)),
-                          _iarr(sext), _iarr(beg), _stream(stream))
+    rc = lib().a4g_insert(len(text), _ptr(tens), ints(text), _ptr(slice_),
+                          ints(sext), ints(beg), _on(stream))
     _check(rc, "a4g_insert")
 
 
 def energy_denominator(index_values, ext0, data0, ext1, e_or_fock, seg_sizes, stream=None):
-    rc = lib().a4g_energy_denominator(_i(len(ext0)), _iarr(index_values), _iarr(ext0),
-                                      ctypes.c_void_p(_ptr(data0)), _i(len(ext1)), _iarr(ext1),
-                                      ctypes.c_void_p(_ptr(e_or_fock)), _i(len(seg_sizes)), _iarr(seg_sizes),
-                                      _stream(stream))
+    rc = lib().a4g_energy_denominator(len(ext0), ints(index_values), ints(ext0),
+                                      _ptr(data0), len(ext1), ints(ext1),
+                                      _ptr(e_or_fock), len(seg_sizes), ints(seg_sizes),
+                                      _on(stream))
     _check(rc, "a4g_energy_denominator")
 
 
@@ -146,10 +163,9 @@ def update_t2(index_values, ext, t2new, t2new_pair, t2old, t2old_pair, diis_err,
               seg_sizes, norm2=None, stream=None):
     """updatet2 for one (a,i,b,j) block (a4g_update_t2): writes the DIIS error
     block and the next T2old block, adds sum(err^2) to norm2 (CUDA float64)."""
-    p = lambda x: ctypes.c_void_p(_ptr(x)) if x is not None else None
-    rc = lib().a4g_update_t2(_iarr(index_values), _iarr(ext), p(t2new), p(t2new_pair), p(t2old), p(t2old_pair),
-                             p(diis_err), p(t2old_next), _i(len(ext1)), _iarr(ext1), p(e_or_fock),
-                             _i(len(seg_sizes)), _iarr(seg_sizes), p(norm2), _stream(stream))
+    rc = lib().a4g_update_t2(ints(index_values), ints(ext), _ptr(t2new), _ptr(t2new_pair), _ptr(t2old), _ptr(t2old_pair),
+                             _ptr(diis_err), _ptr(t2old_next), len(ext1), ints(ext1), _ptr(e_or_fock),
+                             len(seg_sizes), ints(seg_sizes), _ptr(norm2), _on(stream))
     _check(rc, "a4g_update_t2")
 
 
@@ -157,11 +173,11 @@ def energy_contract(index_values, ext0, data0, ext1, e_or_fock, seg_sizes, efact
                     stream=None):
     """esum (1-element CUDA float64 tensor) += efact * sum w * (w / eps): the
     fused (T)-energy pass of one block (a4g_energy_contract)."""
-    order = _iarr(den_order) if den_order is not None else None
-    rc = lib().a4g_energy_contract(_i(len(ext0)), _iarr(index_values), _iarr(ext0), ctypes.c_void_p(_ptr(data0)),
-                                   order, _i(len(ext1)), _iarr(ext1), ctypes.c_void_p(_ptr(e_or_fock)),
-                                   _i(len(seg_sizes)), _iarr(seg_sizes), ctypes.c_double(efact),
-                                   ctypes.c_void_p(_ptr(esum)), _stream(stream))
+    order = ints(den_order) if den_order is not None else None
+    rc = lib().a4g_energy_contract(len(ext0), ints(index_values), ints(ext0), _ptr(data0),
+                                   order, len(ext1), ints(ext1), _ptr(e_or_fock),
+                                   len(seg_sizes), ints(seg_sizes), ctypes.c_double(efact),
+                                   _ptr(esum), _on(stream))
     _check(rc, "a4g_energy_contract")
 
 

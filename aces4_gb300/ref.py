@@ -12,7 +12,7 @@ import ctypes
 
 import numpy as np
 
-from ._lib import last_error, lib
+from ._lib import INT, ints, last_error, lib
 
 _i = ctypes.c_int
 _d = ctypes.c_double
@@ -29,6 +29,17 @@ def _dp(a: np.ndarray):
     return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
+def _addr(a: np.ndarray) -> int:
+    """_dp's address, for the calls with declared arguments."""
+    if a.dtype != np.float64 or not (a.flags.c_contiguous or a.flags.f_contiguous):
+        raise TypeError("blocks must be contiguous float64 arrays")
+    return a.__array_interface__["data"][0]
+
+
+def _int(n: int):
+    return INT[n] if 0 <= n < len(INT) else ctypes.byref(_i(n))
+
+
 def get_contraction_ptrn(drank: int, lrank: int, rrank: int, aces_ptrn) -> tuple[int, list[int]]:
     out = (ctypes.c_int * max(1, lrank + rrank))()
     ierr = _i(0)
@@ -41,9 +52,9 @@ def tensor_block_contract(ptrn, l, lext, r, rext, d, dext, nthreads: int = 8) ->
     """D is overwritten with contract(L, R), like tensor_dil_omp.F90:662."""
     ierr = _i(0)
     lib().tensor_block_contract__(
-        ctypes.byref(_i(nthreads)), _iarr(ptrn), _dp(l), ctypes.byref(_i(len(lext))), _iarr(lext),
-        _dp(r), ctypes.byref(_i(len(rext))), _iarr(rext), _dp(d), ctypes.byref(_i(len(dext))),
-        _iarr(dext), ctypes.byref(ierr))
+        _int(nthreads), ints(ptrn), _addr(l), _int(len(lext)), ints(lext),
+        _addr(r), _int(len(rext)), ints(rext), _addr(d), _int(len(dext)),
+        ints(dext), ctypes.byref(ierr))
     return ierr.value
 
 
@@ -63,51 +74,51 @@ def tensor_block_copy(ext, perm_o2n_1based, tin: np.ndarray, out: np.ndarray | N
     (a new array when None)."""
     out = np.empty_like(tin) if out is None else out
     ierr = _i(0)
-    lib().tensor_block_copy__(ctypes.byref(_i(8)), ctypes.byref(_i(len(ext))), _iarr(ext),
-                              _iarr([1] + list(perm_o2n_1based)), _dp(tin), _dp(out), ctypes.byref(ierr))
+    lib().tensor_block_copy__(_int(8), _int(len(ext)), ints(ext),
+                              ints([1] + list(perm_o2n_1based)), _addr(tin), _addr(out), ctypes.byref(ierr))
     return ierr.value, out
 
 
 def tensor_block_add(ext, t0, t1, scale) -> int:
     ierr = _i(0)
-    lib().tensor_block_add__(ctypes.byref(_i(8)), ctypes.byref(_i(len(ext))), _iarr(ext), _dp(t0),
-                             _dp(t1), ctypes.byref(_d(scale)), ctypes.byref(ierr))
+    lib().tensor_block_add__(_int(8), _int(len(ext)), ints(ext), _addr(t0),
+                             _addr(t1), ctypes.byref(_d(scale)), ctypes.byref(ierr))
     return ierr.value
 
 
 def tensor_block_scale(t, ext, f) -> int:
     ierr = _i(0)
-    lib().tensor_block_scale__(ctypes.byref(_i(8)), _dp(t), ctypes.byref(_i(len(ext))), _iarr(ext),
+    lib().tensor_block_scale__(_int(8), _addr(t), _int(len(ext)), ints(ext),
                                ctypes.byref(_d(f)), ctypes.byref(ierr))
     return ierr.value
 
 
 def tensor_block_init(t, ext, v) -> int:
     ierr = _i(0)
-    lib().tensor_block_init__(ctypes.byref(_i(8)), _dp(t), ctypes.byref(_i(len(ext))), _iarr(ext),
+    lib().tensor_block_init__(_int(8), _addr(t), _int(len(ext)), ints(ext),
                               ctypes.byref(_d(v)), ctypes.byref(ierr))
     return ierr.value
 
 
 def tensor_block_norm2(t, ext) -> tuple[float, int]:
     ierr = _i(0)
-    v = lib().tensor_block_norm2__(ctypes.byref(_i(8)), _dp(t), ctypes.byref(_i(len(ext))),
-                                   _iarr(ext), ctypes.byref(ierr))
+    v = lib().tensor_block_norm2__(_int(8), _addr(t), _int(len(ext)),
+                                   ints(ext), ctypes.byref(ierr))
     return v, ierr.value
 
 
 def tensor_block_slice(t, text, sext, beg) -> tuple[int, np.ndarray]:
     s = np.empty(int(np.prod(sext)) if len(sext) else 1)
     ierr = _i(0)
-    lib().tensor_block_slice__(ctypes.byref(_i(8)), ctypes.byref(_i(len(text))), _dp(t), _iarr(text),
-                               _dp(s), _iarr(sext), _iarr(beg), ctypes.byref(ierr))
+    lib().tensor_block_slice__(_int(8), _int(len(text)), _addr(t), ints(text),
+                               _addr(s), ints(sext), ints(beg), ctypes.byref(ierr))
     return ierr.value, s
 
 
 def tensor_block_insert(t, text, s, sext, beg) -> int:
     ierr = _i(0)
-    lib().tensor_block_insert__(ctypes.byref(_i(8)), ctypes.byref(_i(len(text))), _dp(t), _iarr(text),
-                                _dp(s), _iarr(sext), _iarr(beg), ctypes.byref(ierr))
+    lib().tensor_block_insert__(_int(8), _int(len(text)), _addr(t), ints(text),
+                                _addr(s), ints(sext), ints(beg), ctypes.byref(ierr))
     return ierr.value
 
 
