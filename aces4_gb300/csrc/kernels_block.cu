@@ -721,6 +721,10 @@ __global__ void __launch_bounds__(kUpdThreads, 6) update_t2_kernel(UpdParams p, 
                                                            double* norm2, double* partial, unsigned* counter) {
   __shared__ double pn[kUpdA][kUpdB + 1], po[kUpdA][kUpdB + 1];  // [a][b] of the partner tiles
   __shared__ double sa[kUpdA], sb[kUpdB];  // (e_i + e_j) - e_a of the tile's a, e_b of its b
+  // The next update's CTAs may take their places as this one's leave; they wait
+  // here until it has completed before they read anything.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   double acc = 0.0;
   for (int64_t u = blockIdx.x; u < p.units; u += gridDim.x) {
     int64_t r = u;
@@ -1107,17 +1111,31 @@ int launch_update_t2(const int* off, const int* ext, const double* t2new, const 
   p.ea = ext[0], p.ei = ext[1], p.eb = ext[2], p.ej = ext[3];
   p.oa = off[0], p.oi = off[1], p.ob = off[2], p.oj = off[3];
   p.rank1 = rank1, p.ld1 = ld1;
-  p.tiles_a = (p.ea + kUpdA - 1) / kUpdA, p.tiles_b = (p.eb + kUpdB - 1) / kUpdB;
-  p.ta = (p.ea + p.tiles_a - 1) / p.tiles_a, p.tb = (p.eb + p.tiles_b - 1) / p.tiles_b;
+  // the cut of the plane with the fewest passes over a tile (kUpdGroup x
+  // kUpdThreads elements a pass), a quarter of a pass for each tile's ends;
+  // tiles of 8 and more a side where the plane has them
+  int64_t best = 0;
+  for (int na = (p.ea + kUpdA - 1) / kUpdA, a_end = std::max(na, std::min(na + 3, p.ea / 8)); na <= a_end; ++na)
+    for (int nb = (p.eb + kUpdB - 1) / kUpdB, b_end = std::max(nb, std::min(nb + 3, p.eb / 8)); nb <= b_end; ++nb) {
+      const int ta = (p.ea + na - 1) / na, tb = (p.eb + nb - 1) / nb;
+      const int64_t passes = (ta * tb + kUpdGroup * kUpdThreads - 1) / (kUpdGroup * kUpdThreads);
+      const int64_t cost = int64_t(na) * nb * (4 * passes + 1);
+      if (!best || cost < best) best = cost, p.tiles_a = na, p.tiles_b = nb, p.ta = ta, p.tb = tb;
+    }
   p.mul_a = ((1u << 20) + p.ta - 1) / p.ta, p.mul_b = ((1u << 20) + p.tb - 1) / p.tb;
   p.units = int64_t(p.tiles_a) * p.tiles_b * p.ei * p.ej;
   if (p.units == 0) return A4G_OK;
   // one resident wave (6 CTAs of 128 threads per SM): its CTAs share the units evenly
   const int sms = ctx()->num_sms > 0 ? ctx()->num_sms : 152;
   const int64_t wave = std::min<int64_t>(kDotBlocks, 6 * int64_t(sms));
-  update_t2_kernel<<<unsigned(std::min(p.units, wave)), kUpdThreads, 0, s>>>(
-      p, t2new, t2new_pair, t2old, t2old_pair, err, next, e_or_fock, norm2, slot.partial, slot.counter);
-  A4G_CUDA(cudaGetLastError());
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(std::min(p.units, wave))), cfg.blockDim = dim3(kUpdThreads), cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at, cfg.numAttrs = 1;
+  A4G_CUDA(cudaLaunchKernelEx(&cfg, update_t2_kernel, p, t2new, t2new_pair, t2old, t2old_pair, err, next, e_or_fock, norm2,
+                              slot.partial, slot.counter));
   return A4G_OK;
 }
 
