@@ -1429,26 +1429,25 @@ __device__ __forceinline__ void exp_generic(const OzSplitJob& jb, const OzPanel&
   if (part == 0 && r0 + r < jb.rows && m > 0) atomicMax(&pn.exps[r0 + r], m);
 }
 
-// Row maxima of a column-major [rows x K] block (rows contiguous) over a
-// kExpRowsK-wide k range: a thread owns two rows (one 16-byte load per k) and every
-// KG-th k, KG as many as 256 threads allow for the block's rows (a 144-row
-// block: 96 threads for the rows, 2 k at a time), eight loads in flight; the
-// row maxima meet in shared memory.
-constexpr int kExpRowsK = 32;
+// Row maxima of a column-major [rows x K] block (rows contiguous): 64 rows and
+// up to kExpRowsK k of them.  A thread owns two rows (one 16-byte load per k)
+// and every KG-th k, eight loads in flight; the row maxima meet in shared
+// memory, and a row's k range in one global atomic (pieces of 512 rows x 32 k
+// sent one per row and 32 k: the o=10/v=48 step's
+// pass 19 us instead of 15).
+constexpr int kExpRows = 64, kExpRowsK = 256;
 __device__ __forceinline__ void exp_rows(const OzSplitJob& jb, const OzPanel& pn, int t, int* best) {
   const int ktiles = (jb.K + kExpRowsK - 1) / kExpRowsK;
-  const int r0 = (t / ktiles) * 512, k0 = (t % ktiles) * kExpRowsK;
-  const int rows = min(512, jb.rows - r0), kn = min(kExpRowsK, jb.K - k0);
-  const int rp = ((rows + 1) / 2 + 31) & ~31, kg = 256 / rp;
+  const int r0 = (t / ktiles) * kExpRows, k0 = (t % ktiles) * kExpRowsK;
+  const int rows = min(kExpRows, jb.rows - r0), kn = min(kExpRowsK, jb.K - k0);
+  const int rp = rows > 32 ? 32 : rows > 16 ? 16 : 8, kg = 256 / rp;
   const int lane = threadIdx.x % rp, kq = threadIdx.x / rp;
-  if (kg > 1) {
-    for (int i = threadIdx.x; i < rows; i += 256) best[i] = 0;
-    __syncthreads();
-  }
+  if (threadIdx.x < kExpRows) best[threadIdx.x] = 0;
+  __syncthreads();
   const int r = 2 * lane;
   unsigned long long m0 = 0, m1 = 0;
   constexpr unsigned long long kExp = 0x7FF0000000000000ull;
-  if (kq < kg && r < rows) {
+  if (r < rows) {
     const double* base = jb.src + size_t(k0) * jb.rows + r0 + r;
     if (r + 1 < rows && (jb.rows & 1) == 0) {
 #pragma unroll 8
@@ -1465,15 +1464,11 @@ __device__ __forceinline__ void exp_rows(const OzSplitJob& jb, const OzPanel& pn
         if (two) m1 = max(m1, __double_as_longlong(__ldg(base + size_t(k) * jb.rows + 1)) & kExp);
       }
     }
-    int* e = kg > 1 ? best : pn.exps + r0;
-    if (m0) atomicMax(&e[r], int(m0 >> 52));
-    if (m1) atomicMax(&e[r + 1], int(m1 >> 52));
+    if (m0) atomicMax(&best[r], int(m0 >> 52));
+    if (m1) atomicMax(&best[r + 1], int(m1 >> 52));
   }
-  if (kg > 1) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < rows; i += 256)
-      if (best[i]) atomicMax(&pn.exps[r0 + i], best[i]);
-  }
+  __syncthreads();
+  if (threadIdx.x < rows && best[threadIdx.x]) atomicMax(&pn.exps[r0 + threadIdx.x], best[threadIdx.x]);
 }
 
 // Row maxima of a [K x rows] block (k contiguous): one warp per row.
@@ -2046,7 +2041,7 @@ int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t row
 }
 
 int64_t oz_exp_tiles(int layout, int rows, int K) {
-  if (layout == kOzRowsMajor) return int64_t((rows + 511) / 512) * ((K + kExpRowsK - 1) / kExpRowsK);
+  if (layout == kOzRowsMajor) return int64_t((rows + kExpRows - 1) / kExpRows) * ((K + kExpRowsK - 1) / kExpRowsK);
   if (layout == kOzKMajor) return (rows + 31) / 32;
   return int64_t((rows + 63) / 64) * ((K + 63) / 64);
 }
