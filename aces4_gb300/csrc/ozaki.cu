@@ -1227,6 +1227,11 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
   const int q = warp & 3, h = (warp - 2) >> 2;
   const int row = 32 * q + lane;
   const uint32_t lane_addr = tmem + (uint32_t(32 * q) << 16) + uint32_t(16 * h);
+  // 256^t, hidden from the compiler: a level joins the sum with one 32 x 32 + 64
+  // bit multiply-add instead of five shifts and additions
+  int weight[4];
+  asm volatile("mov.b32 %0, 1;\n\tmov.b32 %1, 256;\n\tmov.b32 %2, 65536;\n\tmov.b32 %3, 16777216;"
+               : "=r"(weight[0]), "=r"(weight[1]), "=r"(weight[2]), "=r"(weight[3]));
   [[maybe_unused]] double eacc = 0.0;
   uint32_t nt = 0;
   for (int g = int(blockIdx.x); g < a.n_tiles; g += int(gridDim.x), ++nt) {
@@ -1254,9 +1259,10 @@ __device__ void lv_epilogue(const OzGemmArgs& a, LvSmem& sm, uint32_t tmem, int 
         long long r = 0;
 #pragma unroll
         for (int t = 0; t < S; ++t) {
-            long long st = __float2int_rz(__uint_as_float(v[lv_acc(t, 0)][j]));
-            if (t >= 3) st += __float2int_rz(__uint_as_float(v[lv_acc(t, 1)][j]));
-            r = r * 256 + st;
+          int st = __float2int_rz(__uint_as_float(v[lv_acc(t, 0)][j]));
+          if (t >= 3) st += __float2int_rz(__uint_as_float(v[lv_acc(t, 1)][j]));
+          if (S - 1 - t == 4) r = (long long)((unsigned long long)uint32_t(st) << 32);
+          else asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(r) : "r"(st), "r"(weight[S - 1 - t]));
         }
         sum[8 * gg + j] = r;
       }
