@@ -41,14 +41,16 @@ __device__ __forceinline__ double ew(double d, double s, double a) {
 }
 
 // Bound by HBM, or by the FP64 pipes where an element takes two operations
-// (add_scaled: 340 us for 96^4 elements, of 338 measured).  Two reads and a
-// write: a CTA per 2 x 256 pairs and no loop (358 us with the grid held to 8
-// CTAs per SM); fewer streams: the held grid (scale_copy 209 us, 241 without).
+// (add_scaled: 340 us for 96^4 elements, of 336 measured).  A CTA per share of
+// 256 threads x 4 pairs (a fill: 8), all loaded before the first is stored, and
+// no loop.  96^4 elements, grid held to 8 CTAs per SM and one pair at a time ->
+// now: scale_copy 234 -> 201 us (24^6: 527 -> 440), add 364 -> 285, fill 108 ->
+// 93; two pairs: scale_copy 252; eight: 198, but a 20^4 block 8.9 us, not 7.4.
 template <EwOp OP>
 struct EwReads {
   static constexpr bool d = !(OP == EwOp::kFill || OP == EwOp::kScaleCopy);
   static constexpr bool s = OP == EwOp::kScaleCopy || OP == EwOp::kAddScaled || OP == EwOp::kAdd || OP == EwOp::kAxpy;
-  static constexpr int pairs = d && s ? 2 : 1;  // a thread's, all loaded before the first is stored
+  static constexpr int pairs = d || s ? 4 : 8;
 };
 template <EwOp OP, bool VEC>
 __global__ void __launch_bounds__(kThreads) ew_kernel(double* __restrict__ d,
@@ -92,8 +94,7 @@ int launch_ew(double* d, const double* s, int64_t n, double a, cudaStream_t st) 
   if (!d) return fail(A4G_ERR_ARG, "null block pointer");
   const bool vec = aligned16(d) && (s == nullptr || aligned16(s));
   constexpr int kShare = EwReads<OP>::pairs * kThreads;
-  const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((n / 2 + kShare - 1) / kShare, 0x7fffffff));
-  const int64_t g = EwReads<OP>::pairs > 1 ? ctas : grid_for(n / 2 + 1);
+  const int64_t g = std::max<int64_t>(1, std::min<int64_t>((n / 2 + kShare - 1) / kShare, 0x7fffffff));
   if (vec) ew_kernel<OP, true><<<unsigned(g), kThreads, 0, st>>>(d, s, n, a);
   else ew_kernel<OP, false><<<grid_for(n), kThreads, 0, st>>>(d, s, n, a);
   A4G_CUDA(cudaGetLastError());
@@ -175,8 +176,73 @@ __device__ __forceinline__ double perm_op(const double* l, int64_t o, double rv)
   else return __dsub_rn(l[o], rv);
 }
 
+// Division of an unsigned below 2^31 by d: x * mul >> 31 + shift, exact.
+struct FastDiv {
+  unsigned mul;
+  int shift;
+};
+FastDiv fast_div(unsigned d) {
+  FastDiv f{0, 0};
+  while ((uint64_t(1) << f.shift) < d) ++f.shift;
+  f.mul = unsigned(((uint64_t(1) << (31 + f.shift)) + d - 1) / d);
+  return f;
+}
+__device__ __forceinline__ unsigned fast_quot(unsigned x, FastDiv f) {
+  return unsigned((uint64_t(x) * f.mul) >> (31 + f.shift));
+}
+
 // Input dim 0 is also output dim 0: runs of dim 0 are contiguous on both
-// sides; a block takes several runs and decodes each run's output offset once.
+// sides.  As T (pairs where every run starts on 16 bytes and has an even length,
+// else single elements), kPermLoads a thread in input order, all loaded before
+// the first is stored; fewer than 2^31 elements.  (A CTA per 96-element run:
+// 432 us on 96^4 elements, 199 now; with an addition 464 and 290.)
+constexpr int kPermLoads = 4;
+struct PermRuns {
+  int rank;
+  unsigned ext[kPermMax];
+  FastDiv div[kPermMax];
+  int64_t sout[kPermMax];
+};
+template <int OP, class T>
+__global__ void __launch_bounds__(kThreads) perm_runs_kernel(PermRuns p, const T* __restrict__ in, T* out, const T* l,
+                                                             unsigned n) {
+  const unsigned first = blockIdx.x * (kThreads * kPermLoads) + threadIdx.x;
+  int64_t at[kPermLoads];
+  T v[kPermLoads], lv[kPermLoads];
+#pragma unroll
+  for (int u = 0; u < kPermLoads; ++u) {
+    const unsigned i = first + u * kThreads;
+    unsigned rem = i;
+    int64_t o = 0;
+    for (int q = 0; q < p.rank - 1; ++q) {
+      const unsigned d = fast_quot(rem, p.div[q]);
+      o += int64_t(rem - d * p.ext[q]) * p.sout[q];
+      rem = d;
+    }
+    at[u] = o + int64_t(rem) * p.sout[p.rank - 1];
+    if (i < n) {
+      v[u] = in[i];
+      if constexpr (OP != 0) lv[u] = l[at[u]];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kPermLoads; ++u) {
+    if (first + u * kThreads >= n) continue;
+    if constexpr (OP == 0) {
+      out[at[u]] = v[u];
+    } else if constexpr (sizeof(T) == sizeof(double2)) {
+      T x;
+      x.x = OP == 1 ? __dadd_rn(lv[u].x, v[u].x) : __dsub_rn(lv[u].x, v[u].x);
+      x.y = OP == 1 ? __dadd_rn(lv[u].y, v[u].y) : __dsub_rn(lv[u].y, v[u].y);
+      out[at[u]] = x;
+    } else {
+      out[at[u]] = OP == 1 ? __dadd_rn(lv[u], v[u]) : __dsub_rn(lv[u], v[u]);
+    }
+  }
+}
+
+// The same beyond 2^31 elements: a block takes several runs and decodes each
+// run's output offset once.
 template <int OP>
 __global__ void __launch_bounds__(kThreads) perm_direct_kernel(PermParams p, const double* __restrict__ in,
                                                                double* out, const double* l, int64_t nruns,
@@ -278,19 +344,38 @@ template <int OP>
 int launch_perm_op(const PermParams& p, const double* in, double* out, const double* l, int64_t total,
                    cudaStream_t s) {
   const int sms = ctx()->num_sms > 0 ? ctx()->num_sms : 152;
-  const int64_t want = int64_t(sms) * 16;  // blocks to aim for
   if (p.rank <= 1 || p.b_dim == p.a_dim) {
+    if (total <= 0) return A4G_OK;
+    if (total <= 0x7fffffff - kThreads * kPermLoads) {
+      PermRuns r{};
+      r.rank = std::max(1, p.rank);
+      bool pairs = aligned16(in) && aligned16(out) && (OP == 0 || aligned16(l)) && (p.ext[0] & 1) == 0;
+      for (int q = 1; q < p.rank; ++q) pairs = pairs && (p.sout[q] & 1) == 0;
+      for (int q = 0; q < r.rank; ++q) {
+        r.ext[q] = unsigned(q == 0 && pairs ? p.ext[0] / 2 : p.ext[q]);
+        r.sout[q] = q > 0 && pairs ? p.sout[q] / 2 : p.sout[q];
+        r.div[q] = fast_div(r.ext[q]);
+      }
+      const unsigned n = unsigned(pairs ? total / 2 : total), grid = (n + kThreads * kPermLoads - 1) / (kThreads * kPermLoads);
+      if (pairs)
+        perm_runs_kernel<OP><<<grid, kThreads, 0, s>>>(r, reinterpret_cast<const double2*>(in), reinterpret_cast<double2*>(out),
+                                                       reinterpret_cast<const double2*>(l), n);
+      else perm_runs_kernel<OP><<<grid, kThreads, 0, s>>>(r, in, out, l, n);
+      A4G_CUDA(cudaGetLastError());
+      return A4G_OK;
+    }
     const int E0 = p.rank >= 1 ? p.ext[0] : 1;
     const int64_t nruns = total / E0;
     const int threads = E0 >= kThreads ? kThreads : (E0 + 31) / 32 * 32;
-    const int rpb = int(std::max<int64_t>(1, std::min<int64_t>(64, nruns / want)));
+    const int rpb = int(std::max<int64_t>(1, std::min<int64_t>(64, nruns / (int64_t(sms) * 16))));
     const int64_t blocks = (nruns + rpb - 1) / rpb;
     if (blocks > 0x7fffffffLL) return fail(A4G_ERR_RANGE, "permute grid too large");
     if (blocks > 0) perm_direct_kernel<OP><<<unsigned(blocks), threads, 0, s>>>(p, in, out, l, nruns, rpb);
   } else {
     const int Ea = p.ext[p.a_dim], Eb = p.ext[p.b_dim];
     const int64_t tiles = int64_t((Ea + kTile - 1) / kTile) * ((Eb + kTile - 1) / kTile);
-    const int rpb = 2 * int(std::max<int64_t>(1, std::min<int64_t>(8, p.n_rest_total * tiles / (2 * want))));
+    // up to four slices a block (sixteen: 33 x 20 x 29 x 20 in 12.0 us instead of 11.3; two: 96^4 in 259, not 248)
+    const int rpb = 2 * int(std::max<int64_t>(1, std::min<int64_t>(2, p.n_rest_total * tiles / (int64_t(sms) * 32))));
     const int64_t blocks = tiles * ((p.n_rest_total + rpb - 1) / rpb);
     if (blocks > 0x7fffffffLL) return fail(A4G_ERR_RANGE, "permute grid too large");
     perm_tiled_kernel<OP><<<unsigned(blocks), dim3(kTile, 8), 0, s>>>(p, in, out, l, rpb);
@@ -398,8 +483,7 @@ struct SliceParams {
   int sext[kPermMax];
   int64_t tstride[kPermMax];
   int64_t tbase;
-  unsigned mul[kPermMax];  // slice_runs_kernel: division by sext
-  int shift[kPermMax];
+  FastDiv div[kPermMax];  // slice_runs_kernel: division by sext
 };
 
 // Beyond 2^31 slice elements: an element at a time, 64-bit divisions.
@@ -421,8 +505,8 @@ __global__ void __launch_bounds__(kThreads) slice_insert_kernel(SliceParams p, i
 
 // Fewer than 2^31 slice elements, as T (pairs where every run starts on 16
 // bytes and has an even length, else single elements): kSliceLoads a thread, all
-// loaded before the first is stored, offsets by multiplications (x / d = x *
-// mul >> 31 + shift, exact below 2^31).  HBM bounds it; an element's 64-bit
+// loaded before the first is stored, offsets by multiplications
+// (FastDiv).  HBM bounds it; an element's 64-bit
 // divisions did: a 72^4 slice of a 96^4
 // block 190 -> 66 us, its insertion 190 -> 60.
 constexpr int kSliceLoads = 4;
@@ -438,7 +522,7 @@ __global__ void __launch_bounds__(kThreads) slice_runs_kernel(SliceParams p, T* 
     unsigned rem = i;
     int64_t o = p.tbase;
     for (int q = 0; q < p.rank - 1; ++q) {
-      const unsigned d = unsigned((uint64_t(rem) * p.mul[q]) >> (31 + p.shift[q]));
+      const unsigned d = fast_quot(rem, p.div[q]);
       o += int64_t(rem - d * unsigned(p.sext[q])) * p.tstride[q];
       rem = d;
     }
@@ -1024,10 +1108,7 @@ int launch_slice_insert(int insert, int rank, double* tens, const int* tens_ext,
     n /= 2, m.sext[0] /= 2, m.tbase /= 2;
     for (int q = 1; q < m.rank; ++q) m.tstride[q] /= 2;
   }
-  for (int q = 0; q < m.rank; ++q) {
-    while ((int64_t(1) << m.shift[q]) < m.sext[q]) ++m.shift[q];
-    m.mul[q] = unsigned(((uint64_t(1) << (31 + m.shift[q])) + uint64_t(m.sext[q]) - 1) / uint64_t(m.sext[q]));
-  }
+  for (int q = 0; q < m.rank; ++q) m.div[q] = fast_div(unsigned(m.sext[q]));
   const unsigned grid = unsigned((n + kThreads * kSliceLoads - 1) / (kThreads * kSliceLoads));
   if (pairs && insert) slice_runs_kernel<1><<<grid, kThreads, 0, s>>>(m, reinterpret_cast<double2*>(tens), reinterpret_cast<double2*>(slice), unsigned(n));
   else if (pairs) slice_runs_kernel<0><<<grid, kThreads, 0, s>>>(m, reinterpret_cast<double2*>(tens), reinterpret_cast<double2*>(slice), unsigned(n));
