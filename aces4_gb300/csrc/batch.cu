@@ -972,8 +972,8 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
     ga.nsplit = nsplit;
     ga.residue = b->residue ? 1 : 0;
     for (int t = 0; t < kOzMaxResidues; ++t)
-      ga.chunk_kb[t] = b->residue ? kOzResidueChunkKb : t < S ? oz_chunk_kb(t) : 1, ga.res_p[t] = b->crt.p[t],
-      ga.res_inv[t] = b->crt.inv[t];
+      ga.chunk_kb[t] = b->residue ? kOzResidueChunkKb : t < S ? oz_chunk_kb(t) : 1, ga.res_p[t] = -b->crt.np[t].x,
+      ga.res_inv[t] = b->crt.inv[t].x;
     ga.err_flag = ctx()->d_error_flag;
     ga.direct = gf.direct ? 1 : 0;
     ga.mode = b->store_mode();

@@ -185,10 +185,12 @@ struct OzResidues {
 struct OzCrt {
   int L, slices;
   int words;  // 32-bit words of the reconstruction: 3 when |sum| < 2^95, else 4
-  float p[kOzMaxResidues], inv[kOzMaxResidues];
-  float cinv[kOzMaxResidues];  // (P / p)^-1 modulo p, P the product of the moduli
+  // each twice, as the packed FP32 instructions take them: -p, the FP32
+  // nearest 1/p, (P / p)^-1 modulo p, P the product of the moduli
+  float2 np[kOzMaxResidues], inv[kOzMaxResidues], cinv[kOzMaxResidues];
   int m[kOzMaxResidues][4];    // P / p modulo 2^128, signed 32-bit words
   int prod[4];                 // P modulo 2^128
+  long long base[4];           // -0x4B400000 sum_i m[i][w]: the integers come with the bits of 1.5 2^23
 };
 
 struct OzGemmArgs {

@@ -273,38 +273,65 @@ constexpr size_t kGenericSmem = kSplitT * (kSplitT + 1) * sizeof(unsigned long l
 //     k = rint(sum_i y_i / p_i)
 // in W signed 32-bit word columns of 64-bit sums, modulo 2^(32 W): three words
 // hold |X| < 2^95, four |X| < 2^127.
+// Two sums at a time: the residue arithmetic in packed FP32.
 template <int W>
-struct Crt {
-  long long col[W];
-  float turns;
-  __device__ __forceinline__ void clear() {
-    turns = 0.0f;
+struct CrtPair {
+  long long col[2][W];
+  F32x2 turns;
+  __device__ __forceinline__ void clear(const OzCrt& T) {
+    turns = 0ull;  // two +0
 #pragma unroll
-    for (int w = 0; w < W; ++w) col[w] = 0;
+    for (int w = 0; w < W; ++w) col[0][w] = col[1][w] = T.base[w];
   }
-  // |s| < 2^14, |cinv| < 2^8: the product is an exact FP32 integer
-  __device__ __forceinline__ void add(const OzCrt& T, int i, int s) {
-    const float v = __fmul_rn(float_of_small(s), T.cinv[i]);
-    const float y = fmaf(-T.p[i], __fsub_rn(fmaf(v, T.inv[i], kRintMagic), kRintMagic), v);
-    turns = fmaf(y, T.inv[i], turns);
-    const int yi = int_of_small(y);
+  // two biased residues (16-bit halves of s, below 2^15 + 2^8) less the bias
+  // in `unbias` = -2^23 - bias; |s| < 2^14, |cinv| < 2^8: the product is an exact
+  // FP32 integer.  The integers enter the columns with the bits of 1.5 2^23 and
+  // T.base takes them out again (modulo 2^64, like every step of a column).
+  __device__ __forceinline__ void add(const OzCrt& T, int i, int s, F32x2 unbias, F32x2 magic, F32x2 unmagic) {
+    const F32x2 x = add2(pack2(__uint_as_float(__byte_perm(uint32_t(s), 0x4B000000u, 0x7610)),
+                               __uint_as_float(__byte_perm(uint32_t(s), 0x4B000000u, 0x7632))),
+                         unbias);
+    const F32x2 v = fma2(x, packed(T.cinv[i]), 0ull);
+    const F32x2 y = fma2(packed(T.np[i]), add2(fma2(v, packed(T.inv[i]), magic), unmagic), v);
+    turns = fma2(y, packed(T.inv[i]), turns);
+    float y0, y1;
+    unpack2(add2(y, magic), y0, y1);
 #pragma unroll
-    for (int w = 0; w < W; ++w) col[w] = mad_wide(yi, T.m[i][w], col[w]);
+    for (int w = 0; w < W; ++w) {
+      col[0][w] = mad_wide(int(__float_as_uint(y0)), T.m[i][w], col[0][w]);
+      col[1][w] = mad_wide(int(__float_as_uint(y1)), T.m[i][w], col[1][w]);
+    }
   }
-  __device__ __forceinline__ double value(const OzCrt& T, int e2, bool neg) {
+  __device__ __forceinline__ void value(const OzCrt& T, const int (&e2)[2], bool neg, double (&out)[2]) {
+    float t0, t1;
+    unpack2(turns, t0, t1);
+    out[0] = one(T, col[0], t0, e2[0], neg);
+    out[1] = one(T, col[1], t1, e2[1], neg);
+  }
+  static __device__ __forceinline__ double one(const OzCrt& T, long long (&c)[W], float turns, int e2, bool neg) {
     const int k = 0x4B400000 - int(__float_as_uint(__fadd_rn(turns, kRintMagic)));
 #pragma unroll
-    for (int w = 0; w < W; ++w) col[w] = mad_wide(k, T.prod[w], col[w]);
-    unsigned __int128 x = (unsigned __int128)(__int128)col[0] + ((unsigned __int128)(__int128)col[1] << 32);
+    for (int w = 0; w < W; ++w) c[w] = mad_wide(k, T.prod[w], c[w]);
+    unsigned __int128 x = (unsigned __int128)(__int128)c[0] + ((unsigned __int128)(__int128)c[1] << 32);
     if constexpr (W == 4) {
-      x += ((unsigned __int128)(__int128)col[2] << 64) + ((unsigned __int128)(unsigned long long)col[3] << 96);
+      x += ((unsigned __int128)(__int128)c[2] << 64) + ((unsigned __int128)(unsigned long long)c[3] << 96);
     } else {
-      const long long hi = (long long)(unsigned long long)(x >> 64) + col[2];
+      const long long hi = (long long)(unsigned long long)(x >> 64) + c[2];
       x = ((unsigned __int128)(unsigned long long)(long long)int(hi) << 64) | (unsigned long long)x;  // 96 bits, signed
     }
     const bool minus = (__int128)x < 0;
     const unsigned __int128 u = minus ? -x : x;
     const unsigned long long hi = (unsigned long long)(u >> 64), lo = (unsigned long long)u;
+    if constexpr (W == 3) {
+      // |X| in [2^64, 2^95) without a branch: its top 62 bits, the last one sticky
+      const uint32_t h = uint32_t(hi), m = uint32_t(lo >> 32), l = uint32_t(lo);
+      const int n = __clz(int(h | 1u));
+      const uint32_t top = __funnelshift_l(m, h, n), low = __funnelshift_l(l, m, n), rest = l << n;
+      const unsigned long long kept = ((unsigned long long)top << 32 | low) >> 2;
+      const long long v = (long long)(kept | ((low & 3u) | rest ? 1ull : 0ull));
+      double r;
+      if (i64_scaled_normal(v, e2 + 34 - n, &r) && h) return minus != neg ? -r : r;
+    }
     // the top 62 bits, what is below them folded into the last (a sticky bit:
     // the rounding position lies above it)
     const int sh = (hi ? 64 - clz64(hi) : -clz64(lo | 1ull)) + 2;
@@ -325,10 +352,12 @@ struct Crt {
 // residues (two non-negative 16-bit sums in one 32-bit one: at most 64 splits
 // of at most 512), reconstructs, scales and
 // stores along D's unit-stride dimension (through shared memory when that is
-// n).
+// n).  About 200 instructions an element and the loads' latency bound it, not
+// HBM: four CTAs per SM (up to 12 moduli; more spill) and packed residue
+// arithmetic took the o=40/v=300 ring step's reconstruction from 2.57 to 2.02 ms.
 constexpr int kRecThreads = 256;
 template <int L, int W>
-__global__ void __launch_bounds__(kRecThreads, 3) oz_residue_recombine_kernel(
+__global__ void __launch_bounds__(kRecThreads, L <= 12 && W == 3 ? 4 : 3) oz_residue_recombine_kernel(
     const __grid_constant__ OzCrt T, const OzTile* __restrict__ tiles, const OzDBlock* __restrict__ dblocks,
     const OzPanel* __restrict__ pa, const OzPanel* __restrict__ pb, const int16_t* __restrict__ ws, int log_rows,
     int log_cols, int nsplit, int mode) {
@@ -337,20 +366,22 @@ __global__ void __launch_bounds__(kRecThreads, 3) oz_residue_recombine_kernel(
   const int tile = blockIdx.x >> (log_rp + log_cp);
   const int piece = blockIdx.x & ((1 << (log_rp + log_cp)) - 1);
   const int sr = (piece & ((1 << log_rp) - 1)) * 64, sc = (piece >> log_rp) * 8;
+  const int rp = 2 * (threadIdx.x & 31), cl = threadIdx.x >> 5;
+  const size_t plane = size_t(1) << (log_rows + log_cols);  // one split's [cols][rows]
+  const int* q = reinterpret_cast<const int*>(ws + size_t(tile) * L * nsplit * plane +
+                                              (size_t(sc + cl) << log_rows) + sr + rp);
+  const size_t step = size_t(nsplit) * plane / 2;
+  // the first split's loads leave before the tile's tables are known (a tile's
+  // workspace is whole, whatever of it lies in D)
+  int s[L];
+#pragma unroll
+  for (int i = 0; i < L; ++i) s[i] = __ldg(q + size_t(i) * step);
   const OzTile tl = tiles[tile];
   const OzDBlock db = dblocks[tl.dblock];
   if (tl.n0 + sc >= db.N || tl.m0 + sr >= db.M) return;  // the piece lies beyond D
-  const int rp = 2 * (threadIdx.x & 31), cl = threadIdx.x >> 5;
   const int m = tl.m0 + sr + rp, n = tl.n0 + sc + cl;
   double v[2] = {0.0, 0.0};
   if (m < db.M && n < db.N) {
-    const size_t plane = size_t(1) << (log_rows + log_cols);  // one split's [cols][rows]
-    const int* q = reinterpret_cast<const int*>(ws + size_t(tile) * L * nsplit * plane +
-                                                (size_t(sc + cl) << log_rows) + sr + rp);
-    const size_t step = size_t(nsplit) * plane / 2;
-    int s[L];
-#pragma unroll
-    for (int i = 0; i < L; ++i) s[i] = __ldg(q + size_t(i) * step);
     for (int sp = 1; sp < nsplit; ++sp)
 #pragma unroll
       for (int i = 0; i < L; ++i) s[i] += __ldg(q + size_t(i) * step + size_t(sp) * (plane / 2));
@@ -358,15 +389,14 @@ __global__ void __launch_bounds__(kRecThreads, 3) oz_residue_recombine_kernel(
     const int e0 = pa[tl.panel_a].exps[m], f = pb[tl.panel_b].exps[n];
     const int e1 = m + 1 < db.M ? pa[tl.panel_a].exps[m + 1] : 0;
     const int F = (f ? f : 1) - 1022 + 2 - 2 * kDigitBits * T.slices;
-    Crt<W> c0, c1;
-    c0.clear(), c1.clear();
+    CrtPair<W> crt;
+    crt.clear(T);
+    const float off = -8388608.0f - float(bias);
+    const F32x2 unbias = pack2(off, off), magic = pack2(kRintMagic, kRintMagic), unmagic = pack2(-kRintMagic, -kRintMagic);
 #pragma unroll
-    for (int i = 0; i < L; ++i) {
-      c0.add(T, i, (s[i] & 0xFFFF) - bias);
-      c1.add(T, i, int(uint32_t(s[i]) >> 16) - bias);
-    }
-    v[0] = c0.value(T, (e0 ? e0 : 1) - 1022 + F, mode & 2);
-    v[1] = c1.value(T, (e1 ? e1 : 1) - 1022 + F, mode & 2);
+    for (int i = 0; i < L; ++i) crt.add(T, i, s[i], unbias, magic, unmagic);
+    const int e2[2] = {(e0 ? e0 : 1) - 1022 + F, (e1 ? e1 : 1) - 1022 + F};
+    crt.value(T, e2, mode & 2, v);
     if (e0 == kNonFiniteExp || f == kNonFiniteExp) v[0] = __longlong_as_double(0x7FF8000000000000ll);
     if (e1 == kNonFiniteExp || f == kNonFiniteExp) v[1] = __longlong_as_double(0x7FF8000000000000ll);
   }
@@ -422,10 +452,8 @@ void oz_residue_tables(int slices, int L, int64_t K, OzResidues* r, OzCrt* t) {
   signed_words(prod, t->prod);
   for (int i = 0; i < L; ++i) {
     const int p = kModuli[i];
-    t->p[i] = float(p);
-    t->inv[i] = 1.0f / float(p);
-    r->np[i] = make_float2(-t->p[i], -t->p[i]);
-    r->inv[i] = make_float2(t->inv[i], t->inv[i]);
+    r->np[i] = t->np[i] = make_float2(-float(p), -float(p));
+    r->inv[i] = t->inv[i] = make_float2(1.0f / float(p), 1.0f / float(p));
     for (int q = 0; q < 3; ++q) {
       const float c = float(symmetric(1ll << (14 * (q + 1)), p));
       r->c[q][i] = make_float2(c, c);
@@ -435,7 +463,10 @@ void oz_residue_tables(int slices, int L, int64_t K, OzResidues* r, OzCrt* t) {
     for (int j = 0; j < L; ++j)
       if (j != i) m *= unsigned(kModuli[j]), mp = mp * kModuli[j] % p;
     signed_words(m, t->m[i]);
-    t->cinv[i] = float(symmetric(inverse_mod(int(mp), p), p));
+    const float c = float(symmetric(inverse_mod(int(mp), p), p));
+    t->cinv[i] = make_float2(c, c);
+    for (int w = 0; w < 4; ++w)
+      t->base[w] = (long long)((unsigned long long)t->base[w] - 0x4B400000ull * (unsigned long long)(long long)t->m[i][w]);
   }
 }
 
