@@ -736,10 +736,10 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
       p.base = static_cast<__nv_bfloat16*>(mem);
       p.exps = b->d_exps + eoff;
       eoff += p.rows_pad;
-      r = oz_make_tensor_map(maps[i].b, mem, p.kpad, int64_t(NP) * p.rows_pad, kOzBM);
+      r = oz_make_tensor_map(maps[i].b, mem, p.kpad, p.rows, p.rows_pad, NP, kOzBM);
       if (r) return r;
-      if (maps2 && (r = oz_make_tensor_map((*maps2)[i].b, mem, p.kpad, int64_t(NP) * p.rows_pad, 64))) return r;
-      if (maps3 && (r = oz_make_tensor_map((*maps3)[i].b, mem, p.kpad, int64_t(NP) * p.rows_pad, 256))) return r;
+      if (maps2 && (r = oz_make_tensor_map((*maps2)[i].b, mem, p.kpad, p.rows, p.rows_pad, NP, 64))) return r;
+      if (maps3 && (r = oz_make_tensor_map((*maps3)[i].b, mem, p.kpad, p.rows, p.rows_pad, NP, 256))) return r;
       dst.push_back(p);
     }
     return A4G_OK;

@@ -821,9 +821,9 @@ int a4g_fused_create(a4g_fused** out, int drank, int lrank, int rrank, const a4g
       hp[i].base = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(p) + at[i]);
       hp[i].exps = f->d_exps + offset_of(hp[i].exps);
       // all-levels form: every slice's 32-wide k box of 128 rows (A) or 64 columns (B)
-      rc = P.levels ? oz_make_levels_map(maps[i].b, hp[i].base, hp[i].kpad, hp[i].rows_pad, S,
+      rc = P.levels ? oz_make_levels_map(maps[i].b, hp[i].base, hp[i].kpad, hp[i].rows, hp[i].rows_pad, S,
                                          int(i) >= P.nA ? kOzLevelsTileCols : kOzBM)
-                    : oz_make_tensor_map(maps[i].b, hp[i].base, hp[i].kpad, int64_t(S) * hp[i].rows_pad, kOzBM);
+                    : oz_make_tensor_map(maps[i].b, hp[i].base, hp[i].kpad, hp[i].rows, hp[i].rows_pad, S, kOzBM);
       if (rc) return rc;
     }
     MapImage* d_maps = nullptr;

@@ -192,13 +192,6 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(p));
   return p != 0;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, uint32_t bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-          dst),
-      "l"(map), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
@@ -248,12 +241,12 @@ __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar_cluster, uin
 }
 // TMA load into this CTA's shared memory that signals an mbarrier which may
 // live in either CTA of the pair
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* map, uint32_t bar_cluster, int c0,
-                                                 int c1) {
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void* map, uint32_t bar_cluster, int c0, int c1,
+                                                 int c2) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::"r"(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
           dst),
-      "l"(map), "r"(bar_cluster), "r"(c0), "r"(c1)
+      "l"(map), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
 template <int N>
@@ -379,30 +372,27 @@ __device__ void producer(const OzGemmArgs& a, OzSmemT<PAIR, BN>& sm, uint32_t ra
     const int level = un.level;
     const void* ma = static_cast<const uint8_t*>(a.maps_a) + size_t(tl.panel_a) * 128;
     const void* mb = static_cast<const uint8_t*>(a.maps_b) + size_t(tl.panel_b) * 128;
-    const int rpa = a.panels_a[tl.panel_a].rows_pad, rpb = a.panels_b[tl.panel_b].rows_pad;
     const int first = RES ? level : 0;
-    const int arow = tl.m0 + int(rank) * kOzBM + first * rpa;  // this CTA's 128 rows of A
-    // this CTA's rows of B (pair form: half of them); slice level - i, or the modulus' own
-    const int brow = tl.n0 + (PAIR ? int(rank) * (BN / 2) : 0) + level * rpb;
+    const int ar = tl.m0 + int(rank) * kOzBM;                       // this CTA's 128 rows of A
+    const int br = tl.n0 + (PAIR ? int(rank) * (BN / 2) : 0);  // and of B (pair form: half of them)
     bool ok = true;
     for_unit_kblocks(a, un, tl, [&](int ka, int kb, int) {
-      int ar = arow, br = brow;
       for (int i = first; i <= level; ++i) {
+        const int j = RES ? level : level - i;  // the B slice, or the modulus' own
         if (!warp_wait(empty0 + 8 * s, free_parity, sm, a.err_flag, 1)) return ok = false;
         if (leader) {
           const uint32_t fb = full0 + 8 * s;
           if constexpr (PAIR) {
             mbar_expect_tx_cluster(fb, kBytes);
-            tma_load_2d_pair(a0 + s * kTileBytes, ma, fb, ka, ar);
-            tma_load_2d_pair(b0 + s * SM::kBBytes, mb, fb, kb, br);
+            tma_load_3d_pair(a0 + s * kTileBytes, ma, fb, ka, ar, i);
+            tma_load_3d_pair(b0 + s * SM::kBBytes, mb, fb, kb, br, j);
           } else {
             mbar_expect_tx(fb, kBytes);
-            tma_load_2d(a0 + s * kTileBytes, ma, fb, ka, ar);
-            tma_load_2d(b0 + s * SM::kBBytes, mb, fb, kb, br);
+            tma_load_3d(a0 + s * kTileBytes, ma, fb, ka, ar, i);
+            tma_load_3d(b0 + s * SM::kBBytes, mb, fb, kb, br, j);
           }
         }
         __syncwarp();
-        ar += rpa, br -= rpb;
         if (++s == uint32_t(SM::kSt)) s = 0, free_parity ^= 1;
       }
       return true;
@@ -2011,16 +2001,21 @@ int oz_chunk_kb(int level) {
   return int(k / kOzBK);
 }
 
-int oz_make_tensor_map(void* map128, const void* base, int64_t kpad, int64_t rows_total, int box_rows) {
+// A panel's planes as a 3-D map.  Its rows end at the last live one: a box that
+// reaches into the padding gets zeros without reading them (the o=10/v=48
+// step's 144 rows a block, padded to 256: its GEMM 43 -> 31 us, panel reads
+// 208 -> 117 MB).
+int oz_make_tensor_map(void* map128, const void* base, int64_t kpad, int64_t rows, int64_t rows_pad, int planes,
+                       int box_rows) {
   EncodeTiled enc = get_encoder();
   if (!enc) return fail(A4G_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   if (kpad % kOzBK != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0)
     return fail(A4G_ERR_ARG, "panel not aligned for TMA");
-  cuuint64_t dims[2] = {cuuint64_t(kpad), cuuint64_t(rows_total)};
-  cuuint64_t strides[1] = {cuuint64_t(kpad) * 2};
-  cuuint32_t box[2] = {cuuint32_t(kOzBK), cuuint32_t(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(reinterpret_cast<CUtensorMap*>(map128), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+  cuuint64_t dims[3] = {cuuint64_t(kpad), cuuint64_t(rows), cuuint64_t(planes)};
+  cuuint64_t strides[2] = {cuuint64_t(kpad) * 2, cuuint64_t(rows_pad) * cuuint64_t(kpad) * 2};
+  cuuint32_t box[3] = {cuuint32_t(kOzBK), cuuint32_t(box_rows), 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(reinterpret_cast<CUtensorMap*>(map128), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -2028,12 +2023,13 @@ int oz_make_tensor_map(void* map128, const void* base, int64_t kpad, int64_t row
   return A4G_OK;
 }
 
-int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t rows_pad, int slices, int box_rows) {
+int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t rows, int64_t rows_pad, int slices,
+                       int box_rows) {
   EncodeTiled enc = get_encoder();
   if (!enc) return fail(A4G_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   if (kpad % kOzBK != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0)
     return fail(A4G_ERR_ARG, "panel not aligned for TMA");
-  cuuint64_t dims[3] = {cuuint64_t(kpad), cuuint64_t(rows_pad), cuuint64_t(slices)};
+  cuuint64_t dims[3] = {cuuint64_t(kpad), cuuint64_t(rows), cuuint64_t(slices)};
   cuuint64_t strides[2] = {cuuint64_t(kpad) * 2, cuuint64_t(rows_pad) * cuuint64_t(kpad) * 2};
   cuuint32_t box[3] = {cuuint32_t(kLvBK), cuuint32_t(box_rows), cuuint32_t(slices)};
   cuuint32_t estr[3] = {1, 1, 1};

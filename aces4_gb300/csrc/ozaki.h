@@ -11,9 +11,11 @@ constexpr int kOzMaxUsableSlices = 7;  // 7 digits x 7 bits = 49 bits <= the 53-
 
 int oz_prepare();  // one-time kernel attributes (call outside stream capture)
 int oz_chunk_kb(int level);  // 64-wide k blocks per exact FP32 flush at a level
-int oz_make_tensor_map(void* map128, const void* base, int64_t kpad, int64_t rows_total, int box_rows);
+int oz_make_tensor_map(void* map128, const void* base, int64_t kpad, int64_t rows, int64_t rows_pad, int planes,
+                       int box_rows);
 // the all-levels form's map of a panel: boxes of 32 k x box_rows rows x every slice (64-byte swizzle)
-int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t rows_pad, int slices, int box_rows);
+int oz_make_levels_map(void* map128, const void* base, int64_t kpad, int64_t rows, int64_t rows_pad, int slices,
+                       int box_rows);
 int oz_max_pairs(int* pairs);  // CTA pairs of the 2-SM kernel that fit on the GPU at once
 // CTA counts of the exponent / split kernels for one job of a given layout, and
 // the list of pieces of a job set's CTAs.
