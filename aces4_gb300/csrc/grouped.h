@@ -184,13 +184,13 @@ struct OzResidues {
 };
 struct OzCrt {
   int L, slices;
-  int words;  // 32-bit words of the reconstruction: 3 when |sum| < 2^95, else 4
+  int words;  // 32-bit words of the reconstruction: 3 when |sum| < 2^95, 4 when |sum| < 2^127, else 5
   // each twice, as the packed FP32 instructions take them: -p, the FP32
   // nearest 1/p, (P / p)^-1 modulo p, P the product of the moduli
   float2 np[kOzMaxResidues], inv[kOzMaxResidues], cinv[kOzMaxResidues];
-  int m[kOzMaxResidues][4];    // P / p modulo 2^128, signed 32-bit words
-  int prod[4];                 // P modulo 2^128
-  long long base[4];           // -0x4B400000 sum_i m[i][w]: the integers come with the bits of 1.5 2^23
+  int m[kOzMaxResidues][5];    // P / p modulo 2^160, signed 32-bit words
+  int prod[5];                 // P modulo 2^160
+  long long base[5];           // -0x4B400000 sum_i m[i][w]: the integers come with the bits of 1.5 2^23
 };
 
 struct OzGemmArgs {

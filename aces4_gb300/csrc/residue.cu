@@ -52,11 +52,21 @@ int inverse_mod(int a, int p) {
   return 0;
 }
 
-// Words of v in base 2^32 with digits in [-2^31, 2^31), modulo 2^128.
-void signed_words(unsigned __int128 v, int (&w)[4]) {
-  for (int j = 0; j < 4; ++j) {
-    w[j] = int(uint32_t(v));
-    v = (v - (unsigned __int128)(__int128)w[j]) >> 32;
+// A number modulo 2^160.
+struct Words160 {
+  uint32_t w[5] = {1, 0, 0, 0, 0};
+  void times(uint32_t f) {
+    uint64_t carry = 0;
+    for (uint32_t& x : w) carry += uint64_t(x) * f, x = uint32_t(carry), carry >>= 32;
+  }
+};
+// Its words in base 2^32 with digits in [-2^31, 2^31), modulo 2^160.
+void signed_words(const Words160& v, int (&w)[5]) {
+  uint64_t carry = 0;
+  for (int j = 0; j < 5; ++j) {
+    const uint64_t t = v.w[j] + carry;
+    w[j] = int(uint32_t(t));
+    carry = (t >> 32) + (w[j] < 0 ? 1 : 0);
   }
 }
 
@@ -272,7 +282,7 @@ constexpr size_t kGenericSmem = kSplitT * (kSplitT + 1) * sizeof(unsigned long l
 //     X = sum_i y_i (P / p_i) - k P,   y_i = s_i (P / p_i)^-1 mod p_i,
 //     k = rint(sum_i y_i / p_i)
 // in W signed 32-bit word columns of 64-bit sums, modulo 2^(32 W): three words
-// hold |X| < 2^95, four |X| < 2^127.
+// hold |X| < 2^95, four |X| < 2^127, five |X| < 2^159.
 // Two sums at a time: the residue arithmetic in packed FP32.
 template <int W>
 struct CrtPair {
@@ -312,6 +322,26 @@ struct CrtPair {
     const int k = 0x4B400000 - int(__float_as_uint(__fadd_rn(turns, kRintMagic)));
 #pragma unroll
     for (int w = 0; w < W; ++w) c[w] = mad_wide(k, T.prod[w], c[w]);
+    if constexpr (W == 5) {
+      uint32_t w[5];
+      long long t = 0;
+#pragma unroll
+      for (int j = 0; j < 5; ++j) t += c[j], w[j] = uint32_t(t), t >>= 32;
+      const bool minus = int(w[4]) < 0;
+      if (minus) {
+        unsigned long long carry = 1;
+#pragma unroll
+        for (int j = 0; j < 5; ++j) carry += uint32_t(~w[j]), w[j] = uint32_t(carry), carry >>= 32;
+      }
+      const unsigned long long a = (unsigned long long)w[4] << 32 | w[3], b = (unsigned long long)w[2] << 32 | w[1];
+      if (a) {  // from 2^96 on: the top 62 bits, the last one sticky
+        const int n = clz64(a);
+        const unsigned long long top = n ? a << n | b >> (64 - n) : a, rest = b << n | w[0];
+        const long long v = (long long)(top >> 2 | ((top & 3u) || rest ? 1ull : 0ull));
+        return i64_scaled_to_double(minus ? -v : v, e2 + 98 - n, neg);
+      }
+      return small((unsigned long long)w[2], (unsigned long long)w[1] << 32 | w[0], minus, e2, neg);
+    }
     unsigned __int128 x = (unsigned __int128)(__int128)c[0] + ((unsigned __int128)(__int128)c[1] << 32);
     if constexpr (W == 4) {
       x += ((unsigned __int128)(__int128)c[2] << 64) + ((unsigned __int128)(unsigned long long)c[3] << 96);
@@ -332,8 +362,12 @@ struct CrtPair {
       double r;
       if (i64_scaled_normal(v, e2 + 34 - n, &r) && h) return minus != neg ? -r : r;
     }
-    // the top 62 bits, what is below them folded into the last (a sticky bit:
-    // the rounding position lies above it)
+    return small(hi, lo, minus, e2, neg);
+  }
+  // (minus ? -1 : 1) (hi 2^64 + lo) 2^e2: the top 62 bits, what is below them
+  // folded into the last (a sticky bit: the rounding position lies above it)
+  static __device__ __forceinline__ double small(unsigned long long hi, unsigned long long lo, bool minus, int e2,
+                                                 bool neg) {
     const int sh = (hi ? 64 - clz64(hi) : -clz64(lo | 1ull)) + 2;
     long long v = (long long)lo;
     if (sh > 0) {
@@ -427,12 +461,12 @@ __global__ void __launch_bounds__(kRecThreads, L <= 12 && W == 3 ? 4 : 3) oz_res
 // Products the residue form needs for K columns at `slices` slices: the
 // smallest count whose moduli hold every sum |sum| <= K 4^(8 slices - 1) below
 // 0.49 of their product; 0 when none does, or when the sum would not stay
-// below 2^127 (the reconstruction's words).  At 5 slices or more and k ranges
+// below 2^158 (the reconstruction's words).  At 5 slices or more and k ranges
 // worth it (batch.cu), 10 to 15.
 int oz_residue_count(int slices, int64_t K) {
   if (K < 1) return 0;
   const double need = 2.0 * (8.0 * slices - 1.0) + std::log2(double(K));
-  if (need >= 127.0) return 0;
+  if (need >= 158.0) return 0;
   double have = std::log2(0.49);
   for (int i = 0; i < kOzMaxResidues; ++i) {
     have += std::log2(double(kModuli[i]));
@@ -446,9 +480,10 @@ void oz_residue_tables(int slices, int L, int64_t K, OzResidues* r, OzCrt* t) {
   *t = OzCrt{};
   r->L = t->L = L;
   r->slices = t->slices = slices;
-  t->words = 2.0 * (8.0 * slices - 1.0) + std::log2(double(K)) < 94.9 ? 3 : 4;
-  unsigned __int128 prod = 1;  // modulo 2^128
-  for (int i = 0; i < L; ++i) prod *= unsigned(kModuli[i]);
+  const double bits = 2.0 * (8.0 * slices - 1.0) + std::log2(double(K));
+  t->words = bits < 94.9 ? 3 : bits < 126.9 ? 4 : 5;
+  Words160 prod;
+  for (int i = 0; i < L; ++i) prod.times(unsigned(kModuli[i]));
   signed_words(prod, t->prod);
   for (int i = 0; i < L; ++i) {
     const int p = kModuli[i];
@@ -458,14 +493,14 @@ void oz_residue_tables(int slices, int L, int64_t K, OzResidues* r, OzCrt* t) {
       const float c = float(symmetric(1ll << (14 * (q + 1)), p));
       r->c[q][i] = make_float2(c, c);
     }
-    unsigned __int128 m = 1;
+    Words160 m;
     long long mp = 1;
     for (int j = 0; j < L; ++j)
-      if (j != i) m *= unsigned(kModuli[j]), mp = mp * kModuli[j] % p;
+      if (j != i) m.times(unsigned(kModuli[j])), mp = mp * kModuli[j] % p;
     signed_words(m, t->m[i]);
     const float c = float(symmetric(inverse_mod(int(mp), p), p));
     t->cinv[i] = make_float2(c, c);
-    for (int w = 0; w < 4; ++w)
+    for (int w = 0; w < 5; ++w)
       t->base[w] = (long long)((unsigned long long)t->base[w] - 0x4B400000ull * (unsigned long long)(long long)t->m[i][w]);
   }
 }
@@ -519,7 +554,10 @@ int oz_launch_residue_recombine(const OzTile* tiles, int ntiles, int tile_rows, 
     case 12: go(std::integral_constant<int, 12>(), w4); break;
     case 13: go(std::integral_constant<int, 13>(), w4); break;
     case 14: go(std::integral_constant<int, 14>(), w4); break;
-    case 15: go(std::integral_constant<int, 15>(), w4); break;
+    case 15:
+      if (t.words == 5) go(std::integral_constant<int, 15>(), std::integral_constant<int, 5>());
+      else go(std::integral_constant<int, 15>(), w4);
+      break;
     default: return fail(A4G_ERR_ARG, "residue form: 10 to 15 moduli");
   }
   A4G_CUDA(cudaGetLastError());
