@@ -583,9 +583,12 @@ int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vect
   // the padded k.  (o=48/v=400 step with 30 % zero blocks, four zero patterns:
   // 45 -> 29.5 GB of panels.)
   Panels lay = lay_panels(groups, plans, right_order, false);
-  {
-    const Panels shared = lay_panels(groups, plans, right_order, true);
-    if (shared.cost_us(b->slices) < lay.cost_us(b->slices)) lay = shared;
+  std::unordered_set<const double*> rights;
+  size_t sliced = 0;
+  for (const auto& p : lay.pb) rights.insert(p.order.begin(), p.order.end()), sliced += p.order.size();
+  if (sliced > rights.size()) {  // some right block is sliced more than once
+    Panels shared = lay_panels(groups, plans, right_order, true);
+    if (shared.cost_us(b->slices) < lay.cost_us(b->slices)) lay = std::move(shared);
   }
   std::vector<PanelBuild>&pa = lay.pa, &pb = lay.pb;
   std::vector<int>&ga = lay.ga, &gb = lay.gb;
