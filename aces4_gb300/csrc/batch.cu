@@ -367,86 +367,6 @@ void for_stretches(const DGroup& g, const PanelBuild& pa, const PanelBuild& pb,
   if (first >= 0) f(first, int(g.pairs.size()) - 1, ka, kb, kk);
 }
 
-// The operand panels of a step: A panels of the left blocks, B panels of the
-// right blocks, and which of them each destination block's group reads.
-struct Panels {
-  std::vector<PanelBuild> pa, pb;
-  std::vector<int> ga, gb;
-  double elems = 0.0;  // sliced elements
-  double macs = 0.0;   // per product, over the padded k
-  // at 1.6 PFLOP/s a product and 5.5 TB/s of panel traffic
-  double cost_us(int slices) const {
-    const int planes = slices < 5 ? slices : 2 * slices + 1, products = slices < 5 ? slices * (slices + 1) / 2 : planes;
-    return elems * (16.0 + 2.0 * planes) / 5.5e6 + products * 2.0 * macs / 1.6e9;
-  }
-};
-
-// share_right: one B panel for all groups whose sets of right blocks overlap
-// (right_order: where a block first appears in the triples), else one per set.
-Panels lay_panels(const std::vector<DGroup>& groups, const std::vector<const DevPlan*>& plans,
-                  const std::unordered_map<const double*, int64_t>& right_order, bool share_right) {
-  Panels P;
-  std::map<std::vector<const double*>, int> ia, ib;
-  P.ga.resize(groups.size()), P.gb.resize(groups.size());
-  std::vector<std::vector<std::pair<const double*, int>>> rights(groups.size());
-  for (size_t gi = 0; gi < groups.size(); ++gi)
-    for (const Pair& p : groups[gi].pairs) rights[gi].push_back({p.r, p.plan});
-  if (share_right) {
-    // components of groups that share a right block, then each one's blocks in order
-    std::unordered_map<const double*, int> owner;
-    std::vector<int> parent(groups.size());
-    for (size_t i = 0; i < parent.size(); ++i) parent[i] = int(i);
-    auto root = [&](int x) {
-      while (parent[size_t(x)] != x) x = parent[size_t(x)] = parent[size_t(parent[size_t(x)])];
-      return x;
-    };
-    for (size_t gi = 0; gi < groups.size(); ++gi)
-      for (const auto& r : rights[gi]) {
-        const int o = owner.emplace(r.first, int(gi)).first->second;
-        parent[size_t(root(int(gi)))] = root(o);
-      }
-    std::map<int, std::map<int64_t, std::pair<const double*, int>>> blocks;  // component -> blocks by order
-    for (size_t gi = 0; gi < groups.size(); ++gi)
-      for (const auto& r : rights[gi]) blocks[root(int(gi))].emplace(right_order.at(r.first), r);
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-      rights[gi].clear();
-      for (const auto& kv : blocks.at(root(int(gi)))) rights[gi].push_back(kv.second);
-    }
-  }
-  for (size_t gi = 0; gi < groups.size(); ++gi) {
-    const DGroup& g = groups[gi];
-    const GemmPlan& h = plans[g.plan]->host;
-    std::vector<std::pair<const double*, int>> ls;
-    for (const Pair& p : g.pairs) ls.push_back({p.l, p.plan});
-    P.ga[gi] = find_or_add_panel(P.pa, ia, ls, int(h.M), plans);
-    P.gb[gi] = find_or_add_panel(P.pb, ib, rights[gi], int(h.N), plans);
-  }
-  // In the A panels, align the first block of every stretch to 64 columns and
-  // pad after its last block; padding only splits stretches, so repeat until
-  // every stretch starts and ends on marked blocks (marks only grow).
-  for (bool changed = true; changed;) {
-    changed = false;
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-      PanelBuild& A = P.pa[P.ga[gi]];
-      for_stretches(groups[gi], A, P.pb[P.gb[gi]], plans, [&](int first, int last, int64_t, int64_t, int64_t) {
-        changed |= A.pad_before.insert(groups[gi].pairs[first].l).second;
-        changed |= A.pad_after.insert(groups[gi].pairs[last].l).second;
-      });
-    }
-    if (changed)
-      for (auto& p : P.pa) layout_panel(p, plans);
-  }
-  for (size_t gi = 0; gi < groups.size(); ++gi) {
-    const GemmPlan& h = plans[groups[gi].plan]->host;
-    for_stretches(groups[gi], P.pa[P.ga[gi]], P.pb[P.gb[gi]], plans, [&](int, int, int64_t, int64_t, int64_t kk) {
-      P.macs += double(h.M) * double(h.N) * double(ceil_to(kk, kOzBK));
-    });
-  }
-  for (const auto* side : {&P.pa, &P.pb})
-    for (const auto& p : *side) P.elems += double(p.rows) * double(p.kpad);
-  return P;
-}
-
 int build_f64(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector<const DevPlan*>& plans) {
   std::vector<GroupedPair> pairs;
   std::vector<F64Shape> shapes;
@@ -568,30 +488,40 @@ int launch_recombine(const a4g_batch* b, const a4g_batch::GemmForm& gf, const Oz
 }
 
 int build_ozaki(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector<const DevPlan*>& plans,
-                const std::unordered_map<const double*, int64_t>& right_order, const int* ptrn, bool allow_residue) {
+                const int* ptrn, bool allow_residue) {
+  std::vector<PanelBuild> pa, pb;
+  std::map<std::vector<const double*>, int> ia, ib;
   std::vector<OzDBlock> dblocks;
   std::vector<OzTile> dinfo;  // one per destination block: m0 = M, n0 = N (tiles are cut per form)
   std::vector<OzTrip> trips;
-  // Panels with their k layouts.  A zero block on one side leaves the
-  // destinations it feeds with different sets of blocks on the other: with
-  // panels of exact sets, a right block that several destinations read is then
-  // sliced once per set.  With shared right panels, sets that overlap make one
-  // panel (in the order of the triples, skipped ones included, so that runs of
-  // live pairs stay contiguous) and every right block is sliced once; a
-  // destination's skipped blocks break its stretches of k, each padded to 64.
-  // The cheaper layout by both costs is taken: sliced bytes, and products over
-  // the padded k.  (o=48/v=400 step with 30 % zero blocks, four zero patterns:
-  // 45 -> 29.5 GB of panels.)
-  Panels lay = lay_panels(groups, plans, right_order, false);
-  std::unordered_set<const double*> rights;
-  size_t sliced = 0;
-  for (const auto& p : lay.pb) rights.insert(p.order.begin(), p.order.end()), sliced += p.order.size();
-  if (sliced > rights.size()) {  // some right block is sliced more than once
-    Panels shared = lay_panels(groups, plans, right_order, true);
-    if (shared.cost_us(b->slices) < lay.cost_us(b->slices)) lay = std::move(shared);
+  // One panel per set of blocks that some destination multiplies, and not one
+  // for sets that overlap: a panel's rows carry one exponent and one
+  // non-finite mark each, and a destination must not take them from a block
+  // that it skips (its partner is a zero block).
+  std::vector<int> ga(groups.size()), gb(groups.size());
+  for (size_t gi = 0; gi < groups.size(); ++gi) {
+    const DGroup& g = groups[gi];
+    const GemmPlan& h = plans[g.plan]->host;
+    std::vector<std::pair<const double*, int>> ls, rs;
+    for (const Pair& p : g.pairs) ls.push_back({p.l, p.plan}), rs.push_back({p.r, p.plan});
+    ga[gi] = find_or_add_panel(pa, ia, ls, int(h.M), plans);
+    gb[gi] = find_or_add_panel(pb, ib, rs, int(h.N), plans);
   }
-  std::vector<PanelBuild>&pa = lay.pa, &pb = lay.pb;
-  std::vector<int>&ga = lay.ga, &gb = lay.gb;
+  // In the A panels, align the first block of every stretch to 64 columns and
+  // pad after its last block; padding only splits stretches, so repeat until
+  // every stretch starts and ends on marked blocks (marks only grow).
+  for (bool changed = true; changed;) {
+    changed = false;
+    for (size_t gi = 0; gi < groups.size(); ++gi) {
+      PanelBuild& A = pa[ga[gi]];
+      for_stretches(groups[gi], A, pb[gb[gi]], plans, [&](int first, int last, int64_t, int64_t, int64_t) {
+        changed |= A.pad_before.insert(groups[gi].pairs[first].l).second;
+        changed |= A.pad_after.insert(groups[gi].pairs[last].l).second;
+      });
+    }
+    if (changed)
+      for (auto& p : pa) layout_panel(p, plans);
+  }
   // Stacks: destination blocks whose pairs multiply the same left blocks at
   // the same k positions of one A panel, whose B panels lay their pairs out
   // alike, and whose rows are addressed alike (equal offDm) are laid side by
@@ -1384,15 +1314,12 @@ static int create_batch(a4g_batch** out, const int* ptrn, int drank, int lrank, 
   std::vector<DGroup> groups;
   std::map<double*, int> gindex;
   std::map<double*, int64_t> all_d;
-  std::unordered_map<const double*, int64_t> order[2];  // first triple naming a left / right block, skipped ones included
   for (int64_t i = 0; i < n; ++i) {
     const a4g_triple& t = trip[i];
     if (!t.d) return fail(A4G_ERR_ARG, "triple with NULL destination");
     int64_t dsize = 1;
     for (int q = 0; q < drank; ++q) dsize *= t.dext[q];
     all_d[t.d] = dsize;
-    if (t.l) order[0].emplace(t.l, i);
-    if (t.r) order[1].emplace(t.r, i);
     if (!t.l || !t.r) continue;  // zero block: skipped
     const DevPlan* p = nullptr;
     if ((rc = get_dev_plan(ptrn, lrank, t.lext, rrank, t.rext, drank, t.dext, &p))) return rc;
@@ -1456,7 +1383,7 @@ static int create_batch(a4g_batch** out, const int* ptrn, int drank, int lrank, 
   for (const DevPlan* p : plans) refs.push_back(plan_ref(*p));
   if ((rc = upload(b.get(), refs, &b->d_plans))) return rc;
   rc = b->precision == A4G_PREC_FP64 ? build_f64(b.get(), groups, plans)
-                                     : build_ozaki(b.get(), groups, plans, order[b->swapped ? 0 : 1], ptrn, allow_residue);
+                                     : build_ozaki(b.get(), groups, plans, ptrn, allow_residue);
   *residue = b->residue;
   if (rc) return rc;
   *out = b.release();
