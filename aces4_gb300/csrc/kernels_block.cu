@@ -786,7 +786,7 @@ struct UpdParams {
 };
 
 __device__ __forceinline__ double eps_at_upd(const UpdParams& p, const double* e, int orb) {
-  return p.rank1 == 2 ? e[int64_t(orb) + int64_t(orb) * p.ld1] : e[orb];
+  return __ldcg(p.rank1 == 2 ? e + int64_t(orb) + int64_t(orb) * p.ld1 : e + orb);
 }
 
 // x / 2 without the FP64 pipe where that is an exponent decrement (normal x
@@ -806,7 +806,11 @@ __global__ void __launch_bounds__(kUpdThreads, 6) update_t2_kernel(UpdParams p, 
   __shared__ double pn[kUpdA][kUpdB + 1], po[kUpdA][kUpdB + 1];  // [a][b] of the partner tiles
   __shared__ double sa[kUpdA], sb[kUpdB];  // (e_i + e_j) - e_a of the tile's a, e_b of its b
   // The next update's CTAs may take their places as this one's leave; they wait
-  // here until it has completed before they read anything.
+  // here until it has completed before they read anything.  All its inputs are
+  // read from L2 (__ldcg): the update before may have written them while this
+  // grid was already there, so they are not read-only for its lifetime, as the
+  // non-coherent loads (__ldg) require, and a line of this
+  // SM's L1 may be from before that write.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   double acc = 0.0;
@@ -835,8 +839,8 @@ __global__ void __launch_bounds__(kUpdThreads, 6) update_t2_kernel(UpdParams p, 
       for (int g = 0; g < kUpdGroup; ++g) {
         const int el = e0 + kUpdThreads * g, b = int((uint32_t(el) * p.mul_a) >> 20), a = el - b * p.ta;
         const bool live = el < n && a < na && b < nb;
-        t[g] = live ? __ldg(xn + qb + a + qsb * b) : 1.0;
-        t1[g] = live ? __ldg(xo + qb + a + qsb * b) : 0.0;
+        t[g] = live ? __ldcg(xn + qb + a + qsb * b) : 1.0;
+        t1[g] = live ? __ldcg(xo + qb + a + qsb * b) : 0.0;
       }
     };
     load_own(threadIdx.x);
@@ -850,8 +854,8 @@ __global__ void __launch_bounds__(kUpdThreads, 6) update_t2_kernel(UpdParams p, 
       for (int g = 0; g < kUpdGroup; ++g) {
         const int el = e0 + kUpdThreads * g, a = int((uint32_t(el) * p.mul_b) >> 20), b = el - a * p.tb;
         const bool live = el < n && a < na && b < nb;
-        vn[g] = live ? __ldg(xnp + pb + b + psa * a) : 0.0;
-        vo[g] = live ? __ldg(xop + pb + b + psa * a) : 0.0;
+        vn[g] = live ? __ldcg(xnp + pb + b + psa * a) : 0.0;
+        vo[g] = live ? __ldcg(xop + pb + b + psa * a) : 0.0;
       }
 #pragma unroll
       for (int g = 0; g < kUpdGroup; ++g) {
