@@ -45,12 +45,11 @@ struct Context {
   // every synchronisation, so a synchronous call would allocate from scratch
   // each time.
   cudaMemPool_t pool = nullptr;
-  // Scratch of the deterministic reductions: rings of slots, one per launch in
-  // turn, so that launches on several streams (or from several threads) that
-  // overlap do not share one.  The counters' ring is the longer one: a counter
-  // that two launches shared would not come back to zero.
-  static constexpr int kReducePartials = 1024, kReduceSlots = 256, kReduceCounters = 65536;
-  double* reduce_partials = nullptr;  // [slot][kReducePartials + 8]
+  // Scratch of the deterministic reductions, one slot per stream or captured
+  // stream (reduction_slots.h): partial sums in chunks, made as slots are first
+  // used, and the counters, zero between launches.
+  static constexpr int kReducePartials = 1024, kReduceChunk = 64;
+  std::vector<double*> reduce_partials;  // chunks of [kReduceChunk][kReducePartials + 8]
   unsigned* reduce_counters = nullptr;
   // Kernels can read and write pageable host memory through the host's page
   // tables (address translation services over the CPU-GPU link): the
@@ -140,8 +139,23 @@ struct ReductionSlot {
   double* result = nullptr;
   unsigned* counter = nullptr;
 };
-// The next slot of the context's rings (after ensure_init).
-ReductionSlot reduction_slot();
+// The scratch of the reductions that the caller launches on `s` while the
+// object lives (after ensure_init).
+class ReductionScratch {
+ public:
+  ReductionScratch() = default;
+  ReductionScratch(const ReductionScratch&) = delete;
+  ReductionScratch& operator=(const ReductionScratch&) = delete;
+  ~ReductionScratch() {
+    if (own_) cudaFreeAsync(own_, stream_);
+  }
+  int acquire(cudaStream_t s);
+  ReductionSlot slot;
+
+ private:
+  void* own_ = nullptr;  // stream-ordered memory, where the stream has no slot
+  cudaStream_t stream_ = nullptr;
+};
 int launch_dot(const double* a, const double* b, const int64_t* offA, const int64_t* offB, int64_t n, double* d_out,
                const ReductionSlot& slot, int beta, cudaStream_t s);
 int launch_norm2(const double* a, int64_t n, double* d_out, const ReductionSlot& slot, cudaStream_t s);

@@ -170,7 +170,9 @@ int contract_device(const int* ptrn, const double* l, int lrank, const int* lext
   int rc = get_dev_plan(ptrn, lrank, lext, rrank, rext, drank, dext, &p);
   if (rc) return rc;
   if (p->host.kind == ContractKind::kTensorTensor) return launch_contract_f64(p, l, r, d, beta, s);
-  return launch_scalar_cases(p, l, r, d, beta, reduction_slot(), s);
+  ReductionScratch scratch;
+  if ((rc = scratch.acquire(s))) return rc;
+  return launch_scalar_cases(p, l, r, d, beta, scratch.slot, s);
 }
 
 }  // namespace
@@ -250,7 +252,8 @@ double tensor_block_norm2__(int* nthreads, double* tens, int* tens_rank, int* ex
   if (!rc) rc = io.in(tens, n, &d);
   if (!rc) {
     double* out = io.scratch(1);
-    rc = launch_norm2(d, n, out, reduction_slot(), io.s);
+    ReductionScratch scratch;
+    if (!(rc = scratch.acquire(io.s))) rc = launch_norm2(d, n, out, scratch.slot, io.s);
     if (!rc) rc = d2h(&result, out, 1, io.s);
     if (!rc) rc = io.finish();
   }
@@ -630,10 +633,11 @@ int a4g_add_sub(int subtract, int rank, const int* d_labels, const int* r_labels
 int a4g_norm2(const double* t, int64_t n, double* h_result, void* stream) {
   int rc = ensure_init();
   if (rc) return rc;
-  const ReductionSlot slot = reduction_slot();
   cudaStream_t s = pick(stream);
-  double* out = slot.result;
-  rc = launch_norm2(t, n, out, slot, s);
+  ReductionScratch scratch;
+  if ((rc = scratch.acquire(s))) return rc;
+  double* out = scratch.slot.result;
+  rc = launch_norm2(t, n, out, scratch.slot, s);
   if (rc) return rc;
   A4G_CUDA(cudaMemcpyAsync(h_result, out, sizeof(double), cudaMemcpyDeviceToHost, s));
   return check_device_flag(s);
@@ -686,8 +690,11 @@ int a4g_update_t2(const int* iv, const int* ext, const double* t2new, const doub
   int off[6];
   rc = denominator_offsets(4, iv, ext, rank1, ext1, std::vector<int>(segs, segs + std::max(nsegs, 0)), off);
   if (rc) return rc;
+  cudaStream_t s = pick(stream);
+  ReductionScratch scratch;
+  if (norm2 && (rc = scratch.acquire(s))) return rc;
   return launch_update_t2(off, ext, t2new, t2new_pair, t2old, t2old_pair, diis_err, t2old_next, rank1, ext1[0],
-                          e_or_fock, norm2, reduction_slot(), pick(stream));
+                          e_or_fock, norm2, scratch.slot, s);
 }
 
 int a4g_selftest_wait_timeout(int limit_ms, int* waited_ms, void* stream) {
@@ -733,8 +740,10 @@ int a4g_energy_contract(int rank0, const int* iv, const int* ext0, const double*
   int off[6];
   rc = denominator_offsets(rank0, iv, ext0, rank1, ext1, std::vector<int>(segs, segs + std::max(nsegs, 0)), off);
   if (rc) return rc;
-  return launch_energy_contract(rank0, off, ext0, pos, data0, rank1, ext1[0], e, efact, esum, reduction_slot(),
-                                pick(stream));
+  cudaStream_t s = pick(stream);
+  ReductionScratch scratch;
+  if ((rc = scratch.acquire(s))) return rc;
+  return launch_energy_contract(rank0, off, ext0, pos, data0, rank1, ext1[0], e, efact, esum, scratch.slot, s);
 }
 
 }  // extern "C"

@@ -1641,11 +1641,15 @@ int a4g_batch_error_bound(a4g_batch* b, double target, double* h_bound, void* st
   const size_t ng = b->err_groups.size();
   double* dev = nullptr;
   if (const int rc_ = async_alloc(reinterpret_cast<void**>(&dev), std::max<size_t>(ng, 1) * sizeof(double), s)) return rc_;
-  const ReductionSlot slot = reduction_slot();  // one block after another on this stream
+  ReductionScratch scratch;  // one block after another on this stream
+  if (const int rc_ = scratch.acquire(s)) {
+    cudaFreeAsync(dev, s);
+    return rc_;
+  }
   int rc = A4G_OK;
   for (size_t i = 0; i < ng && !rc; ++i) {
     const a4g_batch::ErrGroup& eg = b->err_groups[i];
-    rc = launch_norm2(eg.d, eg.size, dev + i, slot, s);
+    rc = launch_norm2(eg.d, eg.size, dev + i, scratch.slot, s);
   }
   std::vector<double> nrm2(ng);
   if (!rc && ng) {

@@ -1,12 +1,12 @@
 // Runtime support: error reporting, the process context, the contraction
 // pattern planner and the device plan cache.
 #include <algorithm>
-#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <unordered_map>
 
 #include "a4g_internal.h"
+#include "reduction_slots.h"
 
 namespace a4g {
 
@@ -31,6 +31,8 @@ static std::mutex g_mu;
 
 Context* ctx() { return &g_ctx; }
 
+constexpr size_t kReduceLen = Context::kReducePartials + 8;  // doubles of a reduction's scratch
+
 int ensure_init() {
   if (g_ctx.device >= 0) return A4G_OK;
   std::lock_guard<std::mutex> lock(g_mu);
@@ -48,10 +50,11 @@ int ensure_init() {
   A4G_CUDA(cudaHostGetDevicePointer(&d_flag, flag, 0));
   g_ctx.h_error_flag = static_cast<volatile int*>(flag), g_ctx.d_error_flag = static_cast<int*>(d_flag);
   *g_ctx.h_error_flag = 0;
-  A4G_CUDA(cudaMalloc(&g_ctx.reduce_partials,
-                      sizeof(double) * (Context::kReducePartials + 8) * size_t(Context::kReduceSlots)));
-  A4G_CUDA(cudaMalloc(&g_ctx.reduce_counters, sizeof(unsigned) * Context::kReduceCounters));
-  A4G_CUDA(cudaMemset(g_ctx.reduce_counters, 0, sizeof(unsigned) * Context::kReduceCounters));
+  A4G_CUDA(cudaMalloc(&g_ctx.reduce_counters, sizeof(unsigned) * SlotTable::kMaxSlots));
+  A4G_CUDA(cudaMemset(g_ctx.reduce_counters, 0, sizeof(unsigned) * SlotTable::kMaxSlots));
+  double* partials = nullptr;
+  A4G_CUDA(cudaMalloc(&partials, sizeof(double) * kReduceLen * Context::kReduceChunk));
+  g_ctx.reduce_partials.push_back(partials);
   A4G_CUDA(cudaDeviceSynchronize());
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
@@ -74,11 +77,80 @@ int async_alloc(void** p, size_t bytes, cudaStream_t s) {
   return A4G_OK;
 }
 
-ReductionSlot reduction_slot() {
-  static std::atomic<unsigned> next{0};
-  const unsigned q = next.fetch_add(1, std::memory_order_relaxed);
-  double* p = g_ctx.reduce_partials + size_t(Context::kReducePartials + 8) * (q % Context::kReduceSlots);
-  return {p, p + Context::kReducePartials, g_ctx.reduce_counters + q % Context::kReduceCounters};
+// ------------------------------------------------------------------ reduction scratch
+// Never destroyed: a graph may outlive the library's statics.
+static SlotTable& g_slots = *new SlotTable;
+static std::mutex g_slots_mu;  // the table and the chunks
+static std::vector<unsigned long long>& g_gone = *new std::vector<unsigned long long>;  // captures whose graphs are gone
+static std::mutex& g_gone_mu = *new std::mutex;  // held for the list alone: CUDA calls graph_gone from any thread
+
+static void CUDART_CB graph_gone(void* p) {
+  unsigned long long* id = static_cast<unsigned long long*>(p);
+  {
+    std::lock_guard<std::mutex> lock(g_gone_mu);
+    g_gone.push_back(*id);
+  }
+  delete id;
+}
+
+// Has the graph that is being captured report its end (and its instances').
+static int watch_graph(cudaGraph_t graph, unsigned long long capture) {
+  unsigned long long* id = new unsigned long long(capture);
+  cudaUserObject_t obj;
+  cudaError_t e = cudaUserObjectCreate(&obj, id, graph_gone, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    delete id;
+    return cuda_fail(e, "cudaUserObjectCreate");
+  }
+  e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(obj, 1);
+    return cuda_fail(e, "cudaGraphRetainUserObject");
+  }
+  return A4G_OK;
+}
+
+int ReductionScratch::acquire(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long capture = 0, id = 0;
+  cudaGraph_t graph = nullptr;
+  A4G_CUDA(cudaStreamGetCaptureInfo(s, &status, &capture, &graph));
+  if (status != cudaStreamCaptureStatusActive) capture = 0;
+  if (capture) id = reinterpret_cast<uintptr_t>(s);  // the id cannot be asked for during capture, nor the stream destroyed
+  else A4G_CUDA(cudaStreamGetId(s, &id));
+  stream_ = s;
+  {
+    std::lock_guard<std::mutex> lock(g_slots_mu);
+    {
+      std::lock_guard<std::mutex> gone(g_gone_mu);
+      for (unsigned long long g : g_gone) g_slots.release(g);
+      g_gone.clear();
+    }
+    if (capture && !g_slots.has_capture(capture))
+      if (const int rc = watch_graph(graph, capture)) return rc;
+    const int q = g_slots.slot(capture, id);
+    if (q >= 0) {
+      const size_t chunk = size_t(q / Context::kReduceChunk);
+      if (chunk >= g_ctx.reduce_partials.size()) {
+        // an allocation that no capture records or forbids
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        A4G_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        double* p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, sizeof(double) * kReduceLen * Context::kReduceChunk);
+        A4G_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
+        g_ctx.reduce_partials.push_back(p);
+      }
+      double* p = g_ctx.reduce_partials[chunk] + kReduceLen * size_t(q % Context::kReduceChunk);
+      slot = {p, p + Context::kReducePartials, g_ctx.reduce_counters + q};
+      return A4G_OK;
+    }
+  }
+  if (const int rc = async_alloc(&own_, sizeof(double) * (kReduceLen + 1), s)) return rc;
+  double* p = static_cast<double*>(own_);
+  slot = {p, p + Context::kReducePartials, reinterpret_cast<unsigned*>(p + kReduceLen)};
+  A4G_CUDA(cudaMemsetAsync(slot.counter, 0, sizeof(unsigned), s));
+  return A4G_OK;
 }
 
 cudaStream_t pick(void* stream) {

@@ -251,8 +251,9 @@ int a4g_update_t2(const int* index_values, const int* ext, const double* t2new, 
  * index_values0 / ext0 follow data0's storage order; den_order[q] names the
  * dimension of data0 at position q of the denominator's order (virtual,
  * occupied, virtual, occupied, ...), NULL when data0 is stored in that order.
- * esum is a device double.  The sum is deterministic on a given GPU; calls
- * share the library's reduction scratch, so keep them on one stream. */
+ * esum is a device double.  The sum is deterministic on a given GPU; calls on
+ * different streams, and replays of captured ones, do not share scratch (they
+ * do share an esum that they are all given). */
 int a4g_energy_contract(int rank0, const int* index_values0, const int* ext0, const double* data0,
                         const int* den_order, int rank1, const int* ext1, const double* e_or_fock,
                         int nsegs, const int* seg_sizes, double efact, double* esum, void* stream);
