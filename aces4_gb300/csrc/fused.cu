@@ -392,6 +392,8 @@ int plan_fused(int drank, int lrank, int rrank, const a4g_term* terms, int nterm
       return fail(A4G_ERR_UNSUPPORTED, "fused energy: the denominator's last term is a fixed (batch) index");
     const int64_t ne = energy->rank1 == 2 ? int64_t(energy->ext1[0]) * energy->ext1[1] : energy->ext1[0];
     if (ne <= 0) return fail(A4G_ERR_ARG, "fused energy: empty energy array");
+    // part of the structure: a rebind with another energy array's shape is refused
+    sig.put(energy->rank1), sig.put(energy->ext1[0]), sig.put(energy->rank1 == 2 ? energy->ext1[1] : 0);
     const std::vector<int> segs(energy->seg_sizes, energy->seg_sizes + std::max(energy->nsegs, 0));
     for (int64_t i = 0; i < energy->n_blocks; ++i) {
       auto it = widx.find(energy->blocks[i]);
@@ -951,7 +953,7 @@ int a4g_fused_rebind(a4g_fused* f, const a4g_term* terms, int nterms, const a4g_
     return rc;
   f->zero_blocks = P.zero_blocks;
   if (f->energy) {
-    f->e_dev = P.e_dev, f->efact = P.efact, f->rank1 = P.rank1, f->ld1 = P.ld1;
+    f->e_dev = P.e_dev, f->efact = P.efact;
     // energies that the default stream is still writing are waited for there
     if (!f->ev_default) A4G_CUDA(cudaEventCreateWithFlags(&f->ev_default, cudaEventDisableTiming));
     A4G_CUDA(cudaEventRecord(f->ev_default, cudaStreamLegacy));
