@@ -1196,6 +1196,7 @@ int launch_update_t2(const int* off, const int* ext, const double* t2new, const 
   p.ea = ext[0], p.ei = ext[1], p.eb = ext[2], p.ej = ext[3];
   p.oa = off[0], p.oi = off[1], p.ob = off[2], p.oj = off[3];
   p.rank1 = rank1, p.ld1 = ld1;
+  if (int64_t(p.ei) * p.ej > 65535) return fail(A4G_ERR_RANGE, "amplitude update: block too large");
   // the cut of the plane with the fewest passes over a tile (kUpdGroup x
   // kUpdThreads elements a pass), a quarter of a pass for each tile's ends;
   // tiles of 8 and more a side where the plane has them
