@@ -26,6 +26,14 @@ inline PlanRef plan_ref(const DevPlan& p) {
 }
 
 // ------------------------------------------------------------ FP64 grouped
+constexpr int kF64Step = 16;  // k of one step
+// n / d rounded up, 1 <= n <= 2^31 - 1.
+__host__ __device__ constexpr int ceil_div(int n, int d) { return (n - 1) / d + 1; }
+// The k at which step `step` of K starts (K beyond the last one); step * 16
+// may pass 2^31 where K is within 16 of it.
+__host__ __device__ constexpr int f64_step_start(int step, int K) {
+  return step <= (K - 1) / kF64Step ? step * kF64Step : K;
+}
 struct GroupedPair {
   const double* l;
   const double* r;

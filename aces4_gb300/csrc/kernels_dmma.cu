@@ -39,7 +39,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int BK = 16;      // a k step: 4 k for each of the four warps
+constexpr int BK = kF64Step;  // a k step: 4 k for each of the four warps
 constexpr int kStage = 32;  // k staged at a time
 constexpr int kThreadsF64 = 128;
 constexpr int kTile = 32;  // rows and columns of the largest tile
@@ -57,17 +57,17 @@ __device__ __forceinline__ void tile_coord(bool kfast, int e, int& r, int& kk) {
   else r = e & 31, kk = e >> 5;
 }
 
-// Gathers one 32 x kStage operand tile (rows x k from k0, below kend).
+// Gathers one 32 x kStage operand tile (rows x the first `left` of the k that
+// offK starts at).
 __device__ __forceinline__ void gather_tile(bool kfast, double (&reg)[kStage / 4], const double* __restrict__ X,
                                             const int64_t* __restrict__ offRow,  // smem, per row
                                             const int64_t* __restrict__ offK,    // global, per k
-                                            int rows, int k0, int kend) {
+                                            int rows, int left) {
 #pragma unroll
   for (int i = 0; i < kStage / 4; ++i) {
     int r, kk;
     tile_coord(kfast, int(threadIdx.x) + kThreadsF64 * i, r, kk);
-    const int k = k0 + kk;
-    reg[i] = (r < rows && k < kend) ? __ldg(&X[offRow[r] + __ldg(&offK[k])]) : 0.0;
+    reg[i] = (r < rows && kk < left) ? __ldg(&X[offRow[r] + __ldg(&offK[kk])]) : 0.0;
   }
 }
 
@@ -134,29 +134,31 @@ __device__ void accumulate_tile(F64Smem& sm, const GroupedPair* __restrict__ pai
   for (int q = pb; q < pe; ++q) {
     const GroupedPair pr = pairs[q];
     const PlanRef pl = plans[pr.plan];
-    const int kend = q == pe - 1 ? min(pl.K, ks1 * BK) : pl.K;
+    const int first = q == pb ? f64_step_start(ks0, pl.K) : 0, end = q == pe - 1 ? f64_step_start(ks1, pl.K) : pl.K;
     const int rows = min(pl.M - m0, 8 * mi), cols = min(pl.N - n0, 8 * NJ + nrem);
-    int kb = q == pb ? ks0 * BK : 0;
+    const int64_t *offLk = pl.offLk + first, *offRk = pl.offRk + first;
+    int left = end - first;  // k to do, from offLk and offRk on
     __syncthreads();  // previous pair done with the tables / tiles
     if (t < kTile) sm.sLm[t] = t < rows ? pl.offLm[m0 + t] : 0;
     else if (t < 2 * kTile) sm.sRn[t - kTile] = t - kTile < cols ? pl.offRn[n0 + t - kTile] : 0;
     __syncthreads();
-    if (kb >= kend) continue;
+    if (left <= 0) continue;
     double ra[kStage / 4], rb[kStage / 4];
-    gather_tile(pl.a_kfast, ra, pr.l, sm.sLm, pl.offLk, rows, kb, kend);
-    gather_tile(pl.b_kfast, rb, pr.r, sm.sRn, pl.offRk, cols, kb, kend);
+    gather_tile(pl.a_kfast, ra, pr.l, sm.sLm, offLk, rows, left);
+    gather_tile(pl.b_kfast, rb, pr.r, sm.sRn, offRk, cols, left);
     store_tile(pl.a_kfast, sm.As[0], ra);
     store_tile(pl.b_kfast, sm.Bs[0], rb);
     __syncthreads();
-    for (int cur = 0; kb < kend; kb += kStage, cur ^= 1) {
-      const bool more = kb + kStage < kend;
+    for (int cur = 0; left > 0; left -= kStage, cur ^= 1) {
+      const bool more = left > kStage;
       if (more) {
-        gather_tile(pl.a_kfast, ra, pr.l, sm.sLm, pl.offLk, rows, kb + kStage, kend);
-        gather_tile(pl.b_kfast, rb, pr.r, sm.sRn, pl.offRk, cols, kb + kStage, kend);
+        offLk += kStage, offRk += kStage;
+        gather_tile(pl.a_kfast, ra, pr.l, sm.sLm, offLk, rows, left - kStage);
+        gather_tile(pl.b_kfast, rb, pr.r, sm.sRn, offRk, cols, left - kStage);
       }
 #pragma unroll
       for (int h = 0; h < kStage / BK; ++h) {
-        if (h && kb + h * BK >= kend) break;
+        if (h && h * BK >= left) break;
         const int k4 = h * BK + 4 * warp;
         if constexpr (NJ > 0) {
           const double *ak = &sm.As[cur][k4 + tig][g], *bk = &sm.Bs[cur][k4 + tig][g];
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(kThreadsF64, 4) contract_f64_kernel(const __gr
   __shared__ __align__(16) F64Smem sm;
   const int ranks = int(cg::this_cluster().num_blocks()), rank = int(cg::this_cluster().block_rank());
   const int tile = int(blockIdx.x) / ranks, tm = tile % a.tiles_m, tn = tile / a.tiles_m;
-  const int um = (a.plan.M + 7) / 8, un = (a.plan.N + 7) / 8, steps = (a.plan.K + BK - 1) / BK;
+  const int um = ceil_div(a.plan.M, 8), un = ceil_div(a.plan.N, 8), steps = ceil_div(a.plan.K, BK);
   const int u0 = int(int64_t(um) * tm / a.tiles_m), u1 = int(int64_t(um) * (tm + 1) / a.tiles_m);
   const int v0 = int(int64_t(un) * tn / a.tiles_n), v1 = int(int64_t(un) * (tn + 1) / a.tiles_n);
   f64_tile(sm, &a.pair, &a.plan, 0, 1, int(int64_t(steps) * rank / ranks), int(int64_t(steps) * (rank + 1) / ranks),
