@@ -24,13 +24,6 @@ A4G_HD int clz64(unsigned long long x) {
   return x ? __builtin_clzll(x) : 64;
 #endif
 }
-A4G_HD unsigned long long mulhi64(unsigned long long a, unsigned long long b) {
-#if defined(__CUDA_ARCH__)
-  return __umul64hi(a, b);
-#else
-  return (unsigned long long)(((unsigned __int128)a * b) >> 64);
-#endif
-}
 A4G_HD unsigned long long bits_of(double x) {
 #if defined(__CUDA_ARCH__)
   return (unsigned long long)__double_as_longlong(x);

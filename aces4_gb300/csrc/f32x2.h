@@ -37,13 +37,6 @@ __device__ __forceinline__ uint32_t bf16x2_of(F32x2 v) {
 
 // x + kRintMagic - kRintMagic rounds |x| < 2^22 to the nearest integer.
 constexpr float kRintMagic = 12582912.0f;  // 1.5 2^23
-// An integer-valued float below 2^22 in magnitude as int, and back.
-__device__ __forceinline__ int int_of_small(float x) {
-  return int(__float_as_uint(__fadd_rn(x, kRintMagic))) - 0x4B400000;
-}
-__device__ __forceinline__ float float_of_small(int x) {
-  return __fsub_rn(__uint_as_float(uint32_t(x + 0x4B400000)), kRintMagic);
-}
 
 __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
   long long r;
