@@ -428,12 +428,18 @@ int build_f64(a4g_batch* b, const std::vector<DGroup>& groups, const std::vector
 // destination (below, the direct forms' digits need no workspace).  Then the
 // products saved have to pay for the wider panels, L instead of S planes
 // written by every run: both sides at measured rates (a tensor-core product
-// at 1.6 PFLOP/s, panel bytes at 5.5 TB/s), with 30 % for the reconstruction.  A 529 x 2304 x 6241 step lies just
-// below the line (381 us with digits, 397 with residues), the o=64/v=512 slab
-// (1024 x 4096 x 262144) well above it (20.8 -> 18.1 ms).  Where the digits'
-// products take less than kResidueSmallUs in all, units and launches count and
-// not bytes: all residue products cost the same, so the GEMM has more and equal
-// units (o=10/v=48 step: 64 -> 44 us).  A pinned variant names a digit form.
+// at 1.6 PFLOP/s, panel bytes at 5.5 TB/s), with 30 % for the reconstruction.
+// A 529 x 2304 x 6241 step lies just below the line (337 us with digits, 388
+// with residues), the o=64/v=512 slab (1024 x 4096 x 262144) well above it
+// (20.8 -> 18.1 ms).  Where the digits' products take less than
+// kResidueSmallUs in all, units and launches count and not bytes: all residue
+// products cost the same, so the GEMM has more and equal units (o=10/v=48 step:
+// 64 -> 44 us; the narrow 3600 x 100 x 3600 step, 9 us of products against 29 of
+// panels by the rates above: 210 us with digits, 192 with residues).  Over 775
+// steps of v 40 to 400, o 5 to 60, 5 to 7 slices, both forms measured of each,
+// the line's picks take 3.5 % more than the better forms (digits alone 23 %,
+// residues alone 1.2 %); three steps are slower than they were with the digits
+// of before the residues, by 2, 5 and 10 %.  A pinned variant names a digit form.
 constexpr int kResidueMinKb = 24;
 constexpr double kResidueSmallUs = 40.0;
 void choose_products(a4g_batch* b, const std::vector<OzTile>& dinfo, const std::vector<PanelBuild>& pa,

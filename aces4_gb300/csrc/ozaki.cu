@@ -855,9 +855,10 @@ __device__ void epilogue_int(const OzGemmArgs& a, OzSmemT<PAIR, 256>& sm, uint32
 }
 
 // Residue form, every tile shape: a chunk (256 k) of the modulus' product is an
-// exact FP32 integer below 2^24 - 256; the thread's running residue (at most
-// p / 2 in magnitude, one FP32 register per column) is added to it, exactly,
-// and the sum reduced modulo p again: four packed FP32 instructions per two
+// exact FP32 integer below 2^24 - 256; the thread's running residue (at most 256
+// in magnitude: p / 2, or one multiple of p off where the reciprocal's error
+// meets a tie; one FP32 register per column) is added to it, exactly, and the
+// sum reduced modulo p again: four packed FP32 instructions per two
 // columns.  (The conversion to int32 that the level form uses runs at a
 // quarter of the FP32 rate's 128 per clock and would take as long as the
 // chunk's MMAs: 2048 clocks for a 128 x 256 accumulator.)  A chunk has to be

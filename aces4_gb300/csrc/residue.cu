@@ -3,7 +3,8 @@
 // numbers, instead of the digit products of the levels 0..S-1.
 //
 // At S slices an operand element is the integer n = round(x 2^(8S - E - 1)),
-// |n| <= 2^(8S-1), as in the digit form (same row scales, same rounding).  The
+// |n| <= 2^(8S-1), as in the digit form (same row scales; both round to the
+// nearest integer, ties here to even up to 6 slices, there away from zero).  The
 // digit form multiplies S (S + 1) / 2 pairs of 8-bit digits and drops the
 // levels i + j >= S.  Here n is reduced modulo L coprime moduli p <= 511 to
 // residues |r| <= 255 (exact BF16 values); one tensor-core product per modulus
@@ -282,7 +283,7 @@ constexpr size_t kGenericSmem = kSplitT * (kSplitT + 1) * sizeof(unsigned long l
 //     X = sum_i y_i (P / p_i) - k P,   y_i = s_i (P / p_i)^-1 mod p_i,
 //     k = rint(sum_i y_i / p_i)
 // in W signed 32-bit word columns of 64-bit sums, modulo 2^(32 W): three words
-// hold |X| < 2^95, four |X| < 2^127, five |X| < 2^159.
+// hold |X| < 2^95, four |X| < 2^127, five any sum that 15 moduli hold (2^133).
 // Two sums at a time: the residue arithmetic in packed FP32.
 template <int W>
 struct CrtPair {
@@ -460,13 +461,11 @@ __global__ void __launch_bounds__(kRecThreads, L <= 12 && W == 3 ? 4 : 3) oz_res
 
 // Products the residue form needs for K columns at `slices` slices: the
 // smallest count whose moduli hold every sum |sum| <= K 4^(8 slices - 1) below
-// 0.49 of their product; 0 when none does, or when the sum would not stay
-// below 2^158 (the reconstruction's words).  At 5 slices or more and k ranges
-// worth it (batch.cu), 10 to 15.
+// 0.49 of their product; 0 when none does (15 hold sums below 2^133).  At 5
+// slices or more and k ranges worth it (batch.cu), 10 to 15.
 int oz_residue_count(int slices, int64_t K) {
   if (K < 1) return 0;
   const double need = 2.0 * (8.0 * slices - 1.0) + std::log2(double(K));
-  if (need >= 158.0) return 0;
   double have = std::log2(0.49);
   for (int i = 0; i < kOzMaxResidues; ++i) {
     have += std::log2(double(kModuli[i]));
@@ -544,13 +543,11 @@ int oz_launch_residue_recombine(const OzTile* tiles, int ntiles, int tile_rows, 
   const std::integral_constant<int, 3> w3;
   const std::integral_constant<int, 4> w4;
   switch (t.L) {
-#define A4G_RESIDUE(N)                                                                                \
-  case N:                                                                                             \
-    if (t.words == 3) go(std::integral_constant<int, N>(), w3);                                       \
-    else go(std::integral_constant<int, N>(), w4);                                                    \
-    break;
-    A4G_RESIDUE(10) A4G_RESIDUE(11)
-#undef A4G_RESIDUE
+    case 10: go(std::integral_constant<int, 10>(), w3); break;  // 10 moduli hold sums below 2^89
+    case 11:
+      if (t.words == 3) go(std::integral_constant<int, 11>(), w3);
+      else go(std::integral_constant<int, 11>(), w4);
+      break;
     case 12: go(std::integral_constant<int, 12>(), w4); break;
     case 13: go(std::integral_constant<int, 13>(), w4); break;
     case 14: go(std::integral_constant<int, 14>(), w4); break;

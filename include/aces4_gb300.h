@@ -290,7 +290,11 @@ typedef struct a4g_batch_opts {
                       near 1e-11, 6 near 1e-13.  At 5 and more slices and k
                       ranges of 1536 and more the products run modulo coprime
                       numbers (a4g_batch_products) unless `variant` names a
-                      digit form; both round the operands alike.            */
+                      digit form.  Both round an operand element to the same
+                      multiple; where two are equally near, the residues take
+                      the even one up to 6 slices, the digits the larger.
+                      Residue panels take 11/5 (13/6, 15/7) of the digits'
+                      bytes: a caller who needs that memory names a form.    */
   int beta;        /* 0: D = sum of products (overwrite); 1: D += sum        */
   int variant;     /* split precision, tensor-core GEMM form: 0 autotuned at
                       creation (each form timed once and scored with the
