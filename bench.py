@@ -60,6 +60,17 @@ def _peaks():
         return {"hbm_gbs": 6800.0, "bf16_tflops": 1900.0, "bf16_tflops_sustained": 1700.0}, "fallback"
 
 
+def _split_dtype(slices, products):
+    if products < slices * (slices + 1) // 2:
+        return f"f64 (split precision: {8 * slices}-bit operands, {products} BF16 residue products)"
+    return f"f64 (Ozaki, {slices} BF16 slices)"
+
+
+def _split_kernel(slices, products):
+    kind = "residue" if products < slices * (slices + 1) // 2 else "slice"
+    return f"oz_gemm_kernel (tcgen05 BF16 {kind} products)"
+
+
 def _traffic(kernel: str):
     try:
         with open(os.path.join(ROOT, "profiles", "traffic_per_launch.json")) as f:
@@ -930,7 +941,7 @@ def run_ladder_full(args, world, rank, local):
         out = {
             "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "strong",
-            "vs_baseline": None, "dtype": f"f64 (Ozaki, {S} BF16 slices)", "data": "synthetic",
+            "vs_baseline": None, "dtype": _split_dtype(S, cold["products"]), "data": "synthetic",
             "config": {"workload": full_workload_name(nv, no, len(all_slabs)), "slices": S,
                        "slabs_per_run": k_run,
                        "products": cold["products"], "slabs": len(all_slabs), "slabs_this_rank": len(slabs),
@@ -941,7 +952,7 @@ def run_ladder_full(args, world, rank, local):
                                    f"550 GB): slab q reads pool[q % {P}]",
                        "parallelism": f"slabs split over {world} rank(s), no collective"},
             "e2e": e2e,
-            "roofline": {"kernel": "oz_gemm_kernel (tcgen05 BF16 slice products)", "bound": "tensor",
+            "roofline": {"kernel": _split_kernel(S, cold["products"]), "bound": "tensor",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_kind": f"{peak_key} of {peak_kind} (timed region {ms * args.steps / 1e3:.1f} s)",
                          "algorithmic_per_launch": f"{cold['products']} BF16 products x {k_run} slab(s) x "
@@ -1558,12 +1569,12 @@ def main():
         out = {
             "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": f"f64 (Ozaki, {S} BF16 slices)", "data": "synthetic",
+            "vs_baseline": None, "dtype": _split_dtype(S, products), "data": "synthetic",
             "config": {"workload": workload, "slices": S, "products": products, "block_pairs": info["pairs"],
                        "l2": f"inputs {n_elem * 8 / 1e9:.2f} GB > 126 MB L2 (no flush needed)",
                        "parallelism": f"replicas x{world}"},
             "e2e": e2e,
-            "roofline": {"kernel": "oz_gemm_kernel (tcgen05 BF16 slice products)", "bound": "tensor",
+            "roofline": {"kernel": _split_kernel(S, products), "bound": "tensor",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_kind": f"{peak_key} of {peak_kind} (timed region {ms * args.steps / 1e3:.2f} s)",
                          "algorithmic_per_launch": f"{products} BF16 products x {flops:.3e} flop",
