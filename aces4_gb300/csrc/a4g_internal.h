@@ -49,8 +49,13 @@ struct Context {
   // stream (reduction_slots.h): partial sums in chunks, made as slots are first
   // used, and the counters, zero between launches.
   static constexpr int kReducePartials = 1024, kReduceChunk = 64;
-  std::vector<double*> reduce_partials;  // chunks of [kReduceChunk][kReducePartials + 8]
+  std::vector<double*> reduce_partials;  // chunks of [kReduceChunk][kReducePartials]
   unsigned* reduce_counters = nullptr;
+  // Results on their way to the host, one per synchronous call in turn: a thread
+  // has one call at a time, so calls of fewer threads than this never meet, on
+  // one stream either.
+  static constexpr int kReduceResults = 4096;
+  double* reduce_results = nullptr;
   // Kernels can read and write pageable host memory through the host's page
   // tables (address translation services over the CPU-GPU link): the
   // drop-ins then run on the caller's host blocks in place.
@@ -132,13 +137,13 @@ int launch_permute(int rank, const int* ext, const int* o2n_1based, const double
                    cudaStream_t s);
 int launch_add_sub_permuted(int subtract, int rank, const int* r_ext, const int* o2n_1based,
                             double* d, const double* l, const double* r, cudaStream_t s);
-// Scratch of one reduction: partial sums of its CTAs, the counter of those that
-// have written theirs (zero between launches) and room for a result.
+// Scratch of one reduction: partial sums of its CTAs and the counter of those
+// that have written theirs (zero between launches).
 struct ReductionSlot {
   double* partial = nullptr;
-  double* result = nullptr;
   unsigned* counter = nullptr;
 };
+double* reduction_result();  // the next of the context's results (after ensure_init)
 // The scratch of the reductions that the caller launches on `s` while the
 // object lives (after ensure_init).
 class ReductionScratch {

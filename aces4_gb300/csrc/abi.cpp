@@ -636,7 +636,7 @@ int a4g_norm2(const double* t, int64_t n, double* h_result, void* stream) {
   cudaStream_t s = pick(stream);
   ReductionScratch scratch;
   if ((rc = scratch.acquire(s))) return rc;
-  double* out = scratch.slot.result;
+  double* out = reduction_result();
   rc = launch_norm2(t, n, out, scratch.slot, s);
   if (rc) return rc;
   A4G_CUDA(cudaMemcpyAsync(h_result, out, sizeof(double), cudaMemcpyDeviceToHost, s));

@@ -1,6 +1,7 @@
 // Runtime support: error reporting, the process context, the contraction
 // pattern planner and the device plan cache.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <unordered_map>
@@ -31,8 +32,6 @@ static std::mutex g_mu;
 
 Context* ctx() { return &g_ctx; }
 
-constexpr size_t kReduceLen = Context::kReducePartials + 8;  // doubles of a reduction's scratch
-
 int ensure_init() {
   if (g_ctx.device >= 0) return A4G_OK;
   std::lock_guard<std::mutex> lock(g_mu);
@@ -53,8 +52,9 @@ int ensure_init() {
   A4G_CUDA(cudaMalloc(&g_ctx.reduce_counters, sizeof(unsigned) * SlotTable::kMaxSlots));
   A4G_CUDA(cudaMemset(g_ctx.reduce_counters, 0, sizeof(unsigned) * SlotTable::kMaxSlots));
   double* partials = nullptr;
-  A4G_CUDA(cudaMalloc(&partials, sizeof(double) * kReduceLen * Context::kReduceChunk));
+  A4G_CUDA(cudaMalloc(&partials, sizeof(double) * Context::kReducePartials * Context::kReduceChunk));
   g_ctx.reduce_partials.push_back(partials);
+  A4G_CUDA(cudaMalloc(&g_ctx.reduce_results, sizeof(double) * Context::kReduceResults));
   A4G_CUDA(cudaDeviceSynchronize());
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
@@ -136,21 +136,26 @@ int ReductionScratch::acquire(cudaStream_t s) {
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         A4G_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
         double* p = nullptr;
-        const cudaError_t e = cudaMalloc(&p, sizeof(double) * kReduceLen * Context::kReduceChunk);
+        const cudaError_t e = cudaMalloc(&p, sizeof(double) * Context::kReducePartials * Context::kReduceChunk);
         A4G_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
         g_ctx.reduce_partials.push_back(p);
       }
-      double* p = g_ctx.reduce_partials[chunk] + kReduceLen * size_t(q % Context::kReduceChunk);
-      slot = {p, p + Context::kReducePartials, g_ctx.reduce_counters + q};
+      slot = {g_ctx.reduce_partials[chunk] + Context::kReducePartials * size_t(q % Context::kReduceChunk),
+              g_ctx.reduce_counters + q};
       return A4G_OK;
     }
   }
-  if (const int rc = async_alloc(&own_, sizeof(double) * (kReduceLen + 1), s)) return rc;
+  if (const int rc = async_alloc(&own_, sizeof(double) * (Context::kReducePartials + 1), s)) return rc;
   double* p = static_cast<double*>(own_);
-  slot = {p, p + Context::kReducePartials, reinterpret_cast<unsigned*>(p + kReduceLen)};
+  slot = {p, reinterpret_cast<unsigned*>(p + Context::kReducePartials)};
   A4G_CUDA(cudaMemsetAsync(slot.counter, 0, sizeof(unsigned), s));
   return A4G_OK;
+}
+
+double* reduction_result() {
+  static std::atomic<unsigned> next{0};
+  return g_ctx.reduce_results + next.fetch_add(1, std::memory_order_relaxed) % Context::kReduceResults;
 }
 
 cudaStream_t pick(void* stream) {
