@@ -761,7 +761,8 @@ __global__ void __launch_bounds__(kThreads) energy_generic_kernel(DenParams p, c
 //   partial[block] = sum of E^2                  (its residual norm, deterministic)
 // eps = ((e_i + e_j) - e_a) - e_b, energy_denominator_rhf's rank-4 order.
 // (0.5 t)/eps is formed as 0.5 (t/eps): both are t/(2 eps) correctly rounded
-// while the quotient is a normal number; below that the division is redone.
+// while the quotient and 0.5 t are normal numbers; below and beyond that (t/eps
+// may overflow where its half does not) the division is redone.
 //
 // A work unit is one (a,b) tile at fixed (i,j).  The plane is cut evenly into
 // tiles of at most 48 x 24 (a 33 x 37 plane is two of 33 x 19, 96 x 96 eight of
@@ -775,6 +776,7 @@ __global__ void __launch_bounds__(kThreads) energy_generic_kernel(DenParams p, c
 // o=40/v=300 (400 blocks of about 33 x 20 x 33 x 20, 48 B an element):
 // 20 us a block before.
 constexpr int kUpdA = 48, kUpdB = 24, kUpdGroup = 4, kUpdThreads = 128;
+constexpr uint32_t kHalvable = 2u << 21;  // the high word, less its sign, of 2^-1021: the least number with a normal half
 struct UpdParams {
   int ea, ei, eb, ej;   // extents
   int oa, oi, ob, oj;   // first orbitals
@@ -888,15 +890,17 @@ __global__ void __launch_bounds__(kUpdThreads, 6) update_t2_kernel(UpdParams p, 
       // FP64 pipe, 16 clocks a warp)
       double ev[kUpdGroup], nx[kUpdGroup];
       bool all = true;
+      uint32_t least = ~0u;  // of |t|'s exponent and upper fraction: below 2^-1021, t loses a bit when it is halved
 #pragma unroll
       for (int g = 0; g < kUpdGroup; ++g) {
         const unsigned long long x = bits_of(__dsub_rn(t1[g], td[g])), y = bits_of(td[g]);
+        least = min(least, uint32_t(bits_of(t[g]) >> 32) << 1);
         ev[g] = double_of((x - (1ull << 52)) ^ (1ull << 63));
         nx[g] = double_of(y - (1ull << 52));
         t1[g] = double_of(x);
         all = all && (uint32_t(x >> 52) & 0x7FFu) - 2u < 2045u && (uint32_t(y >> 52) & 0x7FFu) - 2u < 2045u;
       }
-      if (!all) {
+      if (!all || least < kHalvable) {
 #pragma unroll 1
         for (int g = 0; g < kUpdGroup; ++g) {
           double x = 0.0, y = 0.0, tg = 0.0, eg = 0.0;
@@ -905,7 +909,8 @@ __global__ void __launch_bounds__(kUpdThreads, 6) update_t2_kernel(UpdParams p, 
             if (k == g) x = t1[k], y = td[k], tg = t[k], eg = eps[k];
           const unsigned f = uint32_t(bits_of(y) >> 52) & 0x7FFu;
           x = double_of(bits_of(half_of(x)) ^ (1ull << 63));
-          y = f >= 2u ? half_of(y) : __ddiv_rn(__dmul_rn(tg, 0.5), eg);
+          y = f - 2u < 2045u && (uint32_t(bits_of(tg) >> 32) << 1) >= kHalvable ? half_of(y)
+                                                                                : __ddiv_rn(__dmul_rn(tg, 0.5), eg);
 #pragma unroll
           for (int k = 0; k < kUpdGroup; ++k)
             if (k == g) ev[k] = x, nx[k] = y;
