@@ -590,6 +590,24 @@ __device__ __forceinline__ void den_coords(const DenParams& p, int64_t i, int (&
 // (64-bit divisions are dear) and stepped along dimension 0 with carries.
 constexpr int kDenRun = 4;
 
+// The denominators of the run of elements from x on, the first `live` of them
+// (1 for the rest); x moves to the element behind the last live one.
+__device__ __forceinline__ void den_run(const DenParams& p, const double* e, int (&x)[6], int live,
+                                        double (&d)[kDenRun]) {
+#pragma unroll
+  for (int u = 0; u < kDenRun; ++u) {
+    d[u] = 1.0;
+    if (u >= live) continue;
+    d[u] = den_eps(p, e, x);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {  // next element: x[0] + 1 with carries
+      if (q >= p.rank0) break;
+      if (++x[q] < p.ext[q]) break;
+      x[q] = 0;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kThreads) denominator_kernel(DenParams p, double* data,
                                                                const double* __restrict__ e,
                                                                int64_t n) {
@@ -600,17 +618,12 @@ __global__ void __launch_bounds__(kThreads) denominator_kernel(DenParams p, doub
     double v[kDenRun];
 #pragma unroll
     for (int u = 0; u < kDenRun; ++u) v[u] = i0 + u < n ? data[i0 + u] : 0.0;
+    double d[kDenRun], quot[kDenRun];
+    den_run(p, e, x, int(min(int64_t(kDenRun), n - i0)), d);
+    div_rn_n<kDenRun>(v, d, quot);
 #pragma unroll
-    for (int u = 0; u < kDenRun; ++u) {
-      if (i0 + u >= n) break;
-      data[i0 + u] = div_rn(v[u], den_eps(p, e, x));
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {  // next element: x[0] + 1 with carries
-        if (q >= p.rank0) break;
-        if (++x[q] < p.ext[q]) break;
-        x[q] = 0;
-      }
-    }
+    for (int u = 0; u < kDenRun; ++u)
+      if (i0 + u < n) data[i0 + u] = quot[u];
   }
 }
 
@@ -734,17 +747,15 @@ __global__ void __launch_bounds__(kThreads) energy_generic_kernel(DenParams p, c
     double v[kDenRun];
 #pragma unroll
     for (int u = 0; u < kDenRun; ++u) v[u] = i0 + u < n ? __ldg(w + i0 + u) : 0.0;
+    double d[kDenRun], quot[kDenRun];
+    bool ok[kDenRun];
+    den_run(p, e, x, int(min(int64_t(kDenRun), n - i0)), d);
 #pragma unroll
-    for (int u = 0; u < kDenRun; ++u) {
-      if (i0 + u >= n) break;
-      if (nonzero(v[u])) acc = fma(v[u], div_rn(v[u], den_eps(p, e, x)), acc);
+    for (int u = 0; u < kDenRun; ++u) ok[u] = div_rn_int(v[u], d[u], &quot[u]);
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        if (q >= p.rank0) break;
-        if (++x[q] < p.ext[q]) break;
-        x[q] = 0;
-      }
-    }
+    for (int u = 0; u < kDenRun; ++u)
+      if (ok[u]) acc = fma(v[u], quot[u], acc);
+      else if (nonzero(v[u])) acc = fma(v[u], div_rn_slow(v[u], d[u]), acc);
   }
   double total;
   if (grid_sum(acc, partial, counter, &total)) *esum = __dadd_rn(*esum, __dmul_rn(total, efact));
