@@ -374,8 +374,12 @@ int launch_perm_op(const PermParams& p, const double* in, double* out, const dou
   } else {
     const int Ea = p.ext[p.a_dim], Eb = p.ext[p.b_dim];
     const int64_t tiles = int64_t((Ea + kTile - 1) / kTile) * ((Eb + kTile - 1) / kTile);
-    // up to four slices a block (sixteen: 33 x 20 x 29 x 20 in 12.0 us instead of 11.3; two: 96^4 in 259, not 248)
-    const int rpb = 2 * int(std::max<int64_t>(1, std::min<int64_t>(2, p.n_rest_total * tiles / (int64_t(sms) * 32))));
+    // 2 to 16 slices a block, the most that leave 16 blocks an SM: with fewer
+    // blocks the last wave costs more than the blocks' starts (33 x 20 x 29 x 20:
+    // 6.2 us by 2, 12.4 by 16), with many the starts do (24^6: 1050 us by 2, 962 by
+    // 4, 922 by 16; 96^4 260, 250 and 248; 30 x 100 x 30 x 100 39, 37 and 46)
+    int rpb = 2;
+    while (rpb < 16 && p.n_rest_total * tiles / (int64_t(sms) * 16) >= 2 * rpb) rpb *= 2;
     const int64_t blocks = tiles * ((p.n_rest_total + rpb - 1) / rpb);
     if (blocks > 0x7fffffffLL) return fail(A4G_ERR_RANGE, "permute grid too large");
     perm_tiled_kernel<OP><<<unsigned(blocks), dim3(kTile, 8), 0, s>>>(p, in, out, l, rpb);
