@@ -20,7 +20,7 @@
 // Rows, columns and cluster size come from a model of the makespan (f64_form).
 // Against 64 x 64 (48, 32) tiles padded to their edges, 2 x 2 warps a tile, and
 // partial tiles through a workspace and a second launch: a 660 x 580 x 580 pair
-// 715 -> 502 us (425 at the pipes' rate), the o=10/v=48 step 1488 -> 1124 us
+// 715 -> 497 us (425 at the pipes' rate), the o=10/v=48 step 1488 -> 1120 us
 // (1013), 108 x 96 x 96 pairs 43 -> 12 us.
 //
 // The grouped form runs a whole pardo step: one cluster owns one tile of one
